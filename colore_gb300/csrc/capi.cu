@@ -106,7 +106,7 @@ struct cg_ctx {
   double norm_zlast = 0, norm_idz = 0;
   int norm_nz = 0;
   int bins_nz_cap = 0, bins_nt_cap = 0;
-  float *d_pk = nullptr;
+  float4 *d_pk = nullptr;
   float2 *d_twN = nullptr, *d_twH = nullptr;
   Box box;
   FillParams fill;
@@ -757,10 +757,13 @@ extern "C" int cg_upload_tables(cg_ctx *c, const cg_config *cfg)
     CUDA_TRY(c, cudaStreamSynchronize(c->stream)); /* host staging vectors */
   }
   /* P(k) */
-  std::vector<float> pk(cfg->numk);
-  for (int i = 0; i < cfg->numk; i++) pk[i] = (float)cfg->pkarr[i];
+  std::vector<float4> pk(cfg->numk);
+  for (int i = 0; i < cfg->numk; i++) {
+    const float a = (float)cfg->pkarr[i], b = (float)cfg->pkarr[i + 1 < cfg->numk ? i + 1 : i];
+    pk[i] = make_float4((float)cfg->logkmin + (float)i / (float)cfg->idlogk, a, b - a, 0.0f);
+  }
   if (int rc = dalloc(c, &c->d_pk, pk.size())) return rc;
-  CUDA_TRY(c, cudaMemcpyAsync(c->d_pk, pk.data(), pk.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(c, cudaMemcpyAsync(c->d_pk, pk.data(), pk.size() * sizeof(float4), cudaMemcpyHostToDevice, c->stream));
   /* box and fill parameters */
   const double L = cfg->l_box;
   const int N = c->N;
@@ -789,8 +792,10 @@ extern "C" int cg_upload_tables(cg_ctx *c, const cg_config *cfg)
   f.logkmax = (float)cfg->logkmax;
   f.idlogk = (float)cfg->idlogk;
   f.n_scal = (float)cfg->n_scal;
-  f.key0 = (uint32_t)cfg->seed;
-  f.key1 = (uint32_t)(cfg->seed >> 32) ^ CG_STREAM_FIELD;
+  for (uint32_t r = 0; r < 10; r++) {
+    f.rk0[r] = (uint32_t)cfg->seed + r * 0x9E3779B9u;
+    f.rk1[r] = ((uint32_t)(cfg->seed >> 32) ^ CG_STREAM_FIELD) + r * 0xBB67AE85u;
+  }
   f.lpt_norm = (float)std::pow(std::sqrt(2 * M_PI) / L, 3);
   c->have_fields = c->have_density = c->have_norm = c->have_srcs = 0;
   return CG_OK;

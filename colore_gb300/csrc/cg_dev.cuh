@@ -168,10 +168,10 @@ struct FillParams {
   int N, NH;
   float dk, idk3, prefac, r2s;
   int do_smooth, smooth_pot;
-  const float *pk; /* numk values on logk_i = logkmin + i/idlogk */
+  const float4 *pk; /* numk entries (logk_i = logkmin + i/idlogk, P_i, P_i+1 - P_i, -) */
   int numk;
   float logkmin, logkmax, idlogk, n_scal;
-  uint32_t key0, key1;
+  uint32_t rk0[10], rk1[10]; /* Philox round keys: (seed, stream) plus r times the Weyl constants */
   float lpt_norm; /* (sqrt(2 pi)/L)^3, used by the 1LPT displacement fill */
   int lpt_kind;   /* three-field fill: 0 Psi_x,y,z; 1 phi_xx,xy,xz; 2 phi_yy,yz,zz */
 };

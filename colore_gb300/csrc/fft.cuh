@@ -231,16 +231,47 @@ __host__ __device__ __forceinline__ void stage(float2 *v, int t, const float2 *_
   }
 }
 
+/* Exchange slots.  Stage 0 writes position t r0 + q of thread t, so without
+ * padding the threads of a half-warp (one 128-byte shared-memory wavefront of
+ * float2) hit the same banks.  Slot p sits at p + (p >> sh), 2^sh the largest
+ * power of two dividing r0: thread t's writes then lie (r0 + r0/2^sh) t slots
+ * apart, an odd stride, which spreads over all banks for any number of
+ * columns; reads at consecutive positions stay consecutive but for one slot
+ * per 2^sh.  (y pass at 512^3: 10.9 M conflict wavefronts per launch without
+ * the padding, as many as the accesses themselves.) */
+__host__ __device__ constexpr int pad_shift(int r0)
+{
+  int s = 0;
+  while (r0 % 2 == 0) {
+    r0 /= 2;
+    s++;
+  }
+  return s;
+}
+/* Slots of a padded exchange buffer of length L. */
+__host__ __device__ constexpr int pad_len(int L, int r0) { return L + (L >> pad_shift(r0)); }
+
+/* Slot of position base + off.  off is a constant once loops are unrolled,
+ * and splits off the shift when either part is a multiple of 2^sh. */
+template <int SH>
+__host__ __device__ __forceinline__ int pad_at(int base, int off, bool base_aligned)
+{
+  if (base_aligned || (off & ((1 << SH) - 1)) == 0) return (base + (base >> SH)) + (off + (off >> SH));
+  return base + off + ((base + off) >> SH);
+}
+
 /*
  * Full transform of length L = r0*r1*r2 (r2 = 1 for two stages, r1 = r2 = 1
  * for one) by P = L/R threads.  Ld(pos) -> float2 supplies the input,
- * St(pos, value) consumes the output, Sm(pos) -> float2& addresses this
- * transform's shared-memory exchange slot.  Contains the barriers of the
- * exchanges, so every thread of the block must call it.
+ * St(pos, value) consumes the output, Sm(slot) -> float2& addresses slot
+ * 0..pad_len(L, r0)-1 of this transform's shared-memory exchange buffer.
+ * Contains the barriers of the exchanges, so every thread of the block must
+ * call it.
  */
 template <int L, int R, int r0, int r1, int r2, int S, class Ld, class St, class Sm>
 __device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL, Ld ld, St st, Sm sm)
 {
+  constexpr int SH = pad_shift(r0);
   float2 v[R];
 #pragma unroll
   for (int i = 0; i < R / r0; i++)
@@ -259,12 +290,12 @@ __device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL,
 #pragma unroll
   for (int i = 0; i < R / r0; i++)
 #pragma unroll
-    for (int q = 0; q < r0; q++) sm(out_pos<L, R, r0, 1>(t, i, q)) = v[i * r0 + q];
+    for (int q = 0; q < r0; q++) sm(pad_at<SH>((t + (L / R) * i) * r0, q, true)) = v[i * r0 + q];
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < R / r1c; i++)
 #pragma unroll
-    for (int q = 0; q < r1c; q++) v[i * r1c + q] = sm(in_pos<L, R, r1c>(t, i, q));
+    for (int q = 0; q < r1c; q++) v[i * r1c + q] = sm(pad_at<SH>(t, (L / R) * i + q * (L / r1c), false));
   stage<L, R, r1c, r0, S>(v, t, twL);
   if (r2 == 1) {
 #pragma unroll
@@ -278,12 +309,12 @@ __device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL,
 #pragma unroll
   for (int i = 0; i < R / r1c; i++)
 #pragma unroll
-    for (int q = 0; q < r1c; q++) sm(out_pos<L, R, r1c, r0>(t, i, q)) = v[i * r1c + q];
+    for (int q = 0; q < r1c; q++) sm(pad_at<SH>(out_pos<L, R, r1c, r0>(t, i, 0), q * r0, false)) = v[i * r1c + q];
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < R / r2c; i++)
 #pragma unroll
-    for (int q = 0; q < r2c; q++) v[i * r2c + q] = sm(in_pos<L, R, r2c>(t, i, q));
+    for (int q = 0; q < r2c; q++) v[i * r2c + q] = sm(pad_at<SH>(t, (L / R) * i + q * (L / r2c), false));
   stage<L, R, r2c, r0 * r1c, S>(v, t, twL);
 #pragma unroll
   for (int i = 0; i < R / r2c; i++)

@@ -9,8 +9,8 @@
  *
  *   1. fill + z : a block owns TX consecutive kx at one ky and all kz.  It
  *                 generates the modes of every output field from one set of
- *                 Philox draws (fields after the first are parked in shared
- *                 memory), transforms along z and writes the result.  The
+ *                 Philox draws, kz and -kz together, parks them in shared
+ *                 memory, transforms along z and writes the result.  The
  *                 spectrum is never read back from HBM.
  *   2. y        : the same column transform along y, read-modify-write.
  *   3. x (c2r)  : a group of threads owns one row of N/2+1 complex values;
@@ -55,107 +55,147 @@ constexpr int P = N / PL::CR;       /* threads per column transform (y pass)    
 constexpr int PF = N / PL::FR;      /* threads per column transform (fill + z)    */
 constexpr int LH = N / 2;           /* row transform length         */
 constexpr int PR = LH / PL::RR;     /* threads per row transform    */
-constexpr int ROWS = (NH > LH + LH / 32 + 1) ? NH : (LH + LH / 32 + 1); /* smem per row */
+constexpr int EXF = cgfft::pad_len(N, PL::F0);  /* exchange slots per column (fill + z) */
+constexpr int EXY = cgfft::pad_len(N, PL::C0);  /* exchange slots per column (y pass)   */
+constexpr int EXX = cgfft::pad_len(LH, PL::R0); /* exchange slots per row (x pass)      */
+constexpr int ROWS = NH > EXX ? NH : EXX;       /* smem per row */
 
 /* P(k) at log10 k, pk_linear0 (cosmo.c:291-308).  The interpolation branch
  * stops at numk-2: the reference also takes it for ik = numk-1 and then
  * reads one element past the table. */
 __device__ __forceinline__ float pk_lin(const FillParams &p, float lgk)
 {
-  int ik = (int)((lgk - p.logkmin) * p.idlogk);
-  if (ik < 0) return __ldg(&p.pk[0]) * exp10f(p.n_scal * (lgk - p.logkmin));
+  const int ik = (int)((lgk - p.logkmin) * p.idlogk);
+  if (ik < 0) return __ldg(&p.pk[0]).y * exp10f(p.n_scal * (lgk - p.logkmin));
   if (ik < p.numk - 1) {
-    float lk = p.logkmin + (float)ik / p.idlogk;
-    float a = __ldg(&p.pk[ik]), b = __ldg(&p.pk[ik + 1]);
-    return a + (lgk - lk) * (b - a) * p.idlogk;
+    const float4 q = __ldg(&p.pk[ik]); /* log10 k_ik, P_ik, P_ik+1 - P_ik */
+    return q.y + (lgk - q.x) * q.z * p.idlogk;
   }
-  return __ldg(&p.pk[p.numk - 1]) * exp10f(-3.0f * (lgk - p.logkmax));
+  return __ldg(&p.pk[p.numk - 1]).y * exp10f(-3.0f * (lgk - p.logkmax));
 }
 
 __device__ __forceinline__ float kcomp(int i, int n, float dk) { return (float)(2 * i <= n ? i : i - n) * dk; }
 
-/* Unsmoothed Gaussian mode (rng_delta_gauss, common.c:191-201, with
- * sigma^2 = P(k)/dk^3, fourier.c:343) and its |k|^2 and smoothing factor. */
-__device__ __forceinline__ float2 gen_mode(const FillParams &p, int kx, int ky, int kz, float &k2, float &sm)
+/* What a mode's value needs besides its random draw: |k|^2, P(k)/dk^3, the
+ * smoothing factor and num/|k|^2.  They depend on the components of k through their squares
+ * only, so modes (kx, ky, kz) and (kx, ky, -kz) share one evaluation. */
+struct KAmp {
+  float k2, s2, sm, ik2;
+};
+
+__device__ __forceinline__ KAmp k_amp(const FillParams &p, float num, int kx, int ky, int kz)
 {
-  float kxf = (float)kx * p.dk, kyf = kcomp(ky, N, p.dk), kzf = kcomp(kz, N, p.dk);
-  k2 = kxf * kxf + kyf * kyf + kzf * kzf;
-  sm = 1.0f;
-  if (!(k2 > 0.0f)) return make_float2(0.0f, 0.0f);
-  float lgk = 0.5f * log10f(k2);
-  float s2 = pk_lin(p, lgk) * p.idk3;
-  uint64_t m = (uint64_t)kx + (uint64_t)NH * ((uint64_t)ky + (uint64_t)N * (uint64_t)kz);
-  cg_u32x4 w = cg_philox4x32_10((uint32_t)m, (uint32_t)(m >> 32), 0u, 0u, p.key0, p.key1);
-  float u1 = cg_u01f(w.v[0]), u2 = cg_u01f(w.v[1]);
+  const float kxf = (float)kx * p.dk, kyf = kcomp(ky, N, p.dk), kzf = kcomp(kz, N, p.dk);
+  KAmp a;
+  a.k2 = kxf * kxf + kyf * kyf + kzf * kzf;
+  a.sm = 1.0f;
+  a.s2 = a.ik2 = 0.0f;
+  if (!(a.k2 > 0.0f)) return a;
+  a.ik2 = num / a.k2;
+  const float lgk = 0.5f * log10f(a.k2);
+  a.s2 = pk_lin(p, lgk) * p.idk3;
+  if (p.do_smooth) a.sm = expf(-0.5f * p.r2s * a.k2);
+  return a;
+}
+
+/* Unsmoothed Gaussian mode (rng_delta_gauss, common.c:191-201, with
+ * sigma^2 = P(k)/dk^3, fourier.c:343), k != 0. */
+__device__ __forceinline__ float2 k_draw(const FillParams &p, float s2, int kx, int ky, int kz)
+{
+  uint32_t lo, hi = 0u;
+  if constexpr ((uint64_t)NH * N * N <= 0x100000000ull) { /* the mode number fits 32 bits */
+    lo = (uint32_t)kx + (uint32_t)NH * ((uint32_t)ky + (uint32_t)N * (uint32_t)kz);
+  } else {
+    const uint64_t m = (uint64_t)kx + (uint64_t)NH * ((uint64_t)ky + (uint64_t)N * (uint64_t)kz);
+    lo = (uint32_t)m;
+    hi = (uint32_t)(m >> 32);
+  }
+  /* words 0 and 1 of Philox4x32-10 at counter (lo, hi, 0, 0): cg_philox4x32_10
+   * with the round keys read from the parameters */
+  uint32_t c0 = lo, c1 = hi, c2 = 0u, c3 = 0u;
+#pragma unroll
+  for (int r = 0; r < 10; r++) {
+    uint32_t h0, l0, h1, l1;
+    cg_mulhilo32(0xD2511F53u, c0, &h0, &l0);
+    cg_mulhilo32(0xCD9E8D57u, c2, &h1, &l1);
+    c0 = h1 ^ c1 ^ p.rk0[r];
+    c1 = l1;
+    c2 = h0 ^ c3 ^ p.rk1[r];
+    c3 = l0;
+  }
+  const float u1 = cg_u01f(c0), u2 = cg_u01f(c1);
   float s, c;
   sincospif(2.0f * u1, &s, &c);
-  float mod = sqrtf(-s2 * logf(1.0f - u2));
-  if (p.do_smooth) sm = expf(-0.5f * p.r2s * k2);
+  const float mod = sqrtf(-s2 * logf(1.0f - u2));
   return make_float2(mod * c, mod * s);
 }
 
-/* Field values of one mode of the two-field fill: (delta_k, phi_k)
- * (fourier.c:337-352). */
-template <int F>
-__device__ __forceinline__ void gen_fields(const FillParams &p, int kx, int ky, int kz, float2 *f)
+/* The modes of column (kx, ky) by pairs: put(kz, amplitude) for every kz, the
+ * pair (kz, N - kz) from one amplitude (kz = 0 and N/2 pair up, each with its
+ * own).  Thread t of the PF that share a column takes kz = t, t + PF, ...
+ * below N/2.  Rolled: one copy of the generator in the instruction stream
+ * (inlined per element it overflowed the instruction cache).  The fills are
+ * bound by instruction issue, not HBM (60 % issue-active at 290 instructions
+ * per mode, 20 % of DRAM peak at 1024^3).  One amplitude for two modes, round
+ * keys and the P(k) table's differences formed on the host, and exchange slots
+ * free of conflicts: 7.25 -> 6.58 ms for the two-field fill at 1024^3,
+ * 374 -> 334 us at 384^3. */
+template <class Put>
+__device__ __forceinline__ void k_pairs(const FillParams &p, float num, int kx, int ky, int t, Put put)
 {
-  static_assert(F == 2, "the three-field fills use lpt_base and lpt_field");
-  float k2, sm;
-  float2 d = gen_mode(p, kx, ky, kz, k2, sm);
-  if (!(k2 > 0.0f)) {
-#pragma unroll
-    for (int j = 0; j < F; j++) f[j] = make_float2(0.0f, 0.0f);
-    return;
-  }
-  float g = -p.prefac / k2;
-  float2 phi = make_float2(g * d.x, g * d.y);
-  if (p.do_smooth) {
-    d.x *= sm;
-    d.y *= sm;
-    if (p.smooth_pot) {
-      phi.x *= sm;
-      phi.y *= sm;
+  static_assert(PL::FR % 2 == 0, "an even number of modes per thread");
+#pragma unroll 1
+  for (int e = 0; e < PL::FR / 2; e++) {
+    const int kz = t + PF * e;
+    KAmp a;
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      const int z = h == 0 ? kz : (kz == 0 ? N / 2 : N - kz);
+      if (h == 0 || kz == 0) a = k_amp(p, num, kx, ky, z);
+      put(z, a);
     }
   }
-  f[0] = d;
-  f[1] = phi;
 }
 
-/* Pass 1: fill + z transform of F fields.  grid = (ceil(NH/TX), N).
- * Each thread first generates, in a rolled loop, the modes its stage-0
- * loads will read and parks every field in shared memory (one copy of the
- * generator in the instruction stream: inlined per register element it
- * overflowed the instruction cache); field 0's slot is also the exchange
- * buffer of the transforms, safe because a transform reads all its inputs
- * before its first exchange write. */
-template <int F, int TX>
-__global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, float2 *o2, FillParams p,
+/* Pass 1: fill + z transform of delta_k and phi_k (fourier.c:337-352).
+ * grid = (ceil(NH/TX), N).  The modes of the block's columns are generated by
+ * pairs and parked in shared memory; delta's slot is also the exchange buffer
+ * of the transforms, safe because a transform reads all its inputs before its
+ * first exchange write. */
+template <int TX>
+__global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, FillParams p,
                                                   const float2 *__restrict__ twN)
 {
   extern __shared__ float2 smem[];
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
   const int kx = blockIdx.x * TX + c, ky = blockIdx.y;
   const bool ok = kx < NH;
-#pragma unroll 1
-  for (int e = 0; e < PL::FR; e++) {
-    const int i = e / PL::F0, q = e - i * PL::F0;
-    const int pos = t + (N / PL::FR) * i + q * (N / PL::F0); /* cgfft::in_pos of stage 0 */
-    float2 f[F];
-    if (ok) {
-      gen_fields<F>(p, kx, ky, pos, f);
-    } else {
+  float2 *s0 = smem, *s1 = smem + (size_t)EXF * TX;
+  if (ok)
+    k_pairs(p, -p.prefac, kx, ky, t, [&](int kz, const KAmp &a) {
+      float2 d = make_float2(0.0f, 0.0f), phi = d;
+      if (a.k2 > 0.0f) {
+        d = k_draw(p, a.s2, kx, ky, kz);
+        phi = make_float2(a.ik2 * d.x, a.ik2 * d.y);
+        if (p.do_smooth) {
+          d.x *= a.sm;
+          d.y *= a.sm;
+          if (p.smooth_pot) {
+            phi.x *= a.sm;
+            phi.y *= a.sm;
+          }
+        }
+      }
+      s0[kz * TX + c] = d;
+      s1[kz * TX + c] = phi;
+    });
+  __syncthreads();
+  auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
 #pragma unroll
-      for (int jj = 0; jj < F; jj++) f[jj] = make_float2(0.0f, 0.0f);
-    }
-#pragma unroll
-    for (int jj = 0; jj < F; jj++) smem[(size_t)jj * N * TX + pos * TX + c] = f[jj];
-  }
-  float2 *outs[3] = {o0, o1, o2};
-  auto sm = [&](int pos) -> float2 & { return smem[pos * TX + c]; };
-#pragma unroll
-  for (int j = 0; j < F; j++) {
-    auto ld = [&](int pos) -> float2 { return smem[(size_t)j * N * TX + pos * TX + c]; };
-    float2 *o = outs[j];
+  for (int j = 0; j < 2; j++) {
+    const float2 *in = j == 0 ? s0 : s1;
+    auto ld = [&](int pos) -> float2 { return ok ? in[pos * TX + c] : make_float2(0.0f, 0.0f); };
+    float2 *o = j == 0 ? o0 : o1;
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
@@ -171,24 +211,21 @@ __global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, float
  * i k_i (i k_j delta'_k / (N^3 k^2)) of 2LPT (density.c:704-709), xx xy xz
  * or yy yz zz.  One value per mode is kept, b = delta'_k / (N^3 k^2) with
  * the smoothing (0 at k = 0), and each field is formed from it as the
- * transform loads it. */
-__device__ __forceinline__ float2 lpt_base(const FillParams &p, int kx, int ky, int kz)
+ * transform loads it.  The projection's partner -k has the same amplitude. */
+__device__ __forceinline__ float2 lpt_base(const FillParams &p, const KAmp &a, int kx, int ky, int kz)
 {
-  float k2, sm;
-  float2 d = gen_mode(p, kx, ky, kz, k2, sm);
-  if (!(k2 > 0.0f)) return make_float2(0.0f, 0.0f);
-  d.x *= sm;
-  d.y *= sm;
+  if (!(a.k2 > 0.0f)) return make_float2(0.0f, 0.0f);
+  float2 d = k_draw(p, a.s2, kx, ky, kz);
+  d.x *= a.sm;
+  d.y *= a.sm;
   if (kx == 0 || kx == N / 2) {
-    int ky2 = ky == 0 ? 0 : N - ky, kz2 = kz == 0 ? 0 : N - kz;
-    float k2b, smb;
-    float2 e = gen_mode(p, kx, ky2, kz2, k2b, smb);
-    e.x *= smb;
-    e.y *= smb;
+    const int ky2 = ky == 0 ? 0 : N - ky, kz2 = kz == 0 ? 0 : N - kz;
+    float2 e = k_draw(p, a.s2, kx, ky2, kz2);
+    e.x *= a.sm;
+    e.y *= a.sm;
     d = make_float2(0.5f * (d.x + e.x), 0.5f * (d.y - e.y));
   }
-  const float s = p.lpt_norm / k2;
-  return make_float2(s * d.x, s * d.y);
+  return make_float2(a.ik2 * d.x, a.ik2 * d.y);
 }
 
 __device__ __forceinline__ float2 lpt_field(const FillParams &p, int j, int kx, int ky, int kz, float2 b)
@@ -201,11 +238,10 @@ __device__ __forceinline__ float2 lpt_field(const FillParams &p, int j, int kx, 
   return make_float2(g * b.x, g * b.y);
 }
 
-/* Pass 1 of the three-field fills: as k_fill_z, but each thread parks one
- * value per mode (lpt_base) in the second shared-memory slot and the first
- * stage of each transform forms the field from it (lpt_field); the first
- * slot is the exchange buffer.  Two slots instead of three per block, so
- * three blocks fit on an SM. */
+/* Pass 1 of the three-field fills: as k_fill_z, but one value per mode
+ * (lpt_base) is parked, in the slot after the exchange buffer, and the first
+ * stage of each transform forms the field from it (lpt_field).  Two slots
+ * instead of three per block, so three blocks fit on an SM. */
 template <int TX>
 __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, float2 *o2, FillParams p,
                                                        const float2 *__restrict__ twN)
@@ -214,18 +250,16 @@ __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, f
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
   const int kx = blockIdx.x * TX + c, ky = blockIdx.y;
   const bool ok = kx < NH;
-  float2 *base = smem + (size_t)N * TX;
-#pragma unroll 1
-  for (int e = 0; e < PL::FR; e++) {
-    const int i = e / PL::F0, q = e - i * PL::F0;
-    const int pos = t + (N / PL::FR) * i + q * (N / PL::F0); /* cgfft::in_pos of stage 0 */
-    base[pos * TX + c] = ok ? lpt_base(p, kx, ky, pos) : make_float2(0.0f, 0.0f);
-  }
+  float2 *base = smem + (size_t)EXF * TX;
+  if (ok) k_pairs(p, p.lpt_norm, kx, ky, t, [&](int kz, const KAmp &a) { base[kz * TX + c] = lpt_base(p, a, kx, ky, kz); });
+  __syncthreads();
   float2 *outs[3] = {o0, o1, o2};
-  auto sm = [&](int pos) -> float2 & { return smem[pos * TX + c]; };
+  auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    auto ld = [&](int pos) -> float2 { return lpt_field(p, j, kx, ky, pos, base[pos * TX + c]); };
+    auto ld = [&](int pos) -> float2 {
+      return ok ? lpt_field(p, j, kx, ky, pos, base[pos * TX + c]) : make_float2(0.0f, 0.0f);
+    };
     float2 *o = outs[j];
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
@@ -247,7 +281,7 @@ __global__ void __launch_bounds__(TX *P) k_col_y(float2 *f0, float2 *f1, float2 
   const bool ok = kx < NH;
   float2 *f = blockIdx.z == 0 ? f0 : (blockIdx.z == 1 ? f1 : f2);
   float2 *base = f + (size_t)z * N * NH + kx;
-  auto sm = [&](int pos) -> float2 & { return smem[pos * TX + c]; };
+  auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
   auto ld = [&](int pos) -> float2 { return ok ? base[(size_t)pos * NH] : make_float2(0.0f, 0.0f); };
   auto st = [&](int pos, float2 v) {
     if (ok) base[(size_t)pos * NH] = v;
@@ -275,7 +309,7 @@ __global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 
   float2 *row = smem + rl * ROWS;
   float2 *z = zb + rl * LH;
   auto ld = [&](int j) -> float2 { return rin[j]; };
-  auto sm = [&](int pos) -> float2 & { return row[pos + (pos >> 5)]; };
+  auto sm = [&](int slot) -> float2 & { return row[slot]; };
   auto st = [&](int n, float2 v) { z[n] = v; };
   cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, -1>(t, twH, ld, st, sm);
   __syncthreads();
@@ -300,11 +334,11 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
                                                    const float2 *__restrict__ twN)
 {
   extern __shared__ float2 smem[];
-  float2 *X = smem + (size_t)N * TX;
+  float2 *X = smem + (size_t)EXF * TX;
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
   const int kx = blockIdx.x * TX + c, ky = blockIdx.y;
   const bool ok = kx < NH;
-  auto sm = [&](int pos) -> float2 & { return smem[pos * TX + c]; };
+  auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
   auto ld = [&](int pos) -> float2 { return ok ? src[((size_t)pos * N + ky) * NH + kx] : make_float2(0.0f, 0.0f); };
   auto stx = [&](int pos, float2 v) { X[pos * TX + c] = v; };
   cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, -1>(t, twN, ld, stx, sm);
@@ -364,7 +398,7 @@ __global__ void __launch_bounds__(RB *PR) k_row_c2r(float2 *f0, float2 *f1, floa
     float2 ow = make_float2(o.x * w.x - o.y * w.y, o.x * w.y + o.y * w.x);
     return make_float2(e.x - ow.y, e.y + ow.x);
   };
-  auto sm = [&](int pos) -> float2 & { return row[pos + (pos >> 5)]; };
+  auto sm = [&](int slot) -> float2 & { return row[slot]; };
   float s1 = 0.0f, s2 = 0.0f;
   auto st = [&](int n, float2 v) {
     float2 r = make_float2(v.x * norm, v.y * norm);
@@ -409,15 +443,17 @@ cudaError_t prep(K kern, size_t smem)
 /* ---- tile candidates of the autotuner ----------------------------------
  * Each pass has up to three tile widths: variant 0 is the plan's (fft_plans.h),
  * 1 half of it, 2 twice it.  A variant is valid when its shared memory fits
- * in 200 KiB and its block in 1024 threads (x pass: an even row count, for
+ * in 208 KiB and its block in 1024 threads (x pass: an even row count, for
  * the 16-byte bulk copy).  Only the block shape changes: every column and
  * row goes through the same transform, so all variants give the same bits.
  * The x pass that also sums the moments keeps the plan's RB, since the
  * per-block partial sums depend on it. */
-constexpr size_t SMEM_MAX = 200u * 1024u;
+constexpr size_t SMEM_MAX = 208u * 1024u;
 constexpr int tile_of(int def, int v) { return v == 1 ? def / 2 : (v == 2 ? def * 2 : def); }
-constexpr bool fill_ok(int T) { return T >= 1 && (size_t)2 * N * T * sizeof(float2) <= SMEM_MAX && T * PF <= 1024; }
-constexpr bool y_ok(int T) { return T >= 1 && (size_t)N * T * sizeof(float2) <= SMEM_MAX && T * P <= 1024; }
+constexpr size_t fill_smem(int T) { return (size_t)(EXF + N) * T * sizeof(float2); }
+constexpr size_t y_smem(int T) { return (size_t)EXY * T * sizeof(float2); }
+constexpr bool fill_ok(int T) { return T >= 1 && fill_smem(T) <= SMEM_MAX && T * PF <= 1024; }
+constexpr bool y_ok(int T) { return T >= 1 && y_smem(T) <= SMEM_MAX && T * P <= 1024; }
 constexpr bool x_ok(int R)
 {
   return R >= 2 && R % 2 == 0 && ((size_t)N * N) % R == 0 && (size_t)R * ROWS * sizeof(float2) <= SMEM_MAX &&
@@ -431,11 +467,11 @@ cudaError_t fill2(const cg_field_launch *L)
   if constexpr (!fill_ok(T)) {
     return cudaErrorInvalidValue;
   } else {
-    const size_t sm = (size_t)2 * N * T * sizeof(float2);
-    cudaError_t e = prep(k_fill_z<2, T>, sm);
+    const size_t sm = fill_smem(T);
+    cudaError_t e = prep(k_fill_z<T>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N);
-    k_fill_z<2, T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], nullptr, L->fill, L->twN);
+    k_fill_z<T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], L->fill, L->twN);
     return cudaGetLastError();
   }
 }
@@ -446,7 +482,7 @@ cudaError_t fill3(const cg_field_launch *L)
   if constexpr (!fill_ok(T)) {
     return cudaErrorInvalidValue;
   } else {
-    const size_t sm = (size_t)2 * N * T * sizeof(float2); /* one value per mode + the exchange buffer */
+    const size_t sm = fill_smem(T); /* one value per mode + the exchange buffer */
     cudaError_t e = prep(k_fill_z3<T>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N);
@@ -461,7 +497,7 @@ cudaError_t ypass(const cg_field_launch *L, float2 *a, float2 *b, float2 *c, int
   if constexpr (!y_ok(T)) {
     return cudaErrorInvalidValue;
   } else {
-    const size_t sm = (size_t)N * T * sizeof(float2);
+    const size_t sm = y_smem(T);
     cudaError_t e = prep(k_col_y<T, S>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N, nf);
@@ -564,7 +600,7 @@ extern "C" cudaError_t CG_CAT(cg_field_lpt2_, CG_N)(const cg_field_launch *L)
   using namespace cg;
   constexpr int TX3 = PL::TX3;
   size_t smr = (size_t)PL::RB * (ROWS + LH) * sizeof(float2);
-  size_t smz = (size_t)2 * N * TX3 * sizeof(float2);
+  size_t smz = fill_smem(TX3);
   cudaError_t e;
   if ((e = prep(k_row_r2c, smr)) != cudaSuccess) return e;
   if ((e = prep(k_z_lpt2<TX3>, smz)) != cudaSuccess) return e;
