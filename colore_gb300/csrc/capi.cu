@@ -127,6 +127,7 @@ struct cg_ctx {
   int pending_mode = CG_DMODE_NONE;
   /* sources */
   unsigned short *d_counts = nullptr;
+  cg_pois_seg *d_seg = nullptr; /* table segments of the population being counted */
   long long *d_bsums = nullptr, *d_total = nullptr, *d_ovf_cell = nullptr;
   int *d_ovf_cnt = nullptr, *d_ovf_n = nullptr;
   Cat cat[CG_NPOP_MAX];
@@ -925,7 +926,7 @@ extern "C" void cg_destroy(cg_ctx *c)
     if (q) cudaFree(q);
   void *ptrs[] = {c->d_tabs, c->d_norm, c->d_tabs64, c->d_norm64, c->d_corner, c->d_att, c->d_xstats, c->d_zr, c->d_r2n, c->d_pk, c->d_twN, c->d_twH, c->d_dens, c->d_npot, c->d_disp[0],
                   c->d_disp[1], c->d_disp[2], c->d_part, c->d_stats, c->d_s2f, c->d_err, c->d_ncount,
-                  c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_bsums, c->d_total, c->d_tmpmap, c->d_kmap,
+                  c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_seg, c->d_bsums, c->d_total, c->d_tmpmap, c->d_kmap,
                   c->d_kfac, c->d_kinv, c->d_kir, c->d_ovf_cell, c->d_ovf_cnt, c->d_ovf_n,
                   c->d_recs, c->d_imap_queue,
                   c->d_imap_isw, c->d_ifac, c->d_iir, c->d_cfac, c->d_losfac};
@@ -1439,6 +1440,7 @@ static void srcs_params(cg_ctx *c, int ipop, cg_srcs_params &p)
   for (int k = 0; k < 3; k++) p.cl[k] = c->d_corner + (size_t)(3 + k) * N;
   p.dxh = (float)dx;
   p.dxl = (float)(dx - (double)p.dxh);
+  p.seg = c->d_seg;
   p.force_double = c->force_double;
   p.xstats = c->d_xstats;
 }
@@ -1460,6 +1462,7 @@ static int srcs_run(cg_ctx *c, long long *nsrc, bool readback)
     if (!c->d_bsums && (rc = dalloc(c, &c->d_bsums, (size_t)(cg_srcs_nblocks(c->N) +
                                                              cg_srcs_scan_room(cg_srcs_nblocks(c->N))))))
       return rc;
+    if (!c->d_seg && (rc = dalloc(c, &c->d_seg, (size_t)CG_NA))) return rc;
     if (!c->d_total && (rc = dalloc(c, &c->d_total, (size_t)CG_NPOP_MAX))) return rc;
     if (!c->d_ovf_n && ((rc = dalloc(c, &c->d_ovf_cell, (size_t)CG_OVF_CAP)) ||
                         (rc = dalloc(c, &c->d_ovf_cnt, (size_t)CG_OVF_CAP)) || (rc = dalloc(c, &c->d_ovf_n, (size_t)1))))
@@ -1504,7 +1507,7 @@ static int srcs_run(cg_ctx *c, long long *nsrc, bool readback)
       ProfScope ps(c, "srcs_emit");
       CUDA_TRY(c, cg_srcs_emit(c->stream, c->d_npot, &p));
     }
-    c->launches += 5; /* count, three scan passes, emission */
+    c->launches += 6; /* count tables, count, three scan passes, emission */
   }
   c->have_srcs = 1;
   return CG_OK;

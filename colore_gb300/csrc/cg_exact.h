@@ -723,6 +723,159 @@ CG_HD int cg_lambda_checked(const cg_pois_args *a, int ix, int iy, int iz, float
   return 1;
 }
 
+/* ---- lambda from per-segment tables, with a bound ------------------------
+ * The first tier of the counts: n(r) norm(r) cell_vol and b(r) of the radial
+ * tables as polynomials in the position t in [0, 1) within a table segment,
+ * with one error bound per segment, so that a cell takes two 16-byte loads
+ * and a few multiply-adds where cg_lambda_checked takes eight loads and a
+ * bound per lookup.  The bounds are looser; a cell they leave open goes
+ * through cg_lambda_checked. */
+typedef struct {
+  float c0, c1, c2, e;  /* n norm cell_vol = c0 + t (c1 + t c2) within e */
+  float b0, b1, eb, w;  /* b = b0 + t b1 within eb; w unused */
+} cg_pois_seg;
+
+/* How far the float position s = r idr of cg_seg_pos may be from the double
+ * one, near segment i: r^2 from corners rounded once (2^-24 relative) and
+ * three more roundings, rsqrt 2^-22, two products and idr's rounding, less
+ * than 12 2^-24 relative in all, of s < i + 2. */
+CG_HD double cg_seg_dt(int i) { return (i + 2) * 12.0 * 5.9604644775390625e-08 + 1e-6; }
+
+/* Segment i (0 <= i < na - 1).  The double radius may lie in a neighbouring
+ * segment (dt < 1), so the slopes bound all three; 8 and 4 roundings of the
+ * coefficients and the evaluation, and 2 % for the bound's own arithmetic. */
+CG_HD cg_pois_seg cg_pois_seg_make(const cgx_srcs_tabs *x, int na, int i)
+{
+  const double dt = cg_seg_dt(i);
+  double S = 0, Sb = 0, c0 = 0, c1 = 0, c2 = 0, b0 = 0, b1 = 0;
+  for (int k = i - 1; k <= i + 1; k++) {
+    if (k < 0 || k > na - 2) continue;
+    const double a = x->nz[k], da = x->nz[k + 1] - a, c = x->norm[k], dc = x->norm[k + 1] - c;
+    const double k1 = x->cell_vol * (a * dc + da * c), k2 = x->cell_vol * da * dc;
+    const double s0 = fabs(k1), s1 = fabs(k1 + 2 * k2), sb = fabs(x->bz[k + 1] - x->bz[k]);
+    if (s0 > S) S = s0;
+    if (s1 > S) S = s1;
+    if (sb > Sb) Sb = sb;
+    if (k != i) continue;
+    c0 = x->cell_vol * a * c;
+    c1 = k1;
+    c2 = k2;
+    b0 = x->bz[k];
+    b1 = x->bz[k + 1] - b0;
+  }
+  cg_pois_seg o;
+  o.c0 = (float)c0;
+  o.c1 = (float)c1;
+  o.c2 = (float)c2;
+  o.e = (float)(1.02 * (S * dt + 8 * 5.9604644775390625e-08 * (fabs(c0) + fabs(c1) + fabs(c2))));
+  o.b0 = (float)b0;
+  o.b1 = (float)b1;
+  o.eb = (float)(1.02 * (Sb * dt + 4 * 5.9604644775390625e-08 * (fabs(b0) + fabs(b1))));
+  o.w = 0.0f;
+  return o;
+}
+
+/* 2^x and log2 x: the device's approximate instructions (2^x within 2^-22
+ * relative; log2 within 2^-22 absolute on (1/2, 2) and 2^-22 relative
+ * outside), the libm functions on the host. */
+CG_HD float cg_ex2_fast(float x)
+{
+#if defined(__CUDA_ARCH__)
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+#else
+  return exp2f(x);
+#endif
+}
+
+CG_HD float cg_lg2_fast(float x)
+{
+#if defined(__CUDA_ARCH__)
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+#else
+  return log2f(x);
+#endif
+}
+
+/* lambda of a cell with density d at position t of segment g, and the bound
+ * *elam on its distance to cgx_lambda; *pos is 1 when n(r) > 0 is certain.
+ * An infinite *elam leaves the cell open. */
+CG_HD float cg_lambda_seg(const cg_pois_seg *g, float t, float d, int model, float *elam, int *pos)
+{
+  const float G = CG_FMA(CG_FMA(g->c2, t, g->c1), t, g->c0);
+  const float b = CG_FMA(g->b1, t, g->b0);
+  float v, ev;
+  if (d <= -1.0f) {
+    v = 0.0f;
+    ev = 0.0f;
+  } else if (model == CG_BIAS_POW || (model == CG_BIAS_EXPLIN && d < 0.0f)) {
+    /* v = 2^y: y and the bound ey on it; 2^ey - 1 <= 0.85 ey while ey < 1/4,
+     * and a y certainly below -87 makes v < 2^-87 */
+    const float w = CG_ADD(1.0f, d);
+    float y, ey;
+    if (model == CG_BIAS_POW) {
+      /* b log2(1 + d): 1 + d rounded (2^-24 relative: 8.6e-8 of log2),
+       * lg2 2^-22, the product */
+      const float l = cg_lg2_fast(w);
+      y = CG_MUL(b, l);
+      const float el = CG_FMA(cg_max_nn(1.0f, cg_fabsf(l)), CG_E22, 1e-7f);
+      ey = CG_FMA(cg_fabsf(l), g->eb, CG_FMA(cg_fabsf(b), el, CG_MUL(cg_fabsf(y), CG_E24)));
+    } else {
+      /* b d / (1 + d) log2(e): 1 + d, rcp 2^-22, three products and the
+       * constant, less than 10 2^-24 relative */
+      const float q = CG_MUL(CG_MUL(d, cg_rcp_fast(w)), 1.44269504f);
+      y = CG_MUL(b, q);
+      ey = CG_FMA(cg_fabsf(q), g->eb, CG_MUL(cg_fabsf(y), 10.0f * CG_E24));
+    }
+    v = cg_ex2_fast(y);
+    ev = CG_FMA(v, CG_FMA(0.85f, ey, 3.0f * CG_E22), 1e-37f);
+    if (!(ey < 0.25f)) ev = 3.0e38f;
+    if (CG_ADD(y, ey) < -87.0f) {
+      v = 0.0f;
+      ev = 2e-26f;
+    }
+  } else {
+    v = CG_FMA(b, d, 1.0f);
+    ev = CG_FMA(cg_fabsf(d), g->eb, CG_MUL(4.0f * CG_E24, CG_ADD(cg_fabsf(v), 1.0f)));
+    if (model == CG_BIAS_LIN) v = cg_max_nn(v, 0.0f);
+  }
+  const float l = CG_MUL(G, v);
+  /* |d lambda| <= e (v + ev) + |G| ev, the product's rounding, 2 % */
+  *elam = CG_FMA(1.02f, CG_FMA(g->e, CG_ADD(v, ev), CG_MUL(cg_fabsf(G), ev)), CG_FMA(cg_fabsf(l), 2.0f * CG_E24, 1e-36f));
+  *pos = G > g->e;
+  return l;
+}
+
+/* Position of radius squared r2 > 0 in the tables. */
+CG_HD float cg_seg_pos(float r2, float idr, float *r)
+{
+  *r = CG_MUL(r2, cg_rsqrt_fast(r2));
+  return CG_MUL(*r, idr);
+}
+
+/* First tier of a cell's count: 0 or the count when the segment tables prove
+ * it, -1 when they leave it open (cg_count_cell then decides). */
+CG_HD int cg_count_seg(const cg_pois_seg *segs, const cg_pois_args *a, float r2, float d, float u)
+{
+  float r;
+  if (!(r2 > 0.0f)) return -1;
+  const float s = cg_seg_pos(r2, a->idr, &r);
+  if (r > CG_MUL(a->rlim, 1.000001f)) return 0;
+  if (!(r < CG_MUL(cg_min_nn(a->rlim, a->r_last), 0.999999f))) return -1;
+  const int i = (int)s;
+  float e;
+  int pos;
+  const float l = cg_lambda_seg(&segs[i], CG_SUB(s, (float)i), d, a->bias_model, &e, &pos);
+  /* u < 1 - lambda <= exp(-lambda): no source, whatever the sign of n(r) */
+  const float hi = CG_ADD(cg_max_nn(l, 0.0f), e);
+  if (u < CG_SUB(CG_SUB(1.0f, hi), 2.0f * CG_E24)) return 0;
+  if (!pos || !(hi < 9.99f)) return -1;
+  return cg_poisson_inv_checked(l, e, u);
+}
+
 /* The count of one cell given its Poisson word w: single precision when its
  * margins hold, the double restatement otherwise (*fb set to 1). */
 CG_HD int cg_count_cell(const cg_pois_args *a, int ix, int iy, int iz, float d, long long cid, uint32_t w,

@@ -237,8 +237,8 @@ __host__ __device__ __forceinline__ void stage(float2 *v, int t, const float2 *_
  * power of two dividing r0: thread t's writes then lie (r0 + r0/2^sh) t slots
  * apart, an odd stride, which spreads over all banks for any number of
  * columns; reads at consecutive positions stay consecutive but for one slot
- * per 2^sh.  (y pass at 512^3: 10.9 M conflict wavefronts per launch without
- * the padding, as many as the accesses themselves.) */
+ * per 2^sh.  A tile of 16 or more columns fills the wavefront with one
+ * position and takes no padding (sh = 31). */
 __host__ __device__ constexpr int pad_shift(int r0)
 {
   int s = 0;
@@ -248,14 +248,16 @@ __host__ __device__ constexpr int pad_shift(int r0)
   }
   return s;
 }
-/* Slots of a padded exchange buffer of length L. */
-__host__ __device__ constexpr int pad_len(int L, int r0) { return L + (L >> pad_shift(r0)); }
+constexpr int NO_PAD = 31;
+/* Slots of an exchange buffer of length L. */
+__host__ __device__ constexpr int pad_len(int L, int sh) { return L + (L >> sh); }
 
 /* Slot of position base + off.  off is a constant once loops are unrolled,
  * and splits off the shift when either part is a multiple of 2^sh. */
 template <int SH>
 __host__ __device__ __forceinline__ int pad_at(int base, int off, bool base_aligned)
 {
+  if (SH == NO_PAD) return base + off;
   if (base_aligned || (off & ((1 << SH) - 1)) == 0) return (base + (base >> SH)) + (off + (off >> SH));
   return base + off + ((base + off) >> SH);
 }
@@ -264,14 +266,14 @@ __host__ __device__ __forceinline__ int pad_at(int base, int off, bool base_alig
  * Full transform of length L = r0*r1*r2 (r2 = 1 for two stages, r1 = r2 = 1
  * for one) by P = L/R threads.  Ld(pos) -> float2 supplies the input,
  * St(pos, value) consumes the output, Sm(slot) -> float2& addresses slot
- * 0..pad_len(L, r0)-1 of this transform's shared-memory exchange buffer.
+ * 0..pad_len(L, SH)-1 of this transform's shared-memory exchange buffer
+ * (SH: pad_shift(r0) or NO_PAD).
  * Contains the barriers of the exchanges, so every thread of the block must
  * call it.
  */
-template <int L, int R, int r0, int r1, int r2, int S, class Ld, class St, class Sm>
+template <int L, int R, int r0, int r1, int r2, int S, int SH, class Ld, class St, class Sm>
 __device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL, Ld ld, St st, Sm sm)
 {
-  constexpr int SH = pad_shift(r0);
   float2 v[R];
 #pragma unroll
   for (int i = 0; i < R / r0; i++)

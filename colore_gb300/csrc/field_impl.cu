@@ -55,10 +55,18 @@ constexpr int P = N / PL::CR;       /* threads per column transform (y pass)    
 constexpr int PF = N / PL::FR;      /* threads per column transform (fill + z)    */
 constexpr int LH = N / 2;           /* row transform length         */
 constexpr int PR = LH / PL::RR;     /* threads per row transform    */
-constexpr int EXF = cgfft::pad_len(N, PL::F0);  /* exchange slots per column (fill + z) */
-constexpr int EXY = cgfft::pad_len(N, PL::C0);  /* exchange slots per column (y pass)   */
-constexpr int EXX = cgfft::pad_len(LH, PL::R0); /* exchange slots per row (x pass)      */
-constexpr int ROWS = NH > EXX ? NH : EXX;       /* smem per row */
+/* Exchange slots (fft.cuh).  The fills and the x pass are padded against
+ * bank conflicts; the y pass is not: it waits for HBM, and the padding takes
+ * shared memory from the L1 that holds its loads in flight (512^3, tiles of
+ * 16 columns: 0.406 ms without, 0.546 ms with). */
+constexpr int fill_sh(int TX) { return TX >= 16 ? cgfft::NO_PAD : cgfft::pad_shift(PL::F0); }
+template <int TX>
+constexpr int FSH = fill_sh(TX);
+constexpr int SHX = cgfft::pad_shift(PL::R0);
+constexpr int EXX = cgfft::pad_len(LH, SHX);
+constexpr int ROWS = NH > EXX ? NH : EXX; /* smem per row */
+template <int TX>
+constexpr int EXF = cgfft::pad_len(N, fill_sh(TX)); /* exchange slots per column of the fills */
 
 /* P(k) at log10 k, pk_linear0 (cosmo.c:291-308).  The interpolation branch
  * stops at numk-2: the reference also takes it for ik = numk-1 and then
@@ -170,7 +178,7 @@ __global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, FillP
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
   const int kx = blockIdx.x * TX + c, ky = blockIdx.y;
   const bool ok = kx < NH;
-  float2 *s0 = smem, *s1 = smem + (size_t)EXF * TX;
+  float2 *s0 = smem, *s1 = smem + (size_t)EXF<TX> * TX;
   if (ok)
     k_pairs(p, -p.prefac, kx, ky, t, [&](int kz, const KAmp &a) {
       float2 d = make_float2(0.0f, 0.0f), phi = d;
@@ -199,7 +207,7 @@ __global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, FillP
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1>(t, twN, ld, st, sm);
+    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, twN, ld, st, sm);
     __syncthreads();
   }
 }
@@ -250,7 +258,7 @@ __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, f
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
   const int kx = blockIdx.x * TX + c, ky = blockIdx.y;
   const bool ok = kx < NH;
-  float2 *base = smem + (size_t)EXF * TX;
+  float2 *base = smem + (size_t)EXF<TX> * TX;
   if (ok) k_pairs(p, p.lpt_norm, kx, ky, t, [&](int kz, const KAmp &a) { base[kz * TX + c] = lpt_base(p, a, kx, ky, kz); });
   __syncthreads();
   float2 *outs[3] = {o0, o1, o2};
@@ -264,7 +272,7 @@ __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, f
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1>(t, twN, ld, st, sm);
+    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, twN, ld, st, sm);
     __syncthreads();
   }
 }
@@ -286,7 +294,7 @@ __global__ void __launch_bounds__(TX *P) k_col_y(float2 *f0, float2 *f1, float2 
   auto st = [&](int pos, float2 v) {
     if (ok) base[(size_t)pos * NH] = v;
   };
-  cgfft::transform<N, PL::CR, PL::C0, PL::C1, PL::C2, S>(t, twN, ld, st, sm);
+  cgfft::transform<N, PL::CR, PL::C0, PL::C1, PL::C2, S, cgfft::NO_PAD>(t, twN, ld, st, sm);
 }
 
 /* Forward pass 1 of the 2LPT source: row r2c along x, in place.  A row's N
@@ -311,7 +319,7 @@ __global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 
   auto ld = [&](int j) -> float2 { return rin[j]; };
   auto sm = [&](int slot) -> float2 & { return row[slot]; };
   auto st = [&](int n, float2 v) { z[n] = v; };
-  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, -1>(t, twH, ld, st, sm);
+  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, -1, SHX>(t, twH, ld, st, sm);
   __syncthreads();
   float2 *dst = f + (row0 + rl) * NH;
   for (int k = t; k <= LH; k += PR) {
@@ -334,14 +342,14 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
                                                    const float2 *__restrict__ twN)
 {
   extern __shared__ float2 smem[];
-  float2 *X = smem + (size_t)EXF * TX;
+  float2 *X = smem + (size_t)EXF<TX> * TX;
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
   const int kx = blockIdx.x * TX + c, ky = blockIdx.y;
   const bool ok = kx < NH;
   auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
   auto ld = [&](int pos) -> float2 { return ok ? src[((size_t)pos * N + ky) * NH + kx] : make_float2(0.0f, 0.0f); };
   auto stx = [&](int pos, float2 v) { X[pos * TX + c] = v; };
-  cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, -1>(t, twN, ld, stx, sm);
+  cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, -1, FSH<TX>>(t, twN, ld, stx, sm);
   __syncthreads();
   float2 *outs[3] = {o0, o1, o2};
   const float kxf = (float)kx * dk, kyf = kcomp(ky, N, dk);
@@ -360,7 +368,7 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1>(t, twN, ld2, st, sm);
+    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, twN, ld2, st, sm);
     __syncthreads();
   }
 }
@@ -408,7 +416,7 @@ __global__ void __launch_bounds__(RB *PR) k_row_c2r(float2 *f0, float2 *f1, floa
       s2 += r.x * r.x + r.y * r.y;
     }
   };
-  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, 1>(t, twH, ld, st, sm);
+  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, 1, SHX>(t, twH, ld, st, sm);
   if (STATS) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -443,15 +451,15 @@ cudaError_t prep(K kern, size_t smem)
 /* ---- tile candidates of the autotuner ----------------------------------
  * Each pass has up to three tile widths: variant 0 is the plan's (fft_plans.h),
  * 1 half of it, 2 twice it.  A variant is valid when its shared memory fits
- * in 208 KiB and its block in 1024 threads (x pass: an even row count, for
+ * in 200 KiB and its block in 1024 threads (x pass: an even row count, for
  * the 16-byte bulk copy).  Only the block shape changes: every column and
  * row goes through the same transform, so all variants give the same bits.
  * The x pass that also sums the moments keeps the plan's RB, since the
  * per-block partial sums depend on it. */
-constexpr size_t SMEM_MAX = 208u * 1024u;
+constexpr size_t SMEM_MAX = 200u * 1024u;
 constexpr int tile_of(int def, int v) { return v == 1 ? def / 2 : (v == 2 ? def * 2 : def); }
-constexpr size_t fill_smem(int T) { return (size_t)(EXF + N) * T * sizeof(float2); }
-constexpr size_t y_smem(int T) { return (size_t)EXY * T * sizeof(float2); }
+constexpr size_t fill_smem(int T) { return (size_t)(cgfft::pad_len(N, fill_sh(T)) + N) * T * sizeof(float2); }
+constexpr size_t y_smem(int T) { return (size_t)N * T * sizeof(float2); }
 constexpr bool fill_ok(int T) { return T >= 1 && fill_smem(T) <= SMEM_MAX && T * PF <= 1024; }
 constexpr bool y_ok(int T) { return T >= 1 && y_smem(T) <= SMEM_MAX && T * P <= 1024; }
 constexpr bool x_ok(int R)

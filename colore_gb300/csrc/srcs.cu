@@ -4,10 +4,11 @@
  * redshift-space distortion at each source (srcs.c:425-504, 634-662).
  *
  * Sampling is count -> scan -> emit:
- *   k_pois_count : one block per 2048 consecutive cells; per cell lambda and
- *                  a Poisson deviate keyed by (seed, population, cell), so the
- *                  result does not depend on the launch shape; counts are kept
- *                  as uint16 and the block totals written out.  A cell with
+ *   k_pois_tab   : n(r) norm(r) and b(r) per table segment, with bounds.
+ *   k_pois_count : per cell lambda and a Poisson deviate keyed by (seed,
+ *                  population, cell), so the result does not depend on the
+ *                  launch shape; counts are kept as uint16 and the totals of
+ *                  every 2048 consecutive cells summed up.  A cell with
  *                  CG_COUNT_ESC or more sources stores the escape value and
  *                  appends (cell, count) to a short overflow list.
  *   k_scan_*     : exclusive scan of the block totals (three coalesced passes).
@@ -70,88 +71,235 @@ __device__ __noinline__ int count_double(const cg_srcs_params &p, int ix, int iy
   return cgx_poisson(lam, (double)cg_u01f(w), cid, p.kp0, p.kp1);
 }
 
-/* PTRS in single precision (lambda >= 10: the cells next to the observer,
- * or dense coarse grids), out of line like the double path. */
+/* The table segments of the counts' first tier, from the double tables and
+ * this realisation's normalisation; the overflow list and the block totals
+ * are cleared along the way. */
+__global__ void __launch_bounds__(32) k_pois_tab(cg_srcs_params p, long long nb)
+{
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
+  for (long long i = i0; i < CG_NA - 1; i += st) p.seg[i] = cg_pois_seg_make(&p.pa.x, CG_NA, (int)i);
+  for (long long i = i0; i < nb; i += st) p.block_sums[i] = 0;
+  if (i0 == 0) *p.ovf_n = 0;
+}
+
+/* A cell that the segment tables leave open: lambda with the per-lookup
+ * bounds (cg_lambda_checked), then inversion or PTRS in single precision
+ * where its margins allow, else double (bit 31 set).  Out of line: a few
+ * cells in 10^4, and the cells with lambda >= 10. */
+__device__ __noinline__ unsigned int count_open(const cg_srcs_params &p, const float *__restrict__ grid, long long cid)
+{
+  int ix, iy, iz;
+  cell_of(cid, p.box, ix, iy, iz);
+  const float d = __ldg(grid + pidx(ix, iy, iz, p.box.N));
+  float lam, elam;
+  int st = cg_lambda_checked(&p.pa, ix, iy, iz, d, &lam, &elam);
+  if (p.force_double && (st == 1 || st == 3)) st = 2;
+  if (st == 0) return 0;
+  const uint32_t w = cg_pois_word(cid, p.kp0, p.kp1);
+  int n = st == 1 ? cg_poisson_inv_checked(lam, elam, cg_u01f(w))
+                  : (st == 3 ? cg_poisson_ptrs_checked(lam, elam, cid, p.kp0, p.kp1) : -1);
+  if (n < 0) return (unsigned int)count_double(p, ix, iy, iz, d, cid, w) | 0x80000000u;
+  return (unsigned int)n;
+}
+
+/* PTRS of a cell whose lambda >= 10 is certain (cells next to the observer,
+ * dense coarse grids), out of line like the double path. */
 __device__ __noinline__ int ptrs_float(float lam, float elam, long long cid, uint32_t k0, uint32_t k1)
 {
   return cg_poisson_ptrs_checked(lam, elam, cid, k0, k1);
 }
 
-/* Counts of CPT consecutive cells of one row per thread.  Each cell's lambda
- * is formed in single precision with a bound on its distance to the
- * reference's double lambda, and the Poisson inversion keeps its float
- * count when the uniform lies farther from the bracketing cumulative values
- * than that bound carries them (cg_exact.h); the other cells -- and every
- * cell with lambda >= 10, for PTRS -- take the double arithmetic.  Cells
- * 4m..4m+3 share one Philox block, drawn only when one of them has a
- * positive lambda.  The cell loop is not unrolled (unrolled, the kernel ran
- * instruction-fetch bound); the counts are packed in two 64-bit registers.
- * Each warp adds its total to the block's entry (zeroed before the launch),
- * so warps that finish early do not wait for the block's slowest.  Six
- * blocks per SM (40 registers): the table lookups' latency wants the warps
- * more than the few spills cost (13.1 -> 12.0 ms at 1024^3 against four). */
-__global__ void __launch_bounds__(SB, 6) k_pois_count(const float *__restrict__ grid, cg_srcs_params p)
+constexpr int CWN = 4;  /* warps per block of the count */
+constexpr int CW = 128; /* cells per warp and step: four neighbours per lane */
+
+/* A warp's cells in shared memory: from the front those to be inverted
+ * (lambda, its bound, and the uniform's 24 bits with the cell's place above
+ * them), from the back those for PTRS (the same without a uniform); those
+ * left open by the segment tables; and the counts. */
+struct alignas(16) CountWarp {
+  float lam[CW], elam[CW];
+  unsigned int uc[CW];
+  unsigned char open[CW];
+  unsigned short cnt[CW];
+};
+
+/* Counts, 128 cells per warp and step, `steps` consecutive steps per warp.
+ * First tier: a lane forms lambda of four neighbouring cells of a row from
+ * the segment tables (cg_lambda_seg: two 16-byte loads and about 40
+ * instructions a cell), draws their Philox block when one may hold a source,
+ * and settles u < 1 - lambda on the spot.  The cells left are compacted per
+ * warp in shared memory and inverted (lambda < 10) or sampled by PTRS 32 at a
+ * time, so that the exponential and the search run in full warps (inverted in
+ * place, every warp paid for both in every step: 390 issue slots per cell at
+ * 512^3, now 165).  Cells that the tier's bounds leave open follow in a last
+ * list (count_open); every count is the reference's double decision.  Each
+ * warp adds its total to the entry of its 2048 cells.  Twelve blocks per SM
+ * (40 registers).  1024^3, 1000 sources per deg^2: 11.0 -> 5.3 ms; 512^3, two
+ * populations: 3.04 -> 1.42 ms. */
+__global__ void __launch_bounds__(CWN * 32, 12) k_pois_count(const float *__restrict__ grid, cg_srcs_params p, int steps)
 {
+  __shared__ CountWarp sw[CWN];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned int below = (1u << lane) - 1u;
+  CountWarp &S = sw[wid];
   const int N = p.box.N;
-  const long long ncell = (long long)N * N * N;
-  const long long c0 = (long long)blockIdx.x * CPB + (long long)threadIdx.x * CPT;
+  const float rhi = CG_MUL(p.pa.rlim, 1.000001f), rlo = CG_MUL(cg_min_nn(p.pa.rlim, p.pa.r_last), 0.999999f);
   long long tot = 0;
   unsigned int nfb = 0;
-  if (c0 < ncell) {
+  const long long wbase = ((long long)blockIdx.x * CWN + wid) * steps * CW;
+#pragma unroll 1
+  for (int step = 0; step < steps; step++) {
+    const long long w0 = wbase + step * CW;
+    const long long c0 = w0 + 4 * lane;
     int ix, iy, iz;
     cell_of(c0, p.box, ix, iy, iz);
-    const float *row = grid + pidx(ix, iy, iz, N);
-    unsigned long long lo = 0, hi = 0;
-    long long wm = -1; /* the Philox block held in w */
-    cg_u32x4 w;
-    w.v[0] = w.v[1] = w.v[2] = w.v[3] = 0u;
-#pragma unroll 1
-    for (int h = 0; h < CPT; h++) {
-      const long long cid = c0 + h;
-      const float d = __ldg(row + h);
-      float lam, elam;
-      int st = cg_lambda_checked(&p.pa, ix + h, iy, iz, d, &lam, &elam);
-      if (p.force_double && (st == 1 || st == 3)) st = 2;
-      int n = 0;
-      if (st != 0) {
-        if ((cid >> 2) != wm) {
-          wm = cid >> 2;
-          w = cg_philox4x32_10((uint32_t)wm, (uint32_t)((unsigned long long)wm >> 32), 0u, 0u, p.kp0, p.kp1);
+    float lam[4], elam[4];
+    /* per cell: left open, may hold a source, proper for inversion or PTRS */
+    unsigned int open = 0u, may = 0u, inv = 0u, ptr = 0u;
+    if (p.force_double) {
+      open = 0xfu;
+    } else {
+      /* rows start at an even float (8-byte aligned), ix is a multiple of 4 */
+      const float2 *row = reinterpret_cast<const float2 *>(grid + pidx(ix, iy, iz, N));
+      const float2 da = __ldg(row), db = __ldg(row + 1);
+      const float4 x4 = __ldg(reinterpret_cast<const float4 *>(p.pa.xc + ix));
+      const float d4[4] = {da.x, da.y, db.x, db.y}, xs[4] = {x4.x, x4.y, x4.z, x4.w};
+      const float y = __ldg(p.pa.yc + iy), z = __ldg(p.pa.zc + iz);
+      const float yz2 = CG_FMA(z, z, CG_MUL(y, y));
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float r2 = CG_FMA(xs[q], xs[q], yz2);
+        float r;
+        const float s = cg_seg_pos(r2, p.pa.idr, &r);
+        lam[q] = elam[q] = 0.0f;
+        if (r > rhi) continue;
+        if (!(r2 > 0.0f && r < rlo)) {
+          open |= 1u << q;
+          continue;
         }
-        const int q = (int)(cid & 3);
-        const uint32_t wq = q == 0 ? w.v[0] : (q == 1 ? w.v[1] : (q == 2 ? w.v[2] : w.v[3]));
-        n = st == 1 ? cg_poisson_inv_checked(lam, elam, cg_u01f(wq))
-                    : (st == 3 ? ptrs_float(lam, elam, cid, p.kp0, p.kp1) : -1);
-        if (n < 0) {
-          n = count_double(p, ix + h, iy, iz, d, cid, wq);
-          nfb++;
-        }
+        const int i = (int)s;
+        const float4 *g4 = reinterpret_cast<const float4 *>(p.seg + i);
+        const float4 ga = __ldg(g4), gb = __ldg(g4 + 1);
+        const cg_pois_seg g = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, 0.0f};
+        int pos;
+        lam[q] = cg_lambda_seg(&g, CG_SUB(s, (float)i), d4[q], p.pa.bias_model, &elam[q], &pos);
+        const float hi = CG_ADD(cg_max_nn(lam[q], 0.0f), elam[q]);
+        /* a uniform is at most 1 - 2^-24: lambda below 2^-25 draws nothing */
+        if (!(hi < 0.5f * CG_E24)) may |= 1u << q;
+        if (pos && hi < 9.99f) inv |= 1u << q;
+        else if (pos && CG_SUB(lam[q], elam[q]) > 10.01f) ptr |= 1u << q;
       }
-      unsigned long long v = (unsigned long long)n;
-      if (n >= CG_COUNT_ESC) {
-        const int k = atomicAdd(p.ovf_n, 1);
-        if (k < CG_OVF_CAP) {
-          p.ovf_cell[k] = cid;
-          p.ovf_cnt[k] = n;
-        } else {
-          atomicOr(p.err, ERR_COUNT_OVERFLOW);
-        }
-        v = CG_COUNT_ESC;
-      }
-      if (h < 4) lo |= v << (16 * h);
-      else hi |= v << (16 * (h - 4));
-      tot += n;
     }
-    *reinterpret_cast<uint4 *>(p.counts + c0) =
-        make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+    unsigned int u24[4] = {0u, 0u, 0u, 0u};
+    if (may & ~ptr) {
+      const unsigned long long m = (unsigned long long)c0 >> 2;
+      const cg_u32x4 w = cg_philox4x32_10((uint32_t)m, (uint32_t)(m >> 32), 0u, 0u, p.kp0, p.kp1);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        u24[q] = w.v[q] >> 8;
+        /* u < 1 - lambda <= exp(-lambda): no source, whatever the sign of n(r) */
+        const float hi = CG_ADD(cg_max_nn(lam[q], 0.0f), elam[q]);
+        if (CG_MUL((float)u24[q], CG_E24) < CG_SUB(CG_SUB(1.0f, hi), 2.0f * CG_E24)) may &= ~(1u << q);
+      }
+    }
+    open |= may & ~(inv | ptr);
+    inv &= may;
+    *reinterpret_cast<uint2 *>(&S.cnt[4 * lane]) = make_uint2(0u, 0u);
+    int na = 0, np = 0, no = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bool a = (inv >> q) & 1u;
+      const unsigned int m = __ballot_sync(0xffffffffu, a);
+      if (a) {
+        const int k = na + __popc(m & below);
+        S.lam[k] = lam[q];
+        S.elam[k] = elam[q];
+        S.uc[k] = u24[q] | ((unsigned int)(4 * lane + q) << 24);
+      }
+      na += __popc(m);
+    }
+    if (__any_sync(0xffffffffu, (open | ptr) != 0u)) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const bool o = (open >> q) & 1u, t = (ptr >> q) & 1u;
+        const unsigned int m = __ballot_sync(0xffffffffu, o), mt = __ballot_sync(0xffffffffu, t);
+        if (o) S.open[no + __popc(m & below)] = (unsigned char)(4 * lane + q);
+        if (t) {
+          const int k = CW - 1 - np - __popc(mt & below);
+          S.lam[k] = lam[q];
+          S.elam[k] = elam[q];
+          S.uc[k] = (unsigned int)(4 * lane + q) << 24;
+        }
+        no += __popc(m);
+        np += __popc(mt);
+      }
+    }
+    __syncwarp();
+    /* the inversions, then the PTRS cells */
+#pragma unroll 1
+    for (int k0 = 0; k0 < na; k0 += 32) {
+      const int k = k0 + lane;
+      int n = 0, c = 0;
+      if (k < na) {
+        const unsigned int uc = S.uc[k];
+        c = (int)(uc >> 24);
+        n = cg_poisson_inv_checked(S.lam[k], S.elam[k], CG_MUL((float)(uc & 0xffffffu), CG_E24));
+        if (n > 0) S.cnt[c] = (unsigned short)n; /* below 64 */
+      }
+      const unsigned int m = __ballot_sync(0xffffffffu, n < 0);
+      if (n < 0) S.open[no + __popc(m & below)] = (unsigned char)c;
+      else tot += n;
+      no += __popc(m);
+    }
+    if (np) {
+#pragma unroll 1
+      for (int k0 = 0; k0 < np; k0 += 32) {
+        const int k = CW - 1 - k0 - lane;
+        int n = 0, c = 0;
+        if (k0 + lane < np) {
+          c = (int)(S.uc[k] >> 24);
+          n = ptrs_float(S.lam[k], S.elam[k], w0 + c, p.kp0, p.kp1);
+          if (n >= CG_COUNT_ESC) n = -1; /* the overflow list is count_open's */
+          if (n > 0) S.cnt[c] = (unsigned short)n;
+        }
+        const unsigned int m = __ballot_sync(0xffffffffu, n < 0);
+        if (n < 0) S.open[no + __popc(m & below)] = (unsigned char)c;
+        else tot += n;
+        no += __popc(m);
+      }
+    }
+    if (no) {
+      __syncwarp();
+#pragma unroll 1
+      for (int k = lane; k < no; k += 32) {
+        const int c = S.open[k];
+        const unsigned int o1 = count_open(p, grid, w0 + c);
+        const int n = (int)(o1 & 0x7fffffffu);
+        nfb += o1 >> 31;
+        tot += n;
+        if (n >= CG_COUNT_ESC) {
+          const int o = atomicAdd(p.ovf_n, 1);
+          if (o < CG_OVF_CAP) {
+            p.ovf_cell[o] = w0 + c;
+            p.ovf_cnt[o] = n;
+          } else {
+            atomicOr(p.err, ERR_COUNT_OVERFLOW);
+          }
+        }
+        S.cnt[c] = (unsigned short)(n < CG_COUNT_ESC ? n : CG_COUNT_ESC);
+      }
+    }
+    __syncwarp();
+    *reinterpret_cast<uint2 *>(p.counts + c0) = *reinterpret_cast<const uint2 *>(&S.cnt[4 * lane]);
+    __syncwarp();
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     tot += __shfl_xor_sync(0xffffffffu, tot, o);
     nfb += __shfl_xor_sync(0xffffffffu, nfb, o);
   }
-  if ((threadIdx.x & 31) == 0) {
-    if (tot) atomicAdd(reinterpret_cast<unsigned long long *>(&p.block_sums[blockIdx.x]), (unsigned long long)tot);
+  if (lane == 0) {
+    if (tot) atomicAdd(reinterpret_cast<unsigned long long *>(&p.block_sums[wbase / CPB]), (unsigned long long)tot);
     if (nfb) atomicAdd(p.xstats, (unsigned long long)nfb);
   }
 }
@@ -581,10 +729,13 @@ long long cg_srcs_scan_room(long long nb) { return (nb + SCAN_T - 1) / SCAN_T; }
 cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_params *p, long long *total)
 {
   long long nb = cg_srcs_nblocks(p->box.N);
-  cudaError_t e = cudaMemsetAsync(p->ovf_n, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(p->block_sums, 0, nb * sizeof(long long), s);
-  if (e != cudaSuccess) return e;
-  k_pois_count<<<(unsigned)nb, SB, 0, s>>>(grid, *p);
+  k_pois_tab<<<(CG_NA + 31) / 32, 32, 0, s>>>(*p, nb);
+  /* four steps per warp where the grid has many times the 7296 warps that 152
+   * SMs hold (512^3, two populations: 1.44 ms against 1.50 with two); one on
+   * small grids, whose dense cells near the observer would leave the last
+   * warps alone (128^3) */
+  const int steps = p->box.N > 256 ? 4 : 1;
+  k_pois_count<<<(unsigned)(nb * CPB / (CWN * CW * steps)), CWN * 32, 0, s>>>(grid, *p, steps);
   const long long nt = cg_srcs_scan_room(nb);
   long long *tsum = p->block_sums + nb; /* the tile sums, just past the block totals */
   k_scan_tiles<<<(unsigned)nt, 1024, 0, s>>>(p->block_sums, nb, tsum, p->err);

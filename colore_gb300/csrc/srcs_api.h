@@ -41,6 +41,7 @@ struct cg_srcs_params {
    * the emitted positions; every decision in double when force_double;
    * xstats[0] cells and xstats[1] pixels decided in double */
   cg_pois_args pa;
+  cg_pois_seg *seg;    /* the population's CG_NA - 1 table segments (written by cg_srcs_count) */
   double dx64, p64[3];
   const float *cl[3];  /* low parts of the float corners (pa.xc..: c + l = the double corner) */
   float dxh, dxl;      /* dx as a float pair */

@@ -4,6 +4,8 @@
  * check them against libm, numpy and HEALPix identities on the CPU.
  */
 #include <stdint.h>
+#include <stdlib.h>
+#include <string.h>
 
 #include "../colore_gb300/csrc/cg_exact.h"
 
@@ -149,4 +151,50 @@ void or_ptrs_checked(long n, const float *lam, const float *elam, const double *
     got[i] = cg_poisson_ptrs_checked(lam[i], elam[i], cid[i], k0, k1);
     ref[i] = cgx_poisson_ptrs(lam64[i], cid[i], k0, k1);
   }
+}
+
+/* The counts' first tier (cg_lambda_seg, cg_count_seg) on n cells of a table
+ * of NA nodes at r_i = i / idr: lam[i] within elam[i] of lam64[i]
+ * (cgx_lambda), got[i] the tier's count or -1, ref[i] the double count for
+ * lambda < 10 with the uniform bits[i] 2^-24. */
+void or_count_seg(const double *r, const double *nz, const double *bz, const double *norm, double idr, double dx,
+                  const double *pos, double cell_vol, double rlim, int model, long n, const int *cell, const float *d,
+                  const uint32_t *bits, float *lam, float *elam, double *lam64, int *got, int *ref)
+{
+  cg_pois_args a;
+  memset(&a, 0, sizeof(a));
+  a.x.r = r;
+  a.x.nz = nz;
+  a.x.bz = bz;
+  a.x.norm = norm;
+  a.x.idr = idr;
+  a.x.r_last = r[CG_NA - 1];
+  a.x.bz0 = bz[0];
+  a.x.dx = dx;
+  a.x.cell_vol = cell_vol;
+  a.x.rlim = rlim;
+  for (int k = 0; k < 3; k++) a.x.p[k] = pos[k];
+  a.x.bias_model = model;
+  a.idr = (float)idr;
+  a.r_last = (float)a.x.r_last;
+  a.rlim = (float)rlim;
+  a.bias_model = model;
+  cg_pois_seg *seg = malloc((CG_NA - 1) * sizeof(cg_pois_seg));
+  for (int i = 0; i < CG_NA - 1; i++) seg[i] = cg_pois_seg_make(&a.x, CG_NA, i);
+  for (long i = 0; i < n; i++) {
+    const int *c = cell + 3 * i;
+    const float x = (float)cgx_coord(c[0], dx, pos[0]), y = (float)cgx_coord(c[1], dx, pos[1]);
+    const float z = (float)cgx_coord(c[2], dx, pos[2]);
+    const float r2 = CG_FMA(x, x, CG_FMA(z, z, CG_MUL(y, y)));
+    const float u = CG_MUL((float)bits[i], CG_E24);
+    float rr;
+    const float s = cg_seg_pos(r2, a.idr, &rr);
+    int j = (int)s, pos1;
+    j = r2 > 0.0f && j < CG_NA - 1 ? j : 0;
+    lam[i] = cg_lambda_seg(&seg[j], CG_SUB(s, (float)j), d[i], model, &elam[i], &pos1);
+    lam64[i] = cgx_lambda(&a.x, c[0], c[1], c[2], d[i]);
+    got[i] = cg_count_seg(seg, &a, r2, d[i], u);
+    ref[i] = lam64[i] < 10 ? cgx_poisson(lam64[i], (double)u, i, 1u, 2u) : -1;
+  }
+  free(seg);
 }

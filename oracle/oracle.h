@@ -110,4 +110,8 @@ void or_src_offset_checked(long n, const double *x0, double dx, const uint32_t *
 void or_ptrs_checked(long n, const float *lam, const float *elam, const double *lam64, const long long *cid, uint32_t k0,
                      uint32_t k1, int *got, int *ref);
 
+void or_count_seg(const double *r, const double *nz, const double *bz, const double *norm, double idr, double dx,
+                  const double *pos, double cell_vol, double rlim, int model, long n, const int *cell, const float *d,
+                  const uint32_t *bits, float *lam, float *elam, double *lam64, int *got, int *ref);
+
 #endif

@@ -56,10 +56,11 @@ def lib():
             "or_sht_legendre": [i, i, i, vp, vp, vp, d, vp],
             "or_src_offset_checked": [C.c_long, vp, d, vp, vp, vp, vp],
             "or_ptrs_checked": [C.c_long, vp, vp, vp, vp, C.c_uint32, C.c_uint32, vp, vp],
+            "or_count_seg": [vp, vp, vp, vp, d, d, vp, d, d, i, C.c_long, vp, vp, vp, vp, vp, vp, vp, vp],
         }
         void = ("or_philox", "or_poisson", "or_ang2pix", "or_nest2ring", "or_ring2nest", "or_pix2vec_nest",
                 "or_shell_index", "or_pix_checked", "or_pix_cgx", "or_pix64", "or_pix_ff", "or_ff_ops", "or_src_offset_checked",
-                "or_ptrs_checked")
+                "or_ptrs_checked", "or_count_seg")
         for k, a in sig.items():
             fn = getattr(L, k)
             fn.argtypes = a
@@ -564,3 +565,20 @@ def ptrs_checked(lam, elam, lam64, cid, k0, k1):
     ref = np.empty(n, np.int32)
     lib().or_ptrs_checked(n, P(lam), P(elam), P(lam64), P(cid), k0, k1, P(got), P(ref))
     return got, ref
+
+
+def count_seg(r, nz, bz, norm, idr, dx, pos, cell_vol, rlim, model, cell, d, bits):
+    """The counts' first tier on cells (n x 3): (lam, elam, lam64, got, ref),
+    lam within elam of the double lam64, got the count or -1 where open, ref
+    the double count (-1 for lambda >= 10)."""
+    f8 = [np.ascontiguousarray(a, np.float64) for a in (r, nz, bz, norm, pos)]
+    cell = np.ascontiguousarray(cell, np.int32)
+    d = np.ascontiguousarray(d, np.float32)
+    bits = np.ascontiguousarray(bits, np.uint32)
+    n = len(d)
+    lam, elam = np.empty(n, np.float32), np.empty(n, np.float32)
+    lam64 = np.empty(n, np.float64)
+    got, ref = np.empty(n, np.int32), np.empty(n, np.int32)
+    lib().or_count_seg(P(f8[0]), P(f8[1]), P(f8[2]), P(f8[3]), idr, dx, P(f8[4]), cell_vol, rlim, model, n, P(cell),
+                       P(d), P(bits), P(lam), P(elam), P(lam64), P(got), P(ref))
+    return lam, elam, lam64, got, ref

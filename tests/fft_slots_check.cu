@@ -1,5 +1,5 @@
 // Host check of the exchange slots of colore_gb300/csrc/fft.cuh: for every
-// column and row plan of fft_plans.h, pad_at splits each exchange access into
+// column and row plan of fft_plans.h, padded, pad_at splits each exchange access into
 // base and offset without changing the slot p + (p >> sh), the slots are
 // distinct and below pad_len, and stage 0's writes by 16 consecutive threads
 // of one column fall into 16 different float2 bank pairs.
@@ -18,7 +18,7 @@ static int check_plan()
   std::set<int> seen;
   for (int p = 0; p < L; p++) {
     seen.insert(slot(p));
-    bad += slot(p) >= cgfft::pad_len(L, r0);
+    bad += slot(p) >= cgfft::pad_len(L, SH);
   }
   bad += (int)seen.size() != L;
   for (int t = 0; t < P; t++) {
