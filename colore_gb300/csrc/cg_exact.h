@@ -233,6 +233,14 @@ CG_HD float cgx_src_offset(double x0, double dx, uint32_t bits)
   return (float)X_ADD(x0, X_MUL(dx, X_SUB((double)cg_u01f(bits), 0.5)));
 }
 
+/* The neighbour of finite f towards +infinity (up != 0) or -infinity. */
+CG_HD float cg_next_float(float f, int up)
+{
+  const uint32_t u = cg_f2u(f);
+  if (f == 0.0f) return cg_u2f(up ? 1u : 0x80000001u);
+  return cg_u2f((f > 0.0f) == (up != 0) ? u + 1u : u - 1u);
+}
+
 /* The same float coordinate from single-precision arithmetic: 1 with *out
  * when it is certainly the double expression rounded to float, 0 otherwise.
  * The corner x0 and dx come as float pairs (c + l, dh + dl; each pair
@@ -254,7 +262,7 @@ CG_HD int cg_src_offset_checked(float c, float l, float dh, float dl, uint32_t b
   const float lo = CG_ADD(CG_ADD(e, l), CG_ADD(pe, q));
   const float f = CG_ADD(s, lo);
   const float r = CG_ADD(CG_SUB(s, f), lo); /* s - f exact: f is within an ulp of s */
-  const float nb = nextafterf(f, r >= 0.0f ? 3.0e38f : -3.0e38f);
+  const float nb = cg_next_float(f, r >= 0.0f);
   const float h = CG_MUL(0.5f, cg_fabsf(CG_SUB(nb, f)));
   const float E = CG_FMA(cg_fabsf(r), 1.2e-7f, CG_MUL(5.7e-14f, CG_ADD(CG_ADD(cg_fabsf(c), cg_fabsf(s)), dh)));
   if (!(CG_SUB(h, cg_fabsf(r)) > E)) return 0;
@@ -525,7 +533,9 @@ typedef struct {
   int q;
 } cg_dir;
 
-CG_HD cg_dir cg_dir_of(float x, float y, float z, float ein)
+/* The direction given g, atan(min(|x|, |y|) / max(|x|, |y|)) in quarter turns
+ * (0 on the polar axis). */
+CG_HD cg_dir cg_dir_from(float x, float y, float z, float g, float ein)
 {
   cg_dir o;
   o.rho2 = CG_FMA(x, x, CG_MUL(y, y));
@@ -533,17 +543,13 @@ CG_HD cg_dir cg_dir_of(float x, float y, float z, float ein)
   o.r2 = r2;
   o.rinv = cg_rsqrt_fast(r2);
   o.cth = CG_MUL(z, o.rinv);
-  const float ax = cg_fabsf(x), ay = cg_fabsf(y);
-  const float mx = cg_max_nn(ax, ay), mn = cg_min_nn(ax, ay);
-  const float t = CG_MUL(mn, cg_rcp_fast(cg_max_nn(mx, 1e-30f))); /* atan2(0, 0) = 0 */
-  const float g = cg_atan01_q(t); /* atan(min/max) / (pi/2) */
   /* tt = phi / (pi/2) in [0, 4) is base + g' or base - g' with
    * g' = atan(ay/ax) / (pi/2) (g, or 1 - g when ay > ax) and, by quadrant,
    * (base, sign) = (0, +) x >= 0 y >= 0, (2, -) x < 0 y >= 0, (2, +) x < 0 y < 0,
    * (4, -) x >= 0 y < 0; q and f = tt - q follow without forming tt, so f
    * keeps absolute rounding */
   const int neg = (x < 0.0f) != (y < 0.0f);
-  const int swap = ay > ax;
+  const int swap = cg_fabsf(y) > cg_fabsf(x);
   int q = ((x < 0.0f) ? 2 : ((y < 0.0f) ? 4 : 0)) - neg;
   float f = (swap != neg) ? CG_SUB(1.0f, g) : g;
   if (f >= 1.0f) { /* g' = 0 on the negative side: tt is the next integer */
@@ -556,13 +562,39 @@ CG_HD cg_dir cg_dir_of(float x, float y, float z, float ein)
   /* cos(theta): r^2 (2 roundings), rsqrt (2^-22), product (2^-24); the
    * inputs' error ein (relative to r) moves cos(theta) by at most 2 ein */
   o.ecth = CG_FMA(cg_fabsf(o.cth), 8.0f * CG_E24, CG_MUL(2.0f, ein));
-  /* f: cg_atan01_q within 8.2e-8 of atan / (pi/2) on [0,1]; the ratio's
-   * relative error 2^-22 moves atan by at most that times t/(1+t^2) <= 1/2
-   * (6e-8 rad, 3.8e-8 in quarter turns); the rounding of 1 - g (3e-8):
-   * 1.5e-7 in all, taken as 2.5e-7.  The inputs' share, which depends on
-   * 1/sin(theta), is added by cg_pix_checked. */
+  /* f: g within 1.2e-7 (cg_dir_of: cg_atan01_q within 8.2e-8 of atan / (pi/2)
+   * on [0,1], and the ratio's relative error 2^-22, which moves atan by at
+   * most that times t/(1+t^2) <= 1/2, 3.8e-8 in quarter turns; cg_dir_phi:
+   * cg_atan01 within 1.3 ulp of at most pi/4, 5e-8, its ratio 1.9e-8, 2/pi
+   * and the product 4.5e-8) and the rounding of 1 - g (3e-8): 1.5e-7 in all,
+   * taken as 2.5e-7.  The inputs' share, which depends on 1/sin(theta), is
+   * added by cg_pix_checked. */
   o.ef = 2.5e-7f;
   return o;
+}
+
+CG_HD cg_dir cg_dir_of(float x, float y, float z, float ein)
+{
+  const float ax = cg_fabsf(x), ay = cg_fabsf(y);
+  const float mx = cg_max_nn(ax, ay), mn = cg_min_nn(ax, ay);
+  const float t = CG_MUL(mn, cg_rcp_fast(cg_max_nn(mx, 1e-30f))); /* atan2(0, 0) = 0 */
+  return cg_dir_from(x, y, z, cg_atan01_q(t), ein);
+}
+
+/* The direction and phi = atan2(y, x) in [0, 2 pi] of a source from one
+ * octant angle: phi is cg_cart2sph's, bit for bit (the steps of cg_atan2f). */
+CG_HD cg_dir cg_dir_phi(float x, float y, float z, float *phi)
+{
+  const float ax = cg_fabsf(x), ay = cg_fabsf(y);
+  const float mx = ax > ay ? ax : ay, mn = ax > ay ? ay : ax;
+  const float th = mx > 0.0f ? cg_atan01(CG_DIV(mn, mx)) : 0.0f;
+  float ph = th;
+  if (ay > ax) ph = CG_SUB(CG_HALFPI_F, ph);
+  if (x < 0.0f) ph = CG_SUB(CG_PI_F, ph);
+  if (y < 0.0f) ph = -ph;
+  if (ph < 0.0f) ph = CG_ADD(ph, CG_TWOPI_F);
+  *phi = ph;
+  return cg_dir_from(x, y, z, CG_MUL(th, 0.636619772f), 0.0f);
 }
 
 /* An integer-valued float x with |x| < 2^22 as int: x + 1.5 2^23 holds x in

@@ -378,15 +378,16 @@ __global__ void __launch_bounds__(1024) k_scan_apply(long long *v, long long n, 
   if (i + 1 < n) v[i + 1] = off + a;
 }
 
-/* Centred potential differences at a cell (get_rvel / get_element VEL). */
+/* Centred potential differences at a cell (get_rvel / get_element VEL): the
+ * cell's address once, its neighbours at periodic offsets. */
 __device__ __forceinline__ void grad_phi(const float *__restrict__ phi, int ix, int iy, int iz, int N, float v[3])
 {
-  int xh = wrap(ix + 1, N), xl = wrap(ix - 1, N);
-  int yh = wrap(iy + 1, N), yl = wrap(iy - 1, N);
-  int zh = wrap(iz + 1, N), zl = wrap(iz - 1, N);
-  v[0] = CG_SUB(__ldg(&phi[pidx(xh, iy, iz, N)]), __ldg(&phi[pidx(xl, iy, iz, N)]));
-  v[1] = CG_SUB(__ldg(&phi[pidx(ix, yh, iz, N)]), __ldg(&phi[pidx(ix, yl, iz, N)]));
-  v[2] = CG_SUB(__ldg(&phi[pidx(ix, iy, zh, N)]), __ldg(&phi[pidx(ix, iy, zl, N)]));
+  const int ngx = 2 * (N / 2 + 1), my = (N - 1) * ngx;
+  const long long plane = (long long)ngx * N, mz = plane * (N - 1);
+  const float *c = phi + pidx(ix, iy, iz, N);
+  v[0] = CG_SUB(__ldg(c + (ix == N - 1 ? 1 - N : 1)), __ldg(c + (ix == 0 ? N - 1 : -1)));
+  v[1] = CG_SUB(__ldg(c + (iy == N - 1 ? -my : ngx)), __ldg(c + (iy == 0 ? my : -ngx)));
+  v[2] = CG_SUB(__ldg(c + (iz == N - 1 ? -mz : plane)), __ldg(c + (iz == 0 ? mz : -plane)));
 }
 
 /* Base and count-map pixels of a source by the reference's double
@@ -409,19 +410,26 @@ __device__ __noinline__ unsigned int pixels_double(const cg_srcs_params &p, floa
   return k;
 }
 
-__global__ void __launch_bounds__(SB, 8) k_emit(const float *__restrict__ phi, cg_srcs_params p)
+constexpr int SRC_F = 9; /* floats per source record (Src) */
+
+/* Sources of the block's 2048 cells (blockIdx.x), the share blockIdx.y of
+ * gridDim.y: every share scans the counts again, a few per cent of the work,
+ * so that small grids and dense populations spread over the chip (c1 at
+ * 128^3: 1024 blocks of up to 20000 sources kept the SMs busy 59 % of the
+ * time).  The share's sources are spread evenly over the threads.  Records
+ * of 36 bytes are staged per warp and written as consecutive words: written
+ * field by field they cost L2 ten sectors per source for 56 bytes. */
+__global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, cg_srcs_params p)
 {
-  __shared__ int coff[CPB + 1]; /* exclusive source offset of each cell in the block */
+  __shared__ int coff[CPB]; /* exclusive source offset of each cell in the block */
   __shared__ int ws[SB / 32];
+  __shared__ float stage[SB / 32][32 * SRC_F];
   const int N = p.box.N;
-  const long long ncell = (long long)N * N * N;
   const long long cb = (long long)blockIdx.x * CPB;
   const long long c0 = cb + (long long)threadIdx.x * CPT;
   int n[CPT];
   int tot = 0;
-#pragma unroll
-  for (int h = 0; h < CPT; h++) n[h] = 0;
-  if (c0 < ncell) {
+  {
     const uint4 pk = *reinterpret_cast<const uint4 *>(p.counts + c0);
     const unsigned w4[4] = {pk.x, pk.y, pk.z, pk.w};
 #pragma unroll
@@ -442,88 +450,104 @@ __global__ void __launch_bounds__(SB, 8) k_emit(const float *__restrict__ phi, c
   }
   if (lane == 31) ws[wid] = inc;
   __syncthreads();
-  int woff = 0;
-  for (int w = 0; w < wid; w++) woff += ws[w];
+  int woff = 0, T = 0;
+#pragma unroll
+  for (int w = 0; w < SB / 32; w++) {
+    if (w < wid) woff += ws[w];
+    T += ws[w];
+  }
+  if (T == 0) return;
   int run = woff + inc - tot;
 #pragma unroll
   for (int h = 0; h < CPT; h++) {
     coff[threadIdx.x * CPT + h] = run;
     run += n[h];
   }
-  if (threadIdx.x == SB - 1) coff[CPB] = run;
   __syncthreads();
-  /* the block's sources, spread evenly over its threads: consecutive threads
-   * write consecutive catalogue entries */
-  const int T = coff[CPB];
   const long long base = p.block_sums[blockIdx.x];
   const float dx = p.box.dx;
+  /* the block's first cell; a cell lo < 2048 further on lies lo2 / N rows
+   * below, lo2 = ix0 + lo < 4096, by a product in 32 bits (mdiv / 2^24 is
+   * 1/N + e with e lo2 < 2^-12 < 1/N) */
+  int bx, by, bz;
+  cell_of(cb, p.box, bx, by, bz);
+  const unsigned mdiv = ((1u << 24) + (unsigned)N - 1u) / (unsigned)N;
   unsigned int nfb = 0; /* pixels decided in double */
-  for (int k = threadIdx.x; k < T; k += SB) {
-    /* the cell holding source k: the last cell whose offset is <= k (cells
-     * without sources share their successor's offset) */
-    int lo = 0, hi = CPB - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (coff[mid] <= k) lo = mid;
-      else hi = mid - 1;
-    }
-    const int j = k - coff[lo];
-    const long long cid = cb + lo;
+  const int k1 = (int)((long long)T * (blockIdx.y + 1) / gridDim.y);
+  for (int kb = (int)((long long)T * blockIdx.y / gridDim.y) + wid * 32; kb < k1; kb += SB) {
+    const int k = kb + lane;
     const long long id = base + k;
-    if (id >= p.capacity) {
-      atomicOr(p.err, ERR_CATALOG_OVERFLOW);
-      break;
+    const bool ok = k < k1 && id < p.capacity;
+    if (k < k1 && !ok) atomicOr(p.err, ERR_CATALOG_OVERFLOW);
+    float *q = &stage[wid][lane * SRC_F];
+    if (ok) {
+      /* the cell holding source k: the last cell whose offset is <= k (cells
+       * without sources share their successor's offset) */
+      int lo = 0;
+#pragma unroll
+      for (int st = CPB / 2; st > 0; st >>= 1)
+        if (coff[lo + st] <= k) lo += st;
+      const int j = k - coff[lo];
+      const long long cid = cb + lo;
+      const unsigned lo2 = (unsigned)(bx + lo), dr = (lo2 * mdiv) >> 24;
+      const int ix = (int)(lo2 - dr * (unsigned)N);
+      int iy = by + (int)dr, iz = bz;
+      if (iy >= N) {
+        iy -= N;
+        iz++;
+      }
+      const float x0 = cg_cell_coord(ix, dx, p.box.p0);
+      const float y0 = cg_cell_coord(iy, dx, p.box.p1), z0 = cg_cell_coord(iz, dx, p.box.p2);
+      const float rr = cg_norm3(x0, y0, z0);
+      float v[3];
+      grad_phi(phi, ix, iy, iz, N, v);
+      const float rvel = CG_MUL(p.factor_vel, cg_rvel(v[0], v[1], v[2], x0, y0, z0, rr, p.box.idx));
+      const float dz_rsd = CG_MUL(rvel, bg(p.v1, p.g, rr));
+      cg_u32x4 u = cg_philox4x32_10((uint32_t)cid, (uint32_t)(cid >> 32), (uint32_t)j, 0u, p.kq0, p.kq1);
+      /* the position of the double arithmetic, stored as float (srcs.c:261-263):
+       * in single precision where its rounding is certain, else in double */
+      float px, py, pz;
+      if (p.force_double || !cg_src_offset_checked(p.pa.xc[ix], p.cl[0][ix], p.dxh, p.dxl, u.v[0], &px))
+        px = cgx_src_offset(cgx_coord(ix, p.dx64, p.p64[0]), p.dx64, u.v[0]);
+      if (p.force_double || !cg_src_offset_checked(p.pa.yc[iy], p.cl[1][iy], p.dxh, p.dxl, u.v[1], &py))
+        py = cgx_src_offset(cgx_coord(iy, p.dx64, p.p64[1]), p.dx64, u.v[1]);
+      if (p.force_double || !cg_src_offset_checked(p.pa.zc[iz], p.cl[2][iz], p.dxh, p.dxl, u.v[2], &pz))
+        pz = cgx_src_offset(cgx_coord(iz, p.dx64, p.p64[2]), p.dx64, u.v[2]);
+      p.pos[id] = make_float4(px, py, pz, dz_rsd);
+      /* the base pixel and the count-map pixel: the reference's double
+       * decisions, in single precision where the margins allow */
+      float ph;
+      const cg_dir dr3 = cg_dir_phi(px, py, pz, &ph);
+      long long pr = -1, pc = -1;
+      if (!p.force_double) {
+        pr = cg_pix_checked(&dr3, (int)p.nside_base, 0.0f);
+        if (p.cmap) pc = cg_pix_checked(&dr3, (int)p.nside_count, 0.0f);
+      }
+      if (pr < 0 || (p.cmap && pc < 0)) nfb += pixels_double(p, px, py, pz, &pr, &pc);
+      /* ring2nest costs several 64-bit divisions; nside_base is small, so its
+       * table (built on the host with the same function) replaces them */
+      p.ipix[id] = p.base_r2n ? __ldg(p.base_r2n + pr) : (int)cg_ring2nest(p.nside_base, pr);
+      if (p.cmap) atomicAdd(&p.cmap[pc], 1);
+      cg_radec(px, py, pz, ph, &q[0], &q[1]);              /* ra, dec */
+      q[2] = bg(p.zt, p.g, cg_norm3(px, py, pz));          /* z0  */
+      q[3] = p.need_beaming ? 0.0f : dz_rsd;               /* dz_rsd */
+      q[4] = p.need_beaming ? 0.0f : -1.0f;                /* e1  */
+      q[5] = p.need_beaming ? 0.0f : -1.0f;                /* e2  */
+      q[6] = 0.0f;
+      q[7] = 0.0f;
+      q[8] = 0.0f;
     }
-    int ix, iy, iz;
-    cell_of(cid, p.box, ix, iy, iz);
-    const float x0 = cg_cell_coord(ix, dx, p.box.p0);
-    const float y0 = cg_cell_coord(iy, dx, p.box.p1), z0 = cg_cell_coord(iz, dx, p.box.p2);
-    const float rr = cg_norm3(x0, y0, z0);
-    float v[3];
-    grad_phi(phi, ix, iy, iz, N, v);
-    const float rvel = CG_MUL(p.factor_vel, cg_rvel(v[0], v[1], v[2], x0, y0, z0, rr, p.box.idx));
-    const float dz_rsd = CG_MUL(rvel, bg(p.v1, p.g, rr));
-    cg_u32x4 u = cg_philox4x32_10((uint32_t)cid, (uint32_t)(cid >> 32), (uint32_t)j, 0u, p.kq0, p.kq1);
-    /* the position of the double arithmetic, stored as float (srcs.c:261-263):
-     * in single precision where its rounding is certain, else in double */
-    float px, py, pz;
-    if (p.force_double || !cg_src_offset_checked(p.pa.xc[ix], p.cl[0][ix], p.dxh, p.dxl, u.v[0], &px))
-      px = cgx_src_offset(cgx_coord(ix, p.dx64, p.p64[0]), p.dx64, u.v[0]);
-    if (p.force_double || !cg_src_offset_checked(p.pa.yc[iy], p.cl[1][iy], p.dxh, p.dxl, u.v[1], &py))
-      py = cgx_src_offset(cgx_coord(iy, p.dx64, p.p64[1]), p.dx64, u.v[1]);
-    if (p.force_double || !cg_src_offset_checked(p.pa.zc[iz], p.cl[2][iz], p.dxh, p.dxl, u.v[2], &pz))
-      pz = cgx_src_offset(cgx_coord(iz, p.dx64, p.p64[2]), p.dx64, u.v[2]);
-    p.pos[id] = make_float4(px, py, pz, dz_rsd);
-    float r, cth, ph;
-    cg_cart2sph(px, py, pz, &r, &cth, &ph);
-    /* the base pixel and the count-map pixel: the reference's double
-     * decisions, in single precision where the margins allow */
-    long long pr = -1, pc = -1;
-    if (!p.force_double) {
-      const cg_dir dr = cg_dir_of(px, py, pz, 0.0f);
-      pr = cg_pix_checked(&dr, (int)p.nside_base, 0.0f);
-      if (p.cmap) pc = cg_pix_checked(&dr, (int)p.nside_count, 0.0f);
-    }
-    if (pr < 0 || (p.cmap && pc < 0)) {
-      nfb += pixels_double(p, px, py, pz, &pr, &pc);
-    }
-    /* ring2nest costs several 64-bit divisions; nside_base is small, so its
-     * table (built on the host with the same function) replaces them */
-    p.ipix[id] = p.base_r2n ? __ldg(p.base_r2n + pr) : (int)cg_ring2nest(p.nside_base, pr);
-    float *q = p.src + (size_t)id * 9;
-    cg_radec(px, py, pz, ph, &q[0], &q[1]);                       /* ra, dec */
-    q[2] = bg(p.zt, p.g, r);                                      /* z0  */
-    q[3] = p.need_beaming ? 0.0f : dz_rsd;                        /* dz_rsd */
-    q[4] = p.need_beaming ? 0.0f : -1.0f;                         /* e1  */
-    q[5] = p.need_beaming ? 0.0f : -1.0f;                         /* e2  */
-    q[6] = 0.0f;
-    q[7] = 0.0f;
-    q[8] = 0.0f;
-    if (p.cmap) atomicAdd(&p.cmap[pc], 1);
+    __syncwarp();
+    const int nw = __popc(__ballot_sync(0xffffffffu, ok)) * SRC_F;
+    float *dst = p.src + (size_t)(base + kb) * SRC_F;
+#pragma unroll
+    for (int h = 0; h < SRC_F; h++)
+      if (h * 32 + lane < nw) dst[h * 32 + lane] = stage[wid][h * 32 + lane];
+    __syncwarp();
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) nfb += __shfl_xor_sync(0xffffffffu, nfb, o);
-  if ((threadIdx.x & 31) == 0 && nfb) atomicAdd(p.xstats + 1, (unsigned long long)nfb);
+  if (lane == 0 && nfb) atomicAdd(p.xstats + 1, (unsigned long long)nfb);
 }
 
 /* Trilinear potential gradient at a point with corner cells i0/i1 and
@@ -746,8 +770,15 @@ cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_param
 
 cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p)
 {
-  long long nb = cg_srcs_nblocks(p->box.N);
-  k_emit<<<(unsigned)nb, SB, 0, s>>>(phi, *p);
+  const long long nb = cg_srcs_nblocks(p->box.N);
+  /* shares per block: until there are eight blocks for each of the 152 x 8
+   * that an SM generation holds, while a share keeps a source per thread (the
+   * capacity is the total with an eighth of slack).  c1 at 128^3 with 1 and
+   * 16 shares: 244 and 169 us; 192^3 with 240 sources per block: 74 and 127 us
+   * with 1 and 4. */
+  int sh = 1;
+  while (sh < 16 && nb * sh < 9728 && p->capacity >= nb * sh * 2 * SB) sh *= 2;
+  k_emit<<<dim3((unsigned)nb, (unsigned)sh), SB, 0, s>>>(phi, *p);
   return cudaGetLastError();
 }
 

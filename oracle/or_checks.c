@@ -198,3 +198,22 @@ void or_count_seg(const double *r, const double *nz, const double *bz, const dou
   }
   free(seg);
 }
+
+/* A source's direction from one octant angle (cg_dir_phi): ph its phi and
+ * ref that of cg_cart2sph; pix the RING pixel at nside (-1 where its margin
+ * fails).  Positions are the float xyz. */
+void or_dir_phi(long nside, const float *xyz, long n, float *ph, float *ref, long long *pix)
+{
+  for (long i = 0; i < n; i++) {
+    float r, cth;
+    const cg_dir d = cg_dir_phi(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], &ph[i]);
+    cg_cart2sph(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], &r, &cth, &ref[i]);
+    pix[i] = cg_pix_checked(&d, (int)nside, 0.0f);
+  }
+}
+
+/* cg_next_float of f[i] upwards (up[i] != 0) or downwards. */
+void or_next_float(long n, const float *f, const int *up, float *out)
+{
+  for (long i = 0; i < n; i++) out[i] = cg_next_float(f[i], up[i]);
+}

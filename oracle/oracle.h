@@ -114,4 +114,7 @@ void or_count_seg(const double *r, const double *nz, const double *bz, const dou
                   const double *pos, double cell_vol, double rlim, int model, long n, const int *cell, const float *d,
                   const uint32_t *bits, float *lam, float *elam, double *lam64, int *got, int *ref);
 
+void or_dir_phi(long nside, const float *xyz, long n, float *ph, float *ref, long long *pix);
+void or_next_float(long n, const float *f, const int *up, float *out);
+
 #endif

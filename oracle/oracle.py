@@ -56,11 +56,12 @@ def lib():
             "or_sht_legendre": [i, i, i, vp, vp, vp, d, vp],
             "or_src_offset_checked": [C.c_long, vp, d, vp, vp, vp, vp],
             "or_ptrs_checked": [C.c_long, vp, vp, vp, vp, C.c_uint32, C.c_uint32, vp, vp],
+            "or_dir_phi": [C.c_long, vp, C.c_long, vp, vp, vp], "or_next_float": [C.c_long, vp, vp, vp],
             "or_count_seg": [vp, vp, vp, vp, d, d, vp, d, d, i, C.c_long, vp, vp, vp, vp, vp, vp, vp, vp],
         }
         void = ("or_philox", "or_poisson", "or_ang2pix", "or_nest2ring", "or_ring2nest", "or_pix2vec_nest",
                 "or_shell_index", "or_pix_checked", "or_pix_cgx", "or_pix64", "or_pix_ff", "or_ff_ops", "or_src_offset_checked",
-                "or_ptrs_checked", "or_count_seg")
+                "or_ptrs_checked", "or_count_seg", "or_dir_phi", "or_next_float")
         for k, a in sig.items():
             fn = getattr(L, k)
             fn.argtypes = a
@@ -582,3 +583,22 @@ def count_seg(r, nz, bz, norm, idr, dx, pos, cell_vol, rlim, model, cell, d, bit
     lib().or_count_seg(P(f8[0]), P(f8[1]), P(f8[2]), P(f8[3]), idr, dx, P(f8[4]), cell_vol, rlim, model, n, P(cell),
                        P(d), P(bits), P(lam), P(elam), P(lam64), P(got), P(ref))
     return lam, elam, lam64, got, ref
+
+
+def dir_phi(nside, xyz):
+    """(phi, cart2sph's phi, RING pixel or -1) of float positions (n x 3) by
+    the one-octant-angle direction of the sources."""
+    a = np.ascontiguousarray(xyz, np.float32)
+    n = len(a)
+    ph, ref = np.empty(n, np.float32), np.empty(n, np.float32)
+    pix = np.empty(n, np.int64)
+    lib().or_dir_phi(nside, P(a), n, P(ph), P(ref), P(pix))
+    return ph, ref, pix
+
+
+def next_float(f, up):
+    f = np.ascontiguousarray(f, np.float32)
+    up = np.ascontiguousarray(up, np.int32)
+    out = np.empty_like(f)
+    lib().or_next_float(len(f), P(f), P(up), P(out))
+    return out
