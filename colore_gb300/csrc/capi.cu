@@ -180,6 +180,9 @@ struct cg_ctx {
   cudaGraphExec_t gexec = nullptr;
   cudaEvent_t graph_done = nullptr;
   long long graph_launches = 0; /* kernels per replay */
+  /* page-locked, written by the count's scan: the total, the error word and
+   * the source offsets of EMIT_PARTS equal ranges of cells */
+  long long *h_scan = nullptr;
   /* cg_set_host_*: page-locked host destinations that the stages fill as
    * each output becomes final, with copy-engine transfers on a copy stream
    * that overlap the stages still to run (no SM is taken from them); one
@@ -221,6 +224,9 @@ static int fail(cg_ctx *c, int code, const char *fmt, ...)
 
 static void graph_free(cg_ctx *c);
 static void out_wait_all(cg_ctx *c);
+static int beam_part(cg_ctx *c, int ip, bool async, long long i0, long long n);
+static int out_catalog_part(cg_ctx *c, int ip, long long i0, long long n);
+constexpr int EMIT_PARTS = 16; /* ranges of cells the emission may be cut into */
 
 /* (Re)allocate a device buffer.  A captured graph holds the old addresses,
  * so any reallocation drops the graph: replaying it would touch freed
@@ -244,11 +250,9 @@ static int dalloc(cg_ctx *c, T **p, size_t n)
   return CG_OK;
 }
 
-static int check_device_errors(cg_ctx *c)
+/* The error word h as read from the device. */
+static int error_word(cg_ctx *c, unsigned int h)
 {
-  unsigned int h = 0;
-  CUDA_TRY(c, cudaMemcpyAsync(&h, c->d_err, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   if (h) {
     CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(unsigned int), c->stream));
     return fail(c, CG_EDEVICE, "device error flags 0x%x (1: source count overflow, 2: catalog overflow, "
@@ -257,6 +261,14 @@ static int check_device_errors(cg_ctx *c)
                 h);
   }
   return CG_OK;
+}
+
+static int check_device_errors(cg_ctx *c)
+{
+  unsigned int h = 0;
+  CUDA_TRY(c, cudaMemcpyAsync(&h, c->d_err, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  return error_word(c, h);
 }
 
 /* Event pair around a launch group when profiling is on. */
@@ -939,6 +951,7 @@ extern "C" void cg_destroy(cg_ctx *c)
     for (void *p : q)
       if (p) cudaFree(p);
   }
+  if (c->h_scan) cudaFreeHost(c->h_scan);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
 }
@@ -985,6 +998,7 @@ extern "C" int cg_create(cg_ctx **out, const cg_config *cfg, int device)
       (rc = dalloc(c, &c->d_s2f, (size_t)1)) || (rc = dalloc(c, &c->d_err, (size_t)1)))
     return rc;
   CUDA_TRY(c, cudaMemset(c->d_err, 0, sizeof(unsigned int)));
+  CUDA_TRY(c, cudaHostAlloc((void **)&c->h_scan, (2 + EMIT_PARTS) * sizeof(long long), cudaHostAllocDefault));
   if ((rc = cg_upload_tables(c, cfg))) return rc;
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return CG_OK;
@@ -1445,23 +1459,37 @@ static void srcs_params(cg_ctx *c, int ipop, cg_srcs_params &p)
   p.xstats = c->d_xstats;
 }
 
+static int emit_part(cg_ctx *c, int ip, long long b0, long long b1)
+{
+  cg_srcs_params p;
+  srcs_params(c, ip, p);
+  ProfScope ps(c, "srcs_emit");
+  CUDA_TRY(c, cg_srcs_emit(c->stream, c->d_npot, &p, b0, b1));
+  c->launches++;
+  return CG_OK;
+}
+
 /* srcs_set_cartesian for every population: count -> scan -> emit.  With
  * readback the total is read after the count to size the catalogue (the
  * public entry point); without it the catalogue keeps its capacity, emit
  * drops what does not fit and flags the overflow, and the totals stay on
- * the device until read (the graph-captured sequence). */
-static int srcs_run(cg_ctx *c, long long *nsrc, bool readback)
+ * the device until read (the graph-captured sequence).  With deliver (the
+ * whole sequence) the per-source beam quantities follow and the catalogue
+ * goes to its registered host buffer, part by part: the link is busy from
+ * the first part's end, while the rest and the other populations are made
+ * (c5 at 512^3: 3.9 GB of records, 20 ms of link time that began after 14 ms
+ * of counting, emission and RSD). */
+static int srcs_run(cg_ctx *c, long long *nsrc, bool readback, bool deliver)
 {
   if (!c->have_density) return fail(c, CG_ESTATE, "density not computed");
   if (!c->have_norm) return fail(c, CG_ESTATE, "compute_density_normalization first");
   cudaSetDevice(c->device);
-  const long long ncell = (long long)c->N * c->N * c->N;
+  const long long ncell = (long long)c->N * c->N * c->N, nb = cg_srcs_nblocks(c->N);
+  const long long bpc = (nb + EMIT_PARTS - 1) / EMIT_PARTS; /* blocks of cells per part */
   int rc;
   if (c->cfg.n_srcs > 0) {
     if (!c->d_counts && (rc = dalloc(c, &c->d_counts, (size_t)ncell))) return rc;
-    if (!c->d_bsums && (rc = dalloc(c, &c->d_bsums, (size_t)(cg_srcs_nblocks(c->N) +
-                                                             cg_srcs_scan_room(cg_srcs_nblocks(c->N))))))
-      return rc;
+    if (!c->d_bsums && (rc = dalloc(c, &c->d_bsums, (size_t)(nb + cg_srcs_scan_room(nb))))) return rc;
     if (!c->d_seg && (rc = dalloc(c, &c->d_seg, (size_t)CG_NA))) return rc;
     if (!c->d_total && (rc = dalloc(c, &c->d_total, (size_t)CG_NPOP_MAX))) return rc;
     if (!c->d_ovf_n && ((rc = dalloc(c, &c->d_ovf_cell, (size_t)CG_OVF_CAP)) ||
@@ -1474,13 +1502,16 @@ static int srcs_run(cg_ctx *c, long long *nsrc, bool readback)
     srcs_params(c, ip, p);
     {
       ProfScope ps(c, "srcs_count");
-      CUDA_TRY(c, cg_srcs_count(c->stream, c->d_dens, &p, c->d_total + ip));
+      CUDA_TRY(c, cg_srcs_count(c->stream, c->d_dens, &p, c->d_total + ip, readback ? c->h_scan : nullptr, bpc));
     }
+    c->launches += nb > 8192 ? 5 : 3; /* count tables, count, scan */
+    long long off[EMIT_PARTS + 1]; /* the parts' first sources */
     if (readback) {
-      long long tot = 0;
-      CUDA_TRY(c, cudaMemcpyAsync(&tot, c->d_total + ip, sizeof(tot), cudaMemcpyDeviceToHost, c->stream));
       CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-      if ((rc = check_device_errors(c))) return rc;
+      const long long tot = c->h_scan[0];
+      if ((rc = error_word(c, (unsigned int)c->h_scan[1]))) return rc;
+      for (int k = 0; k < EMIT_PARTS; k++) off[k] = k * bpc < nb ? c->h_scan[2 + k] : tot;
+      off[EMIT_PARTS] = tot;
       if (tot > K.cap) {
         long long cap = tot + tot / 8 + 1024;
         if ((rc = dalloc(c, &K.pos, (size_t)cap)) || (rc = dalloc(c, &K.ipix, (size_t)cap)) ||
@@ -1502,12 +1533,20 @@ static int srcs_run(cg_ctx *c, long long *nsrc, bool readback)
       }
       CUDA_TRY(c, cudaMemsetAsync(K.cmap, 0, np * sizeof(int), c->stream));
     }
-    srcs_params(c, ip, p);
-    {
-      ProfScope ps(c, "srcs_emit");
-      CUDA_TRY(c, cg_srcs_emit(c->stream, c->d_npot, &p));
+    if (!deliver) {
+      if ((rc = emit_part(c, ip, 0, nb))) return rc;
+      continue;
     }
-    c->launches += 6; /* count tables, count, three scan passes, emission */
+    /* a part per 32 MB of records at least; one when timing launch groups */
+    const bool parts = c->h_src[ip] && !c->profiling;
+    if (c->h_src[ip]) *c->h_n[ip] = K.n;
+    for (int k0 = 0, k1; k0 < EMIT_PARTS; k0 = k1) {
+      for (k1 = k0 + 1; k1 < EMIT_PARTS && (!parts || (off[k1] - off[k0]) * 36 < (32 << 20)); k1++) {}
+      if ((rc = emit_part(c, ip, std::min(k0 * bpc, nb), std::min(k1 * bpc, nb)))) return rc;
+      const long long i0 = off[k0], n = off[k1] - off[k0];
+      if (c->cfg.need_beaming && (rc = beam_part(c, ip, false, i0, n))) return rc;
+      if ((rc = out_catalog_part(c, ip, i0, n))) return rc;
+    }
   }
   c->have_srcs = 1;
   return CG_OK;
@@ -1517,7 +1556,7 @@ extern "C" int cg_srcs_set_cartesian(cg_ctx *c, long long *nsrc)
 {
   if (!c) return CG_EINVAL;
   out_join(c, 0); /* the catalogues are rewritten */
-  return srcs_run(c, nsrc, true);
+  return srcs_run(c, nsrc, true, false);
 }
 
 /* Source totals left on the device by a graph launch: wait for it, read
@@ -2034,9 +2073,10 @@ static int los_tables(cg_ctx *c)
   return CG_OK;
 }
 
-/* async: inside a captured sequence, the source total read on the device
- * (the catalogue's capacity bounds the launch). */
-static int srcs_los_run(cg_ctx *c, int ip, bool async)
+/* Sources i0 .. i0 + n - 1 of population ip.  async: inside a captured
+ * sequence, all of them, the source total read on the device (n, the
+ * catalogue's capacity, bounds the launch). */
+static int srcs_los_run(cg_ctx *c, int ip, bool async, long long i0, long long n)
 {
   Cat &K = c->cat[ip];
   const bool lens = c->cfg.lensing_srcs[ip] != 0, skw = c->cfg.skw_srcs[ip] != 0;
@@ -2049,9 +2089,9 @@ static int srcs_los_run(cg_ctx *c, int ip, bool async)
   q.box = c->box;
   q.g = c->g;
   q.d1 = c->d1;
-  q.pos = K.pos;
-  q.src = K.src;
-  q.nsrc = async ? K.cap : K.n;
+  q.pos = K.pos + i0;
+  q.src = K.src + 9 * i0;
+  q.nsrc = n;
   q.nsrc_dev = async ? c->d_total + ip : nullptr;
   q.nr = nr;
   q.dr = (float)(c->cfg.r_max / nr);
@@ -2076,8 +2116,8 @@ static int srcs_los_run(cg_ctx *c, int ip, bool async)
       }
       K.skw_cap = cap;
     }
-    q.skw_d = K.skw_d;
-    q.skw_v = K.skw_v;
+    q.skw_d = K.skw_d + (size_t)i0 * nr;
+    q.skw_v = K.skw_v + (size_t)i0 * nr;
     if (q.nsrc > 0) {
       ProfScope ps(c, "srcs_skewers");
       CUDA_TRY(c, cg_srcs_skewers(c->stream, c->d_dens, c->d_npot, &q, c->nsm));
@@ -2088,32 +2128,49 @@ static int srcs_los_run(cg_ctx *c, int ip, bool async)
   return CG_OK;
 }
 
+/* Records i0 .. i0 + n - 1 of population ip, final, to its registered host
+ * buffer, if it has one. */
+static int out_catalog_part(cg_ctx *c, int ip, long long i0, long long n)
+{
+  if (!c->h_src[ip]) return CG_OK;
+  n = std::min(n, c->h_cap[ip] - i0);
+  if (n <= 0) return CG_OK;
+  if (int rc = out_begin(c)) return rc;
+  CUDA_TRY(c, cudaMemcpyAsync(c->h_src[ip] + 9 * i0, c->cat[ip].src + 9 * i0, (size_t)n * 9 * sizeof(float),
+                              cudaMemcpyDeviceToHost, c->ostream));
+  return out_end(c, 0);
+}
+
 /* Final catalogues to registered host buffers (the counts are current:
  * cg_get_beam_properties reads them first). */
 static int out_catalogs(cg_ctx *c)
 {
   for (int ip = 0; ip < c->cfg.n_srcs; ip++) {
     if (!c->h_src[ip]) continue;
-    const Cat &K = c->cat[ip];
-    const long long k = std::min(K.n, c->h_cap[ip]);
-    *c->h_n[ip] = K.n;
-    if (k <= 0) continue;
-    if (int rc = out_begin(c)) return rc;
-    CUDA_TRY(c, cudaMemcpyAsync(c->h_src[ip], K.src, (size_t)k * 9 * sizeof(float), cudaMemcpyDeviceToHost,
-                                c->ostream));
-    if (int rc = out_end(c, 0)) return rc;
+    *c->h_n[ip] = c->cat[ip].n;
+    if (int rc = out_catalog_part(c, ip, 0, c->cat[ip].n)) return rc;
   }
   return CG_OK;
 }
 
-/* The beam stage (beaming.c:293-374).  async: inside a captured sequence --
- * source totals stay on the device, no host outputs. */
+/* RSD, lensing and skewers of sources i0 .. i0 + n - 1 of population ip
+ * (async: of all, at most n, the total read on the device). */
+static int beam_part(cg_ctx *c, int ip, bool async, long long i0, long long n)
+{
+  cg_srcs_params p;
+  srcs_params(c, ip, p);
+  p.pos += i0;
+  p.src += 9 * i0;
+  ProfScope ps(c, "srcs_beam_rsd");
+  CUDA_TRY(c, cg_srcs_beam_rsd(c->stream, c->d_npot, &p, n, async ? c->d_total + ip : nullptr, c->nsm));
+  if (n > 0) c->launches++;
+  return srcs_los_run(c, ip, async, i0, n);
+}
+
 /* The per-source half of the beam stage (beaming.c:293-374): RSD, lensing
  * and skewers at the sources, then (plain runs) the catalogues to the host.
- * The reference computes the beam quantities last; the passes are
- * independent of the maps, so the mock sequence runs them before the
- * intensity and convergence maps and the catalogues cross the host link
- * while the maps are computed. */
+ * async: inside a captured sequence -- source totals stay on the device, no
+ * host outputs. */
 static int beam_srcs(cg_ctx *c, bool async)
 {
   if (!async) {
@@ -2130,15 +2187,8 @@ static int beam_srcs(cg_ctx *c, bool async)
   }
   if (c->cfg.n_srcs > 0) {
     if (!c->have_srcs) return fail(c, CG_ESTATE, "srcs_set_cartesian first");
-    for (int ip = 0; ip < c->cfg.n_srcs; ip++) {
-      cg_srcs_params p;
-      srcs_params(c, ip, p);
-      const long long n = async ? c->cat[ip].cap : c->cat[ip].n;
-      ProfScope ps(c, "srcs_beam_rsd");
-      CUDA_TRY(c, cg_srcs_beam_rsd(c->stream, c->d_npot, &p, n, async ? c->d_total + ip : nullptr, c->nsm));
-      if (n > 0) c->launches++;
-      if (int rc = srcs_los_run(c, ip, async)) return rc;
-    }
+    for (int ip = 0; ip < c->cfg.n_srcs; ip++)
+      if (int rc = beam_part(c, ip, async, 0, async ? c->cat[ip].cap : c->cat[ip].n)) return rc;
     if (!async)
       if (int rc = out_catalogs(c)) return rc;
   }
@@ -2228,9 +2278,12 @@ extern "C" int cg_run_mock(cg_ctx *c)
   if ((rc = cg_create_cartesian_fields(c))) return rc;
   if ((rc = cg_compute_physical_density_field(c))) return rc;
   if ((rc = cg_compute_density_normalization(c))) return rc;
-  if ((rc = cg_srcs_set_cartesian(c, nullptr))) return rc;
-  /* the sources' beam quantities before the maps (beam_srcs) */
-  if ((rc = beam_srcs(c, false))) return rc;
+  /* the sources, their beam quantities and the catalogues' way to the host
+   * before the maps, on which they do not depend: the reference computes the
+   * beam quantities last */
+  out_join(c, 0);
+  out_join(c, 2);
+  if ((rc = srcs_run(c, nullptr, true, true))) return rc;
   if ((rc = cg_imap_set_cartesian(c))) return rc;
   return beam_maps(c, false);
 }
@@ -2249,7 +2302,7 @@ static int run_mock_async(cg_ctx *c)
   if ((rc = cg_create_cartesian_fields(c))) return rc;
   if ((rc = cg_compute_physical_density_field(c))) return rc;
   if ((rc = cg_compute_density_normalization(c))) return rc;
-  if ((rc = srcs_run(c, nullptr, false))) return rc;
+  if ((rc = srcs_run(c, nullptr, false, false))) return rc;
   if ((rc = beam_srcs(c, true))) return rc;
   if (c->cfg.n_imap > 0 && (rc = imap_run(c, false))) return rc;
   return beam_maps(c, true);

@@ -367,15 +367,70 @@ __global__ void __launch_bounds__(1024) k_scan_top(long long *tsum, long long nt
   if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_apply(long long *v, long long n, const long long *__restrict__ tsum)
+/* Block i's offset to the host when it is one of every bpc-th. */
+__device__ __forceinline__ void tell_offset(long long *host, long long bpc, long long i, long long off)
+{
+  if (host && i % bpc == 0) host[2 + i / bpc] = off;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_apply(long long *v, long long n, const long long *__restrict__ tsum,
+                                                     const long long *__restrict__ total, const unsigned int *err,
+                                                     long long *host, long long bpc)
 {
   __shared__ long long ws[33];
   const long long i = (long long)blockIdx.x * SCAN_T + 2 * (long long)threadIdx.x;
   const long long a = i < n ? v[i] : 0, b = i + 1 < n ? v[i + 1] : 0;
   long long tot;
   const long long off = tsum[blockIdx.x] + block_scan(a + b, ws, &tot);
-  if (i < n) v[i] = off;
-  if (i + 1 < n) v[i + 1] = off + a;
+  if (i < n) {
+    v[i] = off;
+    tell_offset(host, bpc, i, off);
+  }
+  if (i + 1 < n) {
+    v[i + 1] = off + a;
+    tell_offset(host, bpc, i + 1, off + a);
+  }
+  if (host && blockIdx.x == 0 && threadIdx.x == 0) {
+    host[0] = *total;
+    host[1] = (long long)*err;
+  }
+}
+
+/* The whole scan in one block, for up to SCAN_ONE totals: three launches and
+ * their gaps cost more than its few tiles (128^3: 4 us against 12). */
+constexpr long long SCAN_ONE = 4 * SCAN_T;
+
+__global__ void __launch_bounds__(1024) k_scan_one(long long *v, long long n, long long *total, unsigned int *err,
+                                                   long long *host, long long bpc)
+{
+  __shared__ long long ws[33];
+  long long carry = 0;
+  bool big = false;
+  for (long long t0 = 0; t0 < n; t0 += SCAN_T) {
+    const long long i = t0 + 2 * (long long)threadIdx.x;
+    const long long a = i < n ? v[i] : 0, b = i + 1 < n ? v[i + 1] : 0;
+    big |= a > 0x7fffffffLL || b > 0x7fffffffLL; /* k_emit scans a block in int */
+    long long tot;
+    const long long off = carry + block_scan(a + b, ws, &tot);
+    if (i < n) {
+      v[i] = off;
+      tell_offset(host, bpc, i, off);
+    }
+    if (i + 1 < n) {
+      v[i + 1] = off + a;
+      tell_offset(host, bpc, i + 1, off + a);
+    }
+    carry += tot;
+  }
+  if (big) atomicOr(err, ERR_COUNT_OVERFLOW);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *total = carry;
+    if (host) {
+      host[0] = carry;
+      host[1] = (long long)atomicOr(err, 0u);
+    }
+  }
 }
 
 /* Centred potential differences at a cell (get_rvel / get_element VEL): the
@@ -412,20 +467,20 @@ __device__ __noinline__ unsigned int pixels_double(const cg_srcs_params &p, floa
 
 constexpr int SRC_F = 9; /* floats per source record (Src) */
 
-/* Sources of the block's 2048 cells (blockIdx.x), the share blockIdx.y of
+/* Sources of 2048 cells (block b0 + blockIdx.x of them), the share blockIdx.y of
  * gridDim.y: every share scans the counts again, a few per cent of the work,
  * so that small grids and dense populations spread over the chip (c1 at
  * 128^3: 1024 blocks of up to 20000 sources kept the SMs busy 59 % of the
  * time).  The share's sources are spread evenly over the threads.  Records
  * of 36 bytes are staged per warp and written as consecutive words: written
  * field by field they cost L2 ten sectors per source for 56 bytes. */
-__global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, cg_srcs_params p)
+__global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, cg_srcs_params p, long long b0)
 {
   __shared__ int coff[CPB]; /* exclusive source offset of each cell in the block */
   __shared__ int ws[SB / 32];
   __shared__ float stage[SB / 32][32 * SRC_F];
   const int N = p.box.N;
-  const long long cb = (long long)blockIdx.x * CPB;
+  const long long blk = b0 + blockIdx.x, cb = blk * CPB;
   const long long c0 = cb + (long long)threadIdx.x * CPT;
   int n[CPT];
   int tot = 0;
@@ -464,7 +519,7 @@ __global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, c
     run += n[h];
   }
   __syncthreads();
-  const long long base = p.block_sums[blockIdx.x];
+  const long long base = p.block_sums[blk];
   const float dx = p.box.dx;
   /* the block's first cell; a cell lo < 2048 further on lies lo2 / N rows
    * below, lo2 = ix0 + lo < 4096, by a product in 32 bits (mdiv / 2^24 is
@@ -750,9 +805,10 @@ __global__ void __launch_bounds__(256) k_src_skewers(const float *__restrict__ d
 long long cg_srcs_nblocks(int N) { return ((long long)N * N * N + CPB - 1) / CPB; }
 long long cg_srcs_scan_room(long long nb) { return (nb + SCAN_T - 1) / SCAN_T; }
 
-cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_params *p, long long *total)
+cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_params *p, long long *total, long long *host,
+                          long long bpc)
 {
-  long long nb = cg_srcs_nblocks(p->box.N);
+  const long long nb = cg_srcs_nblocks(p->box.N);
   k_pois_tab<<<(CG_NA + 31) / 32, 32, 0, s>>>(*p, nb);
   /* four steps per warp where the grid has many times the 7296 warps that 152
    * SMs hold (512^3, two populations: 1.44 ms against 1.50 with two); one on
@@ -760,25 +816,30 @@ cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_param
    * warps alone (128^3) */
   const int steps = p->box.N > 256 ? 4 : 1;
   k_pois_count<<<(unsigned)(nb * CPB / (CWN * CW * steps)), CWN * 32, 0, s>>>(grid, *p, steps);
+  if (nb <= SCAN_ONE) {
+    k_scan_one<<<1, 1024, 0, s>>>(p->block_sums, nb, total, p->err, host, bpc);
+    return cudaGetLastError();
+  }
   const long long nt = cg_srcs_scan_room(nb);
   long long *tsum = p->block_sums + nb; /* the tile sums, just past the block totals */
   k_scan_tiles<<<(unsigned)nt, 1024, 0, s>>>(p->block_sums, nb, tsum, p->err);
   k_scan_top<<<1, 1024, 0, s>>>(tsum, nt, total);
-  k_scan_apply<<<(unsigned)nt, 1024, 0, s>>>(p->block_sums, nb, tsum);
+  k_scan_apply<<<(unsigned)nt, 1024, 0, s>>>(p->block_sums, nb, tsum, total, p->err, host, bpc);
   return cudaGetLastError();
 }
 
-cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p)
+cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long b0, long long b1)
 {
-  const long long nb = cg_srcs_nblocks(p->box.N);
+  if (b1 <= b0) return cudaSuccess;
   /* shares per block: until there are eight blocks for each of the 152 x 8
    * that an SM generation holds, while a share keeps a source per thread (the
    * capacity is the total with an eighth of slack).  c1 at 128^3 with 1 and
    * 16 shares: 244 and 169 us; 192^3 with 240 sources per block: 74 and 127 us
    * with 1 and 4. */
+  const long long nb = b1 - b0, all = cg_srcs_nblocks(p->box.N);
   int sh = 1;
-  while (sh < 16 && nb * sh < 9728 && p->capacity >= nb * sh * 2 * SB) sh *= 2;
-  k_emit<<<dim3((unsigned)nb, (unsigned)sh), SB, 0, s>>>(phi, *p);
+  while (sh < 16 && nb * sh < 9728 && p->capacity >= all * sh * 2 * SB) sh *= 2;
+  k_emit<<<dim3((unsigned)nb, (unsigned)sh), SB, 0, s>>>(phi, *p, b0);
   return cudaGetLastError();
 }
 

@@ -80,8 +80,13 @@ struct cg_los_params {
 long long cg_srcs_nblocks(int N);
 /* Scan scratch that block_sums needs past its nb entries (the tile sums). */
 long long cg_srcs_scan_room(long long nb);
-cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_params *p, long long *total);
-cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p);
+/* Counts and their scan; *total gets the sum.  With host (page-locked, mapped)
+ * non-NULL it receives the total, the error word, and from host[2] on the
+ * source offset of every bpc-th block of cells. */
+cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_params *p, long long *total, long long *host,
+                          long long bpc);
+/* The sources of blocks [b0, b1) of cells (cg_srcs_nblocks in all). */
+cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long b0, long long b1);
 /* nsrc sources, or with nsrc_dev non-NULL min(*nsrc_dev, nsrc) read on the
  * device (a graph-captured sequence, whose totals stay on the device). */
 cudaError_t cg_srcs_beam_rsd(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long nsrc,
