@@ -605,27 +605,50 @@ __global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, c
   if (lane == 0 && nfb) atomicAdd(p.xstats + 1, (unsigned long long)nfb);
 }
 
-/* Trilinear potential gradient at a point with corner cells i0/i1 and
- * weights h0/h1 (interpolate_from_grid RETURN_VEL, beaming.c:183-265): per z
- * plane the four corners' central differences weighted and summed with FMAs,
- * then the two planes added. */
+/* Trilinear potential gradient at a point with corner cells i0/i1 (i1 the
+ * periodic neighbour above i0) and weights h0/h1 (interpolate_from_grid
+ * RETURN_VEL, beaming.c:183-265): per z plane the four corners' central
+ * differences weighted and summed with FMAs, then the two planes added.  The
+ * eight corners' differences share points: 32 loads instead of 48, at offsets
+ * from one cell's address.  The RSD waits for these loads (L1 wavefronts and
+ * latency): 4.1e7 sources on 256^3 984 -> 791 us, 1.07e8 on 512^3 2.94 ->
+ * 2.14 ms. */
 __device__ __forceinline__ void cic_grad(const float *__restrict__ phi, const int i0[3], const int i1[3],
                                          const float h0[3], const float h1[3], int N, float v[3])
 {
+  const int ngx = 2 * (N / 2 + 1);
+  const int xm = wrap(i0[0] - 1, N) - i0[0], x1 = i1[0] - i0[0], xp = wrap(i1[0] + 1, N) - i0[0];
+  const int ym = (wrap(i0[1] - 1, N) - i0[1]) * ngx, y1 = (i1[1] - i0[1]) * ngx, yp = (wrap(i1[1] + 1, N) - i0[1]) * ngx;
+  const long long plane = (long long)ngx * N;
+  const long long zm = (wrap(i0[2] - 1, N) - i0[2]) * plane, z1 = (i1[2] - i0[2]) * plane,
+                  zp = (wrap(i1[2] + 1, N) - i0[2]) * plane;
+  const float *c = phi + pidx(i0[0], i0[1], i0[2], N);
+  float in[2][4], zo[2][4]; /* [z][y, x]: the corners, and those one plane out */
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int o = ((k & 2) ? y1 : 0) + ((k & 1) ? x1 : 0);
+    in[0][k] = __ldg(c + o);
+    in[1][k] = __ldg(c + z1 + o);
+    zo[0][k] = __ldg(c + zm + o);
+    zo[1][k] = __ldg(c + zp + o);
+  }
   v[0] = v[1] = v[2] = 0.0f;
 #pragma unroll
   for (int hz = 0; hz < 2; hz++) {
-    const int zc = hz ? i1[2] : i0[2];
+    const float *r = c + (hz ? z1 : 0);
     const float wz = hz ? h0[2] : h1[2];
+    const float xo[4] = {__ldg(r + xm), __ldg(r + xp), __ldg(r + y1 + xm), __ldg(r + y1 + xp)};
+    const float yo[4] = {__ldg(r + ym), __ldg(r + ym + x1), __ldg(r + yp), __ldg(r + yp + x1)};
     float acc[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const int yc = (k & 2) ? i1[1] : i0[1], xc = (k & 1) ? i1[0] : i0[0];
       const float w = CG_MUL(CG_MUL(wz, (k & 2) ? h0[1] : h1[1]), (k & 1) ? h0[0] : h1[0]);
-      float g[3];
-      grad_phi(phi, xc, yc, zc, N, g);
-#pragma unroll
-      for (int a = 0; a < 3; a++) acc[a] = CG_FMA(g[a], w, acc[a]);
+      const float gx = (k & 1) ? CG_SUB(xo[k], in[hz][k - 1]) : CG_SUB(in[hz][k + 1], xo[k]);
+      const float gy = (k & 2) ? CG_SUB(yo[k], in[hz][k - 2]) : CG_SUB(in[hz][k + 2], yo[k]);
+      const float gz = hz ? CG_SUB(zo[1][k], in[0][k]) : CG_SUB(in[1][k], zo[0][k]);
+      acc[0] = CG_FMA(gx, w, acc[0]);
+      acc[1] = CG_FMA(gy, w, acc[1]);
+      acc[2] = CG_FMA(gz, w, acc[2]);
     }
 #pragma unroll
     for (int a = 0; a < 3; a++) v[a] = CG_ADD(v[a], acc[a]);
