@@ -102,12 +102,10 @@ CG_HD float cg_pow2i(int k) { return cg_u2f((uint32_t)(k + 127) << 23); }
 /* e^x, |error| <= 2 ulp, flushes to 0 below -103.9 and to +inf above 88.72. */
 CG_HD float cg_expf(float x)
 {
-  if (x > 88.7228317f) return cg_u2f(0x7f800000u);
-  if (x < -103.972084f) return 0.0f;
-  /* j = round-to-nearest(x * log2(e)) through the 1.5*2^23 shifter */
   const float shifter = 12582912.0f;
-  float j = CG_SUB(CG_FMA(x, 1.44269504088896341f, shifter), shifter);
-  int k = (int)j;
+  /* j = round-to-nearest(x * log2(e)) through the 1.5*2^23 shifter */
+  const float t = CG_FMA(x, 1.44269504088896341f, shifter);
+  const float j = CG_SUB(t, shifter);
   /* r = x - j*ln2 with a two-part ln2 (Cody-Waite) */
   float r = CG_FMA(j, -0.693145751953125f, x);
   r = CG_FMA(j, -1.42860682030941723e-06f, r);
@@ -120,7 +118,13 @@ CG_HD float cg_expf(float x)
   p = CG_FMA(p, r, 0.5f);
   p = CG_FMA(p, r, 1.0f);
   p = CG_FMA(p, r, 1.0f);
-  /* scale by 2^k in two steps so that subnormal results are formed once */
+  /* scale by 2^k: in the middle range by adding k to the exponent (the low
+   * bits of t hold it), exact like the product */
+  if (x > -86.5f && x < 88.0f) return cg_u2f(cg_f2u(p) + (cg_f2u(t) << 23));
+  if (x > 88.7228317f) return cg_u2f(0x7f800000u);
+  if (x < -103.972084f) return 0.0f;
+  const int k = (int)j;
+  /* in two steps so that subnormal results are formed once */
   if (k > 126) return CG_MUL(CG_MUL(p, 2.0f), cg_pow2i(k - 1));
   if (k < -125) return CG_MUL(CG_MUL(p, cg_pow2i(k + 64)), 5.42101086242752217e-20f);
   return CG_MUL(p, cg_pow2i(k));

@@ -10,8 +10,8 @@
  *                    the summed redshift and the summed bias_model of every
  *                    tracer.  A warp owns 32 consecutive cells of a row;
  *                    lanes sharing a bin are reduced with shuffles (one pass
- *                    when the 32 cells share a bin, the common case) and lane
- *                    0 adds the sums to the warp's private bins in shared
+ *                    when the 32 cells share a bin) and one lane per value
+ *                    adds the sums to the warp's private bins in shared
  *                    memory: integer counts and compensated (Kahan) FP32
  *                    sums, since FP64 arithmetic is scarce on this GPU.  Each
  *                    block combines its warps' bins in FP64 in a fixed order
@@ -67,14 +67,32 @@ __global__ void k_moments_final(const double2 *__restrict__ part, size_t n, doub
 constexpr int MAXT = 8;      /* tracers per bins launch */
 constexpr int BINS_WARPS = 8; /* warps per block at most  */
 
-/* Warp reduction of v over the lanes whose mask bit is set (others add 0). */
-__device__ __forceinline__ float wsum(float v, bool mine)
+/* Sums of V values (a power of two) over the warp.  While several values are
+ * left, a step exchanges them in pairs: each half of the lanes keeps one value
+ * of a pair and gives the other away; then the plain butterfly.  Every value
+ * is summed over the offsets 16, 8, 4, 2, 1 in this order, as one butterfly
+ * per value would, in 4 (V - 1) + 2 (5 - log2 V) instructions instead of
+ * 10 V.  Lane l returns the sum of value (the bits of l from the top, log2 V
+ * of them). */
+template <int V>
+__device__ __forceinline__ float warp_sums(float *v, int lane)
 {
-  float x = mine ? v : 0.0f;
+  int o = 16;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+  for (int n = V; n > 1; n >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < n / 2; k++) {
+      const float give = up ? v[k] : v[k + n / 2], keep = up ? v[k + n / 2] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
 }
+
+__host__ __device__ constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
 
 /* Compensated FP32 accumulation s += v (c holds the running correction). */
 __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
@@ -117,15 +135,19 @@ __device__ __forceinline__ void fix_add(unsigned long long *a, double x)
  * for the redshift and every tracer. */
 __host__ __device__ inline size_t bins_warp_bytes(int nz, int nt) { return (size_t)nz * (4 + 8 * (1 + nt)); }
 
-/* Up to three tracers the kernel fits 32 registers, eight blocks per SM
- * (11.2 -> 10.8 ms at 1024^3 with two); more tracers keep two. */
+/* Up to three tracers eight blocks per SM (32 registers), more tracers two.
+ * Issue bound (1024^3 with two tracers: 12 % of DRAM peak): row quantities are
+ * formed once per row, a warp's sums take one exchange for all values
+ * (warp_sums) and one compensated addition by as many lanes as there are
+ * values: 10.8 -> 8.5 ms at 1024^3 with two tracers, 2.43 -> 1.74 ms at 512^3
+ * with three. */
 template <int NT>
 __global__ void __launch_bounds__(BINS_WARPS * 32, NT <= 3 ? 8 : 2) k_dens_bins(float *grid, cg_bins_params p)
 {
   extern __shared__ unsigned char sbins[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  constexpr int nt = NT, MT = NT > 0 ? NT : 1;
-  const int nz = p.nz, W = 1 + nt;
+  constexpr int nt = NT, W = 1 + nt, V = pow2_at_least(W);
+  const int nz = p.nz;
   unsigned int *cnt = reinterpret_cast<unsigned int *>(sbins + (size_t)wid * bins_warp_bytes(nz, nt));
   float *acc = reinterpret_cast<float *>(cnt + nz); /* [nz][W] sums, then [nz][W] corrections */
   float *cor = acc + (size_t)nz * W;
@@ -133,27 +155,25 @@ __global__ void __launch_bounds__(BINS_WARPS * 32, NT <= 3 ? 8 : 2) k_dens_bins(
   for (int i = lane; i < 2 * nz * W; i += 32) acc[i] = 0.0f;
   __syncwarp();
   const int N = p.box.N;
-  const int nseg_row = (N + 31) / 32;
   const int nrow = N * N;
   const float s2 = p.sigma2f ? *p.sigma2f : 0.0f;
   const bool need_d1 = (p.mode == CG_DMODE_LGNR || p.mode == CG_DMODE_CLIP);
   const int gw = blockIdx.x * nwb + wid;
   const int nw = gridDim.x * nwb;
-  /* a warp takes whole rows, 32 cells at a time */
-  for (int row = gw; row < nrow; row += nw)
-  for (int sr = 0; sr < nseg_row; sr++) {
-    const int iz = row / N, iy = row - iz * N;
-    const int ix = sr * 32 + lane;
-    int bin = -1;
-    float zz = 0.0f, bs[MT];
-#pragma unroll
-    for (int t = 0; t < MT; t++) bs[t] = 0.0f;
-    if (ix < N) {
-      float *ptr = grid + pidx(ix, iy, iz, N);
+  /* the value whose sum this lane ends up with: 0 the redshift, 1 + t the
+   * bias of tracer t; one lane of each adds it to the bins */
+  const int mine_v = V > 1 ? lane / (32 / V) : 0;
+  const bool adds = lane % (32 / V) == 0 && mine_v < W;
+  /* a warp takes whole rows (N is a multiple of 32), 32 cells at a time */
+  for (int row = gw; row < nrow; row += nw) {
+    const int iz = (int)divN(row, p.box), iy = row - iz * N;
+    const float y0 = cg_cell_coord(iy, p.box.dx, p.box.p1), z0 = cg_cell_coord(iz, p.box.dx, p.box.p2);
+    const float yy = CG_MUL(y0, y0), zz2 = CG_MUL(z0, z0);
+    float *ptr = grid + pidx(lane, iy, iz, N);
+    for (int ix = lane; ix < N; ix += 32, ptr += 32) {
       float d = *ptr;
       const float x0 = cg_cell_coord(ix, p.box.dx, p.box.p0);
-      const float y0 = cg_cell_coord(iy, p.box.dx, p.box.p1), z0 = cg_cell_coord(iz, p.box.dx, p.box.p2);
-      const float r = cg_norm3(x0, y0, z0);
+      const float r = CG_SQRT(CG_ADD(CG_ADD(CG_MUL(x0, x0), yy), zz2)); /* cg_norm3 */
       const BgAt at = bg_at(p.g, r);
       if (p.mode != CG_DMODE_NONE) {
         if (p.mode == CG_DMODE_RHO) {
@@ -166,38 +186,36 @@ __global__ void __launch_bounds__(BINS_WARPS * 32, NT <= 3 ? 8 : 2) k_dens_bins(
         d = cg_dens_transform(p.mode, d, need_d1 ? bgv(p.d1, at) : 0.0f, s2);
         *ptr = d;
       }
-      if (nz > 0) {
-        const float z = bgv(p.zt, at);
-        const int b = (int)CG_MUL(z, p.idz) + 1;
-        if (b >= 0 && b < nz) {
-          bin = b;
-          zz = z;
+      if (nz == 0) continue;
+      float v[V];
 #pragma unroll
-          for (int t = 0; t < nt; t++) bs[t] = cg_bias_model(d, bgv(p.bz[t], at), p.bias_model);
+      for (int k = 0; k < V; k++) v[k] = 0.0f;
+      const float z = bgv(p.zt, at);
+      int bin = (int)CG_MUL(z, p.idz) + 1;
+      if (bin >= 0 && bin < nz) {
+        v[0] = z;
+#pragma unroll
+        for (int t = 0; t < nt; t++) v[1 + t] = cg_bias_model(d, bgv(p.bz[t], at), p.bias_model);
+      } else {
+        bin = -1;
+      }
+      /* segmented reduction by bin; one pass when the 32 cells share a bin */
+      unsigned todo = __ballot_sync(0xffffffffu, bin >= 0);
+      while (todo) {
+        const int lb = __shfl_sync(0xffffffffu, bin, __ffs(todo) - 1);
+        const unsigned grp = __ballot_sync(0xffffffffu, bin == lb);
+        float m[V];
+#pragma unroll
+        for (int k = 0; k < V; k++) m[k] = k < W && bin == lb ? v[k] : 0.0f;
+        const float sum = warp_sums<V>(m, lane);
+        if (adds) {
+          float *a = acc + (size_t)lb * W + mine_v, *c = cor + (size_t)lb * W + mine_v;
+          kahan_add(*a, *c, sum);
+          if (lane == 0) cnt[lb] += (unsigned)__popc(grp);
         }
+        todo &= ~grp;
       }
     }
-    if (nz == 0) continue;
-    /* segmented reduction by bin; one pass when the 32 cells share a bin */
-    unsigned todo = __ballot_sync(0xffffffffu, bin >= 0);
-    while (todo) {
-      const int lb = __shfl_sync(0xffffffffu, bin, __ffs(todo) - 1);
-      const bool mine = (bin == lb);
-      const unsigned grp = __ballot_sync(0xffffffffu, mine);
-      const float zsum = wsum(zz, mine);
-      float bsum[MT];
-#pragma unroll
-      for (int t = 0; t < nt; t++) bsum[t] = wsum(bs[t], mine);
-      if (lane == 0) {
-        float *a = acc + (size_t)lb * W, *c = cor + (size_t)lb * W;
-        cnt[lb] += (unsigned)__popc(grp);
-        kahan_add(a[0], c[0], zsum);
-#pragma unroll
-        for (int t = 0; t < nt; t++) kahan_add(a[1 + t], c[1 + t], bsum[t]);
-      }
-      todo &= ~grp;
-    }
-    __syncwarp();
   }
   __syncthreads();
   /* combine the warps' bins in FP64 in fixed order, one global update each */
