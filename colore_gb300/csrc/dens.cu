@@ -136,11 +136,11 @@ __device__ __forceinline__ void fix_add(unsigned long long *a, double x)
 __host__ __device__ inline size_t bins_warp_bytes(int nz, int nt) { return (size_t)nz * (4 + 8 * (1 + nt)); }
 
 /* Up to three tracers eight blocks per SM (32 registers), more tracers two.
- * Issue bound (1024^3 with two tracers: 12 % of DRAM peak): row quantities are
- * formed once per row, a warp's sums take one exchange for all values
- * (warp_sums) and one compensated addition by as many lanes as there are
- * values: 10.8 -> 8.5 ms at 1024^3 with two tracers, 2.43 -> 1.74 ms at 512^3
- * with three. */
+ * Bound by instruction issue (12 % of DRAM peak at 1024^3 with two tracers),
+ * so row quantities are formed once per row, and a warp's sums take one
+ * exchange for all values (warp_sums) and one compensated addition by as many
+ * lanes as there are values: 10.8 -> 8.5 ms at 1024^3 with two tracers, 2.43
+ * -> 1.74 ms at 512^3 with three. */
 template <int NT>
 __global__ void __launch_bounds__(BINS_WARPS * 32, NT <= 3 ? 8 : 2) k_dens_bins(float *grid, cg_bins_params p)
 {
