@@ -57,8 +57,8 @@ struct Imap {
   int *shell_of = nullptr, *nsub = nullptr;
   long long *base = nullptr, *cap = nullptr;
   unsigned long long *cnt = nullptr, *chunk_off = nullptr;
-  float *data = nullptr;
-  int *nadd = nullptr;
+  float2 *acc = nullptr; /* summed brightness and samples per pixel */
+  int packed = 0;        /* samples held as floats (cg_imap_params) */
   unsigned long long *ctr = nullptr; /* the kernels' counters (5) */
   unsigned long long samples = 0;    /* sub-samples drawn by the last run */
   bool samples_stale = false;        /* a run since samples was read */
@@ -127,6 +127,7 @@ struct cg_ctx {
   int pending_mode = CG_DMODE_NONE;
   /* sources */
   unsigned short *d_counts = nullptr;
+  cg_imap_seg *d_iseg = nullptr; /* table segments of the species being listed */
   cg_pois_seg *d_seg = nullptr; /* table segments of the population being counted */
   long long *d_bsums = nullptr, *d_total = nullptr, *d_ovf_cell = nullptr;
   int *d_ovf_cnt = nullptr, *d_ovf_n = nullptr;
@@ -840,20 +841,34 @@ extern "C" int cg_memory_estimate(const cg_config *cfg, unsigned long long *byte
 }
 
 /* write_imap's normalisation (io.c:738-741): data/nadd where nadd > 0. */
-__device__ __forceinline__ float div_nadd(float d, int k) { return k > 0 ? d / (float)k : d; }
+/* Samples of a map pixel (imap_api.h). */
+__device__ __forceinline__ int hits_of(float2 a, int packed) { return packed ? (int)a.y : __float_as_int(a.y); }
 
-/* data/nadd of m pixels (16-byte vectors; the buffers are cudaMalloc'd). */
-__global__ void k_div_nadd(const float *__restrict__ d, const int *__restrict__ n, float *out, long long m)
+__device__ __forceinline__ float div_nadd(float2 a, int packed)
+{
+  const int k = hits_of(a, packed);
+  return k > 0 ? a.x / (float)k : a.x;
+}
+
+/* data/nadd of m pixels, four at a time (the buffers are cudaMalloc'd). */
+__global__ void k_div_nadd(const float2 *__restrict__ acc, int packed, float *out, long long m)
 {
   const long long m4 = m >> 2, stride = (long long)gridDim.x * blockDim.x;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = t; i < m4; i += stride) {
-    const float4 a = reinterpret_cast<const float4 *>(d)[i];
-    const int4 k = reinterpret_cast<const int4 *>(n)[i];
-    reinterpret_cast<float4 *>(out)[i] = make_float4(div_nadd(a.x, k.x), div_nadd(a.y, k.y), div_nadd(a.z, k.z),
-                                                     div_nadd(a.w, k.w));
+    const float4 a = reinterpret_cast<const float4 *>(acc)[2 * i], b = reinterpret_cast<const float4 *>(acc)[2 * i + 1];
+    reinterpret_cast<float4 *>(out)[i] =
+        make_float4(div_nadd(make_float2(a.x, a.y), packed), div_nadd(make_float2(a.z, a.w), packed),
+                    div_nadd(make_float2(b.x, b.y), packed), div_nadd(make_float2(b.z, b.w), packed));
   }
-  for (long long i = 4 * m4 + t; i < m; i += stride) out[i] = div_nadd(d[i], n[i]);
+  for (long long i = 4 * m4 + t; i < m; i += stride) out[i] = div_nadd(acc[i], packed);
+}
+
+/* The samples per pixel alone. */
+__global__ void k_hits(const float2 *__restrict__ acc, int packed, int *out, long long m)
+{
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x)
+    out[i] = hits_of(acc[i], packed);
 }
 
 /* ---- host outputs (cg_set_host_*) ---- */
@@ -938,7 +953,7 @@ extern "C" void cg_destroy(cg_ctx *c)
     if (q) cudaFree(q);
   void *ptrs[] = {c->d_tabs, c->d_norm, c->d_tabs64, c->d_norm64, c->d_corner, c->d_att, c->d_xstats, c->d_zr, c->d_r2n, c->d_pk, c->d_twN, c->d_twH, c->d_dens, c->d_npot, c->d_disp[0],
                   c->d_disp[1], c->d_disp[2], c->d_part, c->d_stats, c->d_s2f, c->d_err, c->d_ncount,
-                  c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_seg, c->d_bsums, c->d_total, c->d_tmpmap, c->d_kmap,
+                  c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_seg, c->d_iseg, c->d_bsums, c->d_total, c->d_tmpmap, c->d_kmap,
                   c->d_kfac, c->d_kinv, c->d_kir, c->d_ovf_cell, c->d_ovf_cnt, c->d_ovf_n,
                   c->d_recs, c->d_imap_queue,
                   c->d_imap_isw, c->d_ifac, c->d_iir, c->d_cfac, c->d_losfac};
@@ -947,7 +962,7 @@ extern "C" void cg_destroy(cg_ctx *c)
   for (int i = 0; i < CG_NPOP_MAX; i++) {
     void *q[] = {c->cat[i].pos, c->cat[i].ipix, c->cat[i].src, c->cat[i].cmap, c->im[i].b, c->im[i].dxs,
                  c->im[i].dxsl, c->im[i].shell_of, c->im[i].nsub, c->im[i].base, c->im[i].cap, c->im[i].cnt, c->im[i].chunk_off,
-                 c->im[i].data, c->im[i].nadd, c->im[i].ctr, c->d_cmap[i], c->cat[i].skw_d, c->cat[i].skw_v};
+                 c->im[i].acc, c->im[i].ctr, c->d_cmap[i], c->cat[i].skw_d, c->cat[i].skw_v};
     for (void *p : q)
       if (p) cudaFree(p);
   }
@@ -1610,7 +1625,7 @@ static int imap_prepare(cg_ctx *c, int ip)
   const int nside = c->cfg.nside_imap[ip];
   const long long npix = 12LL * nside * nside;
   const double dx = c->cfg.l_box / c->N;
-  const int nbk = nr + 2;
+  const int nbk = CG_IMAP_CLASSES * (nr + 2);
   if (nbk > CG_IMAP_BUCKETS_MAX) return fail(c, CG_EINVAL, "intensity species %d: %d shells", ip, nr);
   std::vector<float> r0f(nr), rff(nr), bb(2 * nr), dxs(nr + 2);
   std::vector<int> shell_of(2 * nr + 1), nsub(nr + 2);
@@ -1624,20 +1639,26 @@ static int imap_prepare(cg_ctx *c, int ip)
         (rc = dalloc(c, &M.nsub, (size_t)nr + 2)) || (rc = dalloc(c, &M.dxs, (size_t)nr + 2)) ||
         (rc = dalloc(c, &M.dxsl, (size_t)nr + 2)) ||
         (rc = dalloc(c, &M.base, (size_t)nbk)) || (rc = dalloc(c, &M.cap, (size_t)nbk)) ||
-        (rc = dalloc(c, &M.cnt, (size_t)nbk)) || (rc = dalloc(c, &M.chunk_off, (size_t)nbk + 1)))
+        (rc = dalloc(c, &M.cnt, (size_t)nbk * CG_IMAP_CNT)) || (rc = dalloc(c, &M.chunk_off, (size_t)nbk + 1)))
       return rc;
   }
   if (M.nr != nr || M.npix != npix) {
-    if ((rc = dalloc(c, &M.data, (size_t)nr * npix)) || (rc = dalloc(c, &M.nadd, (size_t)nr * npix))) return rc;
+    if ((rc = dalloc(c, &M.acc, (size_t)nr * npix))) return rc;
   }
   M.nr = nr;
   M.nside = nside;
   M.npix = npix;
   const double rmin = (double)r0f[0] - 20., rmax = (double)rff[nr - 1] + 20.;
-  /* slots per bucket: the corners of the cells of bucket j + 1 lie in the
-   * radii of the intervals of shell j; each corner's dx-cube lies within
-   * sqrt(3)/2 dx of it, so (expanded shell volume) / dx^3 bounds them */
+  /* slots per bucket: the corners of the cells of shell j's buckets lie in
+   * the radii of its intervals; each corner's dx-cube lies within sqrt(3)/2 dx
+   * of it, so (expanded shell volume) / dx^3 bounds them.  Of these 2/3 lie
+   * at |cos theta| < 2/3 (class 1) and 1/3 beyond (class 2), each up to a
+   * surface layer, about 1 cell deep; class 0 holds the cells on the four
+   * planes between octants and the two cones (t / 2r of a thin shell each for
+   * a layer t: 3.5 cells in r), and all of a shell that a cell may span
+   * (CG_SH_WALK) or leave for none.  Cells past a bucket's room are painted as they are listed. */
   std::vector<double> want(nbk, 0.0);
+  double dense = 0; /* most samples per pixel that a shell's cells hold on average */
   const double h = 0.8660254037844386 * dx, ncell = (double)c->N * c->N * c->N;
   for (int k = -1; k < nb; k++) {
     double lo = k < 0 ? rmin : (double)bb[k], hi = k + 1 < nb ? (double)bb[k + 1] : rmax;
@@ -1645,7 +1666,14 @@ static int imap_prepare(cg_ctx *c, int ip)
     hi = hi > rmax ? rmax : hi;
     if (hi <= lo) continue;
     const double a = lo - h > 0 ? lo - h : 0, z = hi + h;
-    want[shell_of[k + 1] + 1] += 4.0 / 3.0 * M_PI * (z * z * z - a * a * a) / (dx * dx * dx);
+    const double v = 4.0 / 3.0 * M_PI * (z * z * z - a * a * a) / (dx * dx * dx), ir = 1.0 / std::max(a / dx, 1.0);
+    double *w = &want[CG_IMAP_CLASSES * (shell_of[k + 1] + 1)];
+    dense = std::max(dense, v * std::pow((double)nsub[shell_of[k + 1] + 1], 3) / (double)npix);
+    auto painted = [&](int i) { return i >= -1 && i < nb && shell_of[i + 1] >= 0 && shell_of[i + 1] < nr; };
+    const bool plain = painted(k - 1) && painted(k) && painted(k + 1) && bb[k + 1] - bb[k] >= 2.1 * dx;
+    w[0] += plain ? v * std::min(5 * ir + 0.01, 1.0) : v;
+    w[1] += v * std::min(2.0 / 3.0 + ir, 1.0);
+    w[2] += v * std::min(1.0 / 3.0 + ir, 1.0);
   }
   double tot = 0;
   for (int i = 0; i < nbk; i++) {
@@ -1671,6 +1699,7 @@ static int imap_prepare(cg_ctx *c, int ip)
     c->list_cap = acc;
   }
   if (!M.ctr && (rc = dalloc(c, &M.ctr, (size_t)5))) return rc;
+  if (!c->d_iseg && (rc = dalloc(c, &c->d_iseg, (size_t)CG_NA))) return rc;
   if (!c->d_imap_queue) {
     const long long qc = 1LL << 27;
     if ((rc = dalloc(c, &c->d_imap_queue, (size_t)qc))) return rc;
@@ -1691,6 +1720,10 @@ static int imap_prepare(cg_ctx *c, int ip)
   M.contig = cg_imap_contig(r0f.data(), rff.data(), nr, nb);
   M.rmin = rmin;
   M.rmax = rmax;
+  /* samples are spread over the sky like the cells; a pixel of a shell takes
+   * its own cells' and some of its neighbours', so 192 times the mean leaves
+   * a factor 64 to a float's 2^24 whole numbers */
+  M.packed = 192.0 * dense < 16777216.0;
   M.gen = c->tab_gen;
   return CG_OK;
 }
@@ -1701,11 +1734,10 @@ static int imap_prepare(cg_ctx *c, int ip)
 static int imap_launch(cg_ctx *c, int ip)
 {
   Imap &M = c->im[ip];
-  const int nr = M.nr, nside = M.nside, nbk = nr + 2;
+  const int nr = M.nr, nside = M.nside, nbk = CG_IMAP_CLASSES * (nr + 2);
   const long long npix = M.npix;
   const double dx = c->cfg.l_box / c->N;
-  CUDA_TRY(c, cudaMemsetAsync(M.data, 0, (size_t)nr * npix * sizeof(float), c->stream));
-  CUDA_TRY(c, cudaMemsetAsync(M.nadd, 0, (size_t)nr * npix * sizeof(int), c->stream));
+  CUDA_TRY(c, cudaMemsetAsync(M.acc, 0, (size_t)nr * npix * sizeof(float2), c->stream));
   cg_imap_params p;
   memset(&p, 0, sizeof(p));
   p.box = c->box;
@@ -1759,8 +1791,9 @@ static int imap_launch(cg_ctx *c, int ip)
   p.nr = nr;
   p.nbk = nbk;
   p.npix = npix;
-  p.data = M.data;
-  p.nadd = M.nadd;
+  p.seg = c->d_iseg;
+  p.acc = M.acc;
+  p.packed = M.packed;
   p.err = c->d_err;
   p.xstats = c->d_xstats;
   p.force_double = c->force_double;
@@ -1777,7 +1810,7 @@ static int imap_launch(cg_ctx *c, int ip)
     CUDA_TRY(c, cg_imap_paint(c->stream, c->d_dens, c->d_npot, &p, c->nsm));
   }
   M.samples_stale = true;
-  c->launches += 4; /* list, chunks, paint, double */
+  c->launches += 5; /* tables, list, chunks, paint, double */
   return CG_OK;
 }
 
@@ -1801,7 +1834,7 @@ static int imap_run(cg_ctx *c, bool host_out)
       c->imap_out_n[ip] = m;
     }
     k_div_nadd<<<(unsigned)std::min<long long>((m + 255) / 256, (long long)c->nsm * 16), 256, 0, c->stream>>>(
-        M.data, M.nadd, c->d_imap_out[ip], m);
+        M.acc, M.packed, c->d_imap_out[ip], m);
     CUDA_TRY(c, cudaGetLastError());
     c->launches++;
     if (int rc = out_begin(c)) return rc;
@@ -2633,21 +2666,26 @@ extern "C" int cg_download_imap(cg_ctx *c, int ipop, float *map, int *nadd)
 {
   if (!c || ipop < 0 || ipop >= c->cfg.n_imap) return CG_EINVAL;
   const Imap &M = c->im[ipop];
-  if (!M.data) return fail(c, CG_ESTATE, "intensity map %d not painted", ipop);
+  if (!M.acc) return fail(c, CG_ESTATE, "intensity map %d not painted", ipop);
   const long long m = (long long)M.nr * M.npix;
+  const unsigned blocks = (unsigned)std::min<long long>((m + 255) / 256, (long long)c->nsm * 16);
+  if ((map || nadd) && c->tmpmap_n < (size_t)m) {
+    if (int rc = dalloc(c, &c->d_tmpmap, (size_t)m)) return rc;
+    c->tmpmap_n = m;
+  }
   if (map) {
-    if (c->tmpmap_n < (size_t)m) {
-      if (int rc = dalloc(c, &c->d_tmpmap, (size_t)m)) return rc;
-      c->tmpmap_n = m;
-    }
     /* write_imap, io.c:738-741: data/nadd where nadd > 0 */
-    k_div_nadd<<<(unsigned)std::min<long long>((m + 255) / 256, (long long)c->nsm * 16), 256, 0, c->stream>>>(
-        M.data, M.nadd, c->d_tmpmap, m);
+    k_div_nadd<<<blocks, 256, 0, c->stream>>>(M.acc, M.packed, c->d_tmpmap, m);
     CUDA_TRY(c, cudaGetLastError());
     c->launches++;
     CUDA_TRY(c, cudaMemcpyAsync(map, c->d_tmpmap, m * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   }
-  if (nadd) CUDA_TRY(c, cudaMemcpyAsync(nadd, M.nadd, m * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (nadd) { /* through the same buffer, after the map's copy on the stream */
+    k_hits<<<blocks, 256, 0, c->stream>>>(M.acc, M.packed, reinterpret_cast<int *>(c->d_tmpmap), m);
+    CUDA_TRY(c, cudaGetLastError());
+    c->launches++;
+    CUDA_TRY(c, cudaMemcpyAsync(nadd, c->d_tmpmap, m * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  }
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return check_device_errors(c);
 }

@@ -1146,6 +1146,137 @@ CG_HD int cg_imap_cell_checked(const cg_imap_args *a, int ix, int iy, int iz, fl
   return 1;
 }
 
+/* ---- Listing a cell from per-segment tables ------------------------------ */
+
+/* T(r) norm(r), b(r) and the RSD factor fv idx v1(r) ih(r) / 2 of the radial
+ * tables in the position t within a segment (cg_seg_pos), the first quadratic,
+ * the others linear (the factor's curvature is part of its bound); and in kk
+ * the interval of the shells' edges that the segment starts in, 4 (k + 1), and
+ * whether T is certainly positive (1), zero (0) or neither (2) within the
+ * position's error.  A cell takes one 32-byte sector where
+ * cg_imap_cell_checked takes five lookups with a bound each and a search. */
+typedef struct __attribute__((aligned(32))) {
+  float t0, t1, t2;
+  int kk;
+  float b0, b1, g0, g1;
+} cg_imap_seg;
+
+/* Segment i; *eg bounds the distance of its factor to the double one. */
+CG_HD cg_imap_seg cg_imap_seg_make(const cg_imap_args *a, int i, float *eg)
+{
+  const double u = 5.9604644775390625e-08, dt = cg_seg_dt(i), fv = a->fv64 * 0.5 * a->idx64;
+  cg_imap_seg o;
+  int pos = 1, zero = 1;
+  double S = 0, g0 = 0, g1 = 0, curv = 0;
+  for (int k = i - 1; k <= i + 1; k++) {
+    if (k < 0 || k > a->na - 2) continue;
+    for (int e = 0; e < 2; e++) {
+      pos = pos && a->tz64[k + e] > 0;
+      zero = zero && a->tz64[k + e] == 0;
+    }
+    const double v = a->v164[k], dv = a->v164[k + 1] - v, h = a->ih64[k], dh = a->ih64[k + 1] - h;
+    const double k1 = fv * (v * dh + dv * h), k2 = fv * dv * dh;
+    const double s0 = fabs(k1), s1 = fabs(k1 + 2 * k2);
+    if (s0 > S) S = s0;
+    if (s1 > S) S = s1;
+    if (k != i) continue;
+    g0 = fv * v * h;
+    g1 = k1 + k2;          /* the chord */
+    curv = 0.25 * fabs(k2); /* k2 t (1 - t) */
+  }
+  const double t = a->tz64[i], dtz = a->tz64[i + 1] - t, n = a->norm64[i], dn = a->norm64[i + 1] - n;
+  o.t0 = (float)(t * n);
+  o.t1 = (float)(t * dn + dtz * n);
+  o.t2 = (float)(dtz * dn);
+  o.kk = 4 * (cgx_interval(&a->sh, a->r64[i]) + 1) + (pos ? 1 : (zero ? 0 : 2));
+  o.b0 = (float)a->bz64[i];
+  o.b1 = (float)(a->bz64[i + 1] - a->bz64[i]);
+  o.g0 = (float)g0;
+  o.g1 = (float)g1;
+  *eg = (float)(1.02 * (S * dt + curv + 8 * u * (fabs(g0) + fabs(g1))));
+  return o;
+}
+
+/* The listing of cell (corner x0, y0, z0, r2 its squared radius) from the
+ * segments: 0 certainly not listed, 1 with *o, 2 open (cg_imap_cell_checked).
+ * eg: the largest of the segments' bounds; d: the cell's density; v: the
+ * potential's centred differences.  The edges a->sh.b stand between two
+ * sentinels on either side (b[-2], b[-1] below and b[nb], b[nb + 1] above every
+ * radius). */
+CG_HD int cg_imap_cell_seg(const cg_imap_seg *segs, float eg, const cg_imap_args *a, float x0, float y0, float z0,
+                           float r2, float d, const float v[3], cg_imap_cell *o)
+{
+  if (!(r2 > 0.0f)) return 2;
+  const float rinv = cg_rsqrt_fast(r2);
+  const float rc = CG_MUL(r2, rinv);
+  const float erc = CG_MUL(rc, 8.0f * CG_E24);
+  /* rmin and rmax (at most r_last here) with 1e-6 of them to spare */
+  const float hi = cg_min_nn(a->rmax, a->r_last);
+  if (rc > CG_MUL(a->rmax, 1.000001f) || rc < CG_SUB(a->rmin, CG_MUL(1e-6f, cg_fabsf(a->rmin)))) return 0;
+  if (!(rc < CG_MUL(hi, 0.999999f) && rc > CG_FMA(1e-6f, cg_fabsf(a->rmin), a->rmin))) return 2;
+  const float s = CG_MUL(rc, a->idr);
+  const int i = (int)s;
+  const float t = CG_SUB(s, (float)i);
+  const cg_imap_seg g = segs[i];
+  if ((g.kk & 3) != 1) return g.kk & 3;
+  /* the corner's shell: its radius clear of the interval's edges */
+  int k = (g.kk >> 2) - 1;
+  const cg_shells *sh = &a->sh;
+  while (rc >= sh->b[k + 1]) k++;
+  const float b0 = sh->b[k], b1 = sh->b[k + 1];
+  if (!(cg_min_nn(CG_SUB(rc, b0), CG_SUB(b1, rc)) > erc)) return 2;
+  const int j = sh->shell_of[k + 1];
+  o->j = j;
+  const float b = CG_FMA(g.b1, t, g.b0);
+  o->temp = CG_MUL(CG_FMA(CG_FMA(g.t2, t, g.t1), t, g.t0), cg_bias_model(d, b, a->bias_model));
+  const float u0 = CG_MUL(x0, rinv), u1 = CG_MUL(y0, rinv), u2 = CG_MUL(z0, rinv);
+  const float p0 = CG_MUL(v[0], u0), p1 = CG_MUL(v[1], u1), p2 = CG_MUL(v[2], u2);
+  const float dot = CG_ADD(CG_ADD(p0, p1), p2);
+  const float sabs = CG_ADD(CG_ADD(cg_fabsf(p0), cg_fabsf(p1)), cg_fabsf(p2));
+  const float G = CG_FMA(g.g1, t, g.g0);
+  o->drr = CG_MUL(dot, G);
+  /* the dot product within 12 2^-24 sabs (unit vector 7.5, products, sums),
+   * the factor within eg, the product's rounding; 2 % for the rest */
+  o->edrr = CG_MUL(1.02f, CG_FMA(sabs, CG_FMA(12.0f * CG_E24, CG_ADD(cg_fabsf(G), eg), eg),
+                                 CG_MUL(2.0f * CG_E24, cg_fabsf(o->drr))));
+  /* the sample centres' radii: they lie within hs of the cell's centre c on
+   * every axis, so r >= c.w - hs (|w0| + |w1| + |w2|) for the unit vector w of
+   * c, and r <= that sum added plus the square of their distance, 3 hs^2,
+   * over 2 |c| */
+  const float hx = CG_MUL(0.5f, a->dx);
+  const float c0 = CG_ADD(x0, hx), c1 = CG_ADD(y0, hx), c2 = CG_ADD(z0, hx);
+  const float cc = CG_FMA(c2, c2, CG_FMA(c1, c1, CG_MUL(c0, c0)));
+  const float ci = cg_rsqrt_fast(cg_max_nn(cc, 1e-30f));
+  const float rm = CG_MUL(cc, ci);
+  const float hs = CG_SUB(hx, CG_MUL(0.5f, a->dxs[j + 1]));
+  const float w = CG_MUL(hs, CG_MUL(ci, CG_ADD(CG_ADD(cg_fabsf(c0), cg_fabsf(c1)), cg_fabsf(c2))));
+  const float far = CG_MUL(CG_MUL(1.51f, hs), CG_MUL(hs, ci));
+  /* positions within 2^-24 (|x| + 2 dx) per axis, the radius arithmetic */
+  const float er = CG_FMA(CG_ADD(rm, w), 16.0f * CG_E24, CG_MUL(a->dx, 8.0f * CG_E24));
+  const float e = CG_ADD(CG_ADD(er, o->edrr), CG_MUL(1e-6f, a->dx));
+  const float mid = CG_ADD(rm, o->drr);
+  const float slo = CG_SUB(CG_SUB(mid, w), e), shi = CG_ADD(CG_ADD(mid, w), CG_ADD(far, e));
+  /* their intervals: k's or a neighbour's as a rule */
+  int kl = k + (slo >= b1) - (slo < b0), kh = k + (shi >= b1) - (shi < b0);
+  if (!(slo >= sh->b[k - 1] && shi < sh->b[k + 2])) {
+    kl = cg_interval(sh, slo);
+    kh = cg_interval(sh, shi);
+  }
+  o->mode = CG_SH_WALK;
+  o->delta = 0;
+  if (kl == kh) {
+    const int sj = sh->shell_of[kl + 1];
+    if (sj - j >= -1 && sj - j <= 1) {
+      o->mode = CG_SH_SINGLE;
+      o->delta = sj - j;
+    }
+  } else if (kh == kl + 1 && kl - j >= -1 && kl - j <= 1) {
+    o->mode = CG_SH_EDGE;
+    o->delta = kl - j;
+  }
+  return 1;
+}
+
 /* The cell in double (imap.c:184-208): 0 when not painted, 1 with the shell
  * of its corner radius (*j) and the radial shift (*drr). */
 CG_HD int cgx_imap_cell(const cg_imap_args *a, int ix, int iy, int iz, const float v[3], int *j, double *drr)
@@ -1242,6 +1373,204 @@ CG_HD void cgx_imap_sample(const cg_imap_args *a, int ix, int iy, int iz, int ns
   cgx_cart2sph(x, y, z, &r, &cth, &phi);
   *s = a->sh.shell_of[cgx_interval(&a->sh, X_ADD(r, drr)) + 1];
   if (*s >= 0 && *s < a->sh.nr) *pix = cgx_ang2pix(a->nside, cth, phi);
+}
+
+/* ---- Cells whose samples share region, octant and shell edge ------------- */
+
+/* Most cells lie in one octant of phi, on one side of |cos theta| = 2/3 and
+ * of the polar axis' planes, and within one shell or across one edge.  For
+ * those the quadrant, the octant's sign and the region are the cell's, and a
+ * sample's decision is what remains of cg_imap_decide: the octant angle, the
+ * RING coordinates and their floors, with bounds that hold for every such
+ * cell.  A floor comes from adding 1.5 2^23 to x - 1/2, which rounds it to
+ * floor(x), and leaves d = x - 1/2 - floor(x) in [-1/2, 1/2]: x keeps its
+ * distance e to the integers while |d| < 1/2 - e. */
+#define CG_CELL_GENERAL 0
+#define CG_CELL_EQ 1    /* |cos theta| < 2/3 */
+#define CG_CELL_POLAR 2
+
+/* The cells lie 8 cells or more from the observer, where cg_imap_decide's
+ * coordinate error 1.8 2^-24 (1 + 2 dx / r) is at most this. */
+#define CG_CELL_EIN (2.3f * CG_E24)
+
+CG_HD int cg_cell_class(const cg_imap_args *a, const cg_imap_cell *c, float xc, float yc, float zc)
+{
+  const float dx = a->dx;
+  if (c->mode != CG_SH_SINGLE && c->mode != CG_SH_EDGE) return CG_CELL_GENERAL;
+  if (c->mode == CG_SH_EDGE) { /* both sides painted */
+    const int s0 = a->sh.shell_of[c->j + c->delta + 1], s1 = a->sh.shell_of[c->j + c->delta + 2];
+    if (s0 < 0 || s1 < 0 || s0 >= a->sh.nr || s1 >= a->sh.nr) return CG_CELL_GENERAL;
+  }
+  /* |x|, |y|, |z| of the sample centres lie strictly within [mn, mx] */
+  const float xh = CG_ADD(xc, dx), yh = CG_ADD(yc, dx), zh = CG_ADD(zc, dx);
+  const float mnx = cg_max_nn(xc, -xh), mxx = cg_max_nn(-xc, xh);
+  const float mny = cg_max_nn(yc, -yh), mxy = cg_max_nn(-yc, yh);
+  const float mnz = cg_max_nn(cg_max_nn(zc, -zh), 0.0f), mxz = cg_max_nn(-zc, zh);
+  if (!(cg_min_nn(mnx, mny) > CG_MUL(1e-4f, dx))) return CG_CELL_GENERAL; /* one quadrant of phi */
+  if (!(mny >= mxx || mnx >= mxy)) return CG_CELL_GENERAL;                /* one octant */
+  const float rl2 = CG_FMA(mnx, mnx, CG_MUL(mny, mny)), rh2 = CG_FMA(mxx, mxx, CG_MUL(mxy, mxy));
+  const float d2 = CG_MUL(dx, dx);
+  if (!(CG_FMA(mnz, mnz, rl2) > CG_MUL(64.01f, d2))) return CG_CELL_GENERAL;
+  /* region: 5 z^2 against 4 rho^2 with 2e-5 to spare (1.8e-6 of cos theta) */
+  if (CG_MUL(5.0f, CG_MUL(mxz, mxz)) < CG_MUL(3.99992f, rl2)) return CG_CELL_EQ;
+  /* polar cells 4 cells or more from the axis (cg_fast_polar's ip) */
+  if (CG_MUL(5.0f, CG_MUL(mnz, mnz)) > CG_MUL(4.00008f, rh2) && rl2 > CG_MUL(16.01f, d2)) return CG_CELL_POLAR;
+  return CG_CELL_GENERAL;
+}
+
+typedef struct {
+  int ymaj;           /* |y| > |x| */
+  float fb, fs;       /* equatorial: nside (1/2 + f) - 1/2 = fb + fs g; polar: f = fb + fs g */
+  float drr, B, eB;   /* shell: r + drr against the edge B within eB */
+  int s0, s1;         /* shells below and above B */
+  int q, c0, c1;      /* integer constants of the pixel (q: the quadrant, or nside + 1) */
+} cg_imap_fast;
+
+/* The constants of a cell of class cls (CG_CELL_EQ or CG_CELL_POLAR). */
+CG_HD void cg_imap_fast_cell(const cg_imap_args *a, const cg_imap_cell *c, int cls, float xc, float yc, float zc,
+                             cg_imap_fast *F)
+{
+  const float hx = CG_MUL(0.5f, a->dx);
+  const int ymaj = cg_fabsf(CG_ADD(yc, hx)) > cg_fabsf(CG_ADD(xc, hx));
+  const int neg = (xc < 0.0f) != (yc < 0.0f);
+  const int q = (((xc < 0.0f) ? 2 : ((yc < 0.0f) ? 4 : 0)) - neg) & 3;
+  const int back = ymaj != neg; /* f = 1 - g */
+  const int nside = a->nside;
+  F->ymaj = ymaj;
+  F->drr = c->drr;
+  F->s0 = F->s1 = c->j + c->delta;
+  F->B = -3.0e38f;
+  F->eB = 0.0f;
+  if (c->mode == CG_SH_EDGE) {
+    const int kl = c->j + c->delta;
+    F->s0 = a->sh.shell_of[kl + 1];
+    F->s1 = a->sh.shell_of[kl + 2];
+    const float B = a->sh.b[kl + 1];
+    F->B = B;
+    /* cg_imap_shell_checked's bound at r <= B + |drr| + 2 dx (the cell's
+     * shifted radii lie around B) */
+    const float rh = CG_FMA(2.0f, a->dx, CG_ADD(B, cg_fabsf(c->drr)));
+    F->eB = CG_FMA(rh, 10.01f * CG_E24 + 1.0001f * CG_CELL_EIN,
+                   CG_FMA(2.01f * CG_E24, cg_fabsf(c->drr), CG_MUL(1.0001f, c->edrr)));
+  }
+  if (cls == CG_CELL_EQ) {
+    const float ns = (float)nside;
+    F->fb = CG_SUB(CG_MUL(ns, back ? 1.5f : 0.5f), 0.5f); /* exact */
+    F->fs = back ? -ns : ns;
+    /* ip = (2 nside q - nside + 2 - odd + (ua + ub - 2 0x4B400000)) >> 1 and
+     * the pixel 2 nside (nside - 1) + (ir - 1) 4 nside + ip, ir - 1 = nside + ua - ub */
+    F->c0 = (int)((unsigned)(2 * nside * q - nside + 2) - 2u * 0x4B400000u);
+    F->c1 = 2 * nside * (nside - 1) + 4 * nside * nside;
+    F->q = nside + 1; /* ir = q + irm */
+  } else {
+    F->fb = back ? 1.0f : 0.0f;
+    F->fs = back ? -1.0f : 1.0f;
+    F->q = q;
+    /* north 2 ir (ir - 1) + ip, south 12 nside^2 - 2 ir (ir + 1) + ip */
+    F->c0 = zc > 0.0f ? 2 : -2;
+    F->c1 = zc > 0.0f ? 0 : 12 * nside * nside;
+  }
+}
+
+/* 1/2 - e of the equatorial decisions: cg_pix_checked's bound at |cos theta|
+ * <= 2/3 (ecth = 2/3 8 2^-24 + 2 ein). */
+CG_HD float cg_fast_eq_thr(int nside)
+{
+  const float ecth = 5.34f * CG_E24 + 2.0f * CG_CELL_EIN;
+  return CG_SUB(0.5f, CG_FMA((float)nside, 0.751f * ecth + 1.22f * CG_CELL_EIN + 5.0e-7f, 2e-9f));
+}
+
+/* 1/2 - e = k0 - k1 tmp of the polar decisions.  cg_pix_checked: jp and jm
+ * within tmp (ef + 3 2^-24) + es, es = tmp (ecth / 2 + 2 ein / sin + 20
+ * 2^-24), ef = 2.5e-7 + 0.91 ein / sin; ip within ir (ef + 2 2^-24), ir <= tmp
+ * + 1; some roundings.  tmp / sin(theta) <= nside sqrt(3 / (5/3)), and 1 / sin
+ * alone is at most r / (4 dx) < 512. */
+#define CG_FAST_K1 (2.5e-7f + 30.0f * CG_E24 + CG_CELL_EIN)
+CG_HD float cg_fast_polar_k0(int nside)
+{
+  return CG_SUB(0.5f, CG_FMA((float)nside, 1.342f * 2.94f * CG_CELL_EIN, 0.92f * 512.0f * CG_CELL_EIN + 1e-6f));
+}
+
+/* The samples' coordinates are taken as (u, v, z), u the larger of |x| and |y|
+ * over the cell (y when F->ymaj) and v the other.  The octant angle in quarter
+ * turns, as in cg_dir_of. */
+CG_HD float cg_fast_angle(float u, float v)
+{
+  return cg_atan01_q(CG_MUL(cg_fabsf(v), cg_rcp_fast(cg_fabsf(u))));
+}
+
+/* Equatorial sample of the cell: 1 with its pixel when the margins hold;
+ * *above is set when it lies in the shell above B.  vz2 = v^2 + z^2.  Errors
+ * as in cg_pix_checked: r^2 three roundings, cos(theta) 8 2^-24 relative;
+ * nside (1/2 + f) and the two fused multiply-adds 1.8e-7 nside. */
+CG_HD int cg_fast_eq(const cg_imap_fast *F, int nside, float thr, float u, float v, float z, float vz2, int *above,
+                     int *pix)
+{
+  const float M = 12582912.0f;
+  const float r2 = CG_FMA(u, u, vz2);
+  const float rinv = cg_rsqrt_fast(r2);
+  const float cth = CG_MUL(z, rinv);
+  const float db = CG_SUB(CG_FMA(r2, rinv, F->drr), F->B);
+  *above = db >= 0.0f;
+  const float h = CG_FMA(F->fs, cg_fast_angle(u, v), F->fb);
+  const float n34 = CG_MUL(0.75f, (float)nside);
+  const float A = CG_FMA(-n34, cth, h), B = CG_FMA(n34, cth, h);
+  const float ta = CG_ADD(A, M), tb = CG_ADD(B, M);
+  const float da = CG_SUB(A, CG_SUB(ta, M)), dbb = CG_SUB(B, CG_SUB(tb, M));
+  const unsigned ua = cg_f2u(ta), ub = cg_f2u(tb);
+  const int irm = (int)(ua - ub);                  /* ir - 1 - nside */
+  const unsigned odd = (unsigned)(irm + F->q) & 1u; /* ir & 1 */
+  int ip = (int)((unsigned)F->c0 + ua + ub - odd) >> 1;
+  const int m = 4 * nside;
+  if (ip >= m) ip -= m;
+  *pix = F->c1 + irm * m + ip;
+  return cg_max_nn(cg_fabsf(da), cg_fabsf(dbb)) < thr && cg_fabsf(db) > F->eB;
+}
+
+/* What the samples of a polar cell on one line along z share: rho^2,
+ * nside sqrt(3) rho^2, and f and 1 - f. */
+typedef struct {
+  float rho2, c, f, f1;
+} cg_fast_line;
+
+CG_HD cg_fast_line cg_fast_polar_line(const cg_imap_fast *F, int nside, float u, float v)
+{
+  cg_fast_line o;
+  o.rho2 = CG_FMA(u, u, CG_MUL(v, v));
+  o.c = CG_MUL(CG_MUL(1.7320508075688772f, (float)nside), o.rho2);
+  const float g = cg_fast_angle(u, v);
+  o.f = CG_FMA(F->fs, g, F->fb);
+  o.f1 = CG_FMA(-F->fs, g, CG_SUB(1.0f, F->fb));
+  return o;
+}
+
+/* Polar sample: tmp = nside sqrt(3 (1 - |cos theta|)) = nside sqrt(3) rho^2 /
+ * sqrt(rho^2 (r^2 + |z| r)), within 15 2^-24 relative (rho^2 two roundings,
+ * r^2 three, r 6.5, the sum 7.5, the product 10.5; rsqrt 2^-22). */
+CG_HD int cg_fast_polar(const cg_imap_fast *F, const cg_fast_line *l, float k0, float z, int *above, int *pix)
+{
+  const float M = 12582912.0f;
+  const float r2 = CG_FMA(z, z, l->rho2);
+  const float r = CG_MUL(r2, cg_rsqrt_fast(r2));
+  const float db = CG_SUB(CG_ADD(r, F->drr), F->B);
+  *above = db >= 0.0f;
+  const float w = CG_FMA(cg_fabsf(z), r, r2);
+  const float tmp = CG_MUL(l->c, cg_rsqrt_fast(CG_MUL(l->rho2, w)));
+  const float p1 = CG_FMA(l->f, tmp, -0.5f), p2 = CG_FMA(l->f1, tmp, -0.5f);
+  const float t1 = CG_ADD(p1, M), t2 = CG_ADD(p2, M);
+  const float n1 = CG_SUB(t1, M), n2 = CG_SUB(t2, M);
+  const float fir = CG_ADD(CG_ADD(n1, n2), 1.0f); /* ir, exact */
+  const float p3 = CG_FMA(l->f, fir, -0.5f);
+  const float t3 = CG_ADD(p3, M);
+  const float d3 = CG_SUB(p3, CG_SUB(t3, M));
+  const int ir = (int)(cg_f2u(t1) + cg_f2u(t2) - (2u * 0x4B400000u - 1u));
+  int ip = F->q * ir + (int)(cg_f2u(t3) - 0x4B400000u);
+  const int m = 4 * ir;
+  if (ip >= m) ip -= m;
+  *pix = F->c1 + (F->c0 * ir - 2) * ir + ip;
+  return cg_max_nn(cg_max_nn(cg_fabsf(CG_SUB(p1, n1)), cg_fabsf(CG_SUB(p2, n2))), cg_fabsf(d3)) <
+             CG_FMA(-CG_FAST_K1, tmp, k0) &&
+         cg_fabsf(db) > F->eB;
 }
 
 /* ---- The float-float tier ---------------------------------------------- */

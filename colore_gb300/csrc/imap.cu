@@ -13,26 +13,42 @@
  * the hit counts are those of the double arithmetic.
  *
  * nsub is fixed by the shell of the cell's corner radius and grows towards
- * the observer (from 2 at high redshift to ~20 for the nearest shells), so
- * cells are listed per shell -- one bucket per shell, holding cells of one
- * nsub -- and painted bucket after bucket:
+ * the observer (from 2 at high redshift to ~20 for the nearest shells), and
+ * a cell's class says which loop its samples need (cg_cell_class), so cells
+ * are listed per shell and class -- one bucket each, holding cells of one
+ * nsub and one loop -- and painted bucket after bucket:
  *
+ *   k_imap_tab     The radial tables as one 32-byte record per segment.
  *   k_imap_list    Warps take groups of rows from a counter; a lane decides
  *                  one cell (listed or not, its shell, brightness, radial
  *                  shift, and whether all its samples certainly stay in one
- *                  shell, which spares them the radial test) and appends it
- *                  to its bucket: one atomic per bucket present in the warp,
- *                  all issued together.  A cell that finds its bucket full is
- *                  painted by its warp on the spot.
- *   k_imap_chunks  One thread cuts each bucket into chunks of about CHS
+ *                  shell or straddle one edge) from one segment record
+ *                  (cg_imap_cell_seg) and appends it to its bucket: one atomic
+ *                  per bucket present in the warp, all issued together, on
+ *                  counters that have a 128-byte line each (next to each other
+ *                  they sat in one L2 slice, whose atomics bounded the kernel:
+ *                  65 against 54 ms of the stage at 1024^3).  A cell that finds
+ *                  its bucket full is painted by its warp on the spot.
+ *                  456 thread-instructions a cell in range where a lookup with
+ *                  a bound per table took 689: 20.6 -> 13 ms at 1024^3.
+ *   k_imap_chunks  One block cuts each bucket into chunks of about CHS
  *                  samples: whole cells, or slices of one cell.
  *   k_imap_paint   Warps take chunks in bucket order, so the maps' working
- *                  set at any time is a few shells (25 MB per shell at nside
+ *                  set at any time is a few shells (50 MB per shell at nside
  *                  512) and the atomics stay in L2.  Each lane walks one unit
- *                  sample by sample, keeping two (key, count) run slots that
- *                  it evicts with one float and one integer atomic.  Samples
- *                  whose margins fail are staged per warp in shared memory
- *                  and queued in batches.
+ *                  sample by sample, keeping a (key, count) run that it adds to
+ *                  the maps with one two-float reduction.  Cells within one
+ *                  octant, one of the two pixel regions and one shell or edge
+ *                  -- all but the layers on the octants' planes, the cones
+ *                  |cos theta| = 2/3 and the nearest cells -- have these
+ *                  decisions taken once per cell and walk along the line of
+ *                  sight, where the pixel changes least.  Samples whose margins
+ *                  fail are staged per warp in shared memory and queued in
+ *                  batches.  Bound by instruction issue (90 % of the slots): 100
+ *                  thread-instructions a sample where deciding everything per
+ *                  sample took 177, 79 -> 37 ms for the 1.3e10 samples at
+ *                  1024^3; scalar atomics instead of the two-float reduction
+ *                  cost 5.5 ms of it.
  *   k_imap_double  The queued samples: first in float-float, then, for the
  *                  few left, gathered per warp and decided in double 32 at a
  *                  time, the cell's radial shift computed once per run of
@@ -57,14 +73,15 @@ constexpr unsigned F_DOUBLE = 16u; /* flags: mode (2 bits), delta + 1 (2 bits), 
 
 /* Per-block copies of the species' shell tables. */
 struct Sh {
-  float *b, *dxs, *invns;
+  float *b; /* with two sentinels on either side */
+  float *dxs, *invns;
   int *shell_of, *nsub;
   unsigned long long *chunk_off;
 };
 
 __host__ __device__ __forceinline__ size_t shell_smem(int nr, int nbk, bool chunks)
 {
-  size_t n = (size_t)(2 * nr) * 4 + (size_t)(2 * nr + 1) * 4 + 3 * (size_t)(nr + 2) * 4;
+  size_t n = (size_t)(2 * nr + 4) * 4 + (size_t)(2 * nr + 1) * 4 + 3 * (size_t)(nr + 2) * 4;
   n = (n + 7) & ~(size_t)7;
   if (chunks) n += (size_t)(nbk + 1) * 8;
   return n;
@@ -75,8 +92,8 @@ __device__ __forceinline__ Sh shells_at(const cg_imap_params &p, unsigned char *
 {
   const int nr = p.nr;
   Sh s;
-  s.b = reinterpret_cast<float *>(raw);
-  s.shell_of = reinterpret_cast<int *>(s.b + 2 * nr);
+  s.b = reinterpret_cast<float *>(raw) + 2;
+  s.shell_of = reinterpret_cast<int *>(s.b + 2 * nr + 2);
   s.nsub = s.shell_of + 2 * nr + 1;
   s.dxs = reinterpret_cast<float *>(s.nsub + nr + 2);
   s.invns = s.dxs + nr + 2;
@@ -86,7 +103,7 @@ __device__ __forceinline__ Sh shells_at(const cg_imap_params &p, unsigned char *
 
 /* The painting warps' queue stages follow the tables. */
 __host__ __device__ __forceinline__ size_t paint_stage_off(int nr, int nbk) { return (shell_smem(nr, nbk, true) + 15) & ~(size_t)15; }
-__host__ __device__ __forceinline__ size_t paint_smem(int nr, int nbk) { return paint_stage_off(nr, nbk) + (size_t)IW * QB * 8; }
+__host__ __device__ __forceinline__ size_t paint_smem(int nr, int nbk) { return paint_stage_off(nr, nbk) + (size_t)IW * (QB * 8 + 4); }
 /* The double pass keeps the buckets' bases where the painting keeps its
  * chunk table; its per-warp gathers (64 entries) follow. */
 __host__ __device__ __forceinline__ size_t double_stage_off(int nr, int nbk) { return (shell_smem(nr, nbk, true) + 15) & ~(size_t)15; }
@@ -95,7 +112,8 @@ __device__ __forceinline__ Sh load_shells(const cg_imap_params &p, unsigned char
 {
   const int nb = p.a.sh.nb, nr = p.nr;
   const Sh s = shells_at(p, raw);
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s.b[i] = p.a.sh.b[i];
+  for (int i = (int)threadIdx.x - 2; i < nb + 2; i += blockDim.x)
+    s.b[i] = i < 0 ? -3.0e38f : (i < nb ? p.a.sh.b[i] : 3.0e38f);
   for (int i = threadIdx.x; i <= nb; i += blockDim.x) s.shell_of[i] = p.a.sh.shell_of[i];
   for (int i = threadIdx.x; i < nr + 2; i += blockDim.x) {
     s.nsub[i] = p.a.nsub[i];
@@ -131,9 +149,23 @@ __device__ __forceinline__ K key_of(const cg_imap_params &p, int s, long long pi
   return (K)((long long)s * p.npix + pix);
 }
 
+/* n samples of summed brightness t on pixel k of the maps: one two-float
+ * reduction when the counts are floats (p.packed), which halves the L2's
+ * atomic operations, else a float and an integer one. */
+__device__ __forceinline__ void add_to(const cg_imap_params &p, long long k, float t, float n)
+{
+  float2 *a = p.acc + k;
+  if (p.packed) {
+    asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(a), "f"(t), "f"(n) : "memory");
+  } else {
+    atomicAdd(&a->x, t);
+    atomicAdd(reinterpret_cast<int *>(&a->y), (int)n);
+  }
+}
+
 /* The lanes hold consecutive samples: each run of equal (tag, key) is added
- * to the maps once, by its first lane, with its length (data += temp * run,
- * nadd += run).  tag separates cells, whose brightness differs. */
+ * to the maps once, by its first lane, with its length (sum += temp * run,
+ * count += run).  tag separates cells, whose brightness differs. */
 template <typename K>
 __device__ __forceinline__ void add_runs(K key, int tag, float temp, int lane, const cg_imap_params &p)
 {
@@ -145,9 +177,8 @@ __device__ __forceinline__ void add_runs(K key, int tag, float temp, int lane, c
   if (head) {
     const unsigned above = lane == 31 ? 0u : bnd & (FULL << (lane + 1));
     const int end = above ? __ffs(above) - 1 : 32;
-    const unsigned int c = (unsigned int)(end - lane);
-    atomicAdd(&p.data[(long long)key], CG_MUL(temp, (float)c));
-    atomicAdd(&p.nadd[(long long)key], (int)c);
+    const float c = (float)(end - lane);
+    add_to(p, (long long)key, CG_MUL(temp, c), c);
   }
 }
 
@@ -222,10 +253,10 @@ __device__ __forceinline__ cg_imap_cell unpack(const cg_imap_rec &r, int j, int 
 /* A sample of a cell the listing kernel paints itself: its double decision,
  * when needed, on the spot. */
 template <typename K>
-__device__ __noinline__ K sample_key_inline(const cg_imap_params &p, const cg_imap_args &A, const float *phi, int ix,
-                                            int iy, int iz, const cg_imap_cell &c, int dbl, int ns, int q,
-                                            float inv_ns)
+__device__ __noinline__ K sample_key_inline(const cg_imap_params &p, const float *phi, int ix, int iy, int iz,
+                                            const cg_imap_cell &c, int dbl, int ns, int q, float inv_ns)
 {
+  const cg_imap_args &A = p.a;
   int sx, sy, sz, s = -1;
   long long pix = 0;
   sub_of(q, ns, inv_ns, &sx, &sy, &sz);
@@ -241,9 +272,56 @@ __device__ __noinline__ K sample_key_inline(const cg_imap_params &p, const cg_im
   return key_of<K>(p, s, pix);
 }
 
+/* The listing's table segments, with this realisation's normalisation. */
+__global__ void __launch_bounds__(32) k_imap_tab(cg_imap_params p)
+{
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  float eg = 0.0f;
+  if (i < p.a.na - 1) p.seg[i] = cg_imap_seg_make(&p.a, i, &eg);
+  /* non-negative floats order like their bits */
+  const unsigned m = __reduce_max_sync(FULL, __float_as_uint(eg));
+  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned *>(p.seg + p.a.na - 1), m);
+}
+
+/* A cell that the segments leave open: with a bound per lookup
+ * (cg_imap_cell_checked), then in double.  Out of line: rare, and long. */
+struct OpenCell {
+  cg_imap_cell c;
+  int st, dbl, in_double;
+};
+
+__device__ __noinline__ OpenCell cell_open(const cg_imap_params &p, int ix, int iy, int iz, float d, float v0, float v1,
+                                           float v2)
+{
+  const cg_imap_args &A = p.a;
+  OpenCell o;
+  const float v[3] = {v0, v1, v2};
+  o.dbl = o.in_double = 0;
+  o.st = cg_imap_cell_checked(&A, ix, iy, iz, d, v, &o.c);
+  if (p.force_double && o.st == 1) o.st = 2;
+  if (o.st == 2) {
+    o.in_double = 1;
+    int j;
+    double drr;
+    o.st = 0;
+    if (cgx_imap_cell(&A, ix, iy, iz, v, &j, &drr)) {
+      o.c.j = j;
+      o.c.temp = temp32(A, ix, iy, iz, d);
+      o.c.drr = (float)drr;
+      o.c.edrr = 0.0f;
+      o.c.mode = CG_SH_WALK;
+      o.c.delta = 0;
+      o.dbl = o.st = 1;
+    }
+  }
+  return o;
+}
+
+/* 8 blocks per SM (64 registers, some spilled): 5 and 6 without most of the
+ * spills took 1.5 and 1.6 ms more of the stage's 52.5 at 1024^3. */
 template <typename K>
-__global__ void __launch_bounds__(IW * 32) k_imap_list(const float *__restrict__ dens, const float *__restrict__ phi,
-                                                       cg_imap_params p)
+__global__ void __launch_bounds__(IW * 32, 8) k_imap_list(const float *__restrict__ dens, const float *__restrict__ phi,
+                                                               const __grid_constant__ cg_imap_params p)
 {
   extern __shared__ __align__(16) unsigned char sraw[];
   const Sh sh = load_shells(p, sraw, false);
@@ -251,8 +329,12 @@ __global__ void __launch_bounds__(IW * 32) k_imap_list(const float *__restrict__
   const cg_imap_args A = args_with(p, sh);
   const int lane = threadIdx.x & 31;
   const int N = p.box.N;
-  const int nrow = N * N, nch = (N + 31) / 32;
+  const int nrow = N * N, nch = N / 32; /* N is a multiple of 32 */
   const float rlo = A.rmin - 1.0f, rhi = A.rmax + 1.0f;
+  const float rlo2 = rlo > 0.0f ? rlo * rlo : 0.0f, rhi2 = rhi * rhi;
+  const int ngx = 2 * (N / 2 + 1);
+  const long long plane = (long long)ngx * N;
+  const float eg = __uint_as_float(*reinterpret_cast<const unsigned *>(p.seg + A.na - 1));
   unsigned long long drawn = 0, ndbl = 0;
   for (;;) {
     int rbeg = 0;
@@ -260,46 +342,40 @@ __global__ void __launch_bounds__(IW * 32) k_imap_list(const float *__restrict__
     rbeg = __shfl_sync(FULL, rbeg, 0);
     if (rbeg >= nrow) break;
     const int rend = rbeg + ROWS < nrow ? rbeg + ROWS : nrow;
-    for (int row = rbeg; row < rend; row++)
+    for (int row = rbeg; row < rend; row++) {
+      const int iz = (int)divN(row, p.box), iy = row - iz * N;
+      const float y0 = A.yc[iy], z0 = A.zc[iz];
+      const float yz2 = CG_FMA(z0, z0, CG_MUL(y0, y0));
+      if (yz2 > rhi2) continue;
+      const long long r0 = (long long)row * ngx;
+      const int oyh = iy == N - 1 ? -(N - 1) * ngx : ngx, oyl = iy == 0 ? (N - 1) * ngx : -ngx;
+      const long long ozh = iz == N - 1 ? -(N - 1) * plane : plane, ozl = iz == 0 ? (N - 1) * plane : -plane;
       for (int ch = 0; ch < nch; ch++) {
-        const int iz = row / N, iy = row - iz * N;
         const int ix = ch * 32 + lane;
         cg_imap_cell c;
         bool want = false; /* listed and painted */
         int dbl = 0;
-        float d = 0.0f;
-        if (ix < N) {
-          const float x0 = A.xc[ix], y0 = A.yc[iy], z0 = A.zc[iz];
-          const float r2 = CG_FMA(z0, z0, CG_FMA(y0, y0, CG_MUL(x0, x0)));
-          if (r2 >= rlo * rlo * (rlo > 0.0f ? 1.0f : 0.0f) && r2 <= rhi * rhi) {
-            d = __ldg(&dens[pidx(ix, iy, iz, N)]);
-            float v[3];
-            grad_phi(phi, ix, iy, iz, N, v);
-            int st = cg_imap_cell_checked(&A, ix, iy, iz, d, v, &c);
-            if (p.force_double && st == 1) st = 2;
-            if (st == 2) {
-              ndbl++;
-              int j;
-              double drr;
-              if (cgx_imap_cell(&A, ix, iy, iz, v, &j, &drr)) {
-                c.j = j;
-                c.temp = temp32(A, ix, iy, iz, d);
-                c.drr = (float)drr;
-                c.edrr = 0.0f;
-                c.mode = CG_SH_WALK;
-                c.delta = 0;
-                dbl = 1;
-                st = 1;
-              } else {
-                st = 0;
-              }
-            }
-            if (st == 1) {
-              const int ns = A.nsub[c.j + 1];
-              drawn += (unsigned long long)ns * ns * ns;
-              const int sfin = c.j + c.delta;
-              want = !(c.mode == CG_SH_SINGLE && (sfin < 0 || sfin >= p.nr));
-            }
+        const float x0 = A.xc[ix];
+        const float r2 = CG_FMA(x0, x0, yz2);
+        if (r2 >= rlo2 && r2 <= rhi2) {
+          const float d = __ldg(dens + r0 + ix);
+          const float *f = phi + r0 + ix;
+          /* centred potential differences (get_rvel, imap.c:43-74) */
+          const float v[3] = {CG_SUB(__ldg(f + (ix == N - 1 ? 1 - N : 1)), __ldg(f + (ix == 0 ? N - 1 : -1))),
+                              CG_SUB(__ldg(f + oyh), __ldg(f + oyl)), CG_SUB(__ldg(f + ozh), __ldg(f + ozl))};
+          int st = p.force_double ? 2 : cg_imap_cell_seg(p.seg, eg, &A, x0, y0, z0, r2, d, v, &c);
+          if (st == 2) {
+            const OpenCell o = cell_open(p, ix, iy, iz, d, v[0], v[1], v[2]);
+            c = o.c;
+            dbl = o.dbl;
+            st = o.st;
+            ndbl += o.in_double;
+          }
+          if (st == 1) {
+            const int ns = A.nsub[c.j + 1];
+            drawn += (unsigned long long)ns * ns * ns;
+            const int sfin = c.j + c.delta;
+            want = !(c.mode == CG_SH_SINGLE && (sfin < 0 || sfin >= p.nr));
           }
         }
         /* nothing to append (a chunk outside the shells' radial range, about
@@ -309,11 +385,15 @@ __global__ void __launch_bounds__(IW * 32) k_imap_list(const float *__restrict__
          * issued together by each bucket's first lane (one round trip) */
         bool over = false;
         long long slot = 0;
-        const int bk = want ? c.j + 1 : -1;
+        int bk = -1;
+        if (want) {
+          const int cls = dbl ? CG_CELL_GENERAL : cg_cell_class(&A, &c, x0, y0, z0);
+          bk = CG_IMAP_CLASSES * (c.j + 1) + cls;
+        }
         const unsigned same = __match_any_sync(FULL, bk);
         const int leader = __ffs(same) - 1;
         unsigned long long old = 0;
-        if (want && lane == leader) old = atomicAdd(&p.cnt[bk], (unsigned long long)__popc(same));
+        if (want && lane == leader) old = atomicAdd(&p.cnt[(size_t)bk * CG_IMAP_CNT], (unsigned long long)__popc(same));
         old = __shfl_sync(FULL, old, leader);
         if (want) {
           const long long k = (long long)old + __popc(same & ((1u << lane) - 1u));
@@ -343,12 +423,13 @@ __global__ void __launch_bounds__(IW * 32) k_imap_list(const float *__restrict__
           for (int q0 = 0; q0 < n3; q0 += 32) {
             const int q = q0 + lane;
             K key = empty_key<K>();
-            if (q < n3) key = sample_key_inline<K>(p, A, phi, cx, iy, iz, cc, cd, ns, q, inv);
+            if (q < n3) key = sample_key_inline<K>(p, phi, cx, iy, iz, cc, cd, ns, q, inv);
             add_runs(key, tag, cc.temp, lane, p);
           }
           if (lane == 0) atomicAdd(&p.ctr[3], (unsigned long long)n3);
         }
       }
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -362,8 +443,8 @@ __global__ void __launch_bounds__(IW * 32) k_imap_list(const float *__restrict__
 }
 
 /* Work units of a bucket of nsub ns: whole cells for ns <= 4 (8 to 64
- * samples), one z-slab of a cell for ns <= 32 (ns^2 samples), one x-line
- * beyond; each lane of a warp walks one unit. */
+ * samples), one slab of a cell for ns <= 32 (ns^2 samples), one line beyond;
+ * each lane of a warp walks one unit. */
 __host__ __device__ __forceinline__ long long units_per_cell(int ns)
 {
   return ns <= 4 ? 1 : (ns <= 32 ? ns : (long long)ns * ns);
@@ -378,20 +459,48 @@ __host__ __device__ __forceinline__ int groups_per_chunk(int ns)
   return g > 1 ? g : 1;
 }
 
-/* Chunks of every bucket: 32 G units each. */
-__global__ void k_imap_chunks(cg_imap_params p)
+/* Chunks of every bucket, 32 G units each, and their running sum: one block,
+ * a bucket per thread. */
+__global__ void __launch_bounds__(1024) k_imap_chunks(cg_imap_params p)
 {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned long long acc = 0;
-  for (int b = 0; b < p.nbk; b++) {
-    p.chunk_off[b] = acc;
-    const unsigned long long n = p.cnt[b] < (unsigned long long)p.cap[b] ? p.cnt[b] : (unsigned long long)p.cap[b];
-    const int ns = p.a.nsub[b];
-    const unsigned long long nu = n * (unsigned long long)units_per_cell(ns);
-    const unsigned long long per = 32ull * (unsigned long long)groups_per_chunk(ns);
-    acc += (nu + per - 1) / per;
+  __shared__ unsigned long long ws[33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long carry = 0;
+  for (int b0 = 0; b0 < p.nbk; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    unsigned long long x = 0;
+    if (b < p.nbk) {
+      const unsigned long long n = p.cnt[(size_t)b * CG_IMAP_CNT] < (unsigned long long)p.cap[b] ? p.cnt[(size_t)b * CG_IMAP_CNT] : (unsigned long long)p.cap[b];
+      const int ns = p.a.nsub[b / CG_IMAP_CLASSES];
+      const unsigned long long nu = n * (unsigned long long)units_per_cell(ns);
+      const unsigned long long per = 32ull * (unsigned long long)groups_per_chunk(ns);
+      x = (nu + per - 1) / per;
+    }
+    unsigned long long inc = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) ws[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+      const unsigned long long y = ws[lane];
+      unsigned long long yi = y;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(FULL, yi, o);
+        if (lane >= o) yi += t;
+      }
+      ws[lane] = yi - y;
+      if (lane == 31) ws[32] = yi;
+    }
+    __syncthreads();
+    if (b < p.nbk) p.chunk_off[b] = carry + ws[w] + inc - x;
+    carry += ws[32];
+    __syncthreads();
   }
-  p.chunk_off[p.nbk] = acc;
+  if (threadIdx.x == 0) p.chunk_off[p.nbk] = carry;
 }
 
 /* One sample for the double pass, queued on its own. */
@@ -402,83 +511,166 @@ __device__ __noinline__ void queue_one(const cg_imap_params &p, long long rec, i
   else atomicOr(p.err, ERR_IMAP_QUEUE);
 }
 
-/* This warp's queue stage in the painting kernel's shared memory. */
-__device__ __forceinline__ unsigned long long *stage_of(const cg_imap_params &p)
+/* This warp's queue stage in the painting kernel's shared memory: QB entries
+ * and their number. */
+struct Stage {
+  unsigned long long *e;
+  int *n;
+};
+
+__device__ __forceinline__ Stage stage_of(const cg_imap_params &p)
 {
   extern __shared__ __align__(16) unsigned char sraw[];
-  return reinterpret_cast<unsigned long long *>(sraw + paint_stage_off(p.nr, p.nbk)) + (size_t)(threadIdx.x >> 5) * QB;
+  unsigned char *b = sraw + paint_stage_off(p.nr, p.nbk);
+  const int w = threadIdx.x >> 5;
+  return Stage{reinterpret_cast<unsigned long long *>(b) + (size_t)w * QB,
+               reinterpret_cast<int *>(b + (size_t)IW * QB * 8) + w};
 }
 
-/* The warp's staged queue entries (qn of them, in shared memory) to the
- * double queue: one atomic per QB - 128 or more entries. */
-__device__ __forceinline__ void queue_flush(const cg_imap_params &p, const unsigned long long *qb, int qn, int lane)
+/* One sample for the double pass: staged per warp, or queued at once when the
+ * stage is full. */
+__device__ __noinline__ void hold(const cg_imap_params &p, long long rec, int q)
 {
+  const Stage S = stage_of(p);
+  const int k = atomicAdd(S.n, 1);
+  if (k < QB) S.e[k] = ((unsigned long long)rec << 30) | (unsigned long long)q;
+  else queue_one(p, rec, q);
+}
+
+/* The warp's stage to the queue, with one atomic, once it holds min_n. */
+__device__ __forceinline__ void queue_flush(const cg_imap_params &p, int min_n, int lane)
+{
+  const Stage S = stage_of(p);
   __syncwarp();
+  const int qn = *S.n < QB ? *S.n : QB;
+  if (qn < min_n) return;
   unsigned long long q0 = 0;
   if (lane == 0) q0 = atomicAdd(&p.ctr[4], (unsigned long long)qn);
   q0 = __shfl_sync(FULL, q0, 0);
   for (int i = lane; i < qn; i += 32) {
-    if ((long long)(q0 + i) < p.queue_cap) p.queue[q0 + i] = qb[i];
+    if ((long long)(q0 + i) < p.queue_cap) p.queue[q0 + i] = S.e[i];
     else atomicOr(p.err, ERR_IMAP_QUEUE);
   }
+  __syncwarp();
+  if (lane == 0) *S.n = 0;
   __syncwarp();
 }
 
 /* Add a run of cnt samples of brightness temp to key k. */
 template <typename K>
-__device__ __forceinline__ void flush(const cg_imap_params &p, K k, unsigned cnt, float temp)
+__device__ __forceinline__ void flush(const cg_imap_params &p, K k, float cnt, float temp)
 {
-  if (cnt) {
-    atomicAdd(&p.data[(long long)k], CG_MUL(temp, (float)cnt));
-    atomicAdd(&p.nadd[(long long)k], (int)cnt);
+  if (cnt > 0.0f) add_to(p, (long long)k, CG_MUL(temp, cnt), cnt);
+}
+
+/* What a lane carries through a unit: the pixel it is on and its run there.
+ * (A second run slot saves a third of the reductions but costs more in
+ * instructions: 67.0 against 61.7 ms of the stage at 1024^3.) */
+template <typename K>
+struct Lane {
+  K k;
+  float n; /* exact: a unit has at most 1024 samples */
+};
+
+/* A sample on key (ok), or one to hold, of index q0 + step floor(fi): another
+ * key than the run's sends the run to the maps. */
+template <typename K>
+__device__ __forceinline__ void hit(const cg_imap_params &p, Lane<K> &L, K key, bool ok, float temp, long long rec,
+                                    int q0, int step, float fi)
+{
+  if (ok && key == L.k) {
+    L.n = CG_ADD(L.n, 1.0f);
+  } else if (ok) {
+    flush<K>(p, L.k, L.n, temp);
+    L.k = key;
+    L.n = 1.0f;
+  } else {
+    hold(p, rec, q0 + step * (int)fi);
   }
 }
 
-/* One sample at float position (x, y, z), sub-cell index q, of the lane's
- * cell: added to the lane's two (key, count) slots -- a key in a slot adds to
- * it, another key evicts the older slot to the maps -- or, when only double
- * can decide it, held (up to four per unit) or queued. */
+/* One axis of a cell: its corner as a float pair. */
+struct Axis {
+  float c, l;
+};
+__device__ __forceinline__ float at(const Axis &a, float half, float dxs) { return CG_ADD(a.c, CG_FMA(half, dxs, a.l)); }
+
+/* A unit's samples, in rows along x, in the general form. */
 template <typename K>
-__device__ __forceinline__ void paint_sample(const cg_imap_params &p, const cg_imap_args &A, const cg_imap_cell &c,
-                                             int dbl, long long rec, float x, float y, float z, int q, K &k0,
-                                             unsigned &n0, K &k1, unsigned &n1, int &nf, int &f0, int &f1, int &f2,
-                                             int &f3)
+__device__ __forceinline__ void walk_general(const cg_imap_params &p, const cg_imap_args &A, const cg_imap_cell &c,
+                                             int dbl, long long rec, const Axis &ax, const Axis &ay, const Axis &az,
+                                             float dxs, int ns, int z0, int z1, int y0, int y1, Lane<K> &L)
 {
-  int s = -1;
-  long long pix = 0;
-  if (dbl || !cg_imap_decide(&A, &c, x, y, z, &s, &pix)) {
-    if (nf == 0) f0 = q;
-    else if (nf == 1) f1 = q;
-    else if (nf == 2) f2 = q;
-    else if (nf == 3) f3 = q;
-    else queue_one(p, rec, q);
-    nf++;
-    return;
+  const float fns = (float)ns;
+  for (int sz = z0; sz < z1; sz++) {
+    const float z = at(az, CG_ADD((float)sz, 0.5f), dxs);
+    for (int sy = y0; sy < y1; sy++) {
+      const float y = at(ay, CG_ADD((float)sy, 0.5f), dxs);
+#pragma unroll 1
+      for (float fi = 0.5f; fi < fns; fi = CG_ADD(fi, 1.0f)) {
+        int s = -1;
+        long long pix = 0;
+        const bool ok = !dbl && cg_imap_decide(&A, &c, at(ax, fi, dxs), y, z, &s, &pix);
+        const K key = key_of<K>(p, s, pix);
+        if (!ok || key != empty_key<K>()) hit<K>(p, L, key, ok, c.temp, rec, ns * (sy + ns * sz), 1, fi);
+      }
+    }
   }
-  const K key = key_of<K>(p, s, pix);
-  if (key == empty_key<K>()) return;
-  if (key == k0) {
-    n0++;
-  } else if (key == k1) {
-    n1++;
-  } else {
-    flush<K>(p, k1, n1, c.temp);
-    k1 = k0;
-    n1 = n0;
-    k0 = key;
-    n0 = 1;
+}
+
+/* The same for a cell of one octant, region and shell or edge
+ * (cg_imap_fast_cell), along the axis nearest the line of sight, on which
+ * consecutive samples keep their pixel longest: z in the polar caps, where the
+ * octant angle is then the line's, the larger of x and y elsewhere.  Ranges
+ * [o0, o1) and [m0, m1) of the outer and the middle axis. */
+template <typename K, bool EQ>
+__device__ __forceinline__ void walk_fast(const cg_imap_params &p, const cg_imap_fast &F, float temp, long long rec,
+                                          const Axis &x, const Axis &y, const Axis &z, float dxs, int ns, int o0, int o1,
+                                          int m0, int m1, float thr, Lane<K> &L)
+{
+  const int nside = p.a.nside;
+  const K b0 = (K)F.s0 * (K)p.npix, b1 = (K)F.s1 * (K)p.npix;
+  const float fns = (float)ns;
+  Axis u, v;
+  u.c = F.ymaj ? y.c : x.c;
+  u.l = F.ymaj ? y.l : x.l;
+  v.c = F.ymaj ? x.c : y.c;
+  v.l = F.ymaj ? x.l : y.l;
+  const int su = F.ymaj ? ns : 1, sv = F.ymaj ? 1 : ns, sz = ns * ns; /* strides of the sample index */
+  for (int o = o0; o < o1; o++) {
+    const float fo = CG_ADD((float)o, 0.5f);
+    for (int m = m0; m < m1; m++) {
+      const float fm = CG_ADD((float)m, 0.5f);
+      const int q0 = EQ ? o * sz + m * sv : o * sv + m * su;
+      if (EQ) {
+        const float zs = at(z, fo, dxs), vs = at(v, fm, dxs);
+        const float vz2 = CG_FMA(zs, zs, CG_MUL(vs, vs));
+#pragma unroll 1
+        for (float fi = 0.5f; fi < fns; fi = CG_ADD(fi, 1.0f)) {
+          int up, pix;
+          const bool ok = cg_fast_eq(&F, nside, thr, at(u, fi, dxs), vs, zs, vz2, &up, &pix);
+          hit<K>(p, L, (up ? b1 : b0) + (K)pix, ok, temp, rec, q0, su, fi);
+        }
+      } else {
+        const cg_fast_line l = cg_fast_polar_line(&F, nside, at(u, fm, dxs), at(v, fo, dxs));
+#pragma unroll 1
+        for (float fi = 0.5f; fi < fns; fi = CG_ADD(fi, 1.0f)) {
+          int up, pix;
+          const bool ok = cg_fast_polar(&F, &l, thr, at(z, fi, dxs), &up, &pix);
+          hit<K>(p, L, (up ? b1 : b0) + (K)pix, ok, temp, rec, q0, sz, fi);
+        }
+      }
+    }
   }
 }
 
 /* The G unit groups of one chunk of bucket b (nsub ns).  Each lane walks one
- * unit (a cell, a slab or a line) sample by sample with its row coordinates
- * and the cell's fields held in registers.  Every lane of a warp runs the same sample loop,
- * so the samples that only double can decide are staged per warp in shared
- * memory (qb, qn entries) and queued in batches. */
+ * unit (a cell, a slab or a line) sample by sample.  The samples that only
+ * double can decide are staged per warp in shared memory and queued in
+ * batches. */
 template <typename K>
 __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_imap_args &A, int b, int ns,
-                                            unsigned long long u0, int G, unsigned long long nu, float dxs, int lane,
-                                            int &qn)
+                                            unsigned long long u0, int G, unsigned long long nu, float dxs, int lane)
 {
   const int U = (int)units_per_cell(ns);
   /* the chunk's first unit as (record, unit within it); later units are
@@ -488,9 +680,9 @@ __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_im
   for (int g = 0; g < G; g++) {
     const unsigned long long u = u0 + (unsigned long long)g * 32ull + (unsigned long long)lane;
     const bool valid = u < nu;
-    /* the unit: record and its range of (sz, sy) */
+    /* the unit: record and its ranges of the outer and the middle axis */
     long long rl = 0;
-    int z0 = 0, z1 = ns, y0 = 0, y1 = ns;
+    int o0 = 0, o1 = ns, m0 = 0, m1 = ns;
     if (valid) {
       if (U == 1) {
         rl = (long long)u;
@@ -500,87 +692,50 @@ __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_im
         const int w = (int)(t - dr * (unsigned)U);
         rl = r0 + (long long)dr;
         if (ns <= 32) {
-          z0 = w;
-          z1 = w + 1;
+          o0 = w;
+          o1 = w + 1;
         } else {
-          z0 = w / ns;
-          z1 = z0 + 1;
-          y0 = w - z0 * ns;
-          y1 = y0 + 1;
+          o0 = w / ns;
+          o1 = o0 + 1;
+          m0 = w - o0 * ns;
+          m1 = m0 + 1;
         }
       }
     }
     const long long rec = p.base[b] + rl;
-    cg_imap_cell c;
-    int ix = 0, iy = 0, iz = 0, dbl = 0;
-    float xc = 0.0f, xl = 0.0f, yc = 0.0f, yl = 0.0f, zc = 0.0f, zl = 0.0f;
+    float temp = 0.0f;
+    Lane<K> L;
+    L.k = empty_key<K>();
+    L.n = 0.0f;
     if (valid) {
-      c = unpack(p.recs[rec], b - 1, &ix, &iy, &iz, &dbl);
+      int ix, iy, iz, dbl;
+      const cg_imap_cell c = unpack(p.recs[rec], b / CG_IMAP_CLASSES - 1, &ix, &iy, &iz, &dbl);
       dbl |= p.force_double;
-      xc = A.xc[ix];
-      xl = A.xl[ix];
-      yc = A.yc[iy];
-      yl = A.yl[iy];
-      zc = A.zc[iz];
-      zl = A.zl[iz];
-    } else {
-      c.temp = 0.0f;
-      c.drr = 0.0f;
-      c.edrr = 0.0f;
-      c.j = b - 1;
-      c.mode = CG_SH_SINGLE;
-      c.delta = 0;
-    }
-    K k0 = empty_key<K>(), k1 = empty_key<K>();
-    unsigned n0 = 0, n1 = 0;
-    /* samples only double can decide: up to four per lane held here and
-     * queued after the unit, the rest queued at once */
-    int nf = 0, f0 = 0, f1 = 0, f2 = 0, f3 = 0;
-    if (valid) {
-      for (int sz = z0; sz < z1; sz++) {
-        const float z = CG_ADD(zc, CG_FMA(CG_ADD((float)sz, 0.5f), dxs, zl));
-        for (int sy = y0; sy < y1; sy++) {
-          const float y = CG_ADD(yc, CG_FMA(CG_ADD((float)sy, 0.5f), dxs, yl));
-          float fsx = 0.5f; /* sx + 1/2, exact, without a conversion per sample */
-          /* unrolled by 3: half the samples of a 1024^3 run are in cells of
-           * nsub 2 and 3; copies per nsub, or unrolled by 2 or 4, measured
-           * slower (instruction fetch) */
-#pragma unroll 3
-          for (int sx = 0; sx < ns; sx++, fsx = CG_ADD(fsx, 1.0f))
-            paint_sample<K>(p, A, c, dbl, rec, CG_ADD(xc, CG_FMA(fsx, dxs, xl)), y, z, sx + ns * (sy + ns * sz), k0,
-                            n0, k1, n1, nf, f0, f1, f2, f3);
-        }
+      temp = c.temp;
+      const Axis x = {A.xc[ix], A.xl[ix]}, y = {A.yc[iy], A.yl[iy]}, z = {A.zc[iz], A.zl[iz]};
+      /* the bucket's class: one loop for the whole warp */
+      const int cls = dbl ? CG_CELL_GENERAL : b % CG_IMAP_CLASSES;
+      if (cls == CG_CELL_GENERAL) {
+        walk_general<K>(p, A, c, dbl, rec, x, y, z, dxs, ns, o0, o1, m0, m1, L);
+      } else {
+        cg_imap_fast F;
+        cg_imap_fast_cell(&A, &c, cls, x.c, y.c, z.c, &F);
+        if (cls == CG_CELL_EQ)
+          walk_fast<K, true>(p, F, temp, rec, x, y, z, dxs, ns, o0, o1, m0, m1, cg_fast_eq_thr(A.nside), L);
+        else
+          walk_fast<K, false>(p, F, temp, rec, x, y, z, dxs, ns, o0, o1, m0, m1, cg_fast_polar_k0(A.nside), L);
       }
+      flush<K>(p, L.k, L.n, temp);
     }
-    flush<K>(p, k0, n0, c.temp);
-    flush<K>(p, k1, n1, c.temp);
-    /* the held samples (most units hold none) to the warp's stage; at most
-     * 128 per group, so a stage past QB - 128 entries is queued first */
-    const int held = nf < 4 ? nf : 4;
-    if (__any_sync(FULL, held > 0)) {
-      int incl = held;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const int tot = __shfl_sync(FULL, incl, 31);
-      unsigned long long *qb = stage_of(p);
-      if (qn + tot > QB) {
-        queue_flush(p, qb, qn, lane);
-        qn = 0;
-      }
-      const int o = qn + incl - held;
-      for (int h = 0; h < held; h++)
-        qb[o + h] = ((unsigned long long)rec << 30) | (unsigned long long)(h == 0 ? f0 : (h == 1 ? f1 : (h == 2 ? f2 : f3)));
-      qn += tot;
-    }
+    queue_flush(p, QB / 2, lane);
   }
 }
 
-/* Warps take chunks in bucket order; paint_chunk paints one. */
+/* Warps take chunks in bucket order; paint_chunk paints one.  8 blocks per SM:
+ * 5, 6, 7 and 10 took 67.1, 63.5, 62.0 and 64.9 against 61.7 ms of the stage at
+ * 1024^3. */
 template <typename K>
-__global__ void __launch_bounds__(IW * 32, 8) k_imap_paint(cg_imap_params p)
+__global__ void __launch_bounds__(IW * 32, 8) k_imap_paint(const __grid_constant__ cg_imap_params p)
 {
   extern __shared__ __align__(16) unsigned char sraw[];
   const Sh sh = load_shells(p, sraw, true);
@@ -588,7 +743,8 @@ __global__ void __launch_bounds__(IW * 32, 8) k_imap_paint(cg_imap_params p)
   const cg_imap_args A = args_with(p, sh);
   const int lane = threadIdx.x & 31;
   const unsigned long long total = sh.chunk_off[p.nbk];
-  int qn = 0;
+  if (lane == 0) *stage_of(p).n = 0;
+  __syncwarp();
   for (;;) {
     unsigned long long ck = 0;
     if (lane == 0) ck = atomicAdd(&p.ctr[0], 1ull);
@@ -603,15 +759,15 @@ __global__ void __launch_bounds__(IW * 32, 8) k_imap_paint(cg_imap_params p)
     }
     const int b = lo;
     const unsigned long long nrec =
-        p.cnt[b] < (unsigned long long)p.cap[b] ? p.cnt[b] : (unsigned long long)p.cap[b];
-    const int ns = sh.nsub[b];
+        p.cnt[(size_t)b * CG_IMAP_CNT] < (unsigned long long)p.cap[b] ? p.cnt[(size_t)b * CG_IMAP_CNT] : (unsigned long long)p.cap[b];
+    const int ns = sh.nsub[b / CG_IMAP_CLASSES];
     const unsigned long long nu = nrec * (unsigned long long)units_per_cell(ns);
     const int G = groups_per_chunk(ns);
-    const float dxs = sh.dxs[b];
+    const float dxs = sh.dxs[b / CG_IMAP_CLASSES];
     const unsigned long long u0 = (ck - sh.chunk_off[b]) * 32ull * (unsigned long long)G;
-    paint_chunk<K>(p, A, b, ns, u0, G, nu, dxs, lane, qn);
+    paint_chunk<K>(p, A, b, ns, u0, G, nu, dxs, lane);
   }
-  if (qn) queue_flush(p, stage_of(p), qn, lane);
+  queue_flush(p, 1, lane);
 }
 
 /* The samples of one warp batch (n <= 32 entries of the queue's form) in
@@ -641,7 +797,7 @@ __device__ __forceinline__ void double_batch(const float *__restrict__ phi, cons
       else hi = mid - 1;
     }
     int dbl;
-    const cg_imap_cell c = unpack(p.recs[rec], lo - 1, &ix, &iy, &iz, &dbl);
+    const cg_imap_cell c = unpack(p.recs[rec], lo / CG_IMAP_CLASSES - 1, &ix, &iy, &iz, &dbl);
     temp = c.temp;
     float v[3];
     grad_phi(phi, ix, iy, iz, p.box.N, v);
@@ -655,16 +811,13 @@ __device__ __forceinline__ void double_batch(const float *__restrict__ phi, cons
   temp = __shfl_sync(FULL, temp, src);
   drr = __shfl_sync(FULL, drr, src);
   if (!valid) return;
+  lo /= CG_IMAP_CLASSES;
   const int ns = sh.nsub[lo];
   int s = -1, sx, sy, sz;
   sub_of(q, ns, sh.invns[lo], &sx, &sy, &sz);
   long long pix = 0;
   cgx_imap_sample(&A, ix, iy, iz, ns, drr, sx, sy, sz, &s, &pix);
-  if (s >= 0 && s < p.nr) {
-    const long long key = (long long)s * p.npix + pix;
-    atomicAdd(&p.data[key], temp);
-    atomicAdd(&p.nadd[key], 1);
-  }
+  if (s >= 0 && s < p.nr) add_to(p, (long long)s * p.npix + pix, temp, 1.0f);
 }
 
 constexpr int DB_WARPS = 8; /* warps per block of k_imap_double */
@@ -706,19 +859,16 @@ __global__ void __launch_bounds__(DB_WARPS * 32) k_imap_double(const float *__re
         else hi = mid - 1;
       }
       int ix, iy, iz, dbl;
-      const cg_imap_cell c = unpack(p.recs[rec], lo - 1, &ix, &iy, &iz, &dbl);
+      const cg_imap_cell c = unpack(p.recs[rec], lo / CG_IMAP_CLASSES - 1, &ix, &iy, &iz, &dbl);
       if (!dbl) {
+        lo /= CG_IMAP_CLASSES;
         const int ns = sh.nsub[lo];
         int s = -1, sx, sy, sz;
         long long pix = 0;
         sub_of(q, ns, sh.invns[lo], &sx, &sy, &sz);
         if (cg_imap_decide_ff(&A, &c, ix, iy, iz, sx, sy, sz, &s, &pix)) {
           need = false;
-          if (s >= 0 && s < p.nr) {
-            const long long key = (long long)s * p.npix + pix;
-            atomicAdd(&p.data[key], c.temp);
-            atomicAdd(&p.nadd[key], 1);
-          }
+          if (s >= 0 && s < p.nr) add_to(p, (long long)s * p.npix + pix, c.temp, 1.0f);
         }
       }
     }
@@ -744,7 +894,8 @@ template <typename K>
 cudaError_t launch(cudaStream_t s, const float *dens, const float *phi, const cg_imap_params *p, int nsm)
 {
   cudaError_t e = cudaMemsetAsync(p->ctr, 0, 5 * sizeof(unsigned long long), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(p->cnt, 0, (size_t)p->nbk * sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->cnt, 0, (size_t)p->nbk * CG_IMAP_CNT * sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->seg + p->a.na - 1, 0, sizeof(cg_imap_seg), s);
   if (e != cudaSuccess) return e;
   const size_t sm_list = shell_smem(p->nr, p->nbk, false), sm_paint = paint_smem(p->nr, p->nbk);
   const size_t sm_double = double_stage_off(p->nr, p->nbk) + (size_t)DB_WARPS * 64 * 8;
@@ -757,8 +908,9 @@ cudaError_t launch(cudaStream_t s, const float *dens, const float *phi, const cg
   const long long nrow = (long long)p->box.N * p->box.N;
   long long blocks = (nrow + IW * ROWS - 1) / (IW * ROWS);
   if (blocks > (long long)nsm * (per_sm > 0 ? per_sm : 1)) blocks = (long long)nsm * (per_sm > 0 ? per_sm : 1);
+  k_imap_tab<<<(unsigned)((p->a.na + 31) / 32), 32, 0, s>>>(*p);
   k_imap_list<K><<<(unsigned)blocks, IW * 32, sm_list, s>>>(dens, phi, *p);
-  k_imap_chunks<<<1, 32, 0, s>>>(*p);
+  k_imap_chunks<<<1, 1024, 0, s>>>(*p);
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_imap_paint<K>, IW * 32, sm_paint))) return e;
   k_imap_paint<K><<<(unsigned)(nsm * (per_sm > 0 ? per_sm : 1)), IW * 32, sm_paint, s>>>(*p);
   k_imap_double<<<(unsigned)(nsm * 4), DB_WARPS * 32, sm_double, s>>>(phi, *p);

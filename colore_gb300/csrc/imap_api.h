@@ -20,20 +20,26 @@ struct __align__(16) cg_imap_rec {
 };
 
 #define CG_IMAP_REC_BYTES 16
-#define CG_IMAP_BUCKETS_MAX 4100 /* shells -1 .. nr: nr <= 4096 */
+/* A bucket per shell -1 .. nr of the cells' corners and per class of
+ * cg_imap_fast_cell: bucket 3 (j + 1) + class. */
+#define CG_IMAP_CLASSES 3
+#define CG_IMAP_CNT 16 /* stride of the buckets' counters: a 128-byte line each */
+#define CG_IMAP_BUCKETS_MAX (CG_IMAP_CLASSES * 4100) /* nr <= 4096 */
 
 struct cg_imap_params {
   cg::Box box;
   cg_imap_args a;    /* tables, corners, shells (device pointers) */
-  int nr, nbk;       /* shells; buckets nbk = nr + 2, bucket j + 1 for shell j */
+  cg_imap_seg *seg;  /* the tables' segments (na - 1) and, past them, the bits of their
+                        largest factor bound (all written by cg_imap_paint) */
+  int nr, nbk;       /* shells; buckets nbk = CG_IMAP_CLASSES (nr + 2) */
   long long npix;
-  float *data;       /* nr * npix, RING */
-  int *nadd;         /* nr * npix       */
+  float2 *acc;       /* nr * npix, RING: summed brightness, samples */
+  int packed;        /* samples as a float (each below 2^24), else as int bits */
   unsigned int *err;
   unsigned long long *xstats; /* [2] cells, [3] samples decided in double */
   int force_double;
   /* cells are listed per bucket (the shell of their corner, which fixes
-   * nsub), in the slots [base[b], base[b] + cap[b]); cnt[b] counts them
+   * nsub, and the class, which fixes the painting loop), in the slots [base[b], base[b] + cap[b]); cnt[CG_IMAP_CNT b] counts them
    * (may exceed cap: those cells are painted by the listing kernel) */
   cg_imap_rec *recs;
   const long long *base, *cap;

@@ -217,3 +217,76 @@ void or_next_float(long n, const float *f, const int *up, float *out)
 {
   for (long i = 0; i < n; i++) out[i] = cg_next_float(f[i], up[i]);
 }
+
+/* Samples of whole cells by the per-cell constants (cg_imap_fast_cell) against
+ * the double arithmetic: cell (3 ints) of a box of N cells of side dx with the
+ * observer at pos, nsub sub-cells per axis.  edge[i] > 0: the cell crosses the
+ * shell edge edge[i] with radial shift drr[i] known within edrr of drr64[i]
+ * (shells 0 below, 1 above); else one shell.  stat[0..4]: fast cells,
+ * equatorial ones, their samples, samples decided, and decided wrongly. */
+void or_imap_fast(long nside, int N, double dx, const double *pos, long n, const int *cell, const int *nsub,
+                  const float *edge, const float *drr, const double *drr64, float edrr, long long *stat)
+{
+  float b[1];
+  int shell_of[2] = {0, 1};
+  cg_imap_args a;
+  memset(&a, 0, sizeof(a));
+  a.dx = (float)dx;
+  a.nside = (int)nside;
+  a.sh.b = b;
+  a.sh.shell_of = shell_of;
+  a.sh.nb = 1;
+  a.sh.nr = 2;
+  a.sh.contig = 1;
+  for (int k = 0; k < 5; k++) stat[k] = 0;
+  for (long i = 0; i < n; i++) {
+    const int *ci = cell + 3 * i, ns = nsub[i];
+    const float dxs = (float)(dx / ns);
+    cg_imap_cell c;
+    memset(&c, 0, sizeof(c));
+    b[0] = edge[i];
+    c.j = 0;
+    c.drr = drr[i];
+    c.edrr = edrr;
+    c.mode = edge[i] > 0 ? CG_SH_EDGE : CG_SH_SINGLE;
+    c.delta = edge[i] > 0 ? -1 : 0; /* intervals -1 and 0 */
+    float h[3], l[3];
+    for (int k = 0; k < 3; k++) {
+      const double x = cgx_coord(ci[k], dx, pos[k]);
+      h[k] = (float)x;
+      l[k] = (float)(x - (double)h[k]);
+    }
+    cg_imap_fast F;
+    const int cls = cg_cell_class(&a, &c, h[0], h[1], h[2]);
+    if (cls == CG_CELL_GENERAL) continue;
+    cg_imap_fast_cell(&a, &c, cls, h[0], h[1], h[2], &F);
+    stat[0]++;
+    stat[1] += cls == CG_CELL_EQ;
+    for (int q = 0; q < ns * ns * ns; q++) {
+      const int sx = q % ns, sy = q / ns % ns, sz = q / (ns * ns);
+      const float x = cg_imap_coord(&h[0], &l[0], 0, sx, dxs), y = cg_imap_coord(&h[1], &l[1], 0, sy, dxs);
+      const float z = cg_imap_coord(&h[2], &l[2], 0, sz, dxs);
+      const float u = F.ymaj ? y : x, v = F.ymaj ? x : y;
+      int up, pix, ok;
+      if (cls == CG_CELL_EQ) {
+        ok = cg_fast_eq(&F, (int)nside, cg_fast_eq_thr((int)nside), u, v, z, CG_FMA(z, z, CG_MUL(v, v)), &up, &pix);
+      } else {
+        const cg_fast_line line = cg_fast_polar_line(&F, (int)nside, u, v);
+        ok = cg_fast_polar(&F, &line, cg_fast_polar_k0((int)nside), z, &up, &pix);
+      }
+      const int s = up ? F.s1 : F.s0;
+      stat[2]++;
+      if (!ok) continue;
+      stat[3]++;
+      const double step = X_DIV(dx, (double)ns);
+      const double X = X_ADD(cgx_coord(ci[0], dx, pos[0]), X_MUL(X_ADD((double)sx, 0.5), step));
+      const double Y = X_ADD(cgx_coord(ci[1], dx, pos[1]), X_MUL(X_ADD((double)sy, 0.5), step));
+      const double Z = X_ADD(cgx_coord(ci[2], dx, pos[2]), X_MUL(X_ADD((double)sz, 0.5), step));
+      double r, cth, ph;
+      cgx_cart2sph(X, Y, Z, &r, &cth, &ph);
+      const int want = edge[i] > 0 ? (X_ADD(r, drr64[i]) >= (double)edge[i]) : 0;
+      stat[4] += pix != cgx_ang2pix(nside, cth, ph) || s != want;
+    }
+  }
+  (void)N;
+}

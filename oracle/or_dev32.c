@@ -574,6 +574,95 @@ int or_imap32(const cg_config *cfg, int ipop, const float *dens, const float *np
   return 0;
 }
 
+/* The listing of every cell from the per-segment tables (cg_imap_cell_seg)
+ * against the double arithmetic.  stat: [0] cells settled, [1] of them listed,
+ * [2] open; and faults: [3] listed or not, [4] shell of the corner, [5] radial
+ * shift further off than its bound, [6] samples outside the shells that the
+ * cell's mode claims, [7] brightness. */
+static double bias_model64(double d, double b, int model)
+{
+  if (d <= -1) return 0;
+  if (model == CG_BIAS_EXPLIN) return d < 0 ? exp(b * d / (1 + d)) : 1 + b * d;
+  if (model == CG_BIAS_LIN) return b * d > -1 ? 1 + b * d : 0;
+  return pow(1 + d, b);
+}
+
+int or_imap_cells(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
+                  const double *norm64, long long *stat)
+{
+  S32 s;
+  s32_init(&s, cfg);
+  ImapArgs B;
+  imap_args(&B, cfg, &s, ipop, norm32, norm64);
+  cg_imap_args *a = &B.a;
+  const int N = s.N, na = a->na, nb = a->sh.nb;
+  cg_imap_seg *segs = aligned_alloc(32, (size_t)na * sizeof(cg_imap_seg));
+  float eg = 0;
+  for (int i = 0; i < na - 1; i++) {
+    float e;
+    segs[i] = cg_imap_seg_make(a, i, &e);
+    if (e > eg) eg = e;
+  }
+  float *edges = malloc((size_t)(nb + 4) * sizeof(float));
+  edges[0] = edges[1] = -3.0e38f;
+  for (int i = 0; i < nb; i++) edges[i + 2] = a->sh.b[i];
+  edges[nb + 2] = edges[nb + 3] = 3.0e38f;
+  a->sh.b = edges + 2;
+  for (int k = 0; k < 8; k++) stat[k] = 0;
+  for (int iz = 0; iz < N; iz++)
+    for (int iy = 0; iy < N; iy++)
+      for (int ix = 0; ix < N; ix++) {
+        float v[3];
+        grad32(npot, ix, iy, iz, N, v);
+        const float d = dens[pidx(ix, iy, iz, N)];
+        const float x0 = a->xc[ix], y0 = a->yc[iy], z0 = a->zc[iz];
+        const float r2 = CG_FMA(x0, x0, CG_FMA(z0, z0, CG_MUL(y0, y0)));
+        cg_imap_cell c;
+        const int k = cg_imap_cell_seg(segs, eg, a, x0, y0, z0, r2, d, v, &c);
+        int j = 0;
+        double drr = 0;
+        const int k64 = cgx_imap_cell(a, ix, iy, iz, v, &j, &drr);
+        stat[k == 2 ? 2 : 0]++;
+        if (k == 2) continue;
+        stat[3] += k != k64;
+        if (!k || !k64) continue;
+        stat[1]++;
+        stat[4] += c.j != j;
+        stat[5] += !(fabs((double)c.drr - drr) <= (double)c.edrr);
+        const double r = cgx_norm3(cgx_coord(ix, a->dx64, a->p64[0]), cgx_coord(iy, a->dx64, a->p64[1]),
+                                   cgx_coord(iz, a->dx64, a->p64[2]));
+        /* brightness: the tables at a radius 1e-6 (the float position is within
+         * 10 2^-24) to either side, and 24 roundings of the bias factor's
+         * exponent and of the products */
+        double w[3];
+        for (int e = -1; e <= 1; e++) {
+          const double re = r * (1 + 1e-6 * e);
+          w[e + 1] = cgx_bg(a->tz64, a->r64, a->idr64, a->r_last64, 0, 0, re) *
+                     cgx_bg(norm64, a->r64, a->idr64, a->r_last64, 0, 0, re) *
+                     bias_model64(d, cgx_bg(a->bz64, a->r64, a->idr64, a->r_last64, 1, 1, re), a->bias_model);
+        }
+        const double lnf = d > -1 && w[1] > 0 ? fabs((double)d) / (1 + (double)d) * 4 : 0;
+        stat[7] += !(fabs((double)c.temp - w[1]) <=
+                     fabs(w[2] - w[1]) + fabs(w[0] - w[1]) + 24 * 6e-8 * (1 + lnf) * w[1] + 1e-37);
+        if (c.mode == CG_SH_WALK) continue;
+        const int ns = a->nsub[c.j + 1];
+        for (int q = 0; q < ns * ns * ns; q++) {
+          const double step = X_DIV(a->dx64, (double)ns);
+          const double X = X_ADD(cgx_coord(ix, a->dx64, a->p64[0]), X_MUL(X_ADD((double)(q % ns), 0.5), step));
+          const double Y = X_ADD(cgx_coord(iy, a->dx64, a->p64[1]), X_MUL(X_ADD((double)(q / ns % ns), 0.5), step));
+          const double Z = X_ADD(cgx_coord(iz, a->dx64, a->p64[2]), X_MUL(X_ADD((double)(q / (ns * ns)), 0.5), step));
+          const int iv = cgx_interval(&a->sh, X_ADD(cgx_norm3(X, Y, Z), drr));
+          const int kl = c.j + c.delta;
+          stat[6] += c.mode == CG_SH_SINGLE ? a->sh.shell_of[iv + 1] != kl : (iv != kl && iv != kl + 1);
+        }
+      }
+  free(edges);
+  free(segs);
+  imap_args_free(&B);
+  s32_free(&s);
+  return 0;
+}
+
 static int cmp_float(const void *a, const void *b)
 {
   float x = *(const float *)a, y = *(const float *)b;

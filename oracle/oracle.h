@@ -92,6 +92,8 @@ int or_beam_rsd32(const cg_config *cfg, const float *npot, long long n, const fl
  * do not hold); stats: cells and samples decided in double, samples drawn. */
 int or_imap32(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
               const double *norm64, float *data, int *nadd, long long *stats);
+int or_imap_cells(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
+                  const double *norm64, long long *stat);
 int or_kappa32(const cg_config *cfg, const float *npot, float *map);
 int or_isw32(const cg_config *cfg, const float *npot, float *map);
 int or_cstm32(const cg_config *cfg, int ipop, const float *dens, const float *normtab, float n0, float nf,
@@ -116,5 +118,8 @@ void or_count_seg(const double *r, const double *nz, const double *bz, const dou
 
 void or_dir_phi(long nside, const float *xyz, long n, float *ph, float *ref, long long *pix);
 void or_next_float(long n, const float *f, const int *up, float *out);
+
+void or_imap_fast(long nside, int N, double dx, const double *pos, long n, const int *cell, const int *nsub,
+                  const float *edge, const float *drr, const double *drr64, float edrr, long long *stat);
 
 #endif

@@ -37,6 +37,7 @@ def lib():
             "or_counts64": [vp, i, vp, vp, vp, vp],
             "or_emit64": [vp, i, vp, vp, C.c_longlong, vp, vp, vp, vp, vp],
             "or_beam_rsd32": [vp, vp, C.c_longlong, vp, vp], "or_imap32": [vp, i, vp, vp, vp, vp, vp, vp, vp],
+            "or_imap_cells": [vp, i, vp, vp, vp, vp, vp],
             "or_kappa32": [vp, vp, vp], "or_isw32": [vp, vp, vp], "or_isw64": [vp, vp, vp],
             "or_cstm_steps": [vp, i, vp, vp, vp, vp], "or_cstm64": [vp, i, vp, vp, d, d, vp],
             "or_cstm32": [vp, i, vp, vp, f, f, vp],
@@ -56,12 +57,13 @@ def lib():
             "or_sht_legendre": [i, i, i, vp, vp, vp, d, vp],
             "or_src_offset_checked": [C.c_long, vp, d, vp, vp, vp, vp],
             "or_ptrs_checked": [C.c_long, vp, vp, vp, vp, C.c_uint32, C.c_uint32, vp, vp],
+            "or_imap_fast": [C.c_long, i, d, vp, C.c_long, vp, vp, vp, vp, vp, f, vp],
             "or_dir_phi": [C.c_long, vp, C.c_long, vp, vp, vp], "or_next_float": [C.c_long, vp, vp, vp],
             "or_count_seg": [vp, vp, vp, vp, d, d, vp, d, d, i, C.c_long, vp, vp, vp, vp, vp, vp, vp, vp],
         }
         void = ("or_philox", "or_poisson", "or_ang2pix", "or_nest2ring", "or_ring2nest", "or_pix2vec_nest",
                 "or_shell_index", "or_pix_checked", "or_pix_cgx", "or_pix64", "or_pix_ff", "or_ff_ops", "or_src_offset_checked",
-                "or_ptrs_checked", "or_count_seg", "or_dir_phi", "or_next_float")
+                "or_ptrs_checked", "or_count_seg", "or_dir_phi", "or_next_float", "or_imap_fast")
         for k, a in sig.items():
             fn = getattr(L, k)
             fn.argtypes = a
@@ -325,6 +327,18 @@ def imap32(cfg, ipop, dens, npot, tab32, e32, tab64, e64):
     lib().or_imap32(cfgp(cfg), ipop, P(np.ascontiguousarray(dens, np.float32)),
                     P(np.ascontiguousarray(npot, np.float32)), P(t32), P(t64), P(data), P(nadd), P(st))
     return data, nadd, st
+
+
+def imap_cells(cfg, ipop, dens, npot, tab32, e32, tab64, e64):
+    """The listing of every cell from per-segment tables against double:
+    (cells settled, listed, open; faults of listing, shell, radial shift, mode
+    and brightness)."""
+    st = np.zeros(8, np.int64)
+    t32, t64 = _norm_pair(tab32, e32, tab64, e64)
+    lib().or_imap_cells(cfgp(cfg), ipop, P(np.ascontiguousarray(dens, np.float32)),
+                        P(np.ascontiguousarray(npot, np.float32)), P(t32), P(t64), P(st))
+    return tuple(int(v) for v in st)
+
 
 def isw64(cfg, npot):
     ns = cfg.nside_isw
@@ -602,3 +616,16 @@ def next_float(f, up):
     out = np.empty_like(f)
     lib().or_next_float(len(f), P(f), P(up), P(out))
     return out
+
+
+def imap_fast(nside, ng, dx, pos, cell, nsub, edge, drr, drr64, edrr):
+    """Whole cells by the per-cell constants of the painting against double:
+    (fast cells, equatorial ones, samples, decided, decided wrongly)."""
+    pos = np.ascontiguousarray(pos, np.float64)
+    cell = np.ascontiguousarray(cell, np.int32)
+    nsub = np.ascontiguousarray(nsub, np.int32)
+    edge, drr = np.ascontiguousarray(edge, np.float32), np.ascontiguousarray(drr, np.float32)
+    drr64 = np.ascontiguousarray(drr64, np.float64)
+    st = np.zeros(5, np.int64)
+    lib().or_imap_fast(nside, ng, dx, P(pos), len(cell), P(cell), P(nsub), P(edge), P(drr), P(drr64), edrr, P(st))
+    return tuple(int(v) for v in st)
