@@ -263,119 +263,203 @@ __global__ void __launch_bounds__(256) k_bins_finish(const unsigned long long *_
 /* 1LPT: x = q + D(r) Psi (wrapped into the box), then the mass assignment of
  * pos_2_dens (density.c:178-187): NGP (S = 0, density.c:37-62), CIC (S = 1,
  * density.c:64-105) or TSC (S = 2, density.c:107-176).  A block takes a tile
- * of CT_X x CT_Y x CT_Z particles (lattice cells) and deposits into a
- * shared-memory box that extends the tile by CT_H cells on every side; the
- * box is added to the grid at the end with one atomic per non-zero cell.
- * Deposits that fall outside the box (particles displaced by more than about
- * CT_H - 1 cells) go straight to the grid.  Masses are fixed point
- * (DEPOSIT_ONE per particle, integer atomics; the grid holds the int32 bits
- * until the density pass turns them into rho - 1), so the result does not
- * depend on the order of the atomic additions. */
-constexpr int CT_X = 32, CT_Y = 8, CT_Z = 8, CT_H = 2;
+ * of CT_X x CT_Y x CT_Z particles (lattice cells), a thread one column of it
+ * along z, and deposits into a shared-memory box that extends the tile by
+ * CT_H cells on every side; the box is added to the grid at the end, down its
+ * columns, with one atomic per non-zero cell.  Deposits that fall outside the
+ * box (particles displaced by more than about CT_H - 1 cells) go straight to
+ * the grid.  Masses are fixed point (DEPOSIT_ONE per particle, integer atomics;
+ * the grid holds the int32 bits until the density pass turns them into
+ * rho - 1), so the result does not depend on the order of the atomic additions.
+ * Bound by instruction issue (about 190 slots a particle; the box's flush was a
+ * third of 370 when it found every cell's place by divisions): 12.5 -> 7.9 ms
+ * at 1024^3 with the grid's clearing, 207 -> 143 us at 256^3.  Tiles of 8 x 8,
+ * 8 x 16, 16 x 8 and 4 x 32 in y and z took 9.8, 9.1, 10.3 and 10.9 against
+ * 8.4 ms of 4 x 16 before the flush went by columns; 10 and 12 blocks per SM
+ * (registers cut to 48 and 40) 8.1 and 8.3 against 7.9 ms. */
+constexpr int CT_X = 32, CT_Y = 4, CT_Z = 16, CT_H = 2;
 constexpr int CB_X = CT_X + 2 * CT_H, CB_Y = CT_Y + 2 * CT_H, CB_Z = CT_Z + 2 * CT_H;
+constexpr int CT_THREADS = CT_X * CT_Y;
+static_assert(CB_X * CB_Y * CB_Z % 4 == 0, "the box is cleared 16 bytes at a time");
+
+/* A particle's first stencil cell per axis, its weights there, and whether
+ * they are those of a position in the box (no weight above 1). */
+template <int S>
+struct Stencil {
+  int i0[3];
+  float w[3][S + 1];
+  bool plain;
+};
 
 template <int S>
-__global__ void __launch_bounds__(256) k_lpt_deposit(int *grid, const float *__restrict__ dx_,
-                                                     const float *__restrict__ dy_, const float *__restrict__ dz_,
-                                                     cg_lpt_params p)
+__device__ __forceinline__ void stencil_axis(Stencil<S> &t, int a, float q, float po, float L, float iag)
+{
+  constexpr int K = S + 1;
+  q = CG_ADD(q, po);
+  if (q < 0.0f) q = CG_ADD(q, L);
+  if (q >= L) q = CG_SUB(q, L);
+  const float u = CG_MUL(q, iag);
+  t.plain = t.plain && u >= 0.0f;
+  if (S == 0) {
+    t.i0[a] = (int)CG_ADD(u, 0.5f);
+    t.w[a][0] = 1.0f;
+  } else if (S == 1) {
+    t.i0[a] = (int)u;
+    const float a1 = CG_SUB(u, (float)t.i0[a]);
+    t.w[a][0] = CG_SUB(1.0f, a1);
+    t.w[a][K - 1] = a1;
+  } else {
+    const int i0 = (int)floorf(CG_ADD(u, 0.5f));
+    const float a0 = CG_SUB(u, (float)i0);
+    const float hm = CG_SUB(0.5f, a0), hp = CG_ADD(0.5f, a0);
+    t.w[a][0] = CG_MUL(0.5f, CG_MUL(hm, hm));
+    t.w[a][1] = CG_SUB(0.75f, CG_MUL(a0, a0));
+    t.w[a][K - 1] = CG_MUL(0.5f, CG_MUL(hp, hp));
+    t.i0[a] = i0 - 1; /* the stencil starts one cell below the nearest */
+  }
+}
+
+/* A particle that leaves its block's box: straight to the grid. */
+template <int S>
+__device__ __noinline__ void deposit_far(int *grid, int N, Stencil<S> t)
+{
+  constexpr int K = S + 1;
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    /* q is in [0, L) unless the displacement exceeds the box: then a full
+     * modulo keeps the cell index inside the grid */
+    if ((unsigned)t.i0[a] >= (unsigned)N) t.i0[a] = ((t.i0[a] % N) + N) % N;
+#pragma unroll
+  for (int cz = 0; cz < K; cz++)
+#pragma unroll
+    for (int cy = 0; cy < K; cy++)
+#pragma unroll
+      for (int cx = 0; cx < K; cx++) {
+        const int v = __float2int_rn(CG_MUL(CG_MUL(CG_MUL(t.w[0][cx], t.w[1][cy]), t.w[2][cz]), DEPOSIT_ONE));
+        const int gx = t.i0[0] + cx >= N ? t.i0[0] + cx - N : t.i0[0] + cx;
+        const int gy = t.i0[1] + cy >= N ? t.i0[1] + cy - N : t.i0[1] + cy;
+        const int gz = t.i0[2] + cz >= N ? t.i0[2] + cz - N : t.i0[2] + cz;
+        atomicAdd(&grid[pidx(gx, gy, gz, N)], v);
+      }
+}
+
+template <int S, bool TWO>
+__global__ void __launch_bounds__(CT_THREADS, 8) k_lpt_deposit(int *grid, const float *__restrict__ dx_,
+                                                            const float *__restrict__ dy_,
+                                                            const float *__restrict__ dz_,
+                                                            const __grid_constant__ cg_lpt_params p)
 {
   constexpr int K = S + 1; /* cells per axis of the stencil */
-  __shared__ int box[CB_Z][CB_Y][CB_X];
+  __shared__ __align__(16) int box[CB_Z * CB_Y * CB_X];
   const int N = p.box.N;
   const int ntx = (N + CT_X - 1) / CT_X, nty = (N + CT_Y - 1) / CT_Y;
-  const int t = blockIdx.x;
-  const int tx0 = (t % ntx) * CT_X, ty0 = ((t / ntx) % nty) * CT_Y, tz0 = (t / (ntx * nty)) * CT_Z;
-  for (int i = threadIdx.x; i < CB_X * CB_Y * CB_Z; i += blockDim.x) (&box[0][0][0])[i] = 0;
+  const int t = blockIdx.x, tx = t % ntx, tyz = t / ntx;
+  const int tx0 = tx * CT_X, ty0 = (tyz % nty) * CT_Y, tz0 = (tyz / nty) * CT_Z;
+  for (int i = threadIdx.x; i < CB_X * CB_Y * CB_Z / 4; i += CT_THREADS)
+    reinterpret_cast<int4 *>(box)[i] = make_int4(0, 0, 0, 0);
   __syncthreads();
-  const float iag = CG_DIV((float)N, p.box.L);
-  const float po[3] = {p.box.p0, p.box.p1, p.box.p2};
-  const int org[3] = {tx0 - CT_H, ty0 - CT_H, tz0 - CT_H};
-  const int ext[3] = {CB_X, CB_Y, CB_Z};
-  for (int k = threadIdx.x; k < CT_X * CT_Y * CT_Z; k += blockDim.x) {
-    const int ix = tx0 + (k % CT_X), iy = ty0 + (k / CT_X) % CT_Y, iz = tz0 + k / (CT_X * CT_Y);
-    if (ix >= N || iy >= N || iz >= N) continue;
-    const long long id = pidx(ix, iy, iz, N);
-    float xv[3] = {cg_cell_coord(ix, p.box.dx, p.box.p0), cg_cell_coord(iy, p.box.dx, p.box.p1),
-                   cg_cell_coord(iz, p.box.dx, p.box.p2)};
-    const float r = cg_norm3(xv[0], xv[1], xv[2]);
-    const float dg = bg(p.d1, p.g, r);
-    const float dsp[3] = {__ldg(&dx_[id]), __ldg(&dy_[id]), __ldg(&dz_[id])};
-    /* 2LPT: x = q + D1 Psi1 + D2 Psi2 (density.c:890) */
-    const bool two = p.d2x != nullptr;
-    const float d2g = two ? bg(p.d2, p.g, r) : 0.0f;
-    const float ds2[3] = {two ? __ldg(&p.d2x[id]) : 0.0f, two ? __ldg(&p.d2y[id]) : 0.0f,
-                          two ? __ldg(&p.d2z[id]) : 0.0f};
-    int ib[3], bb[3]; /* first stencil cell of each axis, in the grid and in the box */
-    float w[3][K];
-    bool inbox = true;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      float q = CG_FMA(dg, dsp[a], xv[a]);
-      if (two) q = CG_FMA(d2g, ds2[a], q);
-      q = CG_ADD(q, po[a]);
-      if (q < 0.0f) q = CG_ADD(q, p.box.L);
-      if (q >= p.box.L) q = CG_SUB(q, p.box.L);
-      const float u = CG_MUL(q, iag);
-      int i0;
-      if (S == 0) {
-        i0 = (int)CG_ADD(u, 0.5f);
-        w[a][0] = 1.0f;
-      } else if (S == 1) {
-        i0 = (int)u;
-        const float a1 = CG_SUB(u, (float)i0);
-        w[a][0] = CG_SUB(1.0f, a1);
-        w[a][K - 1] = a1;
-      } else {
-        i0 = (int)floorf(CG_ADD(u, 0.5f));
-        const float a0 = CG_SUB(u, (float)i0);
-        const float hm = CG_SUB(0.5f, a0), hp = CG_ADD(0.5f, a0);
-        w[a][0] = CG_MUL(0.5f, CG_MUL(hm, hm));
-        w[a][1] = CG_SUB(0.75f, CG_MUL(a0, a0));
-        w[a][K - 1] = CG_MUL(0.5f, CG_MUL(hp, hp));
-        i0 -= 1; /* the stencil starts one cell below the nearest */
+  const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+  const int ix = tx0 + lane, iy = ty0 + wy;
+  const long long plane = (long long)(2 * (N / 2 + 1)) * N;
+  if (ix < N && iy < N) {
+    const float iag = CG_DIV((float)N, p.box.L);
+    const float po[3] = {p.box.p0, p.box.p1, p.box.p2};
+    const int org[3] = {tx0 - CT_H, ty0 - CT_H, tz0 - CT_H};
+    const int last[3] = {CB_X - K, CB_Y - K, CB_Z - K};
+    float xv[3] = {cg_cell_coord(ix, p.box.dx, p.box.p0), cg_cell_coord(iy, p.box.dx, p.box.p1), 0.0f};
+    long long id = pidx(ix, iy, tz0, N);
+    const int nz = N - tz0 < CT_Z ? N - tz0 : CT_Z;
+    /* the next plane's displacements are loaded a step ahead */
+    float nx[3] = {__ldg(&dx_[id]), __ldg(&dy_[id]), __ldg(&dz_[id])};
+#pragma unroll 1
+    for (int kz = 0; kz < nz; kz++, id += plane) {
+      xv[2] = cg_cell_coord(tz0 + kz, p.box.dx, p.box.p2);
+      const float dsp[3] = {nx[0], nx[1], nx[2]};
+      if (kz + 1 < nz) {
+        nx[0] = __ldg(&dx_[id + plane]);
+        nx[1] = __ldg(&dy_[id + plane]);
+        nx[2] = __ldg(&dz_[id + plane]);
       }
-      /* q is in [0, L) unless the displacement exceeds the box: then a full
-       * modulo keeps the cell index inside the grid */
-      if ((unsigned)i0 >= (unsigned)N) i0 = ((i0 % N) + N) % N;
-      ib[a] = i0;
-      /* position of the first stencil cell in the box, the shorter way round */
-      int d = i0 - org[a];
-      if (d < -N / 2) d += N;
-      if (d >= N / 2) d -= N;
-      bb[a] = d;
-      inbox = inbox && d >= 0 && d + K - 1 < ext[a];
-    }
+      const float r = cg_norm3(xv[0], xv[1], xv[2]);
+      const float dg = bg(p.d1, p.g, r);
+      Stencil<S> st;
+      st.plain = true;
+      if (TWO) { /* 2LPT: x = q + D1 Psi1 + D2 Psi2 (density.c:890) */
+        const float ds2[3] = {__ldg(&p.d2x[id]), __ldg(&p.d2y[id]), __ldg(&p.d2z[id])};
+        const float d2g = bg(p.d2, p.g, r);
 #pragma unroll
-    for (int cz = 0; cz < K; cz++)
+        for (int a = 0; a < 3; a++)
+          stencil_axis<S>(st, a, CG_FMA(d2g, ds2[a], CG_FMA(dg, dsp[a], xv[a])), po[a], p.box.L, iag);
+      } else {
 #pragma unroll
-      for (int cy = 0; cy < K; cy++)
+        for (int a = 0; a < 3; a++) stencil_axis<S>(st, a, CG_FMA(dg, dsp[a], xv[a]), po[a], p.box.L, iag);
+      }
+      /* the first stencil cell in the box: the box may reach over the grid's
+       * end, by less than a period */
+      int at = 0;
+      bool in = st.plain;
 #pragma unroll
-        for (int cx = 0; cx < K; cx++) {
-          /* the weight in units of 2^-20, rounded to nearest (the
-           * scaling by a power of two is exact) */
-          const int v = __float2int_rn(CG_MUL(CG_MUL(CG_MUL(w[0][cx], w[1][cy]), w[2][cz]), DEPOSIT_ONE));
-          if (inbox) {
-            atomicAdd(&box[bb[2] + cz][bb[1] + cy][bb[0] + cx], v);
-          } else {
-            const int gx = ib[0] + cx >= N ? ib[0] + cx - N : ib[0] + cx;
-            const int gy = ib[1] + cy >= N ? ib[1] + cy - N : ib[1] + cy;
-            const int gz = ib[2] + cz >= N ? ib[2] + cz - N : ib[2] + cz;
-            atomicAdd(&grid[pidx(gx, gy, gz, N)], v);
+      for (int a = 2; a >= 0; a--) {
+        int d = st.i0[a] - org[a];
+        if ((unsigned)d >= (unsigned)N) d += d < 0 ? N : -N;
+        in = in && (unsigned)d <= (unsigned)last[a];
+        at = at * (a == 1 ? CB_Y : CB_X) + d;
+      }
+      if (!in) {
+        deposit_far<S>(grid, N, st);
+        continue;
+      }
+#pragma unroll
+      for (int cz = 0; cz < K; cz++)
+#pragma unroll
+        for (int cy = 0; cy < K; cy++)
+#pragma unroll
+          for (int cx = 0; cx < K; cx++) {
+            /* the weight in units of 2^-20, rounded to nearest: the scaling by
+             * a power of two is exact, and 1.5 2^23 added to 0 .. 2^20 rounds
+             * to a whole number in the low bits */
+            const float v = CG_MUL(CG_MUL(st.w[0][cx], st.w[1][cy]), CG_MUL(st.w[2][cz], DEPOSIT_ONE));
+            atomicAdd(&box[at + (cz * CB_Y + cy) * CB_X + cx], __float_as_int(CG_ADD(v, 12582912.0f)) - 0x4b400000);
           }
-        }
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < CB_X * CB_Y * CB_Z; i += blockDim.x) {
-    const int v = (&box[0][0][0])[i];
+  /* the box's tile columns, a lane each, down the planes; then the halo
+   * columns */
+  const int gx = ix >= N ? ix - N : ix, gz0 = tz0 < CT_H ? tz0 - CT_H + N : tz0 - CT_H;
+  for (int by = wy; by < CB_Y; by += CT_THREADS / 32) {
+    int gy = ty0 - CT_H + by;
+    gy = gy < 0 ? gy + N : (gy >= N ? gy - N : gy);
+    int *g = grid + pidx(gx, gy, gz0, N);
+    const int *from = box + by * CB_X + CT_H + lane;
+    int up = N - gz0; /* planes to the grid's end */
+#pragma unroll 4
+    for (int bz = 0; bz < CB_Z; bz++) {
+      if (bz == up) g -= N * plane;
+      const int v = from[bz * (CB_Y * CB_X)];
+      if (v != 0) atomicAdd(g, v);
+      g += plane;
+    }
+  }
+  for (int i = threadIdx.x; i < 2 * CT_H * CB_Y * CB_Z; i += CT_THREADS) {
+    const int row = i / (2 * CT_H), c = i - row * 2 * CT_H, bx = c < CT_H ? c : c + CT_X;
+    const int v = box[row * CB_X + bx];
     if (v == 0) continue;
-    const int bx = i % CB_X, by = (i / CB_X) % CB_Y, bz = i / (CB_X * CB_Y);
-    /* box cells lie within one period of the tile */
-    int gx = org[0] + bx, gy = org[1] + by, gz = org[2] + bz;
+    const int bz = row / CB_Y, by = row - bz * CB_Y;
+    int gx = tx0 - CT_H + bx, gy = ty0 - CT_H + by, gz = tz0 - CT_H + bz;
     gx = gx < 0 ? gx + N : (gx >= N ? gx - N : gx);
     gy = gy < 0 ? gy + N : (gy >= N ? gy - N : gy);
     gz = gz < 0 ? gz + N : (gz >= N ? gz - N : gz);
     atomicAdd(&grid[pidx(gx, gy, gz, N)], v);
   }
+}
+
+template <int S>
+void deposit(unsigned tiles, cudaStream_t s, int *mass, const float *dx, const float *dy, const float *dz,
+             const cg_lpt_params &p)
+{
+  if (p.d2x) k_lpt_deposit<S, true><<<tiles, CT_THREADS, 0, s>>>(mass, dx, dy, dz, p);
+  else k_lpt_deposit<S, false><<<tiles, CT_THREADS, 0, s>>>(mass, dx, dy, dz, p);
 }
 
 /* compute_density_normalization after the bin sums (density.c:1272-1355):
@@ -563,8 +647,8 @@ cudaError_t cg_lpt_cic(cudaStream_t s, float *grid, const float *dx, const float
   /* the grid (zeroed by the caller) holds int32 fixed-point masses until
    * the density pass of mode CG_DMODE_RHO */
   int *mass = reinterpret_cast<int *>(grid);
-  if (p->interp == 0) k_lpt_deposit<0><<<(unsigned)tiles, 256, 0, s>>>(mass, dx, dy, dz, *p);
-  else if (p->interp == 2) k_lpt_deposit<2><<<(unsigned)tiles, 256, 0, s>>>(mass, dx, dy, dz, *p);
-  else k_lpt_deposit<1><<<(unsigned)tiles, 256, 0, s>>>(mass, dx, dy, dz, *p);
+  if (p->interp == 0) deposit<0>((unsigned)tiles, s, mass, dx, dy, dz, *p);
+  else if (p->interp == 2) deposit<2>((unsigned)tiles, s, mass, dx, dy, dz, *p);
+  else deposit<1>((unsigned)tiles, s, mass, dx, dy, dz, *p);
   return cudaGetLastError();
 }
