@@ -107,7 +107,8 @@ struct cg_ctx {
   int norm_nz = 0;
   int bins_nz_cap = 0, bins_nt_cap = 0;
   float4 *d_pk = nullptr;
-  float2 *d_twN = nullptr, *d_twH = nullptr;
+  float2 *d_twN = nullptr;
+  float4 *d_tws = nullptr; /* the field transforms' stage tables */
   Box box;
   FillParams fill;
   /* grids */
@@ -372,6 +373,18 @@ static cudaError_t run_lpt2(int n, const cg_field_launch *L)
 #undef X
   }
   return cudaErrorInvalidValue;
+}
+
+static int field_tables(int n, const float2 *twN, const float2 *twH, float4 *out)
+{
+  switch (n) {
+#define X(k) \
+  case k:    \
+    return cg_field_tables_##k(twN, twH, out);
+    CG_FIELD_SIZES(X)
+#undef X
+  }
+  return 0;
 }
 
 static int field_tile(int n, int pass, int v)
@@ -951,7 +964,7 @@ extern "C" void cg_destroy(cg_ctx *c)
     if (q) cudaFree(q);
   for (float *q : c->d_imap_out)
     if (q) cudaFree(q);
-  void *ptrs[] = {c->d_tabs, c->d_norm, c->d_tabs64, c->d_norm64, c->d_corner, c->d_att, c->d_xstats, c->d_zr, c->d_r2n, c->d_pk, c->d_twN, c->d_twH, c->d_dens, c->d_npot, c->d_disp[0],
+  void *ptrs[] = {c->d_tabs, c->d_norm, c->d_tabs64, c->d_norm64, c->d_corner, c->d_att, c->d_xstats, c->d_zr, c->d_r2n, c->d_pk, c->d_twN, c->d_tws, c->d_dens, c->d_npot, c->d_disp[0],
                   c->d_disp[1], c->d_disp[2], c->d_part, c->d_stats, c->d_s2f, c->d_err, c->d_ncount,
                   c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_seg, c->d_iseg, c->d_bsums, c->d_total, c->d_tmpmap, c->d_kmap,
                   c->d_kfac, c->d_kinv, c->d_kir, c->d_ovf_cell, c->d_ovf_cnt, c->d_ovf_n,
@@ -1003,9 +1016,11 @@ extern "C" int cg_create(cg_ctx **out, const cg_config *cfg, int device)
     std::vector<float2> tw(N), th(H);
     for (int j = 0; j < N; j++) tw[j] = make_float2((float)cos(2 * M_PI * j / N), (float)sin(2 * M_PI * j / N));
     for (int j = 0; j < H; j++) th[j] = make_float2((float)cos(2 * M_PI * j / H), (float)sin(2 * M_PI * j / H));
-    if ((rc = dalloc(c, &c->d_twN, (size_t)N)) || (rc = dalloc(c, &c->d_twH, (size_t)H))) return rc;
+    std::vector<float4> tab(field_tables(N, tw.data(), th.data(), nullptr));
+    field_tables(N, tw.data(), th.data(), tab.data());
+    if ((rc = dalloc(c, &c->d_twN, (size_t)N)) || (rc = dalloc(c, &c->d_tws, tab.size()))) return rc;
     CUDA_TRY(c, cudaMemcpy(c->d_twN, tw.data(), N * sizeof(float2), cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->d_twH, th.data(), H * sizeof(float2), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpy(c->d_tws, tab.data(), tab.size() * sizeof(float4), cudaMemcpyHostToDevice));
   }
   if ((rc = dalloc(c, &c->d_dens, c->grid_floats)) || (rc = dalloc(c, &c->d_npot, c->grid_floats))) return rc;
   c->npart = npartials(c->N);
@@ -1053,7 +1068,7 @@ extern "C" int cg_create_cartesian_fields(cg_ctx *c)
   L.norm = (float)std::pow(std::sqrt(2 * M_PI) / c->cfg.l_box, 3);
   L.partials = c->d_part;
   L.twN = c->d_twN;
-  L.twH = c->d_twH;
+  L.tws = c->d_tws;
   L.src = nullptr;
   L.err = c->d_err;
   L.ev = nullptr;
@@ -1112,7 +1127,7 @@ extern "C" int cg_compute_physical_density_field(cg_ctx *c)
     L.norm = 1.0f;
     L.partials = nullptr;
     L.twN = c->d_twN;
-    L.twH = c->d_twH;
+    L.tws = c->d_tws;
     L.err = c->d_err;
     {
       for (int a = 0; a < 3; a++) L.f[a] = reinterpret_cast<float2 *>(c->d_disp[a]);

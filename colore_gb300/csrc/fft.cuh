@@ -211,22 +211,66 @@ __host__ __device__ __forceinline__ int out_pos(int t, int i, int q)
   return (b / Ns) * Ns * r + (b % Ns) + q * Ns;
 }
 
-/* Twiddles and radix-r butterflies of one stage, data in v[i*r + q]. */
-template <int L, int R, int r, int Ns, int S>
-__host__ __device__ __forceinline__ void stage(float2 *v, int t, const float2 *__restrict__ twL)
+/* Twiddle exp(2 pi i q k / (Ns r)) of a stage, k < Ns, from the roots of unity
+ * of order L. */
+template <int L, int r, int Ns>
+__host__ __device__ __forceinline__ float2 root(const float2 *__restrict__ twL, int k, int q)
+{
+  return CG_LDG(&twL[(q * k) * (L / (Ns * r))]);
+}
+
+/* The same values laid out for a stage: pair p of k, twiddles q = 2p and
+ * 2p + 1, at p Ns + k, so threads of consecutive k read consecutive 16 bytes.
+ * Read from the roots, a warp's twiddles lay q L / (Ns r) apart: half of the y
+ * pass's global loads, at 6.5 sectors each.  y pass 410 -> 356 us at 512^3,
+ * both passes 6.23 -> 5.99 ms at 1024^3; the fills need a quarter fewer
+ * registers (80 -> 60 at 1024^3).  The x pass at 128^3 takes 2 us more. */
+struct StageTw {
+  const float4 *p;
+};
+template <int r0, int r1, int r2>
+constexpr int tw_len = r1 == 1 ? 0 : (r1 * r0 + (r2 == 1 ? 0 : r2 * r0 * r1)) / 2;
+/* The tables of a length-L transform's stages 1 and 2. */
+template <int L, int r0, int r1, int r2>
+void tw_build(const float2 *roots, float4 *out)
+{
+  static_assert((r1 == 1 || r1 % 2 == 0) && (r2 == 1 || r2 % 2 == 0), "twiddles in pairs");
+  for (int s = 1; s < 3; s++) {
+    const int r = s == 1 ? r1 : r2, Ns = s == 1 ? r0 : r0 * r1;
+    for (int p = 0; r > 1 && p < r / 2; p++)
+      for (int k = 0; k < Ns; k++) {
+        const float2 a = roots[2 * p * k * (L / (Ns * r))], b = roots[(2 * p + 1) * k * (L / (Ns * r))];
+        *out++ = make_float4(a.x, a.y, b.x, b.y);
+      }
+  }
+}
+
+template <int L, int r, int Ns, int S>
+__host__ __device__ __forceinline__ void twiddle(float2 *v, int k, const float2 *__restrict__ twL)
+{
+#pragma unroll
+  for (int q = 1; q < r; q++) v[q] = cmulS<S>(v[q], root<L, r, Ns>(twL, k, q));
+}
+template <int L, int r, int Ns, int S>
+__host__ __device__ __forceinline__ void twiddle(float2 *v, int k, StageTw tw)
+{
+#pragma unroll
+  for (int p = 0; p < r / 2; p++) {
+    const float4 w = CG_LDG(&tw.p[p * Ns + k]);
+    if (p > 0) v[2 * p] = cmulS<S>(v[2 * p], make_float2(w.x, w.y));
+    v[2 * p + 1] = cmulS<S>(v[2 * p + 1], make_float2(w.z, w.w));
+  }
+}
+
+/* Twiddles and radix-r butterflies of one stage, data in v[i*r + q].  tw: the
+ * roots, or the stage's table. */
+template <int L, int R, int r, int Ns, int S, class Tw>
+__host__ __device__ __forceinline__ void stage(float2 *v, int t, Tw tw)
 {
   constexpr int NB = R / r;
 #pragma unroll
   for (int i = 0; i < NB; i++) {
-    if (Ns > 1) {
-      int b = t + (L / R) * i;
-      int k = b % Ns;
-#pragma unroll
-      for (int q = 1; q < r; q++) {
-        float2 w = CG_LDG(&twL[(q * k) * (L / (Ns * r))]);
-        v[i * r + q] = cmulS<S>(v[i * r + q], w);
-      }
-    }
+    if (Ns > 1) twiddle<L, r, Ns, S>(&v[i * r], (t + (L / R) * i) % Ns, tw);
     DFT<r, S>::run(&v[i * r]);
   }
 }
@@ -267,19 +311,20 @@ __host__ __device__ __forceinline__ int pad_at(int base, int off, bool base_alig
  * for one) by P = L/R threads.  Ld(pos) -> float2 supplies the input,
  * St(pos, value) consumes the output, Sm(slot) -> float2& addresses slot
  * 0..pad_len(L, SH)-1 of this transform's shared-memory exchange buffer
- * (SH: pad_shift(r0) or NO_PAD).
+ * (SH: pad_shift(r0) or NO_PAD).  tw: the stages' tables (tw_build).
  * Contains the barriers of the exchanges, so every thread of the block must
  * call it.
  */
 template <int L, int R, int r0, int r1, int r2, int S, int SH, class Ld, class St, class Sm>
-__device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL, Ld ld, St st, Sm sm)
+__device__ __forceinline__ void transform(int t, const float4 *__restrict__ tw, Ld ld, St st, Sm sm)
 {
   float2 v[R];
+  const StageTw tw1{tw}, tw2{tw + r0 * r1 / 2};
 #pragma unroll
   for (int i = 0; i < R / r0; i++)
 #pragma unroll
     for (int q = 0; q < r0; q++) v[i * r0 + q] = ld(in_pos<L, R, r0>(t, i, q));
-  stage<L, R, r0, 1, S>(v, t, twL);
+  stage<L, R, r0, 1, S>(v, t, tw1);
   if (r1 == 1) {
 #pragma unroll
     for (int i = 0; i < R / r0; i++)
@@ -298,7 +343,7 @@ __device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL,
   for (int i = 0; i < R / r1c; i++)
 #pragma unroll
     for (int q = 0; q < r1c; q++) v[i * r1c + q] = sm(pad_at<SH>(t, (L / R) * i + q * (L / r1c), false));
-  stage<L, R, r1c, r0, S>(v, t, twL);
+  stage<L, R, r1c, r0, S>(v, t, tw1);
   if (r2 == 1) {
 #pragma unroll
     for (int i = 0; i < R / r1c; i++)
@@ -317,7 +362,7 @@ __device__ __forceinline__ void transform(int t, const float2 *__restrict__ twL,
   for (int i = 0; i < R / r2c; i++)
 #pragma unroll
     for (int q = 0; q < r2c; q++) v[i * r2c + q] = sm(pad_at<SH>(t, (L / R) * i + q * (L / r2c), false));
-  stage<L, R, r2c, r0 * r1c, S>(v, t, twL);
+  stage<L, R, r2c, r0 * r1c, S>(v, t, tw2);
 #pragma unroll
   for (int i = 0; i < R / r2c; i++)
 #pragma unroll

@@ -17,7 +17,7 @@ struct cg_field_launch {
   float norm;           /* real-space scale applied in the x pass    */
   double2 *partials;    /* per-block (sum d, sum d^2) of grid 0       */
   const float2 *twN;    /* exp(+2 pi i j/N), j < N                   */
-  const float2 *twH;    /* exp(+2 pi i j/(N/2)), j < N/2             */
+  const float4 *tws;    /* the transforms' stage tables (cg_field_tables_) */
   float2 *src;          /* 2LPT: the source grid (padded real in, destroyed) */
   unsigned int *err;    /* device error word (bulk-copy timeouts) */
   cudaEvent_t *ev;      /* NULL, or events recorded after each pass (fill+z, y, x) */
@@ -37,6 +37,7 @@ struct cg_field_launch {
   extern "C" cudaError_t cg_field_lpt_##n(const cg_field_launch *L);   \
   extern "C" cudaError_t cg_field_lpt2_##n(const cg_field_launch *L);  \
   extern "C" size_t cg_field_npartials_##n(void);                      \
+  extern "C" int cg_field_tables_##n(const float2 *twN, const float2 *twH, float4 *out); \
   extern "C" int cg_field_tile_##n(int pass, int v);                    \
   extern "C" cudaError_t cg_field_pass_##n(const cg_field_launch *L, int pass, int v, int nf);
 CG_FIELD_SIZES(CG_FIELD_DECL)

@@ -65,6 +65,10 @@ constexpr int FSH = fill_sh(TX);
 constexpr int SHX = cgfft::pad_shift(PL::R0);
 constexpr int EXX = cgfft::pad_len(LH, SHX);
 constexpr int ROWS = NH > EXX ? NH : EXX; /* smem per row */
+/* Stage tables of the column, fill and row transforms, one after the other. */
+constexpr int TW_C = 0, TW_F = TW_C + cgfft::tw_len<PL::C0, PL::C1, PL::C2>;
+constexpr int TW_R = TW_F + cgfft::tw_len<PL::F0, PL::F1, PL::F2>;
+constexpr int TW_LEN = TW_R + cgfft::tw_len<PL::R0, PL::R1, PL::R2>;
 template <int TX>
 constexpr int EXF = cgfft::pad_len(N, fill_sh(TX)); /* exchange slots per column of the fills */
 
@@ -172,7 +176,7 @@ __device__ __forceinline__ void k_pairs(const FillParams &p, float num, int kx, 
  * first exchange write. */
 template <int TX>
 __global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, FillParams p,
-                                                  const float2 *__restrict__ twN)
+                                                  const float4 *__restrict__ tw)
 {
   extern __shared__ float2 smem[];
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, FillP
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, twN, ld, st, sm);
+    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, tw + TW_F, ld, st, sm);
     __syncthreads();
   }
 }
@@ -252,7 +256,7 @@ __device__ __forceinline__ float2 lpt_field(const FillParams &p, int j, int kx, 
  * instead of three per block, so three blocks fit on an SM. */
 template <int TX>
 __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, float2 *o2, FillParams p,
-                                                       const float2 *__restrict__ twN)
+                                                       const float4 *__restrict__ tw)
 {
   extern __shared__ float2 smem[];
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, f
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, twN, ld, st, sm);
+    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, tw + TW_F, ld, st, sm);
     __syncthreads();
   }
 }
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, f
  * S = -1).  grid = (ceil(NH/TX), N, nf). */
 template <int TX, int S>
 __global__ void __launch_bounds__(TX *P) k_col_y(float2 *f0, float2 *f1, float2 *f2,
-                                                 const float2 *__restrict__ twN)
+                                                 const float4 *__restrict__ tw)
 {
   extern __shared__ float2 smem[];
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(TX *P) k_col_y(float2 *f0, float2 *f1, float2 
   auto st = [&](int pos, float2 v) {
     if (ok) base[(size_t)pos * NH] = v;
   };
-  cgfft::transform<N, PL::CR, PL::C0, PL::C1, PL::C2, S, cgfft::NO_PAD>(t, twN, ld, st, sm);
+  cgfft::transform<N, PL::CR, PL::C0, PL::C1, PL::C2, S, cgfft::NO_PAD>(t, tw + TW_C, ld, st, sm);
 }
 
 /* Forward pass 1 of the 2LPT source: row r2c along x, in place.  A row's N
@@ -305,7 +309,7 @@ __global__ void __launch_bounds__(TX *P) k_col_y(float2 *f0, float2 *f1, float2 
  * The half-length spectrum goes to its own shared buffer: the exchange
  * buffer may still be read by other threads when the last stage stores. */
 __global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 *__restrict__ twN,
-                                                        const float2 *__restrict__ twH, unsigned int *err)
+                                                        const float4 *__restrict__ tw, unsigned int *err)
 {
   extern __shared__ __align__(16) float2 smem[];
   __shared__ uint64_t bar;
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 
   auto ld = [&](int j) -> float2 { return rin[j]; };
   auto sm = [&](int slot) -> float2 & { return row[slot]; };
   auto st = [&](int n, float2 v) { z[n] = v; };
-  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, -1, SHX>(t, twH, ld, st, sm);
+  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, -1, SHX>(t, tw + TW_R, ld, st, sm);
   __syncthreads();
   float2 *dst = f + (row0 + rl) * NH;
   for (int k = t; k <= LH; k += PR) {
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 
 template <int TX>
 __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ src, float2 *o0, float2 *o1,
                                                    float2 *o2, float dk, float inv_n3,
-                                                   const float2 *__restrict__ twN)
+                                                   const float4 *__restrict__ tw)
 {
   extern __shared__ float2 smem[];
   float2 *X = smem + (size_t)EXF<TX> * TX;
@@ -349,7 +353,7 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
   auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
   auto ld = [&](int pos) -> float2 { return ok ? src[((size_t)pos * N + ky) * NH + kx] : make_float2(0.0f, 0.0f); };
   auto stx = [&](int pos, float2 v) { X[pos * TX + c] = v; };
-  cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, -1, FSH<TX>>(t, twN, ld, stx, sm);
+  cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, -1, FSH<TX>>(t, tw + TW_F, ld, stx, sm);
   __syncthreads();
   float2 *outs[3] = {o0, o1, o2};
   const float kxf = (float)kx * dk, kyf = kcomp(ky, N, dk);
@@ -368,7 +372,7 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
     auto st = [&](int pos, float2 v) {
       if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
     };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, twN, ld2, st, sm);
+    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, tw + TW_F, ld2, st, sm);
     __syncthreads();
   }
 }
@@ -379,7 +383,7 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
 template <bool STATS, int RB>
 __global__ void __launch_bounds__(RB *PR) k_row_c2r(float2 *f0, float2 *f1, float2 *f2, float norm,
                                                         double2 *partials, const float2 *__restrict__ twN,
-                                                        const float2 *__restrict__ twH, unsigned int *err)
+                                                        const float4 *__restrict__ tw, unsigned int *err)
 {
   extern __shared__ __align__(16) float2 smem[];
   __shared__ uint64_t bar;
@@ -416,7 +420,7 @@ __global__ void __launch_bounds__(RB *PR) k_row_c2r(float2 *f0, float2 *f1, floa
       s2 += r.x * r.x + r.y * r.y;
     }
   };
-  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, 1, SHX>(t, twH, ld, st, sm);
+  cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, 1, SHX>(t, tw + TW_R, ld, st, sm);
   if (STATS) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -479,7 +483,7 @@ cudaError_t fill2(const cg_field_launch *L)
     cudaError_t e = prep(k_fill_z<T>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N);
-    k_fill_z<T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], L->fill, L->twN);
+    k_fill_z<T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], L->fill, L->tws);
     return cudaGetLastError();
   }
 }
@@ -494,7 +498,7 @@ cudaError_t fill3(const cg_field_launch *L)
     cudaError_t e = prep(k_fill_z3<T>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N);
-    k_fill_z3<T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], L->f[2], L->fill, L->twN);
+    k_fill_z3<T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], L->f[2], L->fill, L->tws);
     return cudaGetLastError();
   }
 }
@@ -509,7 +513,7 @@ cudaError_t ypass(const cg_field_launch *L, float2 *a, float2 *b, float2 *c, int
     cudaError_t e = prep(k_col_y<T, S>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N, nf);
-    k_col_y<T, S><<<g, T * P, sm, L->stream>>>(a, b, c, L->twN);
+    k_col_y<T, S><<<g, T * P, sm, L->stream>>>(a, b, c, L->tws);
     return cudaGetLastError();
   }
 }
@@ -524,7 +528,7 @@ cudaError_t xpass(const cg_field_launch *L, float2 *a, float2 *b, float2 *c, int
     cudaError_t e = prep(k_row_c2r<STATS, R>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((unsigned)((size_t)N * N / R), nf);
-    k_row_c2r<STATS, R><<<g, R * PR, sm, L->stream>>>(a, b, c, norm, part, L->twN, L->twH, L->err);
+    k_row_c2r<STATS, R><<<g, R * PR, sm, L->stream>>>(a, b, c, norm, part, L->twN, L->tws, L->err);
     return cudaGetLastError();
   }
 }
@@ -613,16 +617,28 @@ extern "C" cudaError_t CG_CAT(cg_field_lpt2_, CG_N)(const cg_field_launch *L)
   if ((e = prep(k_row_r2c, smr)) != cudaSuccess) return e;
   if ((e = prep(k_z_lpt2<TX3>, smz)) != cudaSuccess) return e;
   dim3 gr((unsigned)((size_t)N * N / PL::RB), 1);
-  k_row_r2c<<<gr, PL::RB * PR, smr, L->stream>>>(L->src, L->twN, L->twH, L->err);
+  k_row_r2c<<<gr, PL::RB * PR, smr, L->stream>>>(L->src, L->twN, L->tws, L->err);
   if ((e = ypass_v<-1>(L, L->var[CG_PASS_Y], L->src, nullptr, nullptr, 1)) != cudaSuccess) return e;
   dim3 gz((NH + TX3 - 1) / TX3, N);
   const float inv_n3 = 1.0f / ((float)N * (float)N * (float)N);
-  k_z_lpt2<TX3><<<gz, TX3 * PF, smz, L->stream>>>(L->src, L->f[0], L->f[1], L->f[2], L->fill.dk, inv_n3, L->twN);
+  k_z_lpt2<TX3><<<gz, TX3 * PF, smz, L->stream>>>(L->src, L->f[0], L->f[1], L->f[2], L->fill.dk, inv_n3, L->tws);
   if ((e = ypass_v<1>(L, L->var[CG_PASS_Y], L->f[0], L->f[1], L->f[2], 3)) != cudaSuccess) return e;
   cg_field_launch L1 = *L;
   L1.norm = 1.0f;
   if ((e = xpass_v(&L1, L->var[CG_PASS_X], L->f[0], L->f[1], L->f[2], 3)) != cudaSuccess) return e;
   return cudaGetLastError();
+}
+
+/* The transforms' stage tables (cg_field_launch.tws) from the roots of unity of
+ * orders N and N/2; out may be NULL.  Returns their number of float4. */
+extern "C" int CG_CAT(cg_field_tables_, CG_N)(const float2 *twN, const float2 *twH, float4 *out)
+{
+  if (out) {
+    cgfft::tw_build<N, PL::C0, PL::C1, PL::C2>(twN, out + TW_C);
+    cgfft::tw_build<N, PL::F0, PL::F1, PL::F2>(twN, out + TW_F);
+    cgfft::tw_build<LH, PL::R0, PL::R1, PL::R2>(twH, out + TW_R);
+  }
+  return TW_LEN;
 }
 
 /* Number of blocks of the moment-sum pass (size of the partials array). */
