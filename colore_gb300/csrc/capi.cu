@@ -1069,7 +1069,7 @@ extern "C" int cg_create_cartesian_fields(cg_ctx *c)
   L.partials = c->d_part;
   L.twN = c->d_twN;
   L.tws = c->d_tws;
-  L.src = nullptr;
+  memset(L.f2, 0, sizeof(L.f2));
   L.err = c->d_err;
   L.ev = nullptr;
   {
@@ -1134,28 +1134,18 @@ extern "C" int cg_compute_physical_density_field(cg_ctx *c)
       const int passes[3] = {CG_PASS_FILL3, CG_PASS_Y, CG_PASS_X}, nfs[3] = {3, 3, 3};
       if (int rc = tune_field_passes(c, &L, passes, nfs, 3)) return rc;
     }
-    if (two) { /* lpt_2, density.c:646-812 */
-      ProfScope ps(c, "lpt2_fft");
-      for (int set = 0; set < 2; set++) { /* xx xy xz, then yy yz zz */
-        L.fill.lpt_kind = 1 + set;
-        for (int a = 0; a < 3; a++) L.f[a] = reinterpret_cast<float2 *>(c->d_lpt2[3 * set + a]);
-        CUDA_TRY(c, run_lpt(c->N, &L));
-      }
-      CUDA_TRY(c, cg_lpt2_source(c->stream, c->d_lpt2[0], c->d_lpt2[1], c->d_lpt2[2], c->d_lpt2[3], c->d_lpt2[4],
-                                 c->d_lpt2[5], c->N, c->nsm));
-      L.src = reinterpret_cast<float2 *>(c->d_lpt2[5]);
-      for (int a = 0; a < 3; a++) L.f[a] = reinterpret_cast<float2 *>(c->d_lpt2[a]);
-      CUDA_TRY(c, run_lpt2(c->N, &L));
-      c->launches += 2 * 3 + 1 + 5;
-    }
-    L.fill.lpt_kind = 0;
-    for (int a = 0; a < 3; a++) L.f[a] = reinterpret_cast<float2 *>(c->d_disp[a]);
+    for (int a = 0; two && a < 6; a++) L.f2[a] = reinterpret_cast<float2 *>(c->d_lpt2[a]);
     {
       ProfScope ps(c, "lpt_fft");
       PassEvents pe(c, "lpt_fill", "lpt_y", "lpt_x");
       L.ev = pe.after();
       CUDA_TRY(c, run_lpt(c->N, &L));
       L.ev = nullptr;
+    }
+    if (two) { /* lpt_2, density.c:646-812 */
+      ProfScope ps(c, "lpt2_fft");
+      CUDA_TRY(c, run_lpt2(c->N, &L));
+      c->launches += 9;
     }
     ProfScope ps2(c, "lpt_cic");
     CUDA_TRY(c, cudaMemsetAsync(c->d_dens, 0, c->grid_floats * sizeof(float), c->stream));

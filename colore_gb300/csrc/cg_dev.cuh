@@ -173,7 +173,6 @@ struct FillParams {
   float logkmin, logkmax, idlogk, n_scal;
   uint32_t rk0[10], rk1[10]; /* Philox round keys: (seed, stream) plus r times the Weyl constants */
   float lpt_norm; /* (sqrt(2 pi)/L)^3, used by the 1LPT displacement fill */
-  int lpt_kind;   /* three-field fill: 0 Psi_x,y,z; 1 phi_xx,xy,xz; 2 phi_yy,yz,zz */
 };
 
 /* Geometry of the Cartesian box. */

@@ -18,7 +18,7 @@ struct cg_field_launch {
   double2 *partials;    /* per-block (sum d, sum d^2) of grid 0       */
   const float2 *twN;    /* exp(+2 pi i j/N), j < N                   */
   const float4 *tws;    /* the transforms' stage tables (cg_field_tables_) */
-  float2 *src;          /* 2LPT: the source grid (padded real in, destroyed) */
+  float2 *f2[6];        /* 2LPT: the second derivatives xx xy xz yy yz zz, else NULL */
   unsigned int *err;    /* device error word (bulk-copy timeouts) */
   cudaEvent_t *ev;      /* NULL, or events recorded after each pass (fill+z, y, x) */
   int var[4];           /* tile variant of each pass (CG_PASS_*): 0 the plan's, 1 half, 2 twice */

@@ -219,9 +219,9 @@ __global__ void __launch_bounds__(TX *PF) k_fill_z(float2 *o0, float2 *o1, FillP
 /* The three-field fills: 1LPT displacements i k_a delta'_k / (N^3 k^2)
  * (density.c:430-436), where delta'_k = r2c(delta_G) = N^3 norm H(delta_k)
  * and H is the Hermitian projection that the c2r applied on the kx = 0 and
- * kx = N/2 planes; with lpt_kind 1 or 2 the second derivatives
+ * kx = N/2 planes; of kind 1 and 2 the second derivatives
  * i k_i (i k_j delta'_k / (N^3 k^2)) of 2LPT (density.c:704-709), xx xy xz
- * or yy yz zz.  One value per mode is kept, b = delta'_k / (N^3 k^2) with
+ * and yy yz zz.  One value per mode is kept, b = delta'_k / (N^3 k^2) with
  * the smoothing (0 at k = 0), and each field is formed from it as the
  * transform loads it.  The projection's partner -k has the same amplitude. */
 __device__ __forceinline__ float2 lpt_base(const FillParams &p, const KAmp &a, int kx, int ky, int kz)
@@ -240,23 +240,29 @@ __device__ __forceinline__ float2 lpt_base(const FillParams &p, const KAmp &a, i
   return make_float2(a.ik2 * d.x, a.ik2 * d.y);
 }
 
-__device__ __forceinline__ float2 lpt_field(const FillParams &p, int j, int kx, int ky, int kz, float2 b)
+__device__ __forceinline__ float2 lpt_field(const FillParams &p, int kind, int j, int kx, int ky, int kz, float2 b)
 {
   const float kv[3] = {(float)kx * p.dk, kcomp(ky, N, p.dk), kcomp(kz, N, p.dk)};
-  if (p.lpt_kind == 0) return make_float2(-kv[j] * b.y, kv[j] * b.x);
-  const float ki[3] = {p.lpt_kind == 1 ? kv[0] : kv[1], p.lpt_kind == 1 ? kv[0] : kv[1], p.lpt_kind == 1 ? kv[0] : kv[2]};
-  const float kj[3] = {p.lpt_kind == 1 ? kv[0] : kv[1], p.lpt_kind == 1 ? kv[1] : kv[2], kv[2]};
+  if (kind == 0) return make_float2(-kv[j] * b.y, kv[j] * b.x);
+  const float ki[3] = {kind == 1 ? kv[0] : kv[1], kind == 1 ? kv[0] : kv[1], kind == 1 ? kv[0] : kv[2]};
+  const float kj[3] = {kind == 1 ? kv[0] : kv[1], kind == 1 ? kv[1] : kv[2], kv[2]};
   const float g = -ki[j] * kj[j];
   return make_float2(g * b.x, g * b.y);
 }
 
+/* Grids of a three-field fill: Psi, then for 2LPT the six second derivatives. */
+struct Lpt9 {
+  float2 *o[9];
+};
+
 /* Pass 1 of the three-field fills: as k_fill_z, but one value per mode
  * (lpt_base) is parked, in the slot after the exchange buffer, and the first
  * stage of each transform forms the field from it (lpt_field).  Two slots
- * instead of three per block, so three blocks fit on an SM. */
-template <int TX>
-__global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, float2 *o2, FillParams p,
-                                                       const float4 *__restrict__ tw)
+ * instead of three per block, so three blocks fit on an SM.  SETS 1 the
+ * displacements, 3 the second derivatives too: the modes are drawn once for
+ * all nine grids (a third of the time of a three-field fill). */
+template <int TX, int SETS>
+__global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(Lpt9 out, FillParams p, const float4 *__restrict__ tw)
 {
   extern __shared__ float2 smem[];
   const int c = threadIdx.x % TX, t = threadIdx.x / TX;
@@ -265,19 +271,21 @@ __global__ void __launch_bounds__(TX *PF, 3) k_fill_z3(float2 *o0, float2 *o1, f
   float2 *base = smem + (size_t)EXF<TX> * TX;
   if (ok) k_pairs(p, p.lpt_norm, kx, ky, t, [&](int kz, const KAmp &a) { base[kz * TX + c] = lpt_base(p, a, kx, ky, kz); });
   __syncthreads();
-  float2 *outs[3] = {o0, o1, o2};
   auto sm = [&](int slot) -> float2 & { return smem[slot * TX + c]; };
+#pragma unroll 1
+  for (int kind = 0; kind < SETS; kind++) {
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    auto ld = [&](int pos) -> float2 {
-      return ok ? lpt_field(p, j, kx, ky, pos, base[pos * TX + c]) : make_float2(0.0f, 0.0f);
-    };
-    float2 *o = outs[j];
-    auto st = [&](int pos, float2 v) {
-      if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
-    };
-    cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, tw + TW_F, ld, st, sm);
-    __syncthreads();
+    for (int j = 0; j < 3; j++) {
+      auto ld = [&](int pos) -> float2 {
+        return ok ? lpt_field(p, SETS == 1 ? 0 : kind, j, kx, ky, pos, base[pos * TX + c]) : make_float2(0.0f, 0.0f);
+      };
+      float2 *o = out.o[3 * kind + j];
+      auto st = [&](int pos, float2 v) {
+        if (ok) o[((size_t)pos * N + ky) * NH + kx] = v;
+      };
+      cgfft::transform<N, PL::FR, PL::F0, PL::F1, PL::F2, 1, FSH<TX>>(t, tw + TW_F, ld, st, sm);
+      __syncthreads();
+    }
   }
 }
 
@@ -301,22 +309,44 @@ __global__ void __launch_bounds__(TX *P) k_col_y(float2 *f0, float2 *f1, float2 
   cgfft::transform<N, PL::CR, PL::C0, PL::C1, PL::C2, S, cgfft::NO_PAD>(t, tw + TW_C, ld, st, sm);
 }
 
-/* Forward pass 1 of the 2LPT source: row r2c along x, in place.  A row's N
- * reals are read as N/2 complex z_j = x_2j + i x_2j+1, transformed forward,
- * and split into the N/2 + 1 modes
+/* Forward pass 1 of the 2LPT source (density.c:739-759): row r2c along x of
+ *   xx yy + xx zz + yy zz - xy^2 - xz^2 - yz^2,
+ * formed as the rows of the six second derivatives (d: xx xy xz yy yz zz) are
+ * loaded, into the rows of zz (a block reads its rows before it writes them).
+ * A row's N reals are read as N/2 complex z_j = x_2j + i x_2j+1, transformed
+ * forward, and split into the N/2 + 1 modes
  *   X_k = (E_k - i e^{-2 pi i k/N} O_k) / 2,  E_k = Z_k + conj Z_{N/2-k},
  *   O_k = Z_k - conj Z_{N/2-k}  (Z_{N/2} = Z_0).
  * The half-length spectrum goes to its own shared buffer: the exchange
- * buffer may still be read by other threads when the last stage stores. */
-__global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 *__restrict__ twN,
-                                                        const float4 *__restrict__ tw, unsigned int *err)
+ * buffer may still be read by other threads when the last stage stores.
+ * Bound by the six reads: 106 us at 256^3, 115 with the source in a kernel of
+ * its own. */
+struct Lpt6 {
+  float2 *d[6];
+};
+
+__device__ __forceinline__ float lpt2_source(float a, float e, float f, float b, float g, float d)
+{
+  const float v = CG_ADD(CG_ADD(CG_MUL(a, b), CG_MUL(a, d)), CG_MUL(b, d));
+  return CG_SUB(CG_SUB(CG_SUB(v, CG_MUL(e, e)), CG_MUL(f, f)), CG_MUL(g, g));
+}
+
+__global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(Lpt6 in, const float2 *__restrict__ twN,
+                                                        const float4 *__restrict__ tw)
 {
   extern __shared__ __align__(16) float2 smem[];
-  __shared__ uint64_t bar;
   float2 *zb = smem + PL::RB * ROWS;
   const int t = threadIdx.x % PR, rl = threadIdx.x / PR;
-  const size_t row0 = (size_t)blockIdx.x * PL::RB;
-  if (!cgtma::stage_rows(smem, f + row0 * NH, (unsigned)(PL::RB * NH * sizeof(float2)), &bar, err)) return;
+  /* the block's rows are contiguous: their source at a stride of NH, as the c2r
+   * rows of k_row_c2r, before the transform exchanges at the stride ROWS */
+  const size_t b0 = (size_t)blockIdx.x * PL::RB * NH;
+#pragma unroll 2
+  for (int i = threadIdx.x; i < PL::RB * NH; i += PL::RB * PR) {
+    const float2 a = in.d[0][b0 + i], e = in.d[1][b0 + i], f = in.d[2][b0 + i];
+    const float2 b = in.d[3][b0 + i], g = in.d[4][b0 + i], d = in.d[5][b0 + i];
+    smem[i] = make_float2(lpt2_source(a.x, e.x, f.x, b.x, g.x, d.x), lpt2_source(a.y, e.y, f.y, b.y, g.y, d.y));
+  }
+  __syncthreads();
   const float2 *rin = smem + rl * NH;
   float2 *row = smem + rl * ROWS;
   float2 *z = zb + rl * LH;
@@ -325,7 +355,7 @@ __global__ void __launch_bounds__(PL::RB *PR) k_row_r2c(float2 *f, const float2 
   auto st = [&](int n, float2 v) { z[n] = v; };
   cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, -1, SHX>(t, tw + TW_R, ld, st, sm);
   __syncthreads();
-  float2 *dst = f + (row0 + rl) * NH;
+  float2 *dst = in.d[5] + b0 + (size_t)rl * NH;
   for (int k = t; k <= LH; k += PR) {
     const float2 a = z[k == LH ? 0 : k], b = z[k == 0 ? 0 : LH - k];
     const float2 e = make_float2(a.x + b.x, a.y - b.y), o = make_float2(a.x - b.x, a.y + b.y);
@@ -488,17 +518,19 @@ cudaError_t fill2(const cg_field_launch *L)
   }
 }
 
-template <int T>
+template <int T, int SETS>
 cudaError_t fill3(const cg_field_launch *L)
 {
   if constexpr (!fill_ok(T)) {
     return cudaErrorInvalidValue;
   } else {
     const size_t sm = fill_smem(T); /* one value per mode + the exchange buffer */
-    cudaError_t e = prep(k_fill_z3<T>, sm);
+    cudaError_t e = prep(k_fill_z3<T, SETS>, sm);
     if (e != cudaSuccess) return e;
     dim3 g((NH + T - 1) / T, N);
-    k_fill_z3<T><<<g, T * PF, sm, L->stream>>>(L->f[0], L->f[1], L->f[2], L->fill, L->tws);
+    Lpt9 o;
+    for (int j = 0; j < 9; j++) o.o[j] = j < 3 ? L->f[j] : L->f2[j - 3];
+    k_fill_z3<T, SETS><<<g, T * PF, sm, L->stream>>>(o, L->fill, L->tws);
     return cudaGetLastError();
   }
 }
@@ -545,9 +577,9 @@ cudaError_t fill2_v(const cg_field_launch *L, int v)
 cudaError_t fill3_v(const cg_field_launch *L, int v)
 {
   switch (v) {
-    case 1: return fill3<tile_of(PL::TX3, 1)>(L);
-    case 2: return fill3<tile_of(PL::TX3, 2)>(L);
-    default: return fill3<PL::TX3>(L);
+    case 1: return fill3<tile_of(PL::TX3, 1), 1>(L);
+    case 2: return fill3<tile_of(PL::TX3, 2), 1>(L);
+    default: return fill3<PL::TX3, 1>(L);
   }
 }
 
@@ -590,12 +622,16 @@ extern "C" cudaError_t CG_CAT(cg_field_gauss_, CG_N)(const cg_field_launch *L)
   return cudaGetLastError();
 }
 
-/* 1LPT displacement fields Psi_x,y,z: passes 1-3 on three grids. */
+/* 1LPT displacement fields Psi_x,y,z: passes 1-3 on three grids; with L->f2[0]
+ * set, pass 1 also of the second derivatives in L->f2 (cg_field_lpt2_). */
 extern "C" cudaError_t CG_CAT(cg_field_lpt_, CG_N)(const cg_field_launch *L)
 {
   using namespace cg;
   cudaError_t e;
-  if ((e = fill3_v(L, L->var[CG_PASS_FILL3])) != cudaSuccess) return e;
+  /* nine fields share the modes of the plan's tile: the half tile that wins with
+   * three fields loses here (256^3: 303 against 248 us, three apart 312) */
+  e = L->f2[0] ? fill3<PL::TX3, 3>(L) : fill3_v(L, L->var[CG_PASS_FILL3]);
+  if (e != cudaSuccess) return e;
   if (L->ev) cudaEventRecord(L->ev[0], L->stream);
   if ((e = ypass_v<1>(L, L->var[CG_PASS_Y], L->f[0], L->f[1], L->f[2], 3)) != cudaSuccess) return e;
   if (L->ev) cudaEventRecord(L->ev[1], L->stream);
@@ -604,9 +640,10 @@ extern "C" cudaError_t CG_CAT(cg_field_lpt_, CG_N)(const cg_field_launch *L)
   return cudaGetLastError();
 }
 
-/* 2LPT second-order displacements from the source grid L->src (padded
- * real, overwritten): r2c along x, forward y, the fused z pass into
- * L->f[0..2], then the inverse y and x passes of those three grids. */
+/* 2LPT second-order displacements from the second derivatives L->f2, which
+ * cg_field_lpt_ has filled (xx xy xz yy yz zz, destroyed): their y and x passes,
+ * the source with its r2c along x, forward y, the fused z pass into L->f2[0..2],
+ * then the inverse y and x passes of those three grids. */
 extern "C" cudaError_t CG_CAT(cg_field_lpt2_, CG_N)(const cg_field_launch *L)
 {
   using namespace cg;
@@ -617,15 +654,23 @@ extern "C" cudaError_t CG_CAT(cg_field_lpt2_, CG_N)(const cg_field_launch *L)
   if ((e = prep(k_row_r2c, smr)) != cudaSuccess) return e;
   if ((e = prep(k_z_lpt2<TX3>, smz)) != cudaSuccess) return e;
   dim3 gr((unsigned)((size_t)N * N / PL::RB), 1);
-  k_row_r2c<<<gr, PL::RB * PR, smr, L->stream>>>(L->src, L->twN, L->tws, L->err);
-  if ((e = ypass_v<-1>(L, L->var[CG_PASS_Y], L->src, nullptr, nullptr, 1)) != cudaSuccess) return e;
-  dim3 gz((NH + TX3 - 1) / TX3, N);
-  const float inv_n3 = 1.0f / ((float)N * (float)N * (float)N);
-  k_z_lpt2<TX3><<<gz, TX3 * PF, smz, L->stream>>>(L->src, L->f[0], L->f[1], L->f[2], L->fill.dk, inv_n3, L->tws);
-  if ((e = ypass_v<1>(L, L->var[CG_PASS_Y], L->f[0], L->f[1], L->f[2], 3)) != cudaSuccess) return e;
   cg_field_launch L1 = *L;
   L1.norm = 1.0f;
-  if ((e = xpass_v(&L1, L->var[CG_PASS_X], L->f[0], L->f[1], L->f[2], 3)) != cudaSuccess) return e;
+  const int vy = L->var[CG_PASS_Y], vx = L->var[CG_PASS_X];
+  Lpt6 in;
+  for (int a = 0; a < 6; a++) in.d[a] = L->f2[a];
+  float2 **f = in.d, *src = in.d[5];
+  for (int a = 0; a < 6; a += 3)
+    if ((e = ypass_v<1>(L, vy, f[a], f[a + 1], f[a + 2], 3)) != cudaSuccess ||
+        (e = xpass_v(&L1, vx, f[a], f[a + 1], f[a + 2], 3)) != cudaSuccess)
+      return e;
+  k_row_r2c<<<gr, PL::RB * PR, smr, L->stream>>>(in, L->twN, L->tws);
+  if ((e = ypass_v<-1>(L, vy, src, nullptr, nullptr, 1)) != cudaSuccess) return e;
+  dim3 gz((NH + TX3 - 1) / TX3, N);
+  const float inv_n3 = 1.0f / ((float)N * (float)N * (float)N);
+  k_z_lpt2<TX3><<<gz, TX3 * PF, smz, L->stream>>>(src, f[0], f[1], f[2], L->fill.dk, inv_n3, L->tws);
+  if ((e = ypass_v<1>(L, vy, f[0], f[1], f[2], 3)) != cudaSuccess) return e;
+  if ((e = xpass_v(&L1, vx, f[0], f[1], f[2], 3)) != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
