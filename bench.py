@@ -121,7 +121,7 @@ MEASURED_DRAM_BYTES_PER_CELL = {"field_fft": 38.5, "lpt_fft": 59.8, "dens_bins":
 # listing kernel per cell in the shells' radial range, the painting kernel per
 # sub-sample.  The stage is bound by instruction issue, not HBM, so its
 # roofline is the issue rate: 4 schedulers x 32 lanes per SM and cycle.
-IMAP_INSTR_PER_CELL = 455.8
+IMAP_INSTR_PER_CELL = 486.6
 IMAP_INSTR_PER_SAMPLE = 99.9
 
 

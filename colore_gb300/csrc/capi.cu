@@ -1796,6 +1796,7 @@ static int imap_launch(cg_ctx *c, int ip)
   p.nr = nr;
   p.nbk = nbk;
   p.npix = npix;
+  p.phi = c->d_npot;
   p.seg = c->d_iseg;
   p.acc = M.acc;
   p.packed = M.packed;

@@ -27,10 +27,11 @@
  *                  per bucket present in the warp, all issued together, on
  *                  counters that have a 128-byte line each (next to each other
  *                  they sat in one L2 slice, whose atomics bounded the kernel:
- *                  65 against 54 ms of the stage at 1024^3).  A cell that finds
- *                  its bucket full is painted by its warp on the spot.
- *                  456 thread-instructions a cell in range where a lookup with
- *                  a bound per table took 689: 20.6 -> 13 ms at 1024^3.
+ *                  65 against 54 ms of the stage at 1024^3).  Cells that the
+ *                  segments leave open, and cells that find their bucket full
+ *                  (painted by the warp), wait until the warp's rows are done.
+ *                  487 thread-instructions a cell in range where a lookup with
+ *                  a bound per table took 689: 20.6 -> 11.5 ms at 1024^3.
  *   k_imap_chunks  One block cuts each bucket into chunks of about CHS
  *                  samples: whole cells, or slices of one cell.
  *   k_imap_paint   Warps take chunks in bucket order, so the maps' working
@@ -66,6 +67,7 @@ using namespace cg;
 
 constexpr int IW = 4;     /* warps per block                     */
 constexpr int ROWS = 2;   /* rows per fetch in k_imap_list        */
+constexpr int LATE_CH = 64; /* words of 32 cells in a row: N <= 2048 */
 constexpr int CHS = 4096; /* samples per painting chunk           */
 constexpr int QB = 256;   /* queue entries staged per painting warp */
 constexpr unsigned FULL = 0xffffffffu;
@@ -253,7 +255,7 @@ __device__ __forceinline__ cg_imap_cell unpack(const cg_imap_rec &r, int j, int 
 /* A sample of a cell the listing kernel paints itself: its double decision,
  * when needed, on the spot. */
 template <typename K>
-__device__ __noinline__ K sample_key_inline(const cg_imap_params &p, const float *phi, int ix, int iy, int iz,
+__device__ __noinline__ K sample_key_inline(const cg_imap_params &p, int ix, int iy, int iz,
                                             const cg_imap_cell &c, int dbl, int ns, int q, float inv_ns)
 {
   const cg_imap_args &A = p.a;
@@ -262,7 +264,7 @@ __device__ __noinline__ K sample_key_inline(const cg_imap_params &p, const float
   sub_of(q, ns, inv_ns, &sx, &sy, &sz);
   if (dbl || p.force_double || !cg_imap_sample_checked(&A, ix, iy, iz, &c, ns, sx, sy, sz, &s, &pix)) {
     float v[3];
-    grad_phi(phi, ix, iy, iz, p.box.N, v);
+    grad_phi(p.phi, ix, iy, iz, p.box.N, v);
     int j;
     double drr = 0;
     cgx_imap_cell(&A, ix, iy, iz, v, &j, &drr);
@@ -317,17 +319,100 @@ __device__ __noinline__ OpenCell cell_open(const cg_imap_params &p, int ix, int 
   return o;
 }
 
-/* 8 blocks per SM (64 registers, some spilled): 5 and 6 without most of the
- * spills took 1.5 and 1.6 ms more of the stage's 52.5 at 1024^3. */
+/* Cells past their bucket's room (m: their lanes), painted by the warp. */
 template <typename K>
-__global__ void __launch_bounds__(IW * 32, 8) k_imap_list(const float *__restrict__ dens, const float *__restrict__ phi,
-                                                               const __grid_constant__ cg_imap_params p)
+__device__ __forceinline__ void paint_over(const cg_imap_params &p, unsigned m, const cg_imap_rec &rec, int bk, int lane)
+{
+  while (m) {
+    const int l = __ffs(m) - 1;
+    m &= m - 1;
+    cg_imap_rec r;
+    r.ixy = __shfl_sync(FULL, rec.ixy, l);
+    r.izf = __shfl_sync(FULL, rec.izf, l);
+    r.temp = __shfl_sync(FULL, rec.temp, l);
+    r.drr = __shfl_sync(FULL, rec.drr, l);
+    const int j = __shfl_sync(FULL, bk, l) / CG_IMAP_CLASSES - 1;
+    int ix, iy, iz, dbl;
+    const cg_imap_cell c = unpack(r, j, &ix, &iy, &iz, &dbl);
+    const int ns = p.a.nsub[j + 1], n3 = ns * ns * ns;
+    const float inv = 1.0f / (float)ns;
+    for (int q0 = 0; q0 < n3; q0 += 32) {
+      const int q = q0 + lane;
+      K key = empty_key<K>();
+      if (q < n3) key = sample_key_inline<K>(p, ix, iy, iz, c, dbl, ns, q, inv);
+      add_runs(key, 0, c.temp, lane, p);
+    }
+    if (lane == 0) atomicAdd(&p.ctr[3], (unsigned long long)n3);
+  }
+}
+
+/* A warp's rows in words of 32 cells: the cells that the segments leave open,
+ * and those that found their bucket full. */
+struct Late {
+  unsigned open[ROWS * LATE_CH], over[ROWS * LATE_CH];
+};
+
+/* Those cells, once per group of rows: out of the listing loop, whose registers
+ * a call would spill. */
+template <typename K>
+__device__ __noinline__ void late_cells(const float *__restrict__ dens, const cg_imap_params &p, const Late &L, int rbeg,
+                                        int rend, int lane)
+{
+  const int N = p.box.N, nch = N / 32, ngx = 2 * (N / 2 + 1);
+  unsigned long long drawn = 0, ndbl = 0;
+  __syncwarp();
+  for (int g = 0; g < (rend - rbeg) * nch; g++) {
+    const unsigned open = L.open[g], any = open | L.over[g];
+    if (!any) continue;
+    const int row = rbeg + g / nch, ix = (g % nch) * 32 + lane;
+    const int iz = (int)divN(row, p.box), iy = row - iz * N;
+    bool over = false;
+    int bk = -1;
+    cg_imap_rec rec = {0u, 0u, 0.0f, 0.0f};
+    if ((any >> lane) & 1u) {
+      float v[3];
+      grad_phi(p.phi, ix, iy, iz, N, v);
+      const OpenCell o = cell_open(p, ix, iy, iz, __ldg(dens + (long long)row * ngx + ix), v[0], v[1], v[2]);
+      if (o.st == 1) {
+        const int sfin = o.c.j + o.c.delta;
+        const bool want = !(o.c.mode == CG_SH_SINGLE && (sfin < 0 || sfin >= p.nr));
+        const int cls = o.dbl ? CG_CELL_GENERAL : cg_cell_class(&p.a, &o.c, p.a.xc[ix], p.a.yc[iy], p.a.zc[iz]);
+        bk = CG_IMAP_CLASSES * (o.c.j + 1) + cls;
+        rec = pack(ix, iy, iz, o.c, (unsigned)o.c.mode | ((unsigned)(o.c.delta + 1) << 2) | (o.dbl ? F_DOUBLE : 0u));
+        over = want;
+        if ((open >> lane) & 1u) {
+          const int ns = p.a.nsub[o.c.j + 1];
+          drawn += (unsigned long long)ns * ns * ns;
+          if (want) {
+            const long long k = (long long)atomicAdd(&p.cnt[(size_t)bk * CG_IMAP_CNT], 1ull);
+            over = k >= p.cap[bk];
+            if (!over) p.recs[p.base[bk] + k] = rec;
+          }
+        }
+      }
+      if ((open >> lane) & 1u) ndbl += o.in_double;
+    }
+    paint_over<K>(p, __ballot_sync(FULL, over), rec, bk, lane);
+  }
+  if (drawn) atomicAdd(&p.ctr[2], drawn);
+  if (ndbl) atomicAdd(p.xstats + 2, ndbl);
+}
+
+/* 12 blocks per SM: 5, 6, 8, 10 and 16 took 55.1, 53.8, 52.5, 51.2 and 50.5
+ * against 50.7 ms of the stage at 1024^3 (16 loses at 256^3: 1194 against 1165
+ * us).  Waiting for the reservations a step later, with the next cells decided
+ * in between, cost more in registers than it hid (52.4 ms). */
+template <typename K>
+__global__ void __launch_bounds__(IW * 32, 12) k_imap_list(const float *__restrict__ dens, const float *__restrict__ phi,
+                                                             const __grid_constant__ cg_imap_params p)
 {
   extern __shared__ __align__(16) unsigned char sraw[];
+  __shared__ Late late[IW];
   const Sh sh = load_shells(p, sraw, false);
   __syncthreads();
   const cg_imap_args A = args_with(p, sh);
   const int lane = threadIdx.x & 31;
+  Late &L = late[threadIdx.x >> 5];
   const int N = p.box.N;
   const int nrow = N * N, nch = N / 32; /* N is a multiple of 32 */
   const float rlo = A.rmin - 1.0f, rhi = A.rmax + 1.0f;
@@ -335,13 +420,16 @@ __global__ void __launch_bounds__(IW * 32, 8) k_imap_list(const float *__restric
   const int ngx = 2 * (N / 2 + 1);
   const long long plane = (long long)ngx * N;
   const float eg = __uint_as_float(*reinterpret_cast<const unsigned *>(p.seg + A.na - 1));
-  unsigned long long drawn = 0, ndbl = 0;
+  unsigned long long drawn = 0;
   for (;;) {
     int rbeg = 0;
     if (lane == 0) rbeg = (int)atomicAdd(&p.ctr[1], (unsigned long long)ROWS);
     rbeg = __shfl_sync(FULL, rbeg, 0);
     if (rbeg >= nrow) break;
     const int rend = rbeg + ROWS < nrow ? rbeg + ROWS : nrow;
+    unsigned any_late = 0;
+    for (int i = lane; i < ROWS * nch; i += 32) L.open[i] = L.over[i] = 0u;
+    __syncwarp();
     for (int row = rbeg; row < rend; row++) {
       const int iz = (int)divN(row, p.box), iy = row - iz * N;
       const float y0 = A.yc[iy], z0 = A.zc[iz];
@@ -353,8 +441,7 @@ __global__ void __launch_bounds__(IW * 32, 8) k_imap_list(const float *__restric
       for (int ch = 0; ch < nch; ch++) {
         const int ix = ch * 32 + lane;
         cg_imap_cell c;
-        bool want = false; /* listed and painted */
-        int dbl = 0;
+        bool want = false, open = false; /* listed and painted; left to late_cells */
         const float x0 = A.xc[ix];
         const float r2 = CG_FMA(x0, x0, yz2);
         if (r2 >= rlo2 && r2 <= rhi2) {
@@ -363,83 +450,50 @@ __global__ void __launch_bounds__(IW * 32, 8) k_imap_list(const float *__restric
           /* centred potential differences (get_rvel, imap.c:43-74) */
           const float v[3] = {CG_SUB(__ldg(f + (ix == N - 1 ? 1 - N : 1)), __ldg(f + (ix == 0 ? N - 1 : -1))),
                               CG_SUB(__ldg(f + oyh), __ldg(f + oyl)), CG_SUB(__ldg(f + ozh), __ldg(f + ozl))};
-          int st = p.force_double ? 2 : cg_imap_cell_seg(p.seg, eg, &A, x0, y0, z0, r2, d, v, &c);
-          if (st == 2) {
-            const OpenCell o = cell_open(p, ix, iy, iz, d, v[0], v[1], v[2]);
-            c = o.c;
-            dbl = o.dbl;
-            st = o.st;
-            ndbl += o.in_double;
-          }
+          const int st = p.force_double ? 2 : cg_imap_cell_seg(p.seg, eg, &A, x0, y0, z0, r2, d, v, &c);
+          open = st == 2;
           if (st == 1) {
             const int ns = A.nsub[c.j + 1];
-            drawn += (unsigned long long)ns * ns * ns;
+            drawn += (unsigned)(ns * ns * ns);
             const int sfin = c.j + c.delta;
             want = !(c.mode == CG_SH_SINGLE && (sfin < 0 || sfin >= p.nr));
           }
         }
         /* nothing to append (a chunk outside the shells' radial range, about
          * half of them): skip the bucket reservation */
+        const unsigned om = __ballot_sync(FULL, open);
+        if (om) {
+          if (lane == 0) L.open[(row - rbeg) * nch + ch] = om;
+          any_late = 1u;
+        }
         if (!__any_sync(FULL, want)) continue;
         /* append to the buckets: one atomic per bucket present in the warp,
          * issued together by each bucket's first lane (one round trip) */
-        bool over = false;
-        long long slot = 0;
         int bk = -1;
-        if (want) {
-          const int cls = dbl ? CG_CELL_GENERAL : cg_cell_class(&A, &c, x0, y0, z0);
-          bk = CG_IMAP_CLASSES * (c.j + 1) + cls;
-        }
+        if (want) bk = CG_IMAP_CLASSES * (c.j + 1) + cg_cell_class(&A, &c, x0, y0, z0);
         const unsigned same = __match_any_sync(FULL, bk);
         const int leader = __ffs(same) - 1;
         unsigned long long old = 0;
         if (want && lane == leader) old = atomicAdd(&p.cnt[(size_t)bk * CG_IMAP_CNT], (unsigned long long)__popc(same));
         old = __shfl_sync(FULL, old, leader);
+        bool over = false;
         if (want) {
           const long long k = (long long)old + __popc(same & ((1u << lane) - 1u));
-          if (k < p.cap[bk]) slot = p.base[bk] + k;
-          else over = true;
+          over = k >= p.cap[bk];
+          if (!over) p.recs[p.base[bk] + k] = pack(ix, iy, iz, c, (unsigned)c.mode | ((unsigned)(c.delta + 1) << 2));
         }
-        if (want && !over)
-          p.recs[slot] = pack(ix, iy, iz, c, (unsigned)c.mode | ((unsigned)(c.delta + 1) << 2) | (dbl ? F_DOUBLE : 0u));
-        /* cells past their bucket's room: painted here by the warp */
-        unsigned om = __ballot_sync(FULL, want && over);
-        while (om) {
-          const int l = __ffs(om) - 1;
-          om &= om - 1;
-          const int cx = __shfl_sync(FULL, ix, l);
-          cg_imap_cell cc;
-          cc.j = __shfl_sync(FULL, c.j, l);
-          cc.temp = __shfl_sync(FULL, c.temp, l);
-          cc.drr = __shfl_sync(FULL, c.drr, l);
-          cc.edrr = __shfl_sync(FULL, c.edrr, l);
-          cc.mode = __shfl_sync(FULL, c.mode, l);
-          cc.delta = __shfl_sync(FULL, c.delta, l);
-          const int cd = __shfl_sync(FULL, dbl, l);
-          const int ns = A.nsub[cc.j + 1];
-          const int n3 = ns * ns * ns;
-          const float inv = sh.invns[cc.j + 1];
-          const int tag = cx;
-          for (int q0 = 0; q0 < n3; q0 += 32) {
-            const int q = q0 + lane;
-            K key = empty_key<K>();
-            if (q < n3) key = sample_key_inline<K>(p, phi, cx, iy, iz, cc, cd, ns, q, inv);
-            add_runs(key, tag, cc.temp, lane, p);
-          }
-          if (lane == 0) atomicAdd(&p.ctr[3], (unsigned long long)n3);
+        const unsigned vm = __ballot_sync(FULL, over);
+        if (vm) {
+          if (lane == 0) L.over[(row - rbeg) * nch + ch] = vm;
+          any_late = 1u;
         }
       }
     }
+    if (any_late) late_cells<K>(dens, p, L, rbeg, rend, lane);
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    drawn += __shfl_xor_sync(FULL, drawn, o);
-    ndbl += __shfl_xor_sync(FULL, ndbl, o);
-  }
-  if (lane == 0) {
-    if (drawn) atomicAdd(&p.ctr[2], drawn);
-    if (ndbl) atomicAdd(p.xstats + 2, ndbl);
-  }
+  for (int o = 16; o > 0; o >>= 1) drawn += __shfl_xor_sync(FULL, drawn, o);
+  if (lane == 0 && drawn) atomicAdd(&p.ctr[2], drawn);
 }
 
 /* Work units of a bucket of nsub ns: whole cells for ns <= 4 (8 to 64

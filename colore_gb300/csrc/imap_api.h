@@ -28,6 +28,7 @@ struct __align__(16) cg_imap_rec {
 
 struct cg_imap_params {
   cg::Box box;
+  const float *phi;  /* the potential */
   cg_imap_args a;    /* tables, corners, shells (device pointers) */
   cg_imap_seg *seg;  /* the tables' segments (na - 1) and, past them, the bits of their
                         largest factor bound (all written by cg_imap_paint) */
