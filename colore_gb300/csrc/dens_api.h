@@ -36,7 +36,7 @@ struct cg_lpt_params {
   cg::Tab d2;
 };
 
-cudaError_t cg_moments_final(cudaStream_t s, const double2 *part, size_t n, double inv_ncell, double *stats,
+cudaError_t cg_moments_final(cudaStream_t s, double2 *part, size_t n, double inv_ncell, double *stats,
                              float *s2f);
 cudaError_t cg_dens_bins(cudaStream_t s, float *grid, const cg_bins_params *p, int nsm);
 int cg_dens_bins_max_tracers(void);
