@@ -1084,7 +1084,8 @@ extern "C" int cg_create_cartesian_fields(cg_ctx *c)
     const double ncell = (double)c->N * c->N * c->N;
     CUDA_TRY(c, cg_moments_final(c->stream, c->d_part, c->npart, 1.0 / ncell, c->d_stats, c->d_s2f));
   }
-  c->launches += 5 + (c->npart > 8192); /* the moments' sums in two launches */
+  /* fill, y, x (one or two), the moments' sums (one or two) */
+  c->launches += 4 + (c->N > CG_FIELD_X_BOTH) + (c->npart > 8192);
   c->have_fields = 1;
   c->have_density = c->have_norm = c->have_srcs = 0;
   c->pending_mode = CG_DMODE_NONE;

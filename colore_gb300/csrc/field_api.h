@@ -30,6 +30,8 @@ struct cg_field_launch {
 #define CG_PASS_Y 2     /* column transforms along y                   */
 #define CG_PASS_X 3     /* row c2r along x (without the moment sums)   */
 
+#define CG_FIELD_X_BOTH 512 /* largest grid whose Gaussian x pass is one launch */
+
 #define CG_FIELD_SIZES(X) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(1024) X(2048)
 
 #define CG_FIELD_DECL(n)                                                 \

@@ -407,8 +407,8 @@ __global__ void __launch_bounds__(TX *PF) k_z_lpt2(const float2 *__restrict__ sr
   }
 }
 
-/* Pass 3: row c2r along x with normalisation and optional moment sums,
- * RB rows per block.  grid = (N*N/RB, nf).  partials[blockIdx.x] =
+/* Pass 3: row c2r along x with normalisation and optional moment sums of the
+ * first field, RB rows per block.  grid = (N*N/RB, nf).  partials[blockIdx.x] =
  * (sum d, sum d^2). */
 template <bool STATS, int RB>
 __global__ void __launch_bounds__(RB *PR) k_row_c2r(float2 *f0, float2 *f1, float2 *f2, float norm,
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(RB *PR) k_row_c2r(float2 *f0, float2 *f1, floa
     }
   };
   cgfft::transform<LH, PL::RR, PL::R0, PL::R1, PL::R2, 1, SHX>(t, tw + TW_R, ld, st, sm);
-  if (STATS) {
+  if (STATS && blockIdx.y == 0) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       s1 += __shfl_xor_sync(0xffffffffu, s1, o);
@@ -616,8 +616,13 @@ extern "C" cudaError_t CG_CAT(cg_field_gauss_, CG_N)(const cg_field_launch *L)
   if (L->ev) cudaEventRecord(L->ev[0], L->stream);
   if ((e = ypass_v<1>(L, L->var[CG_PASS_Y], L->f[0], L->f[1], nullptr, 2)) != cudaSuccess) return e;
   if (L->ev) cudaEventRecord(L->ev[1], L->stream);
-  if ((e = xpass<true, PL::RB>(L, L->f[0], nullptr, nullptr, 1, L->norm, L->partials)) != cudaSuccess) return e;
-  if ((e = xpass_v(L, L->var[CG_PASS_X], L->f[1], nullptr, nullptr, 1)) != cudaSuccess) return e;
+  /* the moments' pass, which keeps the plan's rows, takes the potential along
+   * up to 512^3, where a launch's fill and drain cost more than the tuned row
+   * count gives: both 10.6 -> 7.6 us at 64^3, 60 -> 54 at 256^3, 330 -> 321 at
+   * 512^3, but 2.76 -> 2.79 ms at 1024^3 */
+  constexpr int nf = N <= CG_FIELD_X_BOTH ? 2 : 1;
+  if ((e = xpass<true, PL::RB>(L, L->f[0], L->f[1], nullptr, nf, L->norm, L->partials)) != cudaSuccess) return e;
+  if (nf == 1 && (e = xpass_v(L, L->var[CG_PASS_X], L->f[1], nullptr, nullptr, 1)) != cudaSuccess) return e;
   if (L->ev) cudaEventRecord(L->ev[2], L->stream);
   return cudaGetLastError();
 }
