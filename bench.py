@@ -116,13 +116,14 @@ MEASURED_DRAM_BYTES_PER_CELL = {"field_fft": 38.5, "lpt_fft": 59.8, "dens_bins":
 
 
 # Thread-instructions per unit of work of the intensity-map stage's kernels,
-# from one-kernel ncu captures at 512^3 (smsp__inst_executed.sum x
+# from one-kernel ncu captures at 512^3 with maps at nside 256, which have the
+# 1024^3 workload's sub-samples per cell (smsp__inst_executed.sum x
 # smsp__thread_inst_executed_per_inst_executed.ratio over the units): the
 # listing kernel per cell in the shells' radial range, the painting kernel per
 # sub-sample.  The stage is bound by instruction issue, not HBM, so its
 # roofline is the issue rate: 4 schedulers x 32 lanes per SM and cycle.
 IMAP_INSTR_PER_CELL = 486.6
-IMAP_INSTR_PER_SAMPLE = 99.9
+IMAP_INSTR_PER_SAMPLE = 91.6
 
 
 def issue_roofline(dom, t_step, cfg, m, clocks):

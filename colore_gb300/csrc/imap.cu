@@ -45,11 +45,11 @@
  *                  decisions taken once per cell and walk along the line of
  *                  sight, where the pixel changes least.  Samples whose margins
  *                  fail are staged per warp in shared memory and queued in
- *                  batches.  Bound by instruction issue (90 % of the slots): 100
+ *                  batches.  Bound by instruction issue (87 % of the slots): 92
  *                  thread-instructions a sample where deciding everything per
- *                  sample took 177, 79 -> 37 ms for the 1.3e10 samples at
+ *                  sample took 177, 79 -> 36 ms for the 1.3e10 samples at
  *                  1024^3; scalar atomics instead of the two-float reduction
- *                  cost 5.5 ms of it.
+ *                  cost 5.5 ms, a branch around it 1.7.
  *   k_imap_double  The queued samples: first in float-float, then, for the
  *                  few left, gathered per warp and decided in double 32 at a
  *                  time, the cell's radial shift computed once per run of
@@ -626,19 +626,33 @@ struct Lane {
   float n; /* exact: a unit has at most 1024 samples */
 };
 
+/* One two-float reduction where c holds. */
+__device__ __forceinline__ void red_if(bool c, float2 *a, float t, float n)
+{
+  asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %0, 0;\n@q red.relaxed.gpu.global.add.v2.f32 [%1], {%2, %3};\n}" ::"r"(
+                   (unsigned)c),
+               "l"(a), "f"(t), "f"(n)
+               : "memory");
+}
+
 /* A sample on key (ok), or one to hold, of index q0 + step floor(fi): another
- * key than the run's sends the run to the maps. */
-template <typename K>
+ * key than the run's sends the run to the maps.  With packed sums (P) without a
+ * branch but the rare one: some lane of a warp changes its pixel at nearly
+ * every sample. */
+template <typename K, bool P>
 __device__ __forceinline__ void hit(const cg_imap_params &p, Lane<K> &L, K key, bool ok, float temp, long long rec,
                                     int q0, int step, float fi)
 {
-  if (ok && key == L.k) {
-    L.n = CG_ADD(L.n, 1.0f);
-  } else if (ok) {
+  const bool change = ok && key != L.k;
+  if (P) {
+    red_if(change && L.n > 0.0f, p.acc + L.k, CG_MUL(temp, L.n), L.n);
+  } else if (change) {
     flush<K>(p, L.k, L.n, temp);
-    L.k = key;
-    L.n = 1.0f;
-  } else {
+  }
+  L.k = change ? key : L.k;
+  L.n = change ? 1.0f : CG_ADD(L.n, 1.0f);
+  if (!ok) {
+    L.n = CG_SUB(L.n, 1.0f); /* exact */
     hold(p, rec, q0 + step * (int)fi);
   }
 }
@@ -650,7 +664,7 @@ struct Axis {
 __device__ __forceinline__ float at(const Axis &a, float half, float dxs) { return CG_ADD(a.c, CG_FMA(half, dxs, a.l)); }
 
 /* A unit's samples, in rows along x, in the general form. */
-template <typename K>
+template <typename K, bool P>
 __device__ __forceinline__ void walk_general(const cg_imap_params &p, const cg_imap_args &A, const cg_imap_cell &c,
                                              int dbl, long long rec, const Axis &ax, const Axis &ay, const Axis &az,
                                              float dxs, int ns, int z0, int z1, int y0, int y1, Lane<K> &L)
@@ -666,7 +680,7 @@ __device__ __forceinline__ void walk_general(const cg_imap_params &p, const cg_i
         long long pix = 0;
         const bool ok = !dbl && cg_imap_decide(&A, &c, at(ax, fi, dxs), y, z, &s, &pix);
         const K key = key_of<K>(p, s, pix);
-        if (!ok || key != empty_key<K>()) hit<K>(p, L, key, ok, c.temp, rec, ns * (sy + ns * sz), 1, fi);
+        if (!ok || key != empty_key<K>()) hit<K, P>(p, L, key, ok, c.temp, rec, ns * (sy + ns * sz), 1, fi);
       }
     }
   }
@@ -677,7 +691,7 @@ __device__ __forceinline__ void walk_general(const cg_imap_params &p, const cg_i
  * consecutive samples keep their pixel longest: z in the polar caps, where the
  * octant angle is then the line's, the larger of x and y elsewhere.  Ranges
  * [o0, o1) and [m0, m1) of the outer and the middle axis. */
-template <typename K, bool EQ>
+template <typename K, bool P, bool EQ>
 __device__ __forceinline__ void walk_fast(const cg_imap_params &p, const cg_imap_fast &F, float temp, long long rec,
                                           const Axis &x, const Axis &y, const Axis &z, float dxs, int ns, int o0, int o1,
                                           int m0, int m1, float thr, Lane<K> &L)
@@ -699,19 +713,19 @@ __device__ __forceinline__ void walk_fast(const cg_imap_params &p, const cg_imap
       if (EQ) {
         const float zs = at(z, fo, dxs), vs = at(v, fm, dxs);
         const float vz2 = CG_FMA(zs, zs, CG_MUL(vs, vs));
-#pragma unroll 1
+#pragma unroll 2
         for (float fi = 0.5f; fi < fns; fi = CG_ADD(fi, 1.0f)) {
           int up, pix;
           const bool ok = cg_fast_eq(&F, nside, thr, at(u, fi, dxs), vs, zs, vz2, &up, &pix);
-          hit<K>(p, L, (up ? b1 : b0) + (K)pix, ok, temp, rec, q0, su, fi);
+          hit<K, P>(p, L, (up ? b1 : b0) + (K)pix, ok, temp, rec, q0, su, fi);
         }
       } else {
         const cg_fast_line l = cg_fast_polar_line(&F, nside, at(u, fm, dxs), at(v, fo, dxs));
-#pragma unroll 1
+#pragma unroll 2
         for (float fi = 0.5f; fi < fns; fi = CG_ADD(fi, 1.0f)) {
           int up, pix;
           const bool ok = cg_fast_polar(&F, &l, thr, at(z, fi, dxs), &up, &pix);
-          hit<K>(p, L, (up ? b1 : b0) + (K)pix, ok, temp, rec, q0, sz, fi);
+          hit<K, P>(p, L, (up ? b1 : b0) + (K)pix, ok, temp, rec, q0, sz, fi);
         }
       }
     }
@@ -722,7 +736,7 @@ __device__ __forceinline__ void walk_fast(const cg_imap_params &p, const cg_imap
  * unit (a cell, a slab or a line) sample by sample.  The samples that only
  * double can decide are staged per warp in shared memory and queued in
  * batches. */
-template <typename K>
+template <typename K, bool P>
 __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_imap_args &A, int b, int ns,
                                             unsigned long long u0, int G, unsigned long long nu, float dxs, int lane)
 {
@@ -770,14 +784,14 @@ __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_im
       /* the bucket's class: one loop for the whole warp */
       const int cls = dbl ? CG_CELL_GENERAL : b % CG_IMAP_CLASSES;
       if (cls == CG_CELL_GENERAL) {
-        walk_general<K>(p, A, c, dbl, rec, x, y, z, dxs, ns, o0, o1, m0, m1, L);
+        walk_general<K, P>(p, A, c, dbl, rec, x, y, z, dxs, ns, o0, o1, m0, m1, L);
       } else {
         cg_imap_fast F;
         cg_imap_fast_cell(&A, &c, cls, x.c, y.c, z.c, &F);
         if (cls == CG_CELL_EQ)
-          walk_fast<K, true>(p, F, temp, rec, x, y, z, dxs, ns, o0, o1, m0, m1, cg_fast_eq_thr(A.nside), L);
+          walk_fast<K, P, true>(p, F, temp, rec, x, y, z, dxs, ns, o0, o1, m0, m1, cg_fast_eq_thr(A.nside), L);
         else
-          walk_fast<K, false>(p, F, temp, rec, x, y, z, dxs, ns, o0, o1, m0, m1, cg_fast_polar_k0(A.nside), L);
+          walk_fast<K, P, false>(p, F, temp, rec, x, y, z, dxs, ns, o0, o1, m0, m1, cg_fast_polar_k0(A.nside), L);
       }
       flush<K>(p, L.k, L.n, temp);
     }
@@ -785,11 +799,12 @@ __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_im
   }
 }
 
-/* Warps take chunks in bucket order; paint_chunk paints one.  8 blocks per SM:
- * 5, 6, 7 and 10 took 67.1, 63.5, 62.0 and 64.9 against 61.7 ms of the stage at
- * 1024^3. */
-template <typename K>
-__global__ void __launch_bounds__(IW * 32, 8) k_imap_paint(const __grid_constant__ cg_imap_params p)
+/* Warps take chunks in bucket order; paint_chunk paints one.  7 blocks per SM
+ * with the samples two at a time: 5, 6 and 8 took 51.4, 48.6 and 49.0 against
+ * 47.8 ms of the stage at 1024^3; one, three and four at a time 48.6, 47.9 and
+ * 48.0. */
+template <typename K, bool P>
+__global__ void __launch_bounds__(IW * 32, 7) k_imap_paint(const __grid_constant__ cg_imap_params p)
 {
   extern __shared__ __align__(16) unsigned char sraw[];
   const Sh sh = load_shells(p, sraw, true);
@@ -819,7 +834,7 @@ __global__ void __launch_bounds__(IW * 32, 8) k_imap_paint(const __grid_constant
     const int G = groups_per_chunk(ns);
     const float dxs = sh.dxs[b / CG_IMAP_CLASSES];
     const unsigned long long u0 = (ck - sh.chunk_off[b]) * 32ull * (unsigned long long)G;
-    paint_chunk<K>(p, A, b, ns, u0, G, nu, dxs, lane);
+    paint_chunk<K, P>(p, A, b, ns, u0, G, nu, dxs, lane);
   }
   queue_flush(p, 1, lane);
 }
@@ -953,8 +968,9 @@ cudaError_t launch(cudaStream_t s, const float *dens, const float *phi, const cg
   if (e != cudaSuccess) return e;
   const size_t sm_list = shell_smem(p->nr, p->nbk, false), sm_paint = paint_smem(p->nr, p->nbk);
   const size_t sm_double = double_stage_off(p->nr, p->nbk) + (size_t)DB_WARPS * 64 * 8;
+  auto paint = p->packed ? k_imap_paint<K, true> : k_imap_paint<K, false>;
   if ((e = cudaFuncSetAttribute(k_imap_list<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_list)) ||
-      (e = cudaFuncSetAttribute(k_imap_paint<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_paint)) ||
+      (e = cudaFuncSetAttribute(paint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_paint)) ||
       (e = cudaFuncSetAttribute(k_imap_double, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_double)))
     return e;
   int per_sm = 0;
@@ -965,8 +981,8 @@ cudaError_t launch(cudaStream_t s, const float *dens, const float *phi, const cg
   k_imap_tab<<<(unsigned)((p->a.na + 31) / 32), 32, 0, s>>>(*p);
   k_imap_list<K><<<(unsigned)blocks, IW * 32, sm_list, s>>>(dens, phi, *p);
   k_imap_chunks<<<1, 1024, 0, s>>>(*p);
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_imap_paint<K>, IW * 32, sm_paint))) return e;
-  k_imap_paint<K><<<(unsigned)(nsm * (per_sm > 0 ? per_sm : 1)), IW * 32, sm_paint, s>>>(*p);
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, paint, IW * 32, sm_paint))) return e;
+  paint<<<(unsigned)(nsm * (per_sm > 0 ? per_sm : 1)), IW * 32, sm_paint, s>>>(*p);
   k_imap_double<<<(unsigned)(nsm * 4), DB_WARPS * 32, sm_double, s>>>(phi, *p);
   return cudaGetLastError();
 }
