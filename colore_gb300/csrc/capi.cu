@@ -853,10 +853,10 @@ extern "C" int cg_memory_estimate(const cg_config *cfg, unsigned long long *byte
   return CG_OK;
 }
 
-/* write_imap's normalisation (io.c:738-741): data/nadd where nadd > 0. */
 /* Samples of a map pixel (imap_api.h). */
 __device__ __forceinline__ int hits_of(float2 a, int packed) { return packed ? (int)a.y : __float_as_int(a.y); }
 
+/* write_imap's normalisation (io.c:738-741): data/nadd where nadd > 0. */
 __device__ __forceinline__ float div_nadd(float2 a, int packed)
 {
   const int k = hits_of(a, packed);
@@ -1662,7 +1662,8 @@ static int imap_prepare(cg_ctx *c, int ip)
    * surface layer, about 1 cell deep; class 0 holds the cells on the four
    * planes between octants and the two cones (t / 2r of a thin shell each for
    * a layer t: 3.5 cells in r), and all of a shell that a cell may span
-   * (CG_SH_WALK) or leave for none.  Cells past a bucket's room are painted as they are listed. */
+   * (CG_SH_WALK) or leave for none.  Cells past a bucket's room are painted by
+   * the listing kernel. */
   std::vector<double> want(nbk, 0.0);
   double dense = 0; /* most samples per pixel that a shell's cells hold on average */
   const double h = 0.8660254037844386 * dx, ncell = (double)c->N * c->N * c->N;

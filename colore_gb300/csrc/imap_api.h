@@ -21,7 +21,7 @@ struct __align__(16) cg_imap_rec {
 
 #define CG_IMAP_REC_BYTES 16
 /* A bucket per shell -1 .. nr of the cells' corners and per class of
- * cg_imap_fast_cell: bucket 3 (j + 1) + class. */
+ * cg_cell_class: bucket 3 (j + 1) + class. */
 #define CG_IMAP_CLASSES 3
 #define CG_IMAP_CNT 16 /* stride of the buckets' counters: a 128-byte line each */
 #define CG_IMAP_BUCKETS_MAX (CG_IMAP_CLASSES * 4100) /* nr <= 4096 */
@@ -39,9 +39,10 @@ struct cg_imap_params {
   unsigned int *err;
   unsigned long long *xstats; /* [2] cells, [3] samples decided in double */
   int force_double;
-  /* cells are listed per bucket (the shell of their corner, which fixes
-   * nsub, and the class, which fixes the painting loop), in the slots [base[b], base[b] + cap[b]); cnt[CG_IMAP_CNT b] counts them
-   * (may exceed cap: those cells are painted by the listing kernel) */
+  /* cells are listed per bucket (the shell of their corner, which fixes nsub,
+   * and the class, which fixes the painting loop), in the slots [base[b],
+   * base[b] + cap[b]); cnt[CG_IMAP_CNT b] counts them (may exceed cap: those
+   * cells are painted by the listing kernel) */
   cg_imap_rec *recs;
   const long long *base, *cap;
   unsigned long long *cnt;

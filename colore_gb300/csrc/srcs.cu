@@ -20,7 +20,8 @@
  *                  the NGP velocity (get_rvel, srcs.c:87-118), ra/dec/z, the
  *                  base-pixel id and the count-map increment are fused.
  *
- * Along the line of sight to each source (one thread per source):
+ * Along the line of sight to each source (one thread per source, a warp for
+ * the skewers):
  *   k_beam_rsd    : trilinear RSD at the source.
  *   k_src_lensing : shear, convergence and deflection from the nearest-cell
  *                   tidal tensor and potential gradient at N/2 radial steps.
