@@ -591,12 +591,18 @@ __device__ __noinline__ void hold(const cg_imap_params &p, long long rec, int q)
   else queue_one(p, rec, q);
 }
 
-/* The warp's stage to the queue, with one atomic, once it holds min_n. */
+/* The warp's stage to the queue, with one atomic, once it holds min_n.  One
+ * lane reads the count and the exchange hands it on: the lanes take the same
+ * way out, and none goes on to its next unit, where hold() raises the count,
+ * before it has been read. */
 __device__ __forceinline__ void queue_flush(const cg_imap_params &p, int min_n, int lane)
 {
   const Stage S = stage_of(p);
   __syncwarp();
-  const int qn = *S.n < QB ? *S.n : QB;
+  int qn = 0;
+  if (lane == 0) qn = *S.n;
+  qn = __shfl_sync(FULL, qn, 0);
+  if (qn > QB) qn = QB;
   if (qn < min_n) return;
   unsigned long long q0 = 0;
   if (lane == 0) q0 = atomicAdd(&p.ctr[4], (unsigned long long)qn);
