@@ -1665,7 +1665,6 @@ static int imap_prepare(cg_ctx *c, int ip)
    * (CG_SH_WALK) or leave for none.  Cells past a bucket's room are painted by
    * the listing kernel. */
   std::vector<double> want(nbk, 0.0);
-  double dense = 0; /* most samples per pixel that a shell's cells hold on average */
   const double h = 0.8660254037844386 * dx, ncell = (double)c->N * c->N * c->N;
   for (int k = -1; k < nb; k++) {
     double lo = k < 0 ? rmin : (double)bb[k], hi = k + 1 < nb ? (double)bb[k + 1] : rmax;
@@ -1675,7 +1674,6 @@ static int imap_prepare(cg_ctx *c, int ip)
     const double a = lo - h > 0 ? lo - h : 0, z = hi + h;
     const double v = 4.0 / 3.0 * M_PI * (z * z * z - a * a * a) / (dx * dx * dx), ir = 1.0 / std::max(a / dx, 1.0);
     double *w = &want[CG_IMAP_CLASSES * (shell_of[k + 1] + 1)];
-    dense = std::max(dense, v * std::pow((double)nsub[shell_of[k + 1] + 1], 3) / (double)npix);
     auto painted = [&](int i) { return i >= -1 && i < nb && shell_of[i + 1] >= 0 && shell_of[i + 1] < nr; };
     const bool plain = painted(k - 1) && painted(k) && painted(k + 1) && bb[k + 1] - bb[k] >= 2.1 * dx;
     w[0] += plain ? v * std::min(5 * ir + 0.01, 1.0) : v;
@@ -1727,10 +1725,8 @@ static int imap_prepare(cg_ctx *c, int ip)
   M.contig = cg_imap_contig(r0f.data(), rff.data(), nr, nb);
   M.rmin = rmin;
   M.rmax = rmax;
-  /* samples are spread over the sky like the cells; a pixel of a shell takes
-   * its own cells' and some of its neighbours', so 192 times the mean leaves
-   * a factor 64 to a float's 2^24 whole numbers */
-  M.packed = 192.0 * dense < 16777216.0;
+  /* whole numbers up to 2^24 are floats */
+  M.packed = cg_imap_pixel_max(bb.data(), nb, shell_of.data(), nsub.data(), rmin, rmax, dx, nside) < 16777216.0;
   M.gen = c->tab_gen;
   return CG_OK;
 }

@@ -1809,6 +1809,36 @@ static inline int cg_imap_shells(const double *r0d, const double *rfd, int nr, d
   return nb;
 }
 
+/* The most samples that one pixel of one shell can take.  A sample's pixel is
+ * that of its unshifted direction, so a pixel holds none but the samples of its
+ * cone, and no more of these than fit there, whatever the radial shifts: those
+ * of neighbouring intervals of one nsub, [lo, hi] of the corners' radii, have
+ * radii within sqrt(3) dx of [lo, hi] and lie within rho = CG_PIX_RADIUS / nside
+ * of the pixel's centre, and their sub-cells, which do not overlap, lie within
+ * h = sqrt(3) s / 2, s = dx / nsub, of that piece of a cone.  At x along the axis
+ * the piece thus widened is no wider than tan(rho) (x + h) + h. */
+#define CG_PIX_RADIUS 1.25 /* above any pixel's radius times nside: 0.84 at nside 1, 1.07 at large nside */
+static inline double cg_imap_pixel_max(const float *b, int nb, const int *shell_of, const int *nsub, double rmin,
+                                       double rmax, double dx, int nside)
+{
+  const double pi = 3.14159265358979323846, rho = CG_PIX_RADIUS / nside, tr = tan(rho);
+  double n = 0;
+  for (int k = -1, e; k < nb; k = e) {
+    const int ns = nsub[shell_of[k + 1] + 1];
+    for (e = k + 1; e < nb && nsub[shell_of[e + 1] + 1] == ns;) e++;
+    double lo = k < 0 ? rmin : (double)b[k], hi = e < nb ? (double)b[e] : rmax;
+    lo = lo < rmin ? rmin : lo;
+    hi = hi > rmax ? rmax : hi;
+    if (hi <= lo) continue;
+    const double s = dx / ns, h = 0.8660254037844387 * s, w = 1.7320508075688773 * dx;
+    const double a = lo - w > 0 ? lo - w : 0, z = hi + w, ah = a - h > 0 ? a - h : 0;
+    const double cone = pi / (3 * tr) * (pow(tr * (z + 2 * h) + h, 3) - pow(a * sin(rho) + h, 3));
+    const double all = 4.0 / 3.0 * pi * (pow(z + h, 3) - pow(ah, 3));
+    n += (cone < all ? cone : all) / (s * s * s);
+  }
+  return 1.001 * n + 64; /* corners, edges and directions within 1e-6 of the above */
+}
+
 /* Whether the sorted shells are contiguous (each rf the next r0): then
  * interval k is shell k. */
 static inline int cg_imap_contig(const float *r0f, const float *rff, int nr, int nb)

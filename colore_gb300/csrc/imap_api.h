@@ -35,7 +35,7 @@ struct cg_imap_params {
   int nr, nbk;       /* shells; buckets nbk = CG_IMAP_CLASSES (nr + 2) */
   long long npix;
   float2 *acc;       /* nr * npix, RING: summed brightness, samples */
-  int packed;        /* samples as a float (each below 2^24), else as int bits */
+  int packed;        /* samples as a float (cg_imap_pixel_max below 2^24), else as int bits */
   unsigned int *err;
   unsigned long long *xstats; /* [2] cells, [3] samples decided in double */
   int force_double;

@@ -494,6 +494,19 @@ static void imap_args_free(ImapArgs *B)
   free(B->dxsl);
 }
 
+/* cg_imap_pixel_max of species ipop. */
+double or_imap_pixel_max(const cg_config *cfg, int ipop)
+{
+  S32 s;
+  ImapArgs B;
+  s32_init(&s, cfg);
+  imap_args(&B, cfg, &s, ipop, NULL, NULL);
+  const double n = cg_imap_pixel_max(B.b, B.a.sh.nb, B.shell_of, B.nsub, B.a.rmin64, B.a.rmax64, B.a.dx64, B.a.nside);
+  imap_args_free(&B);
+  s32_free(&s);
+  return n;
+}
+
 /* The intensity map of species ipop as the GPU paints it: cells and samples
  * decided in single precision where the margins hold, then in float-float,
  * and in double otherwise (cg_exact.h); brightness summed in cell order in

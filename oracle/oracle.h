@@ -122,4 +122,6 @@ void or_next_float(long n, const float *f, const int *up, float *out);
 void or_imap_fast(long nside, int N, double dx, const double *pos, long n, const int *cell, const int *nsub,
                   const float *edge, const float *drr, const double *drr64, float edrr, long long *stat);
 
+double or_imap_pixel_max(const cg_config *cfg, int ipop);
+
 #endif

@@ -37,7 +37,7 @@ def lib():
             "or_counts64": [vp, i, vp, vp, vp, vp],
             "or_emit64": [vp, i, vp, vp, C.c_longlong, vp, vp, vp, vp, vp],
             "or_beam_rsd32": [vp, vp, C.c_longlong, vp, vp], "or_imap32": [vp, i, vp, vp, vp, vp, vp, vp, vp],
-            "or_imap_cells": [vp, i, vp, vp, vp, vp, vp],
+            "or_imap_cells": [vp, i, vp, vp, vp, vp, vp], "or_imap_pixel_max": [vp, i],
             "or_kappa32": [vp, vp, vp], "or_isw32": [vp, vp, vp], "or_isw64": [vp, vp, vp],
             "or_cstm_steps": [vp, i, vp, vp, vp, vp], "or_cstm64": [vp, i, vp, vp, d, d, vp],
             "or_cstm32": [vp, i, vp, vp, f, f, vp],
@@ -69,7 +69,7 @@ def lib():
             fn.argtypes = a
             if k in ("or_imap_samples", "or_poisson_total64"):
                 fn.restype = C.c_longlong
-            elif k == "or_atan_q_maxerr":
+            elif k in ("or_atan_q_maxerr", "or_imap_pixel_max"):
                 fn.restype = C.c_double
             elif k.startswith("or_vec") or k in void:
                 fn.restype = None
@@ -338,6 +338,11 @@ def imap_cells(cfg, ipop, dens, npot, tab32, e32, tab64, e64):
     lib().or_imap_cells(cfgp(cfg), ipop, P(np.ascontiguousarray(dens, np.float32)),
                         P(np.ascontiguousarray(npot, np.float32)), P(t32), P(t64), P(st))
     return tuple(int(v) for v in st)
+
+
+def imap_pixel_max(cfg, ipop):
+    """The bound on the samples of one pixel of species ipop's maps."""
+    return lib().or_imap_pixel_max(cfgp(cfg), ipop)
 
 
 def isw64(cfg, npot):
