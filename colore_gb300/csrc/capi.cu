@@ -52,10 +52,11 @@ struct Imap {
   int nr = 0, nside = 0;
   long long npix = 0;
   /* shells (cg_imap_shells): edges, shell of each interval, nsub and
-   * dx/nsub per bucket; bucket slots and counts */
+   * dx/nsub per shell; the rooms' slots and counts */
   float *b = nullptr, *dxs = nullptr, *dxsl = nullptr;
   int *shell_of = nullptr, *nsub = nullptr;
-  long long *base = nullptr, *cap = nullptr;
+  long long *at = nullptr, *cap = nullptr;
+  longlong2 *buckets = nullptr;
   unsigned long long *cnt = nullptr, *chunk_off = nullptr;
   float2 *acc = nullptr; /* summed brightness and samples per pixel */
   int packed = 0;        /* samples held as floats (cg_imap_params) */
@@ -259,7 +260,7 @@ static int error_word(cg_ctx *c, unsigned int h)
     CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(unsigned int), c->stream));
     return fail(c, CG_EDEVICE, "device error flags 0x%x (1: source count overflow, 2: catalog overflow, "
                                "4: shell search, 8: imap sub-sampling, 16: imap double-decision queue full, 32: bulk copy timeout, "
-                               "64: particle deposit overflow)",
+                               "64: particle deposit overflow, 128: imap list room)",
                 h);
   }
   return CG_OK;
@@ -974,7 +975,7 @@ extern "C" void cg_destroy(cg_ctx *c)
     if (p) cudaFree(p);
   for (int i = 0; i < CG_NPOP_MAX; i++) {
     void *q[] = {c->cat[i].pos, c->cat[i].ipix, c->cat[i].src, c->cat[i].cmap, c->im[i].b, c->im[i].dxs,
-                 c->im[i].dxsl, c->im[i].shell_of, c->im[i].nsub, c->im[i].base, c->im[i].cap, c->im[i].cnt, c->im[i].chunk_off,
+                 c->im[i].dxsl, c->im[i].shell_of, c->im[i].nsub, c->im[i].at, c->im[i].cap, c->im[i].cnt, c->im[i].chunk_off, c->im[i].buckets,
                  c->im[i].acc, c->im[i].ctr, c->d_cmap[i], c->cat[i].skw_d, c->cat[i].skw_v};
     for (void *p : q)
       if (p) cudaFree(p);
@@ -1618,7 +1619,7 @@ static int not_capturing(cg_ctx *c, const char *what)
 
 /* Tables of intensity species ip (imap_preproc, imap.c:105-133, and the
  * sub-sampling factors, imap.c:153-174): shells sorted by r0 and their edges
- * as intervals, the buckets' slots, the cell list and the queue.  Built
+ * as intervals, the cells' rooms, the cell list and the queue.  Built
  * once per table generation (or list bound), with host round trips; never
  * inside a stream capture. */
 static int imap_prepare(cg_ctx *c, int ip)
@@ -1644,8 +1645,9 @@ static int imap_prepare(cg_ctx *c, int ip)
     if ((rc = dalloc(c, &M.b, (size_t)2 * nr)) || (rc = dalloc(c, &M.shell_of, (size_t)2 * nr + 1)) ||
         (rc = dalloc(c, &M.nsub, (size_t)nr + 2)) || (rc = dalloc(c, &M.dxs, (size_t)nr + 2)) ||
         (rc = dalloc(c, &M.dxsl, (size_t)nr + 2)) ||
-        (rc = dalloc(c, &M.base, (size_t)nbk)) || (rc = dalloc(c, &M.cap, (size_t)nbk)) ||
-        (rc = dalloc(c, &M.cnt, (size_t)nbk * CG_IMAP_CNT)) || (rc = dalloc(c, &M.chunk_off, (size_t)nbk + 1)))
+        (rc = dalloc(c, &M.at, (size_t)4 * (nr + 2))) || (rc = dalloc(c, &M.cap, (size_t)4 * (nr + 2))) ||
+        (rc = dalloc(c, &M.cnt, (size_t)4 * (nr + 2) * CG_IMAP_CNT)) ||
+        (rc = dalloc(c, &M.chunk_off, (size_t)nbk + 1)) || (rc = dalloc(c, &M.buckets, (size_t)nbk)))
       return rc;
   }
   if (M.nr != nr || M.npix != npix) {
@@ -1655,49 +1657,30 @@ static int imap_prepare(cg_ctx *c, int ip)
   M.nside = nside;
   M.npix = npix;
   const double rmin = (double)r0f[0] - 20., rmax = (double)rff[nr - 1] + 20.;
-  /* slots per bucket: the corners of the cells of shell j's buckets lie in
-   * the radii of its intervals; each corner's dx-cube lies within sqrt(3)/2 dx
-   * of it, so (expanded shell volume) / dx^3 bounds them.  Of these 2/3 lie
-   * at |cos theta| < 2/3 (class 1) and 1/3 beyond (class 2), each up to a
-   * surface layer, about 1 cell deep; class 0 holds the cells on the four
-   * planes between octants and the two cones (t / 2r of a thin shell each for
-   * a layer t: 3.5 cells in r), and all of a shell that a cell may span
-   * (CG_SH_WALK) or leave for none.  Cells past a bucket's room are painted by
-   * the listing kernel. */
-  std::vector<double> want(nbk, 0.0);
-  const double h = 0.8660254037844386 * dx, ncell = (double)c->N * c->N * c->N;
-  for (int k = -1; k < nb; k++) {
-    double lo = k < 0 ? rmin : (double)bb[k], hi = k + 1 < nb ? (double)bb[k + 1] : rmax;
-    lo = lo < rmin ? rmin : lo;
-    hi = hi > rmax ? rmax : hi;
-    if (hi <= lo) continue;
-    const double a = lo - h > 0 ? lo - h : 0, z = hi + h;
-    const double v = 4.0 / 3.0 * M_PI * (z * z * z - a * a * a) / (dx * dx * dx), ir = 1.0 / std::max(a / dx, 1.0);
-    double *w = &want[CG_IMAP_CLASSES * (shell_of[k + 1] + 1)];
-    auto painted = [&](int i) { return i >= -1 && i < nb && shell_of[i + 1] >= 0 && shell_of[i + 1] < nr; };
-    const bool plain = painted(k - 1) && painted(k) && painted(k + 1) && bb[k + 1] - bb[k] >= 2.1 * dx;
-    w[0] += plain ? v * std::min(5 * ir + 0.01, 1.0) : v;
-    w[1] += v * std::min(2.0 / 3.0 + ir, 1.0);
-    w[2] += v * std::min(1.0 / 3.0 + ir, 1.0);
-  }
+  const double ncell = (double)c->N * c->N * c->N;
+  const int nrm = 2 * (nr + 2);
+  std::vector<double> want(nrm), part(nrm);
+  cg_imap_rooms(bb.data(), nb, shell_of.data(), nr, rmin, rmax, dx, ncell, want.data(), part.data());
   double tot = 0;
-  for (int i = 0; i < nbk; i++) {
-    want[i] = std::min(want[i], ncell) + 64;
-    tot += want[i];
-  }
-  /* room: every cell, within a quarter of the free memory and the
-   * caller's bound (cells beyond are painted by the listing kernel) */
+  for (double w : want) tot += w;
+  /* room for every cell, within a quarter of the free memory and the caller's
+   * bound: a cut room is divided between its ends, and the cells that find
+   * their part full are painted by the listing kernel */
   size_t fr = 0, tt = 0;
   CUDA_TRY(c, cudaMemGetInfo(&fr, &tt));
   double room = (double)(fr + (size_t)c->list_cap * CG_IMAP_REC_BYTES) * 0.25 / CG_IMAP_REC_BYTES;
   if (c->list_cap_max > 0 && room > (double)c->list_cap_max) room = (double)c->list_cap_max;
-  const double scale = tot > room ? room / tot : 1.0;
-  std::vector<long long> base(nbk), capv(nbk);
+  const bool cut = tot > room;
+  std::vector<long long> at(2 * nrm), capv(2 * nrm);
   long long acc = 0;
-  for (int i = 0; i < nbk; i++) {
-    base[i] = acc;
-    capv[i] = (long long)(want[i] * scale);
-    acc += capv[i];
+  for (int i = 0; i < nrm; i++) {
+    const long long n = (long long)(want[i] * (cut ? room / tot : 1.0));
+    capv[2 * i] = cut ? (long long)((double)n * part[i]) : n;
+    capv[2 * i + 1] = cut ? n - capv[2 * i] : n;
+    /* the shell's rooms meet at their general ends */
+    at[2 * i + (i & 1 ? 0 : 1)] = acc;
+    at[2 * i + (i & 1 ? 1 : 0)] = acc + n - 1;
+    acc += n;
   }
   if (acc > c->list_cap) {
     if ((rc = dalloc(c, &c->d_recs, (size_t)acc))) return rc;
@@ -1718,8 +1701,8 @@ static int imap_prepare(cg_ctx *c, int ip)
   for (int i = 0; i < nr + 2; i++) dxsl[i] = (float)(dx / nsub[i] - (double)dxs[i]);
   CUDA_TRY(c, cudaMemcpyAsync(M.dxsl, dxsl.data(), (nr + 2) * sizeof(float), cudaMemcpyHostToDevice, c->stream));
 
-  CUDA_TRY(c, cudaMemcpyAsync(M.base, base.data(), nbk * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
-  CUDA_TRY(c, cudaMemcpyAsync(M.cap, capv.data(), nbk * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(c, cudaMemcpyAsync(M.at, at.data(), at.size() * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(c, cudaMemcpyAsync(M.cap, capv.data(), capv.size() * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream)); /* host staging vectors */
   M.nb = nb;
   M.contig = cg_imap_contig(r0f.data(), rff.data(), nr, nb);
@@ -1802,10 +1785,11 @@ static int imap_launch(cg_ctx *c, int ip)
   p.xstats = c->d_xstats;
   p.force_double = c->force_double;
   p.recs = c->d_recs;
-  p.base = M.base;
+  p.at = M.at;
   p.cap = M.cap;
   p.cnt = M.cnt;
   p.chunk_off = M.chunk_off;
+  p.buckets = M.buckets;
   p.ctr = M.ctr;
   p.queue = c->d_imap_queue;
   p.queue_cap = c->queue_cap;
@@ -1864,7 +1848,7 @@ extern "C" int cg_set_imap_list_cap(cg_ctx *c, long long cap)
 {
   if (!c || cap < 0) return CG_EINVAL;
   c->list_cap_max = cap;
-  for (int ip = 0; ip < CG_NPOP_MAX; ip++) c->im[ip].gen = 0; /* bucket room is recomputed */
+  for (int ip = 0; ip < CG_NPOP_MAX; ip++) c->im[ip].gen = 0; /* the rooms are recomputed */
   return CG_OK;
 }
 

@@ -23,6 +23,7 @@ enum : unsigned int {
   ERR_IMAP_NSUB = 8u,        /* sub-sampling factor out of range       */
   ERR_IMAP_QUEUE = 16u,      /* intensity-map double-decision queue full */
   ERR_DEPOSIT_OVERFLOW = 64u, /* a cell of the particle deposit holds 2^11 or more */
+  ERR_IMAP_ROOM = 128u,      /* more cells listed than a shell's room holds */
 };
 
 /* The particle deposit accumulates mass in fixed point, 2^20 units per

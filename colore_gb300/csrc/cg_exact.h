@@ -1393,6 +1393,11 @@ CG_HD void cgx_imap_sample(const cg_imap_args *a, int ix, int iy, int iz, int ns
  * coordinate error 1.8 2^-24 (1 + 2 dx / r) is at most this. */
 #define CG_CELL_EIN (2.3f * CG_E24)
 
+/* Whether a cell's corner (r2 its squared radius) lies at |cos theta| > 2/3, as
+ * those of CG_CELL_POLAR do and those of CG_CELL_EQ do not (both by 1e-5 of
+ * rho^2). */
+CG_HD int cg_corner_polar(float zc, float r2) { return CG_MUL(9.0f, CG_MUL(zc, zc)) > CG_MUL(4.0f, r2); }
+
 CG_HD int cg_cell_class(const cg_imap_args *a, const cg_imap_cell *c, float xc, float yc, float zc)
 {
   const float dx = a->dx;
@@ -1807,6 +1812,45 @@ static inline int cg_imap_shells(const double *r0d, const double *rfd, int nr, d
     dxs[i + 1] = (float)(dx / nsub[i + 1]);
   }
   return nb;
+}
+
+/* Rooms for the listed cells: two per shell of the corners, -1 .. nr, one for
+ * the cells whose corner lies at |cos theta| <= 2/3 and one for those beyond
+ * (cg_corner_polar).  Each holds every such cell: their dx-cubes about the
+ * corners lie within h = sqrt(3)/2 dx of the shell's intervals, so the shell
+ * widened by h bounds their number, and with sin(h's angle) <= 0.87 dx / r the
+ * parts of it are at most 2/3 + dx / r and 1/3 + dx / r.  The cells painted by
+ * the general loop fill a room from one end, those of a per-cell loop
+ * (CG_CELL_EQ, CG_CELL_POLAR: each in its own room) from the other, so neither
+ * can run out while the other leaves room, however many cells span shells.
+ * part: the general cells' part of a room that is cut (a bounded list) -- those
+ * on the four planes between octants and the two cones, 3.5 cells deep, where
+ * shells are thick and their neighbours painted, else half. */
+static inline void cg_imap_rooms(const float *b, int nb, const int *shell_of, int nr, double rmin, double rmax,
+                                 double dx, double ncell, double *room, double *part)
+{
+  const double pi = 3.14159265358979323846, h = 0.8660254037844387 * dx;
+  for (int i = 0; i < 2 * (nr + 2); i++) room[i] = part[i] = 0;
+  for (int k = -1; k < nb; k++) {
+    double lo = k < 0 ? rmin : (double)b[k], hi = k + 1 < nb ? (double)b[k + 1] : rmax;
+    lo = lo < rmin ? rmin : lo;
+    hi = hi > rmax ? rmax : hi;
+    if (hi <= lo) continue;
+    const double a = lo - h > 0 ? lo - h : 0, z = hi + h, ir = dx / (a > dx ? a : dx);
+    const double v = 4.0 / 3.0 * pi * (z * z * z - a * a * a) / (dx * dx * dx);
+    int plain = k > -1 && k + 1 < nb && (double)b[k + 1] - (double)b[k] >= 2.1 * dx;
+    for (int i = k - 1; i <= k + 1 && plain; i++) plain = i >= -1 && shell_of[i + 1] >= 0 && shell_of[i + 1] < nr;
+    const double f = plain && 5 * ir + 0.01 < 0.5 ? 5 * ir + 0.01 : 0.5;
+    const double w[2] = {fmin(2.0 / 3.0 + ir, 1.0) * v, fmin(1.0 / 3.0 + ir, 1.0) * v};
+    for (int q = 0; q < 2; q++) {
+      room[2 * (shell_of[k + 1] + 1) + q] += w[q];
+      part[2 * (shell_of[k + 1] + 1) + q] += f * w[q];
+    }
+  }
+  for (int i = 0; i < 2 * (nr + 2); i++) {
+    part[i] = room[i] > 0 ? part[i] / room[i] : 0.5;
+    room[i] = fmin(room[i], ncell) + 64;
+  }
 }
 
 /* The most samples that one pixel of one shell can take.  A sample's pixel is

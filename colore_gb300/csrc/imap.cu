@@ -16,23 +16,25 @@
  * the observer (from 2 at high redshift to ~20 for the nearest shells), and
  * a cell's class says which loop its samples need (cg_cell_class), so cells
  * are listed per shell and class -- one bucket each, holding cells of one
- * nsub and one loop -- and painted bucket after bucket:
+ * nsub and one loop -- and painted bucket after bucket.  The buckets of a shell
+ * share two rooms from both ends (cg_imap_rooms), which no share of general
+ * cells overfills:
  *
  *   k_imap_tab     The radial tables as one 32-byte record per segment.
  *   k_imap_list    Warps take groups of rows from a counter; a lane decides
  *                  one cell (listed or not, its shell, brightness, radial
  *                  shift, and whether all its samples certainly stay in one
  *                  shell or straddle one edge) from one segment record
- *                  (cg_imap_cell_seg) and appends it to its bucket: one atomic
- *                  per bucket present in the warp, all issued together, on
+ *                  (cg_imap_cell_seg) and appends it to its room: one atomic
+ *                  per counter present in the warp, all issued together, on
  *                  counters that have a 128-byte line each (next to each other
  *                  they sat in one L2 slice, whose atomics bounded the kernel:
  *                  65 against 54 ms of the stage at 1024^3).  Cells that the
- *                  segments leave open, and cells that find their bucket full
+ *                  segments leave open, and cells that find their room full
  *                  (painted by the warp), wait until the warp's rows are done.
  *                  487 thread-instructions a cell in range where a lookup with
  *                  a bound per table took 689: 20.6 -> 11.5 ms at 1024^3.
- *   k_imap_chunks  One block cuts each bucket into chunks of about CHS
+ *   k_imap_chunks  One block finds each bucket's records and cuts it into chunks of about CHS
  *                  samples: whole cells, or slices of one cell.
  *   k_imap_paint   Warps take chunks in bucket order, so the maps' working
  *                  set at any time is a few shells (50 MB per shell at nside
@@ -106,7 +108,7 @@ __device__ __forceinline__ Sh shells_at(const cg_imap_params &p, unsigned char *
 /* The painting warps' queue stages follow the tables. */
 __host__ __device__ __forceinline__ size_t paint_stage_off(int nr, int nbk) { return (shell_smem(nr, nbk, true) + 15) & ~(size_t)15; }
 __host__ __device__ __forceinline__ size_t paint_smem(int nr, int nbk) { return paint_stage_off(nr, nbk) + (size_t)IW * (QB * 8 + 4); }
-/* The double pass keeps the buckets' bases where the painting keeps its
+/* The double pass keeps the shells' bases where the painting keeps its
  * chunk table; its per-warp gathers (64 entries) follow. */
 __host__ __device__ __forceinline__ size_t double_stage_off(int nr, int nbk) { return (shell_smem(nr, nbk, true) + 15) & ~(size_t)15; }
 
@@ -136,6 +138,55 @@ __device__ __forceinline__ cg_imap_args args_with(const cg_imap_params &p, const
   A.dxs = s.dxs;
   return A;
 }
+
+/* The counter of a listed cell: its room (shell j, polar corner or not) and the
+ * end it is listed from. */
+__device__ __forceinline__ int counter_of(int j, int polar, int cls)
+{
+  return 4 * (j + 1) + (cls == CG_CELL_GENERAL ? 2 * polar : 2 * cls - 1);
+}
+
+/* Slot k of counter ct: the fast equatorial and the general polar cells upwards
+ * from their room's begin, the others downwards from its end. */
+__device__ __forceinline__ long long slot_of(const cg_imap_params &p, int ct, long long k)
+{
+  return p.at[ct] + (((ct ^ (ct >> 1)) & 1) ? k : -k);
+}
+
+/* Cells listed on counter ct.  None when both ends hold more than the room,
+ * which bounds their sum unless the list is cut, and then the caps do. */
+__device__ __forceinline__ long long listed(const cg_imap_params &p, int ct)
+{
+  long long n[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int c = (ct & ~1) + k;
+    const long long m = (long long)p.cnt[(size_t)c * CG_IMAP_CNT];
+    n[k] = m < p.cap[c] ? m : p.cap[c];
+  }
+  const long long room = llabs(p.at[ct | 1] - p.at[ct & ~1]) + 1;
+  if (n[0] + n[1] > room) {
+    atomicOr(p.err, ERR_IMAP_ROOM);
+    return 0;
+  }
+  return n[ct & 1];
+}
+
+/* A bucket's records, one after the other: the first and their number.  The
+ * shell's rooms lie next to each other, with the general cells at the ends that
+ * meet. */
+__device__ __forceinline__ longlong2 bucket_of(const cg_imap_params &p, int b)
+{
+  const int s = b / CG_IMAP_CLASSES, cls = b - s * CG_IMAP_CLASSES;
+  if (cls == CG_CELL_GENERAL) {
+    const long long n = listed(p, 4 * s);
+    return make_longlong2(p.at[4 * s + 2] - n, n + listed(p, 4 * s + 2));
+  }
+  const long long n = listed(p, 4 * s + 2 * cls - 1);
+  return make_longlong2(cls == CG_CELL_EQ ? p.at[4 * s + 1] : p.at[4 * s + 3] + 1 - n, n);
+}
+
+static_assert(CG_CELL_GENERAL == 0 && CG_CELL_EQ == 1 && CG_CELL_POLAR == 2, "rooms by class");
 
 template <typename K>
 __device__ __forceinline__ K empty_key()
@@ -319,9 +370,9 @@ __device__ __noinline__ OpenCell cell_open(const cg_imap_params &p, int ix, int 
   return o;
 }
 
-/* Cells past their bucket's room (m: their lanes), painted by the warp. */
+/* Cells past their room (m: their lanes), painted by the warp. */
 template <typename K>
-__device__ __forceinline__ void paint_over(const cg_imap_params &p, unsigned m, const cg_imap_rec &rec, int bk, int lane)
+__device__ __forceinline__ void paint_over(const cg_imap_params &p, unsigned m, const cg_imap_rec &rec, int ct, int lane)
 {
   while (m) {
     const int l = __ffs(m) - 1;
@@ -331,7 +382,7 @@ __device__ __forceinline__ void paint_over(const cg_imap_params &p, unsigned m, 
     r.izf = __shfl_sync(FULL, rec.izf, l);
     r.temp = __shfl_sync(FULL, rec.temp, l);
     r.drr = __shfl_sync(FULL, rec.drr, l);
-    const int j = __shfl_sync(FULL, bk, l) / CG_IMAP_CLASSES - 1;
+    const int j = __shfl_sync(FULL, ct, l) / 4 - 1;
     int ix, iy, iz, dbl;
     const cg_imap_cell c = unpack(r, j, &ix, &iy, &iz, &dbl);
     const int ns = p.a.nsub[j + 1], n3 = ns * ns * ns;
@@ -347,7 +398,7 @@ __device__ __forceinline__ void paint_over(const cg_imap_params &p, unsigned m, 
 }
 
 /* A warp's rows in words of 32 cells: the cells that the segments leave open,
- * and those that found their bucket full. */
+ * and those that found their room full. */
 struct Late {
   unsigned open[ROWS * LATE_CH], over[ROWS * LATE_CH];
 };
@@ -367,7 +418,7 @@ __device__ __noinline__ void late_cells(const float *__restrict__ dens, const cg
     const int row = rbeg + g / nch, ix = (g % nch) * 32 + lane;
     const int iz = (int)divN(row, p.box), iy = row - iz * N;
     bool over = false;
-    int bk = -1;
+    int ct = 0;
     cg_imap_rec rec = {0u, 0u, 0.0f, 0.0f};
     if ((any >> lane) & 1u) {
       float v[3];
@@ -376,23 +427,24 @@ __device__ __noinline__ void late_cells(const float *__restrict__ dens, const cg
       if (o.st == 1) {
         const int sfin = o.c.j + o.c.delta;
         const bool want = !(o.c.mode == CG_SH_SINGLE && (sfin < 0 || sfin >= p.nr));
-        const int cls = o.dbl ? CG_CELL_GENERAL : cg_cell_class(&p.a, &o.c, p.a.xc[ix], p.a.yc[iy], p.a.zc[iz]);
-        bk = CG_IMAP_CLASSES * (o.c.j + 1) + cls;
+        const float x0 = p.a.xc[ix], y0 = p.a.yc[iy], z0 = p.a.zc[iz];
+        ct = counter_of(o.c.j, cg_corner_polar(z0, CG_FMA(x0, x0, CG_FMA(z0, z0, CG_MUL(y0, y0)))),
+                        o.dbl ? CG_CELL_GENERAL : cg_cell_class(&p.a, &o.c, x0, y0, z0));
         rec = pack(ix, iy, iz, o.c, (unsigned)o.c.mode | ((unsigned)(o.c.delta + 1) << 2) | (o.dbl ? F_DOUBLE : 0u));
         over = want;
         if ((open >> lane) & 1u) {
           const int ns = p.a.nsub[o.c.j + 1];
           drawn += (unsigned long long)ns * ns * ns;
           if (want) {
-            const long long k = (long long)atomicAdd(&p.cnt[(size_t)bk * CG_IMAP_CNT], 1ull);
-            over = k >= p.cap[bk];
-            if (!over) p.recs[p.base[bk] + k] = rec;
+            const long long k = (long long)atomicAdd(&p.cnt[(size_t)ct * CG_IMAP_CNT], 1ull);
+            over = k >= p.cap[ct];
+            if (!over) p.recs[slot_of(p, ct, k)] = rec;
           }
         }
       }
       if ((open >> lane) & 1u) ndbl += o.in_double;
     }
-    paint_over<K>(p, __ballot_sync(FULL, over), rec, bk, lane);
+    paint_over<K>(p, __ballot_sync(FULL, over), rec, ct, lane);
   }
   if (drawn) atomicAdd(&p.ctr[2], drawn);
   if (ndbl) atomicAdd(p.xstats + 2, ndbl);
@@ -467,20 +519,20 @@ __global__ void __launch_bounds__(IW * 32, 12) k_imap_list(const float *__restri
           any_late = 1u;
         }
         if (!__any_sync(FULL, want)) continue;
-        /* append to the buckets: one atomic per bucket present in the warp,
-         * issued together by each bucket's first lane (one round trip) */
-        int bk = -1;
-        if (want) bk = CG_IMAP_CLASSES * (c.j + 1) + cg_cell_class(&A, &c, x0, y0, z0);
-        const unsigned same = __match_any_sync(FULL, bk);
+        /* append to the rooms: one atomic per counter present in the warp,
+         * issued together by each counter's first lane (one round trip) */
+        int ct = -1;
+        if (want) ct = counter_of(c.j, cg_corner_polar(z0, r2), cg_cell_class(&A, &c, x0, y0, z0));
+        const unsigned same = __match_any_sync(FULL, ct);
         const int leader = __ffs(same) - 1;
         unsigned long long old = 0;
-        if (want && lane == leader) old = atomicAdd(&p.cnt[(size_t)bk * CG_IMAP_CNT], (unsigned long long)__popc(same));
+        if (want && lane == leader) old = atomicAdd(&p.cnt[(size_t)ct * CG_IMAP_CNT], (unsigned long long)__popc(same));
         old = __shfl_sync(FULL, old, leader);
         bool over = false;
         if (want) {
           const long long k = (long long)old + __popc(same & ((1u << lane) - 1u));
-          over = k >= p.cap[bk];
-          if (!over) p.recs[p.base[bk] + k] = pack(ix, iy, iz, c, (unsigned)c.mode | ((unsigned)(c.delta + 1) << 2));
+          over = k >= p.cap[ct];
+          if (!over) p.recs[slot_of(p, ct, k)] = pack(ix, iy, iz, c, (unsigned)c.mode | ((unsigned)(c.delta + 1) << 2));
         }
         const unsigned vm = __ballot_sync(FULL, over);
         if (vm) {
@@ -524,9 +576,10 @@ __global__ void __launch_bounds__(1024) k_imap_chunks(cg_imap_params p)
     const int b = b0 + threadIdx.x;
     unsigned long long x = 0;
     if (b < p.nbk) {
-      const unsigned long long n = p.cnt[(size_t)b * CG_IMAP_CNT] < (unsigned long long)p.cap[b] ? p.cnt[(size_t)b * CG_IMAP_CNT] : (unsigned long long)p.cap[b];
       const int ns = p.a.nsub[b / CG_IMAP_CLASSES];
-      const unsigned long long nu = n * (unsigned long long)units_per_cell(ns);
+      const longlong2 B = bucket_of(p, b);
+      p.buckets[b] = B;
+      const unsigned long long nu = (unsigned long long)B.y * (unsigned long long)units_per_cell(ns);
       const unsigned long long per = 32ull * (unsigned long long)groups_per_chunk(ns);
       x = (nu + per - 1) / per;
     }
@@ -776,7 +829,7 @@ __device__ __forceinline__ void paint_chunk(const cg_imap_params &p, const cg_im
         }
       }
     }
-    const long long rec = p.base[b] + rl;
+    const long long rec = p.buckets[b].x + rl;
     float temp = 0.0f;
     Lane<K> L;
     L.k = empty_key<K>();
@@ -833,10 +886,8 @@ __global__ void __launch_bounds__(IW * 32, 7) k_imap_paint(const __grid_constant
       else hi = mid - 1;
     }
     const int b = lo;
-    const unsigned long long nrec =
-        p.cnt[(size_t)b * CG_IMAP_CNT] < (unsigned long long)p.cap[b] ? p.cnt[(size_t)b * CG_IMAP_CNT] : (unsigned long long)p.cap[b];
     const int ns = sh.nsub[b / CG_IMAP_CLASSES];
-    const unsigned long long nu = nrec * (unsigned long long)units_per_cell(ns);
+    const unsigned long long nu = (unsigned long long)p.buckets[b].y * (unsigned long long)units_per_cell(ns);
     const int G = groups_per_chunk(ns);
     const float dxs = sh.dxs[b / CG_IMAP_CLASSES];
     const unsigned long long u0 = (ck - sh.chunk_off[b]) * 32ull * (unsigned long long)G;
@@ -864,15 +915,15 @@ __device__ __forceinline__ void double_batch(const float *__restrict__ phi, cons
   float temp = 0.0f;
   double drr = 0;
   if (lead) {
-    /* the record's bucket: last b with base[b] <= rec */
-    int hi = p.nbk - 1;
+    /* the record's shell: the last whose rooms begin at or before it */
+    int hi = p.nr + 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (sbase[mid] <= rec) lo = mid;
       else hi = mid - 1;
     }
     int dbl;
-    const cg_imap_cell c = unpack(p.recs[rec], lo / CG_IMAP_CLASSES - 1, &ix, &iy, &iz, &dbl);
+    const cg_imap_cell c = unpack(p.recs[rec], lo - 1, &ix, &iy, &iz, &dbl);
     temp = c.temp;
     float v[3];
     grad_phi(phi, ix, iy, iz, p.box.N, v);
@@ -886,7 +937,6 @@ __device__ __forceinline__ void double_batch(const float *__restrict__ phi, cons
   temp = __shfl_sync(FULL, temp, src);
   drr = __shfl_sync(FULL, drr, src);
   if (!valid) return;
-  lo /= CG_IMAP_CLASSES;
   const int ns = sh.nsub[lo];
   int s = -1, sx, sy, sz;
   sub_of(q, ns, sh.invns[lo], &sx, &sy, &sz);
@@ -907,8 +957,8 @@ __global__ void __launch_bounds__(DB_WARPS * 32) k_imap_double(const float *__re
 {
   extern __shared__ __align__(16) unsigned char sraw[];
   const Sh sh = load_shells(p, sraw, false);
-  long long *sbase = reinterpret_cast<long long *>(sh.chunk_off); /* the buckets' first records */
-  for (int i = threadIdx.x; i < p.nbk; i += blockDim.x) sbase[i] = p.base[i];
+  long long *sbase = reinterpret_cast<long long *>(sh.chunk_off); /* the shells' first records */
+  for (int i = threadIdx.x; i < p.nr + 2; i += blockDim.x) sbase[i] = p.at[4 * i + 1];
   __syncthreads();
   const cg_imap_args A = args_with(p, sh);
   unsigned long long *db = reinterpret_cast<unsigned long long *>(sraw + double_stage_off(p.nr, p.nbk)) +
@@ -927,16 +977,15 @@ __global__ void __launch_bounds__(DB_WARPS * 32) k_imap_double(const float *__re
     if (valid && !p.force_double) {
       const long long rec = (long long)(e >> 30);
       const int q = (int)(e & ((1ull << 30) - 1));
-      int lo = 0, hi = p.nbk - 1;
+      int lo = 0, hi = p.nr + 1;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (sbase[mid] <= rec) lo = mid;
         else hi = mid - 1;
       }
       int ix, iy, iz, dbl;
-      const cg_imap_cell c = unpack(p.recs[rec], lo / CG_IMAP_CLASSES - 1, &ix, &iy, &iz, &dbl);
+      const cg_imap_cell c = unpack(p.recs[rec], lo - 1, &ix, &iy, &iz, &dbl);
       if (!dbl) {
-        lo /= CG_IMAP_CLASSES;
         const int ns = sh.nsub[lo];
         int s = -1, sx, sy, sz;
         long long pix = 0;
@@ -969,7 +1018,7 @@ template <typename K>
 cudaError_t launch(cudaStream_t s, const float *dens, const float *phi, const cg_imap_params *p, int nsm)
 {
   cudaError_t e = cudaMemsetAsync(p->ctr, 0, 5 * sizeof(unsigned long long), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(p->cnt, 0, (size_t)p->nbk * CG_IMAP_CNT * sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->cnt, 0, (size_t)4 * (p->nr + 2) * CG_IMAP_CNT * sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(p->seg + p->a.na - 1, 0, sizeof(cg_imap_seg), s);
   if (e != cudaSuccess) return e;
   const size_t sm_list = shell_smem(p->nr, p->nbk, false), sm_paint = paint_smem(p->nr, p->nbk);

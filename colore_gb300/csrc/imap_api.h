@@ -23,7 +23,7 @@ struct __align__(16) cg_imap_rec {
 /* A bucket per shell -1 .. nr of the cells' corners and per class of
  * cg_cell_class: bucket 3 (j + 1) + class. */
 #define CG_IMAP_CLASSES 3
-#define CG_IMAP_CNT 16 /* stride of the buckets' counters: a 128-byte line each */
+#define CG_IMAP_CNT 16 /* stride of the rooms' counters: a 128-byte line each */
 #define CG_IMAP_BUCKETS_MAX (CG_IMAP_CLASSES * 4100) /* nr <= 4096 */
 
 struct cg_imap_params {
@@ -40,14 +40,17 @@ struct cg_imap_params {
   unsigned long long *xstats; /* [2] cells, [3] samples decided in double */
   int force_double;
   /* cells are listed per bucket (the shell of their corner, which fixes nsub,
-   * and the class, which fixes the painting loop), in the slots [base[b],
-   * base[b] + cap[b]); cnt[CG_IMAP_CNT b] counts them (may exceed cap: those
-   * cells are painted by the listing kernel) */
+   * and the class, which fixes the painting loop).  Shell j has two rooms
+   * (cg_imap_rooms) next to each other, w = 2 (j + 1) + (polar corner): general
+   * cells on counter 2 w, the others on 2 w + 1 (CG_IMAP_CNT apart), from slot
+   * at[counter] on, one upwards and one downwards.  Either may exceed its cap:
+   * those cells are painted by the listing kernel */
   cg_imap_rec *recs;
-  const long long *base, *cap;
+  const long long *at, *cap;
   unsigned long long *cnt;
-  /* chunks of the painting pass: chunk_off[b] the first chunk of bucket b
-   * (nbk + 1 entries, set on the device) */
+  /* set on the device: the first record of every bucket and their number, and
+   * the painting pass's chunks, chunk_off[b] the first of bucket b (nbk + 1) */
+  longlong2 *buckets;
   unsigned long long *chunk_off;
   /* ctr: [0] chunks taken, [1] rows taken, [2] samples drawn, [3] samples
    * painted by the listing kernel, [4] double-queue entries */

@@ -587,6 +587,73 @@ int or_imap32(const cg_config *cfg, int ipop, const float *dens, const float *np
   return 0;
 }
 
+/* The listing's tables: the segments, their largest factor bound, and the
+ * shells' edges between sentinels, which a->sh.b then points to. */
+static cg_imap_seg *listing_tables(cg_imap_args *a, float *eg, float **edges)
+{
+  const int na = a->na, nb = a->sh.nb;
+  cg_imap_seg *segs = aligned_alloc(32, (size_t)na * sizeof(cg_imap_seg));
+  *eg = 0;
+  for (int i = 0; i < na - 1; i++) {
+    float e;
+    segs[i] = cg_imap_seg_make(a, i, &e);
+    if (e > *eg) *eg = e;
+  }
+  float *b = malloc((size_t)(nb + 4) * sizeof(float));
+  b[0] = b[1] = -3.0e38f;
+  for (int i = 0; i < nb; i++) b[i + 2] = a->sh.b[i];
+  b[nb + 2] = b[nb + 3] = 3.0e38f;
+  *edges = b;
+  a->sh.b = b + 2;
+  return segs;
+}
+
+/* The listed cells per room and end (cells: 4 (nr + 2), the kernel's counters)
+ * and the rooms (cg_imap_rooms, 2 (nr + 2)). */
+int or_imap_rooms(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
+                  const double *norm64, long long *cells, double *room, double *part)
+{
+  S32 s;
+  s32_init(&s, cfg);
+  ImapArgs B;
+  imap_args(&B, cfg, &s, ipop, norm32, norm64);
+  cg_imap_args *a = &B.a;
+  const int N = s.N, nr = a->sh.nr;
+  cg_imap_rooms(a->sh.b, a->sh.nb, a->sh.shell_of, nr, a->rmin64, a->rmax64, a->dx64, (double)N * N * N, room, part);
+  float eg, *edges;
+  cg_imap_seg *segs = listing_tables(a, &eg, &edges);
+  for (int k = 0; k < 4 * (nr + 2); k++) cells[k] = 0;
+  for (int iz = 0; iz < N; iz++)
+    for (int iy = 0; iy < N; iy++)
+      for (int ix = 0; ix < N; ix++) {
+        float v[3];
+        grad32(npot, ix, iy, iz, N, v);
+        const float d = dens[pidx(ix, iy, iz, N)];
+        const float x0 = a->xc[ix], y0 = a->yc[iy], z0 = a->zc[iz];
+        const float r2 = CG_FMA(x0, x0, CG_FMA(z0, z0, CG_MUL(y0, y0)));
+        cg_imap_cell c;
+        int dbl = 0;
+        int k = cg_imap_cell_seg(segs, eg, a, x0, y0, z0, r2, d, v, &c);
+        if (k == 2) k = cg_imap_cell_checked(a, ix, iy, iz, d, v, &c);
+        if (k == 2) {
+          double drr;
+          k = cgx_imap_cell(a, ix, iy, iz, v, &c.j, &drr);
+          dbl = 1;
+        }
+        if (!k) continue;
+        const int sf = c.j + c.delta;
+        if (!dbl && c.mode == CG_SH_SINGLE && (sf < 0 || sf >= nr)) continue;
+        const int cls = dbl ? CG_CELL_GENERAL : cg_cell_class(a, &c, x0, y0, z0), pol = cg_corner_polar(z0, r2);
+        if ((cls == CG_CELL_EQ && pol) || (cls == CG_CELL_POLAR && !pol)) return 1;
+        cells[4 * (c.j + 1) + 2 * pol + (cls != CG_CELL_GENERAL)]++;
+      }
+  free(edges);
+  free(segs);
+  imap_args_free(&B);
+  s32_free(&s);
+  return 0;
+}
+
 /* The listing of every cell from the per-segment tables (cg_imap_cell_seg)
  * against the double arithmetic.  stat: [0] cells settled, [1] of them listed,
  * [2] open; and faults: [3] listed or not, [4] shell of the corner, [5] radial
@@ -608,19 +675,9 @@ int or_imap_cells(const cg_config *cfg, int ipop, const float *dens, const float
   ImapArgs B;
   imap_args(&B, cfg, &s, ipop, norm32, norm64);
   cg_imap_args *a = &B.a;
-  const int N = s.N, na = a->na, nb = a->sh.nb;
-  cg_imap_seg *segs = aligned_alloc(32, (size_t)na * sizeof(cg_imap_seg));
-  float eg = 0;
-  for (int i = 0; i < na - 1; i++) {
-    float e;
-    segs[i] = cg_imap_seg_make(a, i, &e);
-    if (e > eg) eg = e;
-  }
-  float *edges = malloc((size_t)(nb + 4) * sizeof(float));
-  edges[0] = edges[1] = -3.0e38f;
-  for (int i = 0; i < nb; i++) edges[i + 2] = a->sh.b[i];
-  edges[nb + 2] = edges[nb + 3] = 3.0e38f;
-  a->sh.b = edges + 2;
+  const int N = s.N;
+  float eg, *edges;
+  cg_imap_seg *segs = listing_tables(a, &eg, &edges);
   for (int k = 0; k < 8; k++) stat[k] = 0;
   for (int iz = 0; iz < N; iz++)
     for (int iy = 0; iy < N; iy++)

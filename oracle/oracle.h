@@ -94,6 +94,8 @@ int or_imap32(const cg_config *cfg, int ipop, const float *dens, const float *np
               const double *norm64, float *data, int *nadd, long long *stats);
 int or_imap_cells(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
                   const double *norm64, long long *stat);
+int or_imap_rooms(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
+                  const double *norm64, long long *cells, double *room, double *part);
 int or_kappa32(const cg_config *cfg, const float *npot, float *map);
 int or_isw32(const cg_config *cfg, const float *npot, float *map);
 int or_cstm32(const cg_config *cfg, int ipop, const float *dens, const float *normtab, float n0, float nf,

@@ -38,6 +38,7 @@ def lib():
             "or_emit64": [vp, i, vp, vp, C.c_longlong, vp, vp, vp, vp, vp],
             "or_beam_rsd32": [vp, vp, C.c_longlong, vp, vp], "or_imap32": [vp, i, vp, vp, vp, vp, vp, vp, vp],
             "or_imap_cells": [vp, i, vp, vp, vp, vp, vp], "or_imap_pixel_max": [vp, i],
+            "or_imap_rooms": [vp, i, vp, vp, vp, vp, vp, vp, vp],
             "or_kappa32": [vp, vp, vp], "or_isw32": [vp, vp, vp], "or_isw64": [vp, vp, vp],
             "or_cstm_steps": [vp, i, vp, vp, vp, vp], "or_cstm64": [vp, i, vp, vp, d, d, vp],
             "or_cstm32": [vp, i, vp, vp, f, f, vp],
@@ -338,6 +339,20 @@ def imap_cells(cfg, ipop, dens, npot, tab32, e32, tab64, e64):
     lib().or_imap_cells(cfgp(cfg), ipop, P(np.ascontiguousarray(dens, np.float32)),
                         P(np.ascontiguousarray(npot, np.float32)), P(t32), P(t64), P(st))
     return tuple(int(v) for v in st)
+
+
+def imap_rooms(cfg, ipop, dens, npot, tab32, e32, tab64, e64):
+    """Listed cells (shells -1 .. nr, equatorial and polar corners, general and
+    fast) and the rooms for them (shells, corners), with the general cells'
+    part where the list is cut."""
+    nr = cfg.imap_nr[ipop]
+    cells = np.zeros((nr + 2, 2, 2), np.int64)
+    room, part = np.zeros((nr + 2, 2)), np.zeros((nr + 2, 2))
+    t32, t64 = _norm_pair(tab32, e32, tab64, e64)
+    assert lib().or_imap_rooms(cfgp(cfg), ipop, P(np.ascontiguousarray(dens, np.float32)),
+                               P(np.ascontiguousarray(npot, np.float32)), P(t32), P(t64), P(cells), P(room),
+                               P(part)) == 0
+    return cells, room, part
 
 
 def imap_pixel_max(cfg, ipop):
