@@ -27,7 +27,7 @@
  *                  shell or straddle one edge) from one segment record
  *                  (cg_imap_cell_seg) and appends it to its room: one atomic
  *                  per counter present in the warp, all issued together, on
- *                  counters that have a 128-byte line each (next to each other
+ *                  counters that lie 256 bytes apart (next to each other
  *                  they sat in one L2 slice, whose atomics bounded the kernel:
  *                  65 against 54 ms of the stage at 1024^3).  Cells that the
  *                  segments leave open, and cells that find their room full
