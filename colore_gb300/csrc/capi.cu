@@ -413,17 +413,18 @@ static cudaError_t field_pass(int n, const cg_field_launch *L, int pass, int v, 
 }
 
 /* ---- tile autotuner of the transform passes ------------------------------
- * The first time a grid size runs on a device, each pass (the two fills,
- * the y and the x pass) is timed with every valid tile variant on the
+ * The first time a pass of a grid size runs on a device (the fills, the y and
+ * the x pass; not the Gaussian x pass up to 512^3, which keeps the plan's rows
+ * unless a width is forced), it is timed with every valid tile variant on the
  * context's own grids (before the real passes overwrite them): one launch to
  * warm up, then the mean of three with CUDA events.  The fastest variant is
  * kept for the life of the process, for every context of that size on that
  * device.  Variants differ only in block shape, so the choice never changes
  * a result.  COLORE_GB300_TUNE=0 keeps the plans' tiles. */
 struct FieldTune {
-  bool done[4] = {false, false, false, false};
-  int var[4] = {0, 0, 0, 0};
-  float ms[4][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
+  bool done[5] = {};
+  int var[5] = {};
+  float ms[5][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
 };
 static std::mutex g_tune_mu;
 static std::vector<std::pair<long long, FieldTune>> g_tune; /* key: device * 65536 + N */
@@ -442,6 +443,9 @@ static bool tuning_enabled()
   const char *e = getenv("COLORE_GB300_TUNE");
   return !(e && e[0] == '0');
 }
+
+/* The variant forced for a pass, or -1. */
+static int forced_variant(const cg_ctx *c, int pass) { return c->fforce[pass == CG_PASS_FILL9 ? CG_PASS_FILL3 : pass]; }
 
 /* Tune the passes listed (nf grids each) unless done; fills L->var. */
 static int tune_field_passes(cg_ctx *c, cg_field_launch *L, const int *passes, const int *nfs, int np)
@@ -484,7 +488,8 @@ static int tune_field_passes(cg_ctx *c, cg_field_launch *L, const int *passes, c
     t->var[pass] = bv;
     t->done[pass] = true;
   }
-  for (int p = 0; p < 4; p++) L->var[p] = c->fforce[p] >= 0 ? c->fforce[p] : t->var[p];
+  for (int p = 0; p < 5; p++) L->var[p] = forced_variant(c, p) >= 0 ? forced_variant(c, p) : t->var[p];
+  L->x_own = c->fforce[CG_PASS_X] > 0;
   return CG_OK;
 }
 
@@ -506,9 +511,10 @@ extern "C" int cg_field_plan(cg_ctx *c, char *buf, size_t len)
   std::lock_guard<std::mutex> lock(g_tune_mu);
   const FieldTune *t = tune_entry(c->device, c->N);
   size_t o = (size_t)snprintf(buf, len, "{\"n_grid\": %d, \"tuned\": %s", c->N, tuning_enabled() ? "true" : "false");
-  for (int p = 0; p < 4 && o < len; p++) {
-    const int v = c->fforce[p] >= 0 ? c->fforce[p] : t->var[p];
-    o += (size_t)snprintf(buf + o, len - o, ", \"%s\": {\"%s\": %d, \"timed\": %s, \"ms\": {", names[p], tiles[p],
+  for (int q = 0; q < 4 && o < len; q++) {
+    const int p = q == CG_PASS_FILL3 && c->cfg.dens_type == CG_DENS_2LPT ? CG_PASS_FILL9 : q;
+    const int v = forced_variant(c, p) >= 0 ? forced_variant(c, p) : t->var[p];
+    o += (size_t)snprintf(buf + o, len - o, ", \"%s\": {\"%s\": %d, \"timed\": %s, \"ms\": {", names[q], tiles[q],
                           field_tile(c->N, p, v), t->done[p] ? "true" : "false");
     bool first = true;
     for (int w = 0; w < 3 && o < len; w++) {
@@ -1075,7 +1081,7 @@ extern "C" int cg_create_cartesian_fields(cg_ctx *c)
   L.ev = nullptr;
   {
     const int passes[3] = {CG_PASS_FILL2, CG_PASS_Y, CG_PASS_X}, nfs[3] = {2, 2, 1};
-    if (int rc = tune_field_passes(c, &L, passes, nfs, 3)) return rc;
+    if (int rc = tune_field_passes(c, &L, passes, nfs, c->N > CG_FIELD_X_BOTH ? 3 : 2)) return rc;
   }
   {
     ProfScope ps(c, "field_fft");
@@ -1086,7 +1092,7 @@ extern "C" int cg_create_cartesian_fields(cg_ctx *c)
     CUDA_TRY(c, cg_moments_final(c->stream, c->d_part, c->npart, 1.0 / ncell, c->d_stats, c->d_s2f));
   }
   /* fill, y, x (one or two), the moments' sums (one or two) */
-  c->launches += 4 + (c->N > CG_FIELD_X_BOTH) + (c->npart > 8192);
+  c->launches += 4 + (c->N > CG_FIELD_X_BOTH || L.x_own) + (c->npart > 8192);
   c->have_fields = 1;
   c->have_density = c->have_norm = c->have_srcs = 0;
   c->pending_mode = CG_DMODE_NONE;
@@ -1131,12 +1137,12 @@ extern "C" int cg_compute_physical_density_field(cg_ctx *c)
     L.twN = c->d_twN;
     L.tws = c->d_tws;
     L.err = c->d_err;
+    for (int a = 0; a < 3; a++) L.f[a] = reinterpret_cast<float2 *>(c->d_disp[a]);
+    for (int a = 0; two && a < 6; a++) L.f2[a] = reinterpret_cast<float2 *>(c->d_lpt2[a]);
     {
-      for (int a = 0; a < 3; a++) L.f[a] = reinterpret_cast<float2 *>(c->d_disp[a]);
-      const int passes[3] = {CG_PASS_FILL3, CG_PASS_Y, CG_PASS_X}, nfs[3] = {3, 3, 3};
+      const int passes[3] = {two ? CG_PASS_FILL9 : CG_PASS_FILL3, CG_PASS_Y, CG_PASS_X}, nfs[3] = {3, 3, 3};
       if (int rc = tune_field_passes(c, &L, passes, nfs, 3)) return rc;
     }
-    for (int a = 0; two && a < 6; a++) L.f2[a] = reinterpret_cast<float2 *>(c->d_lpt2[a]);
     {
       ProfScope ps(c, "lpt_fft");
       PassEvents pe(c, "lpt_fill", "lpt_y", "lpt_x");

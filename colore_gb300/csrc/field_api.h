@@ -21,7 +21,8 @@ struct cg_field_launch {
   float2 *f2[6];        /* 2LPT: the second derivatives xx xy xz yy yz zz, else NULL */
   unsigned int *err;    /* device error word (bulk-copy timeouts) */
   cudaEvent_t *ev;      /* NULL, or events recorded after each pass (fill+z, y, x) */
-  int var[4];           /* tile variant of each pass (CG_PASS_*): 0 the plan's, 1 half, 2 twice */
+  int var[5];           /* tile variant of each pass (CG_PASS_*): 0 the plan's, 1 half, 2 twice */
+  int x_own;            /* the Gaussian potential's x pass alone, with its variant (a forced width) */
 };
 
 /* Passes whose tile width the autotuner picks. */
@@ -29,6 +30,7 @@ struct cg_field_launch {
 #define CG_PASS_FILL3 1 /* fill + z of the 1LPT displacements          */
 #define CG_PASS_Y 2     /* column transforms along y                   */
 #define CG_PASS_X 3     /* row c2r along x (without the moment sums)   */
+#define CG_PASS_FILL9 4 /* 2LPT's fill + z of nine grids, pass 1 to callers */
 
 #define CG_FIELD_X_BOTH 512 /* largest grid whose Gaussian x pass is one launch */
 

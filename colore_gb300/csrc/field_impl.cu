@@ -574,12 +574,13 @@ cudaError_t fill2_v(const cg_field_launch *L, int v)
   }
 }
 
+template <int SETS>
 cudaError_t fill3_v(const cg_field_launch *L, int v)
 {
   switch (v) {
-    case 1: return fill3<tile_of(PL::TX3, 1), 1>(L);
-    case 2: return fill3<tile_of(PL::TX3, 2), 1>(L);
-    default: return fill3<PL::TX3, 1>(L);
+    case 1: return fill3<tile_of(PL::TX3, 1), SETS>(L);
+    case 2: return fill3<tile_of(PL::TX3, 2), SETS>(L);
+    default: return fill3<PL::TX3, SETS>(L);
   }
 }
 
@@ -619,8 +620,9 @@ extern "C" cudaError_t CG_CAT(cg_field_gauss_, CG_N)(const cg_field_launch *L)
   /* the moments' pass, which keeps the plan's rows, takes the potential along
    * up to 512^3, where a launch's fill and drain cost more than the tuned row
    * count gives: both 10.6 -> 7.6 us at 64^3, 60 -> 54 at 256^3, 330 -> 321 at
-   * 512^3, but 2.76 -> 2.79 ms at 1024^3 */
-  constexpr int nf = N <= CG_FIELD_X_BOTH ? 2 : 1;
+   * 512^3, but 2.76 -> 2.79 ms at 1024^3.  A width forced for the potential's
+   * pass keeps that pass to itself. */
+  const int nf = N <= CG_FIELD_X_BOTH && !L->x_own ? 2 : 1;
   if ((e = xpass<true, PL::RB>(L, L->f[0], L->f[1], nullptr, nf, L->norm, L->partials)) != cudaSuccess) return e;
   if (nf == 1 && (e = xpass_v(L, L->var[CG_PASS_X], L->f[1], nullptr, nullptr, 1)) != cudaSuccess) return e;
   if (L->ev) cudaEventRecord(L->ev[2], L->stream);
@@ -633,9 +635,9 @@ extern "C" cudaError_t CG_CAT(cg_field_lpt_, CG_N)(const cg_field_launch *L)
 {
   using namespace cg;
   cudaError_t e;
-  /* nine fields share the modes of the plan's tile: the half tile that wins with
-   * three fields loses here (256^3: 303 against 248 us, three apart 312) */
-  e = L->f2[0] ? fill3<PL::TX3, 3>(L) : fill3_v(L, L->var[CG_PASS_FILL3]);
+  /* nine fields from one draw are tuned apart from three: the half tile that
+   * wins with three loses with nine (256^3: 303 against 248 us, three fills 312) */
+  e = L->f2[0] ? fill3_v<3>(L, L->var[CG_PASS_FILL9]) : fill3_v<1>(L, L->var[CG_PASS_FILL3]);
   if (e != cudaSuccess) return e;
   if (L->ev) cudaEventRecord(L->ev[0], L->stream);
   if ((e = ypass_v<1>(L, L->var[CG_PASS_Y], L->f[0], L->f[1], L->f[2], 3)) != cudaSuccess) return e;
@@ -701,7 +703,8 @@ extern "C" int CG_CAT(cg_field_tile_, CG_N)(int pass, int v)
   if (v < 0 || v > 2) return 0;
   switch (pass) {
     case CG_PASS_FILL2: return fill_ok(tile_of(PL::TX2, v)) ? tile_of(PL::TX2, v) : 0;
-    case CG_PASS_FILL3: return fill_ok(tile_of(PL::TX3, v)) ? tile_of(PL::TX3, v) : 0;
+    case CG_PASS_FILL3:
+    case CG_PASS_FILL9: return fill_ok(tile_of(PL::TX3, v)) ? tile_of(PL::TX3, v) : 0;
     case CG_PASS_Y: return y_ok(tile_of(PL::TXY, v)) ? tile_of(PL::TXY, v) : 0;
     case CG_PASS_X: return x_ok(tile_of(PL::RB, v)) ? tile_of(PL::RB, v) : 0;
   }
@@ -709,13 +712,14 @@ extern "C" int CG_CAT(cg_field_tile_, CG_N)(int pass, int v)
 }
 
 /* One pass alone with variant v, for timing: the fills write f[0..1] (two
- * fields) or f[0..2] (three); the y and x passes transform f[0..nf-1] in
+ * fields), f[0..2] (three) or these and f2[0..5] (nine); the y and x passes transform f[0..nf-1] in
  * place (inverse, no moment sums). */
 extern "C" cudaError_t CG_CAT(cg_field_pass_, CG_N)(const cg_field_launch *L, int pass, int v, int nf)
 {
   switch (pass) {
     case CG_PASS_FILL2: return fill2_v(L, v);
-    case CG_PASS_FILL3: return fill3_v(L, v);
+    case CG_PASS_FILL3: return fill3_v<1>(L, v);
+    case CG_PASS_FILL9: return fill3_v<3>(L, v);
     case CG_PASS_Y: return ypass_v<1>(L, v, L->f[0], nf > 1 ? L->f[1] : nullptr, nf > 2 ? L->f[2] : nullptr, nf);
     case CG_PASS_X: return xpass_v(L, v, L->f[0], nf > 1 ? L->f[1] : nullptr, nf > 2 ? L->f[2] : nullptr, nf);
   }

@@ -330,15 +330,18 @@ int cg_kernel_times(cg_ctx *ctx, char *names, size_t names_len, float *ms, int c
 
 /* Tile autotuner of the transform passes (no counterpart in the reference;
  * the reference plans with FFTW_ESTIMATE, src/fourier.c:84-91).  The first
- * time a grid size runs on a device, each pass -- pass 0 the fill + z of the
- * Gaussian field and potential, 1 the fill + z of the 1LPT displacements,
- * 2 the y columns, 3 the x rows -- is timed with each valid tile width (the
- * plan's, half, twice) on the context's grids and the fastest is kept for
- * the process.  Tile widths change only the block shape: results are the
- * same bits.  Environment COLORE_GB300_TUNE=0 keeps the plans' widths.
- * cg_set_field_variant forces variant v (0 plan, 1 half, 2 twice; -1 back to
- * the tuner) of one pass for this context; cg_field_plan writes the widths
- * in use and the timings as a JSON object. */
+ * time a pass of a grid size runs on a device -- pass 0 the fill + z of the
+ * Gaussian field and potential, 1 the fill + z of the LPT displacements (of
+ * 2LPT with its second derivatives), 2 the y columns, 3 the x rows -- it is
+ * timed with each valid tile width (the plan's, half, twice) on the context's
+ * grids and the fastest is kept for the process.  The x pass of the Gaussian
+ * fields keeps the plan's rows for the density, and up to 512^3 for the
+ * potential too, unless a width is forced.  Tile widths change only the block
+ * shape: results are the same bits.  Environment COLORE_GB300_TUNE=0 keeps the
+ * plans' widths.  cg_set_field_variant forces variant v (0 plan, 1 half,
+ * 2 twice; -1 back to the tuner) of one pass for this context; cg_field_plan
+ * writes the widths in use and the timings as a JSON object (pass 1 that of
+ * the context's density type). */
 int cg_set_field_variant(cg_ctx *ctx, int pass, int v);
 int cg_field_plan(cg_ctx *ctx, char *buf, size_t len);
 
