@@ -137,6 +137,7 @@ struct cg_ctx {
   /* intensity maps */
   Imap im[CG_NPOP_MAX];
   float *d_tmpmap = nullptr;
+  int *d_hits = nullptr; /* HITS_CHUNK samples on their way to the host */
   size_t tmpmap_n = 0;
   cg_imap_rec *d_recs = nullptr;         /* listed cells of one species */
   unsigned long long *d_imap_queue = nullptr; /* samples for the double pass */
@@ -230,6 +231,7 @@ static void out_wait_all(cg_ctx *c);
 static int beam_part(cg_ctx *c, int ip, bool async, long long i0, long long n);
 static int out_catalog_part(cg_ctx *c, int ip, long long i0, long long n);
 constexpr int EMIT_PARTS = 16; /* ranges of cells the emission may be cut into */
+constexpr long long HITS_CHUNK = 1 << 22; /* map pixels whose samples go to the host at a time */
 
 /* (Re)allocate a device buffer.  A captured graph holds the old addresses,
  * so any reallocation drops the graph: replaying it would touch freed
@@ -884,7 +886,7 @@ __global__ void k_div_nadd(const float2 *__restrict__ acc, int packed, float *ou
   for (long long i = 4 * m4 + t; i < m; i += stride) out[i] = div_nadd(acc[i], packed);
 }
 
-/* The samples per pixel alone. */
+/* The samples of m pixels alone. */
 __global__ void k_hits(const float2 *__restrict__ acc, int packed, int *out, long long m)
 {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x)
@@ -973,7 +975,7 @@ extern "C" void cg_destroy(cg_ctx *c)
     if (q) cudaFree(q);
   void *ptrs[] = {c->d_tabs, c->d_norm, c->d_tabs64, c->d_norm64, c->d_corner, c->d_att, c->d_xstats, c->d_zr, c->d_r2n, c->d_pk, c->d_twN, c->d_tws, c->d_dens, c->d_npot, c->d_disp[0],
                   c->d_disp[1], c->d_disp[2], c->d_part, c->d_stats, c->d_s2f, c->d_err, c->d_ncount,
-                  c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_seg, c->d_iseg, c->d_bsums, c->d_total, c->d_tmpmap, c->d_kmap,
+                  c->d_zsum, c->d_bsum, c->d_bacc, c->d_counts, c->d_seg, c->d_iseg, c->d_bsums, c->d_total, c->d_tmpmap, c->d_hits, c->d_kmap,
                   c->d_kfac, c->d_kinv, c->d_kir, c->d_ovf_cell, c->d_ovf_cnt, c->d_ovf_n,
                   c->d_recs, c->d_imap_queue,
                   c->d_imap_isw, c->d_ifac, c->d_iir, c->d_cfac, c->d_losfac};
@@ -1694,6 +1696,7 @@ static int imap_prepare(cg_ctx *c, int ip)
   }
   if (!M.ctr && (rc = dalloc(c, &M.ctr, (size_t)5))) return rc;
   if (!c->d_iseg && (rc = dalloc(c, &c->d_iseg, (size_t)CG_NA))) return rc;
+  if (!c->d_hits && (rc = dalloc(c, &c->d_hits, (size_t)HITS_CHUNK))) return rc;
   if (!c->d_imap_queue) {
     const long long qc = 1LL << 27;
     if ((rc = dalloc(c, &c->d_imap_queue, (size_t)qc))) return rc;
@@ -2660,10 +2663,11 @@ extern "C" int cg_download_imap(cg_ctx *c, int ipop, float *map, int *nadd)
 {
   if (!c || ipop < 0 || ipop >= c->cfg.n_imap) return CG_EINVAL;
   const Imap &M = c->im[ipop];
-  if (!M.acc) return fail(c, CG_ESTATE, "intensity map %d not painted", ipop);
+  if (!M.acc || !c->d_hits) return fail(c, CG_ESTATE, "intensity map %d not painted", ipop);
   const long long m = (long long)M.nr * M.npix;
   const unsigned blocks = (unsigned)std::min<long long>((m + 255) / 256, (long long)c->nsm * 16);
-  if ((map || nadd) && c->tmpmap_n < (size_t)m) {
+  if (map && c->tmpmap_n < (size_t)m) {
+    c->tmpmap_n = 0;
     if (int rc = dalloc(c, &c->d_tmpmap, (size_t)m)) return rc;
     c->tmpmap_n = m;
   }
@@ -2674,11 +2678,15 @@ extern "C" int cg_download_imap(cg_ctx *c, int ipop, float *map, int *nadd)
     c->launches++;
     CUDA_TRY(c, cudaMemcpyAsync(map, c->d_tmpmap, m * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   }
-  if (nadd) { /* through the same buffer, after the map's copy on the stream */
-    k_hits<<<blocks, 256, 0, c->stream>>>(M.acc, M.packed, reinterpret_cast<int *>(c->d_tmpmap), m);
+  /* the samples by pieces through a buffer that the painting has allocated, so
+   * that nothing is allocated here and a captured sequence keeps its graph */
+  for (long long i = 0; nadd && i < m; i += HITS_CHUNK) {
+    const long long k = std::min(m - i, HITS_CHUNK);
+    k_hits<<<(unsigned)std::min<long long>((k + 255) / 256, (long long)c->nsm * 16), 256, 0, c->stream>>>(
+        M.acc + i, M.packed, c->d_hits, k);
     CUDA_TRY(c, cudaGetLastError());
     c->launches++;
-    CUDA_TRY(c, cudaMemcpyAsync(nadd, c->d_tmpmap, m * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(nadd + i, c->d_hits, k * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   }
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return check_device_errors(c);
