@@ -888,24 +888,43 @@ CG_HD float cg_seg_pos(float r2, float idr, float *r)
   return CG_MUL(*r, idr);
 }
 
-/* First tier of a cell's count: 0 or the count when the segment tables prove
- * it, -1 when they leave it open (cg_count_cell then decides). */
-CG_HD int cg_count_seg(const cg_pois_seg *segs, const cg_pois_args *a, float r2, float d, float u)
+/* The first tier's verdicts on a cell, as bits: it may hold a source, and its
+ * double lambda is certainly below 10 (inversion) or above (PTRS).  A cell that
+ * may hold a source and is neither is left open. */
+#define CG_TIER_MAY 1
+#define CG_TIER_INV 2
+#define CG_TIER_PTRS 4
+
+/* Radii below lo lie certainly inside the tables and the sources' limit, above
+ * hi certainly beyond the limit (both by more than r's 8 2^-24). */
+CG_HD void cg_tier_limits(const cg_pois_args *a, float *lo, float *hi)
 {
-  float r;
-  if (!(r2 > 0.0f)) return -1;
-  const float s = cg_seg_pos(r2, a->idr, &r);
-  if (r > CG_MUL(a->rlim, 1.000001f)) return 0;
-  if (!(r < CG_MUL(cg_min_nn(a->rlim, a->r_last), 0.999999f))) return -1;
-  const int i = (int)s;
-  float e;
-  int pos;
-  const float l = cg_lambda_seg(&segs[i], CG_SUB(s, (float)i), d, a->bias_model, &e, &pos);
-  /* u < 1 - lambda <= exp(-lambda): no source, whatever the sign of n(r) */
-  const float hi = CG_ADD(cg_max_nn(l, 0.0f), e);
-  if (u < CG_SUB(CG_SUB(1.0f, hi), 2.0f * CG_E24)) return 0;
-  if (!pos || !(hi < 9.99f)) return -1;
-  return cg_poisson_inv_checked(l, e, u);
+  *lo = CG_MUL(cg_min_nn(a->rlim, a->r_last), 0.999999f);
+  *hi = CG_MUL(a->rlim, 1.000001f);
+}
+
+/* A radius r (r2 its square) that lies in a table segment and within the limit;
+ * one that is neither beyond hi nor such is left open. */
+CG_HD int cg_tier_inside(float r2, float r, float lo) { return r2 > 0.0f && r < lo; }
+
+/* By lambda (cg_lambda_seg).  A uniform is at most 1 - 2^-24, so lambda below
+ * 2^-25 draws nothing. */
+CG_HD int cg_tier_lambda(float lam, float elam, int pos)
+{
+  const float hi = CG_ADD(cg_max_nn(lam, 0.0f), elam);
+  int t = 0;
+  if (!(hi < 0.5f * CG_E24)) t |= CG_TIER_MAY;
+  if (pos && hi < 9.99f) t |= CG_TIER_INV;
+  else if (pos && CG_SUB(lam, elam) > 10.01f) t |= CG_TIER_PTRS;
+  return t;
+}
+
+/* By the uniform: u < 1 - lambda <= exp(-lambda) leaves no source, whatever the
+ * sign of n(r). */
+CG_HD int cg_tier_uniform(float lam, float elam, float u)
+{
+  const float hi = CG_ADD(cg_max_nn(lam, 0.0f), elam);
+  return u < CG_SUB(CG_SUB(1.0f, hi), 2.0f * CG_E24);
 }
 
 /* The count of one cell given its Poisson word w: single precision when its

@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(CWN * 32, 12) k_pois_count(const float *__rest
   const unsigned int below = (1u << lane) - 1u;
   CountWarp &S = sw[wid];
   const int N = p.box.N;
-  const float rhi = CG_MUL(p.pa.rlim, 1.000001f), rlo = CG_MUL(cg_min_nn(p.pa.rlim, p.pa.r_last), 0.999999f);
+  float rlo, rhi;
+  cg_tier_limits(&p.pa, &rlo, &rhi);
   long long tot = 0;
   unsigned int nfb = 0;
   const long long wbase = ((long long)blockIdx.x * CWN + wid) * steps * CW;
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(CWN * 32, 12) k_pois_count(const float *__rest
         const float s = cg_seg_pos(r2, p.pa.idr, &r);
         lam[q] = elam[q] = 0.0f;
         if (r > rhi) continue;
-        if (!(r2 > 0.0f && r < rlo)) {
+        if (!cg_tier_inside(r2, r, rlo)) {
           open |= 1u << q;
           continue;
         }
@@ -184,11 +185,10 @@ __global__ void __launch_bounds__(CWN * 32, 12) k_pois_count(const float *__rest
         const cg_pois_seg g = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, 0.0f};
         int pos;
         lam[q] = cg_lambda_seg(&g, CG_SUB(s, (float)i), d4[q], p.pa.bias_model, &elam[q], &pos);
-        const float hi = CG_ADD(cg_max_nn(lam[q], 0.0f), elam[q]);
-        /* a uniform is at most 1 - 2^-24: lambda below 2^-25 draws nothing */
-        if (!(hi < 0.5f * CG_E24)) may |= 1u << q;
-        if (pos && hi < 9.99f) inv |= 1u << q;
-        else if (pos && CG_SUB(lam[q], elam[q]) > 10.01f) ptr |= 1u << q;
+        const int t = cg_tier_lambda(lam[q], elam[q], pos);
+        if (t & CG_TIER_MAY) may |= 1u << q;
+        if (t & CG_TIER_INV) inv |= 1u << q;
+        if (t & CG_TIER_PTRS) ptr |= 1u << q;
       }
     }
     unsigned int u24[4] = {0u, 0u, 0u, 0u};
@@ -198,9 +198,7 @@ __global__ void __launch_bounds__(CWN * 32, 12) k_pois_count(const float *__rest
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         u24[q] = w.v[q] >> 8;
-        /* u < 1 - lambda <= exp(-lambda): no source, whatever the sign of n(r) */
-        const float hi = CG_ADD(cg_max_nn(lam[q], 0.0f), elam[q]);
-        if (CG_MUL((float)u24[q], CG_E24) < CG_SUB(CG_SUB(1.0f, hi), 2.0f * CG_E24)) may &= ~(1u << q);
+        if (cg_tier_uniform(lam[q], elam[q], CG_MUL((float)u24[q], CG_E24))) may &= ~(1u << q);
       }
     }
     open |= may & ~(inv | ptr);

@@ -153,10 +153,11 @@ void or_ptrs_checked(long n, const float *lam, const float *elam, const double *
   }
 }
 
-/* The counts' first tier (cg_lambda_seg, cg_count_seg) on n cells of a table
+/* The counts' first tier (cg_lambda_seg, cg_tier_*) on n cells of a table
  * of NA nodes at r_i = i / idr: lam[i] within elam[i] of lam64[i]
- * (cgx_lambda), got[i] the tier's count or -1, ref[i] the double count for
- * lambda < 10 with the uniform bits[i] 2^-24. */
+ * (cgx_lambda), got[i] the tier's count, -1 when it leaves the cell open or -2
+ * when it leaves it to PTRS, ref[i] the double count for lambda < 10 with the
+ * uniform bits[i] 2^-24. */
 void or_count_seg(const double *r, const double *nz, const double *bz, const double *norm, double idr, double dx,
                   const double *pos, double cell_vol, double rlim, int model, long n, const int *cell, const float *d,
                   const uint32_t *bits, float *lam, float *elam, double *lam64, int *got, int *ref)
@@ -179,6 +180,8 @@ void or_count_seg(const double *r, const double *nz, const double *bz, const dou
   a.r_last = (float)a.x.r_last;
   a.rlim = (float)rlim;
   a.bias_model = model;
+  float lo, hi;
+  cg_tier_limits(&a, &lo, &hi);
   cg_pois_seg *seg = malloc((CG_NA - 1) * sizeof(cg_pois_seg));
   for (int i = 0; i < CG_NA - 1; i++) seg[i] = cg_pois_seg_make(&a.x, CG_NA, i);
   for (long i = 0; i < n; i++) {
@@ -193,7 +196,14 @@ void or_count_seg(const double *r, const double *nz, const double *bz, const dou
     j = r2 > 0.0f && j < CG_NA - 1 ? j : 0;
     lam[i] = cg_lambda_seg(&seg[j], CG_SUB(s, (float)j), d[i], model, &elam[i], &pos1);
     lam64[i] = cgx_lambda(&a.x, c[0], c[1], c[2], d[i]);
-    got[i] = cg_count_seg(seg, &a, r2, d[i], u);
+    got[i] = rr > hi ? 0 : -1;
+    if (!(rr > hi) && cg_tier_inside(r2, rr, lo)) {
+      int t = cg_tier_lambda(lam[i], elam[i], pos1);
+      if (cg_tier_uniform(lam[i], elam[i], u)) t &= ~CG_TIER_MAY;
+      if (t & CG_TIER_PTRS) got[i] = -2;
+      else if (!(t & CG_TIER_MAY)) got[i] = 0;
+      else if (t & CG_TIER_INV) got[i] = cg_poisson_inv_checked(lam[i], elam[i], u);
+    }
     ref[i] = lam64[i] < 10 ? cgx_poisson(lam64[i], (double)u, i, 1u, 2u) : -1;
   }
   free(seg);

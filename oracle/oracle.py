@@ -604,8 +604,8 @@ def ptrs_checked(lam, elam, lam64, cid, k0, k1):
 
 def count_seg(r, nz, bz, norm, idr, dx, pos, cell_vol, rlim, model, cell, d, bits):
     """The counts' first tier on cells (n x 3): (lam, elam, lam64, got, ref),
-    lam within elam of the double lam64, got the count or -1 where open, ref
-    the double count (-1 for lambda >= 10)."""
+    lam within elam of the double lam64, got the count, -1 where open or -2 where
+    left to PTRS, ref the double count (-1 for lambda >= 10)."""
     f8 = [np.ascontiguousarray(a, np.float64) for a in (r, nz, bz, norm, pos)]
     cell = np.ascontiguousarray(cell, np.int32)
     d = np.ascontiguousarray(d, np.float32)
