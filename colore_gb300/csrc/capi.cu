@@ -1494,7 +1494,7 @@ static int emit_part(cg_ctx *c, int ip, long long b0, long long b1)
   cg_srcs_params p;
   srcs_params(c, ip, p);
   ProfScope ps(c, "srcs_emit");
-  CUDA_TRY(c, cg_srcs_emit(c->stream, c->d_npot, &p, b0, b1));
+  CUDA_TRY(c, cg_srcs_emit(c->stream, c->d_npot, &p, b0, b1, c->nsm));
   c->launches++;
   return CG_OK;
 }

@@ -467,17 +467,18 @@ __device__ __noinline__ unsigned int pixels_double(const cg_srcs_params &p, floa
 constexpr int SRC_F = 9; /* floats per source record (Src) */
 
 /* Sources of 2048 cells (block b0 + blockIdx.x of them), the share blockIdx.y of
- * gridDim.y: every share scans the counts again, a few per cent of the work,
- * so that small grids and dense populations spread over the chip (c1 at
- * 128^3: 1024 blocks of up to 20000 sources kept the SMs busy 59 % of the
- * time).  The share's sources are spread evenly over the threads.  Records
- * of 36 bytes are staged per warp and written as consecutive words: written
- * field by field they cost L2 ten sectors per source for 56 bytes. */
+ * gridDim.y, a power of two: every share scans the counts again, a few per cent
+ * of the work, so that small grids and dense populations spread over the chip
+ * (c1 at 128^3: 1024 blocks of up to 20000 sources kept the SMs busy 59 % of
+ * the time).  The share's sources are spread evenly over the threads.  STAGED:
+ * records of 36 bytes are staged per warp and written as consecutive words;
+ * written field by field they cost L2 ten sectors per source for 56 bytes. */
+template <bool STAGED>
 __global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, cg_srcs_params p, long long b0)
 {
   __shared__ int coff[CPB]; /* exclusive source offset of each cell in the block */
   __shared__ int ws[SB / 32];
-  __shared__ float stage[SB / 32][32 * SRC_F];
+  __shared__ float stage[STAGED ? SB / 32 : 1][STAGED ? 32 * SRC_F : 1];
   const int N = p.box.N;
   const long long blk = b0 + blockIdx.x, cb = blk * CPB;
   const long long c0 = cb + (long long)threadIdx.x * CPT;
@@ -527,13 +528,14 @@ __global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, c
   cell_of(cb, p.box, bx, by, bz);
   const unsigned mdiv = ((1u << 24) + (unsigned)N - 1u) / (unsigned)N;
   unsigned int nfb = 0; /* pixels decided in double */
-  const int k1 = (int)((long long)T * (blockIdx.y + 1) / gridDim.y);
-  for (int kb = (int)((long long)T * blockIdx.y / gridDim.y) + wid * 32; kb < k1; kb += SB) {
+  const int lg = 31 - __clz((int)gridDim.y);
+  const int k1 = (int)(((long long)T * (blockIdx.y + 1)) >> lg);
+  for (int kb = (int)(((long long)T * blockIdx.y) >> lg) + wid * 32; kb < k1; kb += SB) {
     const int k = kb + lane;
     const long long id = base + k;
     const bool ok = k < k1 && id < p.capacity;
     if (k < k1 && !ok) atomicOr(p.err, ERR_CATALOG_OVERFLOW);
-    float *q = &stage[wid][lane * SRC_F];
+    float *q = STAGED ? &stage[wid][lane * SRC_F] : p.src + (size_t)id * SRC_F;
     if (ok) {
       /* the cell holding source k: the last cell whose offset is <= k (cells
        * without sources share their successor's offset) */
@@ -591,6 +593,7 @@ __global__ void __launch_bounds__(SB, 6) k_emit(const float *__restrict__ phi, c
       q[7] = 0.0f;
       q[8] = 0.0f;
     }
+    if (!STAGED) continue;
     __syncwarp();
     const int nw = __popc(__ballot_sync(0xffffffffu, ok)) * SRC_F;
     float *dst = p.src + (size_t)(base + kb) * SRC_F;
@@ -856,18 +859,22 @@ cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_param
   return cudaGetLastError();
 }
 
-cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long b0, long long b1)
+cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long b0, long long b1,
+                         int nsm)
 {
   if (b1 <= b0) return cudaSuccess;
-  /* shares per block: until there are eight blocks for each of the 152 x 8
-   * that an SM generation holds, while a share keeps a source per thread (the
-   * capacity is the total with an eighth of slack).  c1 at 128^3 with 1 and
-   * 16 shares: 244 and 169 us; 192^3 with 240 sources per block: 74 and 127 us
-   * with 1 and 4. */
+  /* shares per block: until there are 64 blocks per SM, ten times those it
+   * holds, while a share keeps a source per thread (the capacity is the total
+   * with an eighth of slack).  c1 at 128^3 with 1 and 16 shares: 244 and
+   * 169 us; 192^3 with 240 sources per block: 74 and 127 us with 1 and 4. */
   const long long nb = b1 - b0, all = cg_srcs_nblocks(p->box.N);
   int sh = 1;
-  while (sh < 16 && nb * sh < 9728 && p->capacity >= all * sh * 2 * SB) sh *= 2;
-  k_emit<<<dim3((unsigned)nb, (unsigned)sh), SB, 0, s>>>(phi, *p, b0);
+  while (sh < 16 && nb * sh < 64ll * nsm && p->capacity >= all * sh * 2 * SB) sh *= 2;
+  /* records written directly and staged, by sources per block of cells: 13
+   * (512^3) 187 and 264 us, 79 (1024^3) 2.62 and 2.85 ms, 118 (1024^3) 3.29 and
+   * 3.34 ms, 151 (256^3) 74 and 71 us, 197 (1024^3) 4.60 and 4.40 ms */
+  const auto k = p->capacity < 144 * all ? k_emit<false> : k_emit<true>;
+  k<<<dim3((unsigned)nb, (unsigned)sh), SB, 0, s>>>(phi, *p, b0);
   return cudaGetLastError();
 }
 

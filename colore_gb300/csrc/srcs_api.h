@@ -86,7 +86,8 @@ long long cg_srcs_scan_room(long long nb);
 cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_params *p, long long *total, long long *host,
                           long long bpc);
 /* The sources of blocks [b0, b1) of cells (cg_srcs_nblocks in all). */
-cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long b0, long long b1);
+cudaError_t cg_srcs_emit(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long b0, long long b1,
+                         int nsm);
 /* nsrc sources, or with nsrc_dev non-NULL min(*nsrc_dev, nsrc) read on the
  * device (a graph-captured sequence, whose totals stay on the device). */
 cudaError_t cg_srcs_beam_rsd(cudaStream_t s, const float *phi, const cg_srcs_params *p, long long nsrc,
