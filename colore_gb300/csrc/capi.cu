@@ -1938,7 +1938,7 @@ static int kappa_run(cg_ctx *c)
   p.map = c->d_kmap;
   {
     ProfScope ps(c, "kappa");
-    CUDA_TRY(c, cg_kappa_integrate(c->stream, c->d_npot, &p));
+    CUDA_TRY(c, cg_kappa_integrate(c->stream, c->d_npot, &p, c->nsm));
   }
   c->launches++;
   return CG_OK;

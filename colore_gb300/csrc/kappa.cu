@@ -258,11 +258,11 @@ static cudaError_t kappa_launch(cudaStream_t s, const float *phi, const cg_kappa
   return cudaGetLastError();
 }
 
-cudaError_t cg_kappa_integrate(cudaStream_t s, const float *phi, const cg_kappa_params *p)
+cudaError_t cg_kappa_integrate(cudaStream_t s, const float *phi, const cg_kappa_params *p, int nsm)
 {
   /* blocks of 256 neighbouring pixels share rows in L1 (nside 512 on 1024^3:
-   * 12.9 ms, with 64 13.8 ms); maps of less than two waves of them, whose
-   * rays are bound by latency, take 64 for the balance (nside 128 on 256^3:
-   * 271 and 246 us) */
-  return p->npix <= 2ll * 152 * 1024 ? kappa_launch<64>(s, phi, p) : kappa_launch<256>(s, phi, p);
+   * 12.9 ms, with 64 13.8 ms); maps of less than two waves of them (1024 rays
+   * an SM), whose rays are bound by latency, take 64 for the balance (nside 128
+   * on 256^3: 271 and 246 us) */
+  return p->npix <= 2ll * nsm * 1024 ? kappa_launch<64>(s, phi, p) : kappa_launch<256>(s, phi, p);
 }

@@ -21,7 +21,7 @@ struct cg_kappa_params {
   float *map;             /* nplanes * npix, RING order */
 };
 
-cudaError_t cg_kappa_integrate(cudaStream_t s, const float *phi, const cg_kappa_params *p);
+cudaError_t cg_kappa_integrate(cudaStream_t s, const float *phi, const cg_kappa_params *p, int nsm);
 /* Custom map (cstm_get_beam_properties, cstm.c:68-145): per pixel,
  * dr * sum over ir_min..ir_max of kz (bias_model(d, bz) norm - 1), with d the
  * CIC-interpolated density at the step (interpolate_from_grid, beaming.c:183-265). */

@@ -841,10 +841,11 @@ cudaError_t cg_srcs_count(cudaStream_t s, const float *grid, const cg_srcs_param
 {
   const long long nb = cg_srcs_nblocks(p->box.N);
   k_pois_tab<<<(CG_NA + 31) / 32, 32, 0, s>>>(*p, nb);
-  /* four steps per warp where the grid has many times the 7296 warps that 152
-   * SMs hold (512^3, two populations: 1.44 ms against 1.50 with two); one on
-   * small grids, whose dense cells near the observer would leave the last
-   * warps alone (128^3) */
+  /* steps per warp: four where the grid has many times the warps that the chip
+   * holds (384^3 308 us, with two and one 317 and 342; 1024^3 5.2, 5.5 and
+   * 6.1 ms), one on small grids, whose dense cells near the observer would leave
+   * the last warps alone (128^3 77 us, with two and four 88 and 119; 256^3 with
+   * 1000 sources per deg^2 347, 361 and 369) */
   const int steps = p->box.N > 256 ? 4 : 1;
   k_pois_count<<<(unsigned)(nb * CPB / (CWN * CW * steps)), CWN * 32, 0, s>>>(grid, *p, steps);
   if (nb <= SCAN_ONE) {
