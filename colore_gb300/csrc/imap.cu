@@ -78,14 +78,14 @@ constexpr unsigned F_DOUBLE = 16u; /* flags: mode (2 bits), delta + 1 (2 bits), 
 /* Per-block copies of the species' shell tables. */
 struct Sh {
   float *b; /* with two sentinels on either side */
-  float *dxs, *invns;
+  float *dxs;
   int *shell_of, *nsub;
   unsigned long long *chunk_off;
 };
 
 __host__ __device__ __forceinline__ size_t shell_smem(int nr, int nbk, bool chunks)
 {
-  size_t n = (size_t)(2 * nr + 4) * 4 + (size_t)(2 * nr + 1) * 4 + 3 * (size_t)(nr + 2) * 4;
+  size_t n = (size_t)(2 * nr + 4) * 4 + (size_t)(2 * nr + 1) * 4 + 2 * (size_t)(nr + 2) * 4;
   n = (n + 7) & ~(size_t)7;
   if (chunks) n += (size_t)(nbk + 1) * 8;
   return n;
@@ -100,7 +100,6 @@ __device__ __forceinline__ Sh shells_at(const cg_imap_params &p, unsigned char *
   s.shell_of = reinterpret_cast<int *>(s.b + 2 * nr + 2);
   s.nsub = s.shell_of + 2 * nr + 1;
   s.dxs = reinterpret_cast<float *>(s.nsub + nr + 2);
-  s.invns = s.dxs + nr + 2;
   s.chunk_off = reinterpret_cast<unsigned long long *>(raw + shell_smem(nr, p.nbk, false));
   return s;
 }
@@ -122,7 +121,6 @@ __device__ __forceinline__ Sh load_shells(const cg_imap_params &p, unsigned char
   for (int i = threadIdx.x; i < nr + 2; i += blockDim.x) {
     s.nsub[i] = p.a.nsub[i];
     s.dxs[i] = p.a.dxs[i];
-    s.invns[i] = 1.0f / (float)p.a.nsub[i];
   }
   if (chunks)
     for (int i = threadIdx.x; i <= p.nbk; i += blockDim.x) s.chunk_off[i] = p.chunk_off[i];
@@ -216,16 +214,15 @@ __device__ __forceinline__ void add_to(const cg_imap_params &p, long long k, flo
   }
 }
 
-/* The lanes hold consecutive samples: each run of equal (tag, key) is added
+/* The lanes hold consecutive samples of one cell: each run of one key is added
  * to the maps once, by its first lane, with its length (sum += temp * run,
- * count += run).  tag separates cells, whose brightness differs. */
+ * count += run). */
 template <typename K>
-__device__ __forceinline__ void add_runs(K key, int tag, float temp, int lane, const cg_imap_params &p)
+__device__ __forceinline__ void add_runs(K key, float temp, int lane, const cg_imap_params &p)
 {
   const K pk = __shfl_up_sync(FULL, key, 1);
-  const int pt = __shfl_up_sync(FULL, tag, 1);
   const bool valid = key != empty_key<K>();
-  const bool head = valid && (lane == 0 || pk != key || pt != tag);
+  const bool head = valid && (lane == 0 || pk != key);
   const unsigned bnd = __ballot_sync(FULL, head || !valid);
   if (head) {
     const unsigned above = lane == 31 ? 0u : bnd & (FULL << (lane + 1));
@@ -236,8 +233,9 @@ __device__ __forceinline__ void add_runs(K key, int tag, float temp, int lane, c
 }
 
 /* Sub-cell (sx, sy, sz) of sample q < ns^3, x fastest. */
-__device__ __forceinline__ void sub_of(int q, int ns, float inv_ns, int *sx, int *sy, int *sz)
+__device__ __forceinline__ void sub_of(int q, int ns, int *sx, int *sy, int *sz)
 {
+  const float inv_ns = 1.0f / (float)ns;
   int line, z;
   if (ns <= 128) {
     /* (q + 1/2)/ns is at least 1/(2 ns) from an integer and the float
@@ -307,12 +305,12 @@ __device__ __forceinline__ cg_imap_cell unpack(const cg_imap_rec &r, int j, int 
  * when needed, on the spot. */
 template <typename K>
 __device__ __noinline__ K sample_key_inline(const cg_imap_params &p, int ix, int iy, int iz,
-                                            const cg_imap_cell &c, int dbl, int ns, int q, float inv_ns)
+                                            const cg_imap_cell &c, int dbl, int ns, int q)
 {
   const cg_imap_args &A = p.a;
   int sx, sy, sz, s = -1;
   long long pix = 0;
-  sub_of(q, ns, inv_ns, &sx, &sy, &sz);
+  sub_of(q, ns, &sx, &sy, &sz);
   if (dbl || p.force_double || !cg_imap_sample_checked(&A, ix, iy, iz, &c, ns, sx, sy, sz, &s, &pix)) {
     float v[3];
     grad_phi(p.phi, ix, iy, iz, p.box.N, v);
@@ -386,12 +384,11 @@ __device__ __forceinline__ void paint_over(const cg_imap_params &p, unsigned m, 
     int ix, iy, iz, dbl;
     const cg_imap_cell c = unpack(r, j, &ix, &iy, &iz, &dbl);
     const int ns = p.a.nsub[j + 1], n3 = ns * ns * ns;
-    const float inv = 1.0f / (float)ns;
     for (int q0 = 0; q0 < n3; q0 += 32) {
       const int q = q0 + lane;
       K key = empty_key<K>();
-      if (q < n3) key = sample_key_inline<K>(p, ix, iy, iz, c, dbl, ns, q, inv);
-      add_runs(key, 0, c.temp, lane, p);
+      if (q < n3) key = sample_key_inline<K>(p, ix, iy, iz, c, dbl, ns, q);
+      add_runs(key, c.temp, lane, p);
     }
     if (lane == 0) atomicAdd(&p.ctr[3], (unsigned long long)n3);
   }
@@ -939,7 +936,7 @@ __device__ __forceinline__ void double_batch(const float *__restrict__ phi, cons
   if (!valid) return;
   const int ns = sh.nsub[lo];
   int s = -1, sx, sy, sz;
-  sub_of(q, ns, sh.invns[lo], &sx, &sy, &sz);
+  sub_of(q, ns, &sx, &sy, &sz);
   long long pix = 0;
   cgx_imap_sample(&A, ix, iy, iz, ns, drr, sx, sy, sz, &s, &pix);
   if (s >= 0 && s < p.nr) add_to(p, (long long)s * p.npix + pix, temp, 1.0f);
@@ -989,7 +986,7 @@ __global__ void __launch_bounds__(DB_WARPS * 32) k_imap_double(const float *__re
         const int ns = sh.nsub[lo];
         int s = -1, sx, sy, sz;
         long long pix = 0;
-        sub_of(q, ns, sh.invns[lo], &sx, &sy, &sz);
+        sub_of(q, ns, &sx, &sy, &sz);
         if (cg_imap_decide_ff(&A, &c, ix, iy, iz, sx, sy, sz, &s, &pix)) {
           need = false;
           if (s >= 0 && s < p.nr) add_to(p, (long long)s * p.npix + pix, c.temp, 1.0f);
