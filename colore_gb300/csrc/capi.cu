@@ -1687,7 +1687,7 @@ static int imap_prepare(cg_ctx *c, int ip)
     capv[2 * i + 1] = cut ? n - capv[2 * i] : n;
     /* the shell's rooms meet at their general ends */
     at[2 * i + (i & 1 ? 0 : 1)] = acc;
-    at[2 * i + (i & 1 ? 1 : 0)] = acc + n - 1;
+    at[2 * i + (i & 1 ? 1 : 0)] = acc + n;
     acc += n;
   }
   if (acc > c->list_cap) {

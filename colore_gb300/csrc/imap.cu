@@ -141,14 +141,15 @@ __device__ __forceinline__ cg_imap_args args_with(const cg_imap_params &p, const
  * end it is listed from. */
 __device__ __forceinline__ int counter_of(int j, int polar, int cls)
 {
-  return 4 * (j + 1) + (cls == CG_CELL_GENERAL ? 2 * polar : 2 * cls - 1);
+  return 4 * (j + 1) + 2 * polar + (cls != CG_CELL_GENERAL);
 }
 
 /* Slot k of counter ct: the fast equatorial and the general polar cells upwards
  * from their room's begin, the others downwards from its end. */
 __device__ __forceinline__ long long slot_of(const cg_imap_params &p, int ct, long long k)
 {
-  return p.at[ct] + (((ct ^ (ct >> 1)) & 1) ? k : -k);
+  const int down = ((ct ^ (ct >> 1)) & 1) - 1; /* 0 or -1 */
+  return p.at[ct] + (k ^ (long long)down);
 }
 
 /* Cells listed on counter ct.  None when both ends hold more than the room,
@@ -162,7 +163,7 @@ __device__ __forceinline__ long long listed(const cg_imap_params &p, int ct)
     const long long m = (long long)p.cnt[(size_t)c * CG_IMAP_CNT];
     n[k] = m < p.cap[c] ? m : p.cap[c];
   }
-  const long long room = llabs(p.at[ct | 1] - p.at[ct & ~1]) + 1;
+  const long long room = llabs(p.at[ct | 1] - p.at[ct & ~1]);
   if (n[0] + n[1] > room) {
     atomicOr(p.err, ERR_IMAP_ROOM);
     return 0;
@@ -181,7 +182,7 @@ __device__ __forceinline__ longlong2 bucket_of(const cg_imap_params &p, int b)
     return make_longlong2(p.at[4 * s + 2] - n, n + listed(p, 4 * s + 2));
   }
   const long long n = listed(p, 4 * s + 2 * cls - 1);
-  return make_longlong2(cls == CG_CELL_EQ ? p.at[4 * s + 1] : p.at[4 * s + 3] + 1 - n, n);
+  return make_longlong2(cls == CG_CELL_EQ ? p.at[4 * s + 1] : p.at[4 * s + 3] - n, n);
 }
 
 static_assert(CG_CELL_GENERAL == 0 && CG_CELL_EQ == 1 && CG_CELL_POLAR == 2, "rooms by class");

@@ -43,9 +43,9 @@ struct cg_imap_params {
   /* cells are listed per bucket (the shell of their corner, which fixes nsub,
    * and the class, which fixes the painting loop).  Shell j has two rooms
    * (cg_imap_rooms) next to each other, w = 2 (j + 1) + (polar corner): general
-   * cells on counter 2 w, the others on 2 w + 1 (CG_IMAP_CNT apart), from slot
-   * at[counter] on, one upwards and one downwards.  Either may exceed its cap:
-   * those cells are painted by the listing kernel */
+   * cells on counter 2 w, the others on 2 w + 1 (CG_IMAP_CNT apart), one upwards
+   * from the room's begin and one downwards from its end, at[counter].  Either
+   * may exceed its cap: those cells are painted by the listing kernel */
   cg_imap_rec *recs;
   const long long *at, *cap;
   unsigned long long *cnt;
