@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(256) k_bins_finish(const unsigned long long *_
  * the grid.  Masses are fixed point (DEPOSIT_ONE per particle, integer atomics;
  * the grid holds the int32 bits until the density pass turns them into
  * rho - 1), so the result does not depend on the order of the atomic additions.
- * Bound by instruction issue (about 190 slots a particle; the box's flush was a
- * third of 370 when it found every cell's place by divisions): 12.5 -> 7.9 ms
+ * Bound by instruction issue (238 issue slots a particle at 512^3; the box's
+ * flush found every cell's place by divisions before): 12.5 -> 7.9 ms
  * at 1024^3 with the grid's clearing, 207 -> 143 us at 256^3.  Tiles of 8 x 8,
  * 8 x 16, 16 x 8 and 4 x 32 in y and z took 9.8, 9.1, 10.3 and 10.9 against
  * 8.4 ms of 4 x 16 before the flush went by columns; 10 and 12 blocks per SM

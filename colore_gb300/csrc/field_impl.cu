@@ -146,9 +146,10 @@ __device__ __forceinline__ float2 k_draw(const FillParams &p, float s2, int kx, 
  * pair (kz, N - kz) from one amplitude (kz = 0 and N/2 pair up, each with its
  * own).  Thread t of the PF that share a column takes kz = t, t + PF, ...
  * below N/2.  Rolled: one copy of the generator in the instruction stream
- * (inlined per element it overflowed the instruction cache).  The fills are
- * bound by instruction issue, not HBM (60 % issue-active at 290 instructions
- * per mode, 20 % of DRAM peak at 1024^3).  One amplitude for two modes, round
+ * (inlined per element it overflowed the instruction cache).  The fills wait
+ * for issue slots and for the transform's exchanges, not for HBM (20 % of DRAM
+ * peak at 1024^3; with the generation left out 5.4 of 6.5 ms, at 512^3 0.42 of
+ * 0.68).  One amplitude for two modes, round
  * keys and the P(k) table's differences formed on the host, and exchange slots
  * free of conflicts: 7.25 -> 6.58 ms for the two-field fill at 1024^3,
  * 374 -> 334 us at 384^3. */

@@ -32,10 +32,10 @@
  *                  65 against 54 ms of the stage at 1024^3).  Cells that the
  *                  segments leave open, and cells that find their room full
  *                  (painted by the warp), wait until the warp's rows are done.
- *                  487 thread-instructions a cell in range where a lookup with
- *                  a bound per table took 689: 20.6 -> 11.5 ms at 1024^3.
- *   k_imap_chunks  One block finds each bucket's records and cuts it into chunks of about CHS
- *                  samples: whole cells, or slices of one cell.
+ *                  504 thread-instructions a cell in range where a lookup with
+ *                  a bound per table took 689: 20.6 -> 10.4 ms at 1024^3.
+ *   k_imap_chunks  One block finds each bucket's records and cuts them into
+ *                  chunks of about CHS samples: whole cells, or slices of one.
  *   k_imap_paint   Warps take chunks in bucket order, so the maps' working
  *                  set at any time is a few shells (50 MB per shell at nside
  *                  512) and the atomics stay in L2.  Each lane walks one unit
@@ -43,11 +43,11 @@
  *                  the maps with one two-float reduction.  Cells within one
  *                  octant, one of the two pixel regions and one shell or edge
  *                  -- all but the layers on the octants' planes, the cones
- *                  |cos theta| = 2/3 and the nearest cells -- have these
- *                  decisions taken once per cell and walk along the line of
- *                  sight, where the pixel changes least.  Samples whose margins
- *                  fail are staged per warp in shared memory and queued in
- *                  batches.  Bound by instruction issue (87 % of the slots): 92
+ *                  |cos theta| = 2/3, the nearest cells and those that span
+ *                  several thin shells -- have these decisions taken once per
+ *                  cell and walk along the line of sight, where the pixel
+ *                  changes least.  Samples whose margins fail are staged per
+ *                  warp in shared memory and queued in batches.  Bound by instruction issue (87 % of the slots): 91
  *                  thread-instructions a sample where deciding everything per
  *                  sample took 177, 79 -> 36 ms for the 1.3e10 samples at
  *                  1024^3; scalar atomics instead of the two-float reduction

@@ -131,8 +131,8 @@ struct alignas(16) CountWarp {
  * and settles u < 1 - lambda on the spot.  The cells left are compacted per
  * warp in shared memory and inverted (lambda < 10) or sampled by PTRS 32 at a
  * time, so that the exponential and the search run in full warps (inverted in
- * place, every warp paid for both in every step: 390 issue slots per cell at
- * 512^3, now 165).  Cells that the tier's bounds leave open follow in a last
+ * place, every warp paid for both in every step: 261 thread-instructions per
+ * cell at 512^3, now 148).  Cells that the tier's bounds leave open follow in a last
  * list (count_open); every count is the reference's double decision.  Each
  * warp adds its total to the entry of its 2048 cells.  Twelve blocks per SM
  * (40 registers).  1024^3, 1000 sources per deg^2: 11.0 -> 5.3 ms; 512^3, two

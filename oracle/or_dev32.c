@@ -208,8 +208,9 @@ static void pois_args(PoisArgs *P, const cg_config *cfg, const S32 *s, int ipop,
   x->bias_model = cfg->bias_model;
 }
 
-/* Counts of population ipop as the GPU computes them (cg_count_cell: float
- * margins, double decisions where they do not hold); *fallbacks counts the
+/* Counts of population ipop in the GPU's float arithmetic (cg_count_cell: the
+ * margins of its general tier, double decisions where they do not hold; the
+ * kernel settles most cells by the looser bounds of cg_lambda_seg before it); *fallbacks counts the
  * cells decided in double. */
 int or_counts32(const cg_config *cfg, int ipop, const float *dens, const float *norm32, const double *norm64,
                 int *counts, long long *total, long long *fallbacks)
@@ -241,7 +242,7 @@ int or_counts32(const cg_config *cfg, int ipop, const float *dens, const float *
   return 0;
 }
 
-/* The catalogue as the GPU writes it: positions in double rounded to float
+/* The catalogue bit for bit as the GPU's: positions in double rounded to float
  * (the reference's), the base and count-map pixels by cg_src_pixels, the
  * velocity, RA, Dec and redshift in single precision. */
 int or_emit32(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
@@ -507,7 +508,7 @@ double or_imap_pixel_max(const cg_config *cfg, int ipop)
   return n;
 }
 
-/* The intensity map of species ipop as the GPU paints it: cells and samples
+/* The intensity map of species ipop by the GPU's general tier: cells and samples
  * decided in single precision where the margins hold, then in float-float,
  * and in double otherwise (cg_exact.h); brightness summed in cell order in
  * float.  stats:

@@ -78,8 +78,8 @@ int or_run_mock64(const cg_config *cfg, int nthreads_hint, long long *nsrc_total
 int or_density32(const cg_config *cfg, float *dens, float sigma2f, int mode);
 int or_bins32(const cg_config *cfg, const float *dens, int nz, double idz, unsigned long long *narr, double *zarr,
               double *bsum);
-/* Source counts and catalogue as the GPU computes them: float margins with
- * double decisions where they do not hold (cg_exact.h).  norm32 / norm64:
+/* Source counts and catalogue in the GPU's float arithmetic: the margins of
+ * its general tier with double decisions where they do not hold (cg_exact.h).  norm32 / norm64:
  * the normalisation table (CG_NA values, then the two edges) in float and
  * double; *fallbacks: cells (counts) or pixels (emit) decided in double. */
 int or_counts32(const cg_config *cfg, int ipop, const float *dens, const float *norm32, const double *norm64,
@@ -88,7 +88,7 @@ int or_emit32(const cg_config *cfg, int ipop, const float *dens, const float *np
               const double *norm64, long long cap, float *pos4, int *ipix, float *src9, int *cmap, long long *nsrc,
               long long *fallbacks);
 int or_beam_rsd32(const cg_config *cfg, const float *npot, long long n, const float *pos4, float *src9);
-/* The intensity map as the GPU paints it (float margins, double where they
+/* The intensity map by the GPU's general tier (float margins, double where they
  * do not hold); stats: cells and samples decided in double, samples drawn. */
 int or_imap32(const cg_config *cfg, int ipop, const float *dens, const float *npot, const float *norm32,
               const double *norm64, float *data, int *nadd, long long *stats);

@@ -250,7 +250,7 @@ def _norm_pair(tab32, e32, tab64, e64):
 
 
 def counts32(cfg, ipop, dens, tab32, e32, tab64, e64):
-    """Counts as the GPU computes them (float margins, double where they do
+    """Counts by the GPU's general tier (float margins, double where they do
     not hold): (counts [N][N][N], total, cells decided in double)."""
     n = cfg.n_grid
     cnt = np.empty((n, n, n), np.int32)
@@ -317,7 +317,7 @@ def beam_rsd32(cfg, npot, pos, src):
 
 
 def imap32(cfg, ipop, dens, npot, tab32, e32, tab64, e64):
-    """The intensity map as the GPU paints it: (summed brightness, hit
+    """The intensity map by the GPU's general tier: (summed brightness, hit
     counts, stats) with stats = (cells and samples decided in double,
     samples drawn)."""
     ns, nr = cfg.nside_imap[ipop], cfg.imap_nr[ipop]
