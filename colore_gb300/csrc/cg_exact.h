@@ -888,7 +888,7 @@ CG_HD float cg_seg_pos(float r2, float idr, float *r)
   return CG_MUL(*r, idr);
 }
 
-/* The first tier's verdicts on a cell, as bits: it may hold a source, and its
+/* What the first tier says of a cell, as bits: it may hold a source, and its
  * double lambda is certainly below 10 (inversion) or above (PTRS).  A cell that
  * may hold a source and is neither is left open. */
 #define CG_TIER_MAY 1

@@ -1,4 +1,4 @@
-"""The first tier's verdicts that the counting kernel takes, over densities from
+"""The first tier's decisions that the counting kernel takes, over densities from
 nothing to hundreds of sources a cell: a cell without a source has none in
 double, one for inversion has the double count where the margins keep it, one
 left to PTRS has a double lambda of 10 or more, and few cells stay open."""
@@ -10,7 +10,7 @@ NA = 5001
 
 @pytest.mark.parametrize("model", [1, 2, 3])
 @pytest.mark.parametrize("scale", [1e-12, 1e-3, 0.1, 3.0])
-def test_verdicts(built, model, scale):
+def test_decisions(built, model, scale):
     import oracle as orc
     g = np.random.default_rng(int(1000 * scale) + model)
     ng, l_box = 128, 1300.0
